@@ -7,139 +7,75 @@
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;
+constexpr int LK = 16, LPAD = 4;
 
-__global__ void __launch_bounds__(256)
-sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M,
-                int N, int K, int lda, int ldw, int ldc, int vec_ok) {
-  __shared__ __align__(16) float As[BK][BM + PAD];
-  __shared__ __align__(16) float Ws[BK][BN + PAD];
-  const int t = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int lrow = t >> 2, lk = (t & 3) * 4;  // loader: 64 rows x 4 quads of k
-  const int ty = t >> 4, tx = t & 15;         // compute: 16 x 16 threads, 4 x 4 each
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
-    const int gm = m0 + lrow, gn = n0 + lrow, gk = k0 + lk;
-    if (gm < M) {
-      const float* p = A + (size_t)gm * lda + gk;
-      if (vec_ok && gk + 3 < K) {
-        float4 v = *reinterpret_cast<const float4*>(p);
-        a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (gk + i < K) a[i] = p[i];
-      }
-    }
-    if (gn < N) {
-      const float* p = W + (size_t)gn * ldw + gk;
-      if (vec_ok && gk + 3 < K) {
-        float4 v = *reinterpret_cast<const float4*>(p);
-        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (gk + i < K) w[i] = p[i];
-      }
-    }
-    __syncthreads();  // the previous tile has been consumed
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      As[lk + i][lrow] = a[i];
-      Ws[lk + i][lrow] = w[i];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      const float4 av = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      const float4 wv = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-      const float ar[4] = {av.x, av.y, av.z, av.w};
-      const float wr[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
-    }
-  }
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 
-// The same sums for many rows (prompts): tiles of 128 x 128 outputs, 8 x 8 per thread (as four blocks
-// of 4 x 4, so that a thread's reads of shared memory are whole float4s), the next tile's operands
-// fetched into registers while this one is multiplied, two buffers in shared memory.  An output is
-// still one accumulator that walks k = 0..K-1 in order: the same bits as from the kernels above and below.
-constexpr int LM = 128, LN = 128, LK = 16, LPAD = 4;
-
-__global__ void __launch_bounds__(256, 2)
-sgemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M,
-                      int N, int K, int lda, int ldw, int ldc, int vec_ok) {
-  __shared__ __align__(16) float As[2][LK][LM + LPAD];
-  __shared__ __align__(16) float Ws[2][LK][LN + LPAD];
+// Tiles of BM x BN outputs, TM x TN per thread (as blocks of 4 x 4, so that a thread's reads of shared memory are
+// whole float4s), the next tile's operands fetched into registers while this one is multiplied, two buffers in
+// shared memory.  Two neighbouring columns share a packed multiply-add (each half rounds as fmaf does), which halves
+// the instructions beside the reads of shared memory.  An output is one accumulator that walks k = 0..K-1 in order,
+// so every tile shape gives the same bits, and so does the kernel of few rows below.
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 512 / ((BM / TM) * (BN / TN)))
+sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M,
+                int N, int K, int lda, int ldw, int ldc, int vec_ok) {
+  constexpr int TX = BN / TN, THREADS = (BM / TM) * TX;
+  constexpr int MB = TM / 4, NB = TN / 4;        // blocks of four rows, of four columns a thread
+  constexpr int ROWS = THREADS / 4;              // rows a pass of the loader covers: four quads of k a row
+  constexpr int PA = BM / ROWS, PW = BN / ROWS;  // its passes over A and over W
+  static_assert(BM % ROWS == 0 && BN % ROWS == 0, "whole passes");
+  __shared__ __align__(16) float As[2][LK][BM + LPAD];
+  __shared__ __align__(16) float Ws[2][LK][BN + LPAD];
   const int t = threadIdx.x;
-  const int m0 = blockIdx.y * LM, n0 = blockIdx.x * LN;
-  const int ty = t >> 4, tx = t & 15;  // 16 x 16 threads; rows ty*4.. and 64 + ty*4.., columns likewise
-  // loader: 128 rows x 4 quads of k, two rows per thread (row, row + 64)
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  // a warp's lanes lie 4 x 8 in the tile: the fewest distinct words of shared memory a read asks for
+  const int warp = t >> 5, lane = t & 31;
+  const int tx = (warp % (TX / 8)) * 8 + (lane & 7), ty = (warp / (TX / 8)) * 4 + (lane >> 3);
   const int lrow = t >> 2, lk = (t & 3) * 4;
-  float acc[8][8];
+  uint64_t acc[TM][TN / 2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  float ra[2][4], rw[2][4];
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = pair(0.f, 0.f);
+  float ra[PA][4], rw[PW][4];
+  auto row_quad = [&](float (&r)[4], const float* base, int row, int rows, int ld, int k) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = 0.f;
+    if (row >= rows) return;
+    const float* p = base + (size_t)row * ld + k;
+    if (vec_ok && k + 3 < K) {
+      const float4 v = *reinterpret_cast<const float4*>(p);
+      r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (k + i < K) r[i] = p[i];
+    }
+  };
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gm = m0 + lrow + 64 * h, gn = n0 + lrow + 64 * h, gk = k0 + lk;
+    for (int h = 0; h < PA; ++h) row_quad(ra[h], A, m0 + lrow + ROWS * h, M, lda, k0 + lk);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ra[h][i] = rw[h][i] = 0.f;
-      if (gm < M) {
-        const float* p = A + (size_t)gm * lda + gk;
-        if (vec_ok && gk + 3 < K) {
-          const float4 v = *reinterpret_cast<const float4*>(p);
-          ra[h][0] = v.x; ra[h][1] = v.y; ra[h][2] = v.z; ra[h][3] = v.w;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (gk + i < K) ra[h][i] = p[i];
-        }
-      }
-      if (gn < N) {
-        const float* p = W + (size_t)gn * ldw + gk;
-        if (vec_ok && gk + 3 < K) {
-          const float4 v = *reinterpret_cast<const float4*>(p);
-          rw[h][0] = v.x; rw[h][1] = v.y; rw[h][2] = v.z; rw[h][3] = v.w;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (gk + i < K) rw[h][i] = p[i];
-        }
-      }
-    }
+    for (int h = 0; h < PW; ++h) row_quad(rw[h], W, n0 + lrow + ROWS * h, N, ldw, k0 + lk);
   };
   auto stash = [&](int buf) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int i = 0; i < 4; ++i) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        As[buf][lk + i][lrow + 64 * h] = ra[h][i];
-        Ws[buf][lk + i][lrow + 64 * h] = rw[h][i];
-      }
+      for (int h = 0; h < PA; ++h) As[buf][lk + i][lrow + ROWS * h] = ra[h][i];
+#pragma unroll
+      for (int h = 0; h < PW; ++h) Ws[buf][lk + i][lrow + ROWS * h] = rw[h][i];
+    }
   };
   fetch(0);
   stash(0);
@@ -150,16 +86,24 @@ sgemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     if (more) fetch(k0 + LK);  // on its way while this tile is multiplied
 #pragma unroll
     for (int k = 0; k < LK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][64 + ty * 4]);
-      const float4 w0 = *reinterpret_cast<const float4*>(&Ws[buf][k][tx * 4]);
-      const float4 w1 = *reinterpret_cast<const float4*>(&Ws[buf][k][64 + tx * 4]);
-      const float ar[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float wr[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+      float ar[TM];
+      uint64_t wr[TN / 2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int b = 0; b < MB; ++b) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][b * (BM / MB) + ty * 4]);
+        ar[4 * b] = v.x; ar[4 * b + 1] = v.y; ar[4 * b + 2] = v.z; ar[4 * b + 3] = v.w;
+      }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+      for (int b = 0; b < NB; ++b) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Ws[buf][k][b * (BN / NB) + tx * 4]);
+        wr[2 * b] = v.x; wr[2 * b + 1] = v.y;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const uint64_t aa = pair(ar[i], ar[i]);
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma_pair(aa, wr[j], acc[i][j]);
+      }
     }
     if (more) {
       stash(buf ^ 1);  // the other buffer: its last readers passed the barrier below one tile ago
@@ -168,15 +112,34 @@ sgemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + (i >> 2) * (BM / MB) + ty * 4 + (i & 3);
     if (gm >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
+    for (int j = 0; j < TN / 2; ++j) {
+      const int gn = n0 + (j >> 1) * (BN / NB) + tx * 4 + 2 * (j & 1);
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][j]));
+      if (gn < N) C[(size_t)gm * ldc + gn] = lo;
+      if (gn + 1 < N) C[(size_t)gm * ldc + gn + 1] = hi;
     }
   }
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_tiles(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int vec_ok, cudaStream_t st) {
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+  sgemm_nt_kernel<BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, st>>>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok);
+  return KVF_LAUNCH_STATUS();
+}
+
+// Time of the SM with the most tiles, in units of an output of a 128 x 128 tile on a full SM: `cost` is what an output of
+// the shape costs beside that, and an SM that holds few warps (four warps a scheduler hide everything, one little) takes longer.
+double busiest(int M, int N, int bm, int bn, int warps, int resident, double cost) {
+  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn), per_sm = (tiles + 147) / 148;
+  const long long held = (per_sm < resident ? per_sm : resident) * warps;
+  return (double)per_sm * bm * bn * cost * (held <= 4 ? 1.55 : held <= 8 ? 1.16 : held <= 12 ? 1.06 : 1.0);
 }
 
 // The same sums for a handful of rows (decoding): with M <= 16 the tiles above are nearly empty and
@@ -184,7 +147,7 @@ sgemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, 
 // threads takes MR rows of A (8 or 16) and 256 / MR rows of W, four outputs per thread (two rows of
 // A by two rows of W); W and A come in through a cp.async pipeline, k contiguous in shared memory,
 // and each output is one accumulator that walks k = 0..K-1 in order, exactly as above: the bits are
-// the same whichever of the two kernels runs.  (Entries past K are filled with zeros and add
+// the same whichever of the kernels runs.  (Entries past K are filled with zeros and add
 // nothing.)  What bounds a warp is its chains of dependent FMAs, so a thread has four of them.
 // Needs K % 4 == 0 and 16-byte aligned rows.
 constexpr int SBK = 64, SSTAGES = 6, SLD = SBK + 4, STHREADS = 64;
@@ -284,14 +247,15 @@ KVF_API int kvf_gemm_nt_f32(const float* A, const float* W, float* C, int M, int
     if (M <= 8) return launch_small<8>(A, W, C, M, N, K, lda, ldw, ldc, st);
     return launch_small<16>(A, W, C, M, N, K, lda, ldw, ldc, st);
   }
-  if (M > 64 && N > 64) {
-    dim3 large((N + LN - 1) / LN, (M + LM - 1) / LM);
-    if (large.y > 65535) return (int)cudaErrorInvalidValue;
-    sgemm_nt_large_kernel<<<large, 256, 0, st>>>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok);
-    return KVF_LAUNCH_STATUS();
-  }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-  sgemm_nt_kernel<<<grid, 256, 0, st>>>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok);
-  return KVF_LAUNCH_STATUS();
+  // Large tiles read shared memory least per output, small ones leave fewer outputs to rows and SMs that have none.  Costs and
+  // the factor for few warps were measured (B200; the four shapes in turn, one kernel of 128 x 128 or 64 x 64 tiles before):
+  // 515 x 16,384 x 2,048: 907, 788, 871, 1,159 us (1,022 before); 515 x 2,048 x 8,192: 829, 612, 504, 655 us (954);
+  // 2,048 x 16,384 x 2,048: 2,530, 2,665, 2,995, 4,258 us (2,855: 48 TFLOP/s, now 54); 48 x 2,048 x 2,048: 201, 152, 82, 62 us (103).
+  const double t0 = busiest(M, N, 128, 128, 8, 2, 1.0), t1 = busiest(M, N, 64, 128, 4, 4, 1.08), t2 = busiest(M, N, 64, 64, 4, 4, 1.18),
+               t3 = busiest(M, N, 32, 64, 4, 4, 1.68);
+  // (a grid's second dimension ends at 65,535: beyond two million rows only the highest tiles remain)
+  if (M > 65535 * 32 || (t0 <= t1 && t0 <= t2 && t0 <= t3)) return launch_tiles<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok, st);
+  if (t1 <= t2 && t1 <= t3) return launch_tiles<64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok, st);
+  if (t2 <= t3) return launch_tiles<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok, st);
+  return launch_tiles<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec_ok, st);
 }

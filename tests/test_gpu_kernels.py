@@ -119,6 +119,23 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch(ops, n, k):
         assert torch.equal(part, full[lo:hi]), (lo, hi)
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 18944, 20), (129, 16500, 36), (300, 16383, 17), (130, 9500, 52), (200, 4101, 130), (65, 20100, 16), (33, 1000, 64), (17, 67, 9)])
+def test_gemm_f32_every_tile_shape_gives_the_bits_of_few_rows(ops, m, n, k):
+    """Shapes that take each of the four tile shapes (128 x 128, twice 64 x 128, twice 64 x 64, three times 32 x 64), with
+    ragged last tiles, odd columns and a K that is no multiple of the tile's depth."""
+    g = torch.Generator().manual_seed(m + n + k)
+    a, w = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g)
+    wide = torch.full((m, n + 3), float("nan"), device="cuda")
+    ops.gemm_nt_f32(dev(a), dev(w), wide[:, :n])
+    assert torch.isnan(wide[:, n:]).all()
+    ref = a.double() @ w.double().t()
+    assert float((wide[:, :n].cpu().double() - ref).abs().max()) < 2e-6 * math.sqrt(k) * float(ref.abs().max())
+    for lo in (0, (m - 11) // 2, m - 11):
+        part = torch.empty(11, n, device="cuda")
+        ops.gemm_nt_f32(dev(a[lo : lo + 11]), dev(w), part)
+        assert torch.equal(part, wide[lo : lo + 11, :n]), lo
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("many", [False, True])  # a few tokens and many tokens take different kernels
 @pytest.mark.parametrize("nh,nkv,d,rot,bs", [(4, 2, 16, 16, 16), (3, 1, 32, 32, 8), (6, 3, 48, 24, 4), (5, 5, 128, 128, 32)])
