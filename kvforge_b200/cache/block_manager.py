@@ -66,6 +66,20 @@ class _Pool:
         self.free: list[int] = list(range(num_blocks - 1, -1, -1))
         self.held = [False] * num_blocks
         self.tables: dict[str, list[int]] = {}
+        # the same tables as int32 arrays (with room to grow), so that a step copies a table instead of converting a list
+        self.arrays: dict[str, np.ndarray] = {}
+
+    def put(self, seq_id: str, i: int, b: int) -> None:
+        """Entry ``i`` of a request's table, at most one past its end."""
+        table, array = self.tables[seq_id], self.arrays[seq_id]
+        if i == len(table):
+            table.append(b)
+            if i == len(array):
+                array = np.resize(array, 2 * i + 8)
+                self.arrays[seq_id] = array
+        else:
+            table[i] = b
+        array[i] = b
 
     def pop(self) -> int:
         if not self.free:
@@ -117,6 +131,11 @@ class BlockManager:
     def get_block_table(self, seq_id: str, group: int = 0) -> list[int]:
         return self._pools[group].tables[seq_id]
 
+    def table_array(self, seq_id: str, group: int = 0) -> np.ndarray:
+        """The block table as an int32 array, to be read before the next change to the request."""
+        pool = self._pools[group]
+        return pool.arrays[seq_id][: len(pool.tables[seq_id])]
+
     def blocks_needed(self, num_tokens: int) -> int:
         return -(-num_tokens // self.block_size)
 
@@ -134,11 +153,11 @@ class BlockManager:
 
     def slots_array(self, seq_id: str, start: int, end: int, group: int = 0) -> np.ndarray:
         """The same as an int32 array (a prompt portion has thousands of positions)."""
-        table, bs = self._pools[group].tables[seq_id], self.block_size
+        table, bs = self.table_array(seq_id, group), self.block_size
         if end <= start:
             return np.empty(0, dtype=np.int32)
         first, last = start // bs, (end - 1) // bs
-        pages = np.asarray(table[first : last + 1], dtype=np.int64)
+        pages = table[first : last + 1].astype(np.int64)
         if (pages < 0).any():
             p = (first + int(np.argmax(pages < 0))) * bs
             raise RuntimeError(f"position {max(p, start)} of {seq_id} lies in a page that was given back")
@@ -209,6 +228,7 @@ class BlockManager:
             plan.append(need)
         for pool, need in zip(self._pools, plan):
             pool.tables[seq_id] = [pool.pop() for _ in range(need)]
+            pool.arrays[seq_id] = np.array(pool.tables[seq_id], dtype=np.int32)
         self._num_tokens[seq_id] = num_tokens
         return 0
 
@@ -233,19 +253,19 @@ class BlockManager:
             table = pool.tables[seq_id]
             if pool.spec.kind == "full":
                 while len(table) < want:
-                    table.append(pool.pop())
+                    pool.put(seq_id, len(table), pool.pop())
                 continue
             first = self._first_live_block(pool, write_start)
             kept = min(self._kept_blocks(pool), first)
             for i in range(kept, min(first, len(table))):
                 if table[i] >= 0:
                     pool.release(table[i])
-                    table[i] = RELEASED
+                    pool.put(seq_id, i, RELEASED)
             while len(table) < want:
-                table.append(RELEASED if kept <= len(table) < first else pool.pop())
+                pool.put(seq_id, len(table), RELEASED if kept <= len(table) < first else pool.pop())
             for i in [*range(min(kept, want)), *range(first, want)]:
                 if table[i] < 0:
-                    table[i] = pool.pop()
+                    pool.put(seq_id, i, pool.pop())
         self._num_tokens[seq_id] = max(self._num_tokens[seq_id], total_tokens)
         return []
 
@@ -262,6 +282,7 @@ class BlockManager:
             return
         for pool in self._pools:
             table = pool.tables.pop(seq_id, [])
+            pool.arrays.pop(seq_id, None)
             for b in reversed(table):
                 if b >= 0:
                     pool.release(b)
@@ -272,6 +293,8 @@ class BlockManager:
         for gi, pool in enumerate(self._pools):
             seen: dict[int, str] = {}
             for seq, table in pool.tables.items():
+                if pool.arrays[seq][: len(table)].tolist() != table:
+                    raise AssertionError(f"group {gi}: the table of {seq} and its array differ")
                 for b in table:
                     if b < 0:
                         continue

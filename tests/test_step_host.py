@@ -110,3 +110,61 @@ def test_slices_of_the_decode_product_and_ranges_of_the_decode_attention():
     assert ops.attention_wave_target(8, 8, 64) == 888 and ops.attention_wave_target(8, 8, 128) == 444 and ops.attention_wave_target(64, 8, 128) == 3072
     # and never more ranges than the merge takes
     assert -(-(1 << 20) // ops.attention_split_size(8, 8, 1 << 20)) <= ops.MAX_ATTN_SPLITS
+
+
+def test_a_step_of_single_tokens_is_laid_out_as_its_tables_say():
+    """The arrays of a step whose requests bring one token each, against the block manager's lists: full, window and
+    chunk groups whose pages have grown and come back, tokens from the host and from the device, a padded layout."""
+    import pytest
+    import torch
+
+    from kvforge_b200.cache.block_manager import BlockManager, GroupSpec
+    from kvforge_b200.cache.state_slots import StateSlotPool
+
+    rng = random.Random(9)
+    for case in range(20):
+        bs = rng.choice([4, 16, 24])
+        bm = BlockManager(400, bs, 0.0, [GroupSpec(), GroupSpec("window", 40, rng.choice([0, 9])), GroupSpec("chunk", 48)])
+        runner = object.__new__(ModelRunner)
+        runner.block_manager, runner.block_size, runner._copy_done, runner.n_groups = bm, bs, None, 3
+        runner.max_model_len, runner.state_slots, runner.token_feedback = 300, StateSlotPool(8), object()
+        items = []
+        for i in range(rng.randint(1, 6)):
+            start = rng.randint(0, 250)
+            bm.allocate(f"r{i}", 1, 1)
+            for at in range(0, start + 1, 7):
+                bm.append_slots(f"r{i}", min(at + 7, start + 1), at)
+            if rng.random() < 0.7:
+                runner.state_slots.allocate(f"r{i}")
+            wanted = rng.choice(["last", "all", "none", [0]])
+            items.append(BatchItem(f"r{i}", [rng.randrange(1000)], start, wanted, feedback_row=rng.choice([None, 3])))
+        bm.check_invariants()
+        nb = len(items)
+        cap = nb + rng.randint(0, 3)
+        lay = _Layout(cap, cap, 80, 3, cap)
+        runner._host = torch.full((lay.total,), 7, dtype=torch.int32)
+        n, b, r, max_q, max_ctx = runner._fill(items, lay, padded=True, tiles=False)
+        host, o = runner._host.numpy(), lay.off
+        view = lambda name, size: host[o[name] : o[name] + size].tolist()  # noqa: E731
+        rows = [i for i, it in enumerate(items) if it.wanted()]
+        assert (n, b, r, max_q, max_ctx) == (nb, nb, len(rows), 1, max(it.start_pos for it in items) + 1)
+        assert view("token_ids", cap) == [0 if it.feedback_row is not None else it.token_ids[0] for it in items] + [0] * (cap - nb)
+        assert view("feedback_rows", cap) == [-1 if it.feedback_row is None else 3 for it in items] + [-1] * (cap - nb)
+        assert view("positions", nb) == [it.start_pos for it in items]
+        assert view("ctx", cap) == [it.start_pos + 1 for it in items] + [0] * (cap - nb)
+        assert view("qsl", cap + 1) == [min(i, nb) for i in range(cap + 1)]
+        assert view("logit_rows", r) == rows
+        assert view("state_slots", cap) == [runner.state_slots.slot(it.seq_id) if runner.state_slots.has(it.seq_id) else -1 for it in items] + [-1] * (cap - nb)
+        for g in range(3):
+            at = o["slots"] + g * cap
+            assert host[at : at + cap].tolist() == [bm.slots(it.seq_id, it.start_pos, it.start_pos + 1, g)[0] for it in items] + [-1] * (cap - nb)
+            for i, it in enumerate(items):
+                used = it.start_pos // bs + 1
+                at = o["tables"] + (g * cap + i) * 80
+                assert host[at : at + used].tolist() == bm.get_block_table(it.seq_id, g)[:used]
+        with pytest.raises(ValueError):
+            runner._fill([BatchItem("r0", [1], 300, "last")], lay)
+        with pytest.raises(RuntimeError):  # the token's page was given back
+            bm.allocate("gone", 1, 1)
+            bm.append_slots("gone", 250, 249)
+            runner._fill([BatchItem("gone", [1], 20, "last")], lay)
