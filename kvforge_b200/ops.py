@@ -28,6 +28,7 @@ _SIGNATURES = {
     "kvf_paged_attention_mma_bf16": "pppppppiiiiiiiiifiiiippp",
     "kvf_paged_attention_mma_biased_bf16": "pppppppiiiiiiiiifiipifpp",
     "kvf_latent_attention_bf16": "ppppppiiiiiiiiifiiiippp",
+    "kvf_latent_attention_tcgen05_bf16": "ppppppiiiiiiiiilfipipp",
     "kvf_paged_attention_decode_biased_bf16": "pppppppiiiiiiiifiiiipppipifpp",
     "kvf_paged_attention_tcgen05_bf16": "pppppppiiiiiiiiilfipippp",
     "kvf_paged_attention_decode_fused_bf16": "pppppppiiiiiiiifiiiipppp",
@@ -794,16 +795,33 @@ def latent_attention_supported(dtype: torch.dtype, d: int, dv: int) -> bool:
     return dtype == torch.bfloat16 and d % 16 == 0 and d <= MAX_KEY_DIM and dv % 32 == 0 and dv // 32 in (2, 3, 4, 8, 16) and dv <= d
 
 
+def latent_tcgen05_supported(dtype: torch.dtype, nh: int, d: int, dv: int, block_size: int) -> bool:
+    """Whether the tcgen05 kernel for many queries over such a cache (``csrc/attention_latent_tcgen05.cu``) takes the shape: a row
+    of at most 576 numbers (128 queries of it and two tiles of 64 keys fill an SM's shared memory), pages that come as whole
+    tensor-map boxes."""
+    return dtype == torch.bfloat16 and d % 16 == 0 and dv <= d <= 576 and dv in (64, 128, 256, 512) and 0 < nh <= 128 and block_size % 16 == 0
+
+
+def latent_query_tile(nh: int) -> int:
+    """Query tokens of one sequence that a CTA of that kernel takes."""
+    return 128 // nh
+
+
 def latent_attention(
     q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor, qsl: torch.Tensor, ctx_lens: torch.Tensor,
     num_seqs: int, max_q_len: int, nh: int, d: int, dv: int, scale: float, window: int = 0,
-    scratch: tuple[torch.Tensor, ...] | None = None, max_context: int | None = None, split_size: int = 128,
+    scratch: tuple[torch.Tensor, ...] | None = None, max_context: int | None = None, split_size: int = 128, kernel: str = "auto",
+    err: torch.Tensor | None = None, query_tiles: tuple[torch.Tensor, int] | None = None,
 ) -> None:  # fmt: skip
     """Attention of a flat batch over a paged cache of ONE row of ``d`` numbers per token (``cache [blocks, 1,
     block_size, d]``): the row is every head's key and its first ``dv`` numbers every head's value.  ``q [N, nh*d]``,
     ``out [N, nh*dv]``, bfloat16, on the tensor cores.  With ``scratch`` (partial results ``[B, nh, splits, dv]`` and
     their maxima and sums ``[B, nh, splits, 2]``, float) and one query a sequence the decode form runs: ranges of
-    ``split_size`` keys in parallel, then a merge."""
+    ``split_size`` keys in parallel, then a merge.  Without it and with more than one query in some sequence the tcgen05
+    kernel runs where it takes the shape (``kernel``: ``"mma"`` or ``"tcgen05"`` force one; ``err`` and ``query_tiles``, tiles of
+    ``latent_query_tile`` queries, as in ``paged_attention``)."""
+    if kernel not in ("auto", "mma", "tcgen05"):
+        raise ValueError("latent_attention: kernel is 'auto', 'mma' or 'tcgen05'")
     if not latent_attention_supported(q.dtype, d, dv):
         raise ValueError("latent_attention: the kernel does not take this shape")
     _need(q, torch.bfloat16, "q")
@@ -815,6 +833,31 @@ def latent_attention(
     if cache.dim() != 4 or cache.shape[1] != 1 or cache.shape[3] != d or q.shape[-1] != nh * d or out.shape[-1] != nh * dv:
         raise ValueError("latent_attention: shapes do not agree")
     bt_stride = block_tables.shape[-1] if block_tables.dim() == 2 else block_tables.numel() // max(1, num_seqs)
+    takes = (
+        latent_tcgen05_supported(q.dtype, nh, d, dv, int(cache.shape[2])) and scratch is None and window >= 0 and float(scale) > 0.0
+        and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0 and cache.shape[0] * cache.shape[2] < 2**31 - 64
+        and (0 < query_tiles[1] <= 65535 if query_tiles is not None else num_seqs <= 65535 and max_q_len <= 65535 * latent_query_tile(nh))
+    )  # fmt: skip
+    if kernel == "tcgen05" and not takes:
+        raise ValueError("latent_attention: the tcgen05 kernel does not take this call")
+    # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 240 us here, 591 us on
+    # the mma.sync kernel; single queries go to its key ranges, which a CTA of 128 rows would leave empty
+    if takes and (kernel == "tcgen05" or (kernel == "auto" and max_q_len > 1)):
+        tiles, n_tiles = None, 0
+        if query_tiles is not None:
+            tiles, n_tiles = query_tiles
+            _need(tiles, torch.int32, "query tiles")
+            if tiles.numel() < 2 * n_tiles:
+                raise ValueError("latent_attention: the list holds fewer query tiles than it says")
+        name = "kvf_latent_attention_tcgen05_bf16"
+        _check(
+            _fn(name)(
+                _ptr(q), _ptr(out), _ptr(cache), _ptr(block_tables), _ptr(qsl), _ptr(ctx_lens), num_seqs, max_q_len, q.shape[-1], out.shape[-1],
+                bt_stride, nh, d, dv, int(cache.shape[2]), int(cache.shape[0]), float(scale), int(window), _ptr(tiles), n_tiles, _ptr(err), _stream(),
+            ),
+            name,
+        )  # fmt: skip
+        return
     split, max_splits, grid_splits, pa, pm = 0, 0, 0, None, None
     if scratch is not None:
         pa, pm = scratch[:2]

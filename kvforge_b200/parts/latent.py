@@ -122,6 +122,11 @@ class LatentAttention(Mixer):
         table = self.position.table() if self.position is not None else None
         self.interleaved = bool(getattr(self.position, "pairs_interleaved", False))
         self.inv_freq = table
+        # the kernel of prompts and mixed batches takes its tiles of queries from a list made with the step
+        self._query_tile = None
+        if ops.latent_tcgen05_supported(rt.dtype, self.nh, self.d, self.rank, 16):
+            self._query_tile = ops.latent_query_tile(self.nh)
+            rt.query_tile_sizes.add(self._query_tile)
 
     def _per_head(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         """``out[:, h] = a[:, h] @ W[h]`` for every head: ``a [N, H, K]`` and ``out [N, H, M]`` are views
@@ -169,9 +174,11 @@ class LatentAttention(Mixer):
             (acc, ml, _), bound, split = decode_scratch(rt, ctx, h, 1, d, r, None, TENSOR_CORE_RANGE if tensor_cores else FP32_PIPE_RANGE)
             scratch = (acc, ml)
         if tensor_cores:
+            tiles = ctx.query_tiles.get(self._query_tile)
             ops.latent_attention(
                 qa, o_lat, cache.k, ctx.block_tables[cache.group], ctx.query_start_loc, ctx.context_lens, ctx.num_seqs, ctx.max_query_len,
-                h, d, r, self.scale, window=int(self.window or 0), scratch=scratch, max_context=bound, split_size=split,
+                h, d, r, self.scale, window=int(self.window or 0), scratch=scratch, max_context=bound, split_size=split, err=rt.err,
+                query_tiles=(tiles.tiles, tiles.count) if tiles is not None else None,
             )  # fmt: skip
         else:
             # 32-bit, or a latent whose size the tensor-core kernel does not take: the FP32 pipes

@@ -927,3 +927,87 @@ def test_sampling_is_reproducible_and_follows_the_distribution(ops):
     freq = torch.bincount(out1.cpu().long(), minlength=5).double() / 4000
     ref = torch.softmax(logits[0].double() / 0.8, -1)
     assert float((freq - ref).abs().max()) < 0.03
+
+
+# ------------------------------------------------------------------ attention over one row a token, many queries
+
+
+def paged_latent_case(lens, starts, nh, d, dv, block_size, window, seed, sharp=1.0):
+    """Queries, a cache on shuffled pages with NaN wherever no key lies, tables, and the 64-bit result with the bound on
+    what rounding the weights (relative 2^-9 each) and the result (2^-9) to bfloat16 may change, times two."""
+    g = torch.Generator().manual_seed(seed)
+    ctx = [n + s for n, s in zip(lens, starts)]
+    per = [-(-c // block_size) for c in ctx]
+    order = torch.randperm(sum(per) + 3, generator=g).tolist()
+    cache = torch.full((sum(per) + 3, 1, block_size, d), float("nan"))
+    tables = torch.zeros((len(lens), max(per)), dtype=torch.int32)
+    q = (sharp * torch.randn((sum(lens), nh * d), generator=g)).bfloat16()
+    outs, bounds, at, row = [], [], 0, 0
+    for b, (n, c) in enumerate(zip(lens, ctx)):
+        keys = torch.randn((c, d), generator=g).bfloat16()
+        pages = order[at : at + per[b]]
+        at += per[b]
+        for j in range(c):
+            cache[pages[j // block_size], 0, j % block_size] = keys[j].float()
+        gone = max(0, c - n - window + 1) // block_size if window else 0  # pages that no query of the step sees come back
+        tables[b, : per[b]] = torch.tensor([-1] * gone + pages[gone:], dtype=torch.int32)
+        k = keys.double()
+        qs = q[row : row + n].double().view(n, nh, d)
+        row += n
+        i, j = torch.arange(c - n, c)[:, None], torch.arange(c)[None]
+        seen = (j <= i) & ((i - j < window) if window else True)
+        w = torch.softmax((torch.einsum("nhd,jd->hnj", qs, k) * d**-0.5).masked_fill(~seen, -math.inf), -1)
+        o, a = (w @ k[:, :dv]).transpose(0, 1), (w @ k[:, :dv].abs()).transpose(0, 1)
+        outs.append(o.reshape(n, -1))
+        bounds.append((2**-8 * (a + o.abs())).reshape(n, -1))
+    return q, cache.bfloat16(), tables, ctx, torch.cat(outs), torch.cat(bounds)
+
+
+@pytest.mark.parametrize(
+    "nh,d,dv,block_size,window,lens,starts",
+    [
+        (16, 576, 512, 16, 0, [130, 1, 17], [0, 70, 31]),  # two value halves, four query blocks in tensor memory; a single token among prompts
+        (16, 576, 512, 16, 50, [9, 200], [300, 40]),  # a window whose pages have come back
+        (5, 576, 512, 32, 0, [26, 51], [0, 13]),  # 125 of the 128 rows, tiles of 25 tokens, an odd last page
+        (128, 320, 256, 48, 0, [3, 2], [126, 61]),  # a token a CTA, one value half, pages of three boxes
+        (3, 80, 64, 64, 0, [64, 65], [0, 63]),  # a last block of 16 numbers, pages of a whole tile
+        (1, 64, 64, 16, 7, [300], [5]),  # a row of one block: nothing of the queries in tensor memory, no part outside the values
+        (7, 192, 128, 16, 0, [2], [127]),
+        (128, 576, 512, 16, 0, [4, 1], [126, 255]),  # a last tile that is seen whole: 128 and 256 keys
+        (16, 512, 512, 16, 0, [8, 16], [120, 112]),  # keys that are values whole
+    ],
+)
+def test_latent_attention_of_many_queries_on_tcgen05(ops, nh, d, dv, block_size, window, lens, starts):
+    for sharp in (1.0, 4.0):
+        q, cache, tables, ctx, ref, bound = paged_latent_case(lens, starts, nh, d, dv, block_size, window, nh + d, sharp)
+        qsl = [0]
+        for n in lens:
+            qsl.append(qsl[-1] + n)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        tq = ops.latent_query_tile(nh)
+        tiles = [(b, t) for b, n in enumerate(lens) for t in range(0, n, tq)]
+        tiles = sorted(tiles, key=lambda t: -(starts[t[0]] + t[1])) + [(-1, 0), (len(lens) + 2, 0)]  # dead entries
+        for work in (None, (i32(tiles).reshape(-1), len(tiles))):
+            out = torch.full((sum(lens), nh * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+            ops.latent_attention(
+                dev(q), out, dev(cache), dev(tables), i32(qsl), i32(ctx), len(lens), max(lens), nh, d, dv, d**-0.5, window=window,
+                kernel="tcgen05", err=err, query_tiles=work,
+            )  # fmt: skip
+            assert int(err.item()) == 0
+            over = (out.cpu().double() - ref).abs() - bound
+            assert float(over.max()) <= 0.0, (sharp, work is None, float(over.max()))
+
+
+def test_latent_attention_routes_by_shape(ops):
+    """What the tcgen05 kernel does not take stays with the mma.sync kernel, whose result it shares to rounding."""
+    assert ops.latent_tcgen05_supported(torch.bfloat16, 16, 576, 512, 16)
+    for nh, d, dv, bs in ((16, 640, 512, 16), (16, 576, 96, 16), (129, 576, 512, 16), (16, 576, 512, 8), (16, 72, 64, 16)):
+        assert not ops.latent_tcgen05_supported(torch.bfloat16, nh, d, dv, bs)
+    q, cache, tables, ctx, ref, bound = paged_latent_case([40], [3], 6, 128, 96, 8, 0, 1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    out = torch.empty((40, 6 * 96), device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, 40]), i32(ctx), 1, 40, 6, 128, 96, 128**-0.5)
+    assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
+    with pytest.raises(ValueError):
+        ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, 40]), i32(ctx), 1, 40, 6, 128, 96, 128**-0.5, kernel="tcgen05")
