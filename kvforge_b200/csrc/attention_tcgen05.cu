@@ -29,6 +29,12 @@
 // S(t+2), which is all its group waits for, then P(t) V(t).  Two CTAs fit an SM at head size 64
 // (112 KB of shared memory and 256 tensor-memory columns each), one at 128.
 //
+// Shaped scores (a soft cap, a bias by distance and head, kept first keys under a window; sinks beside them) are a form of their own:
+// scores are finished in place before the maximum is taken, kept tiles are walked first, and a group stages the
+// biases of its next tile (128 / g + 63 distances a head, in log2 units) in shared memory behind a barrier of its own, so that a
+// score's bias is one conflict-free word; one stage of keys makes room for them.  2,048 tokens in two sequences, 32 heads of 64 on 8,
+// a window of 1,024, a bias and 64 kept keys: 76 us against 149 us of the mma.sync tile kernel.
+//
 // Every mbarrier wait is bounded; if one runs out the kernel raises bit 4 of the error flag and
 // winds down.  No cluster launch, no multicast.
 #include "tcgen05.cuh"
@@ -46,14 +52,17 @@ constexpr int BN = 64;   // keys per tile
 constexpr int SOFTMAX_WARPS = 8;                    // two groups of four: even and odd key tiles
 constexpr int LOADER_WARP = SOFTMAX_WARPS, MMA_WARP = SOFTMAX_WARPS + 1;
 constexpr int THREADS = (SOFTMAX_WARPS + 2) * 32;
-template <int D> struct Shape {
+// a tile's biases: 128 / g + 63 distances for each of g <= 8 heads, each head's padded to a multiple of 32 words plus 32 / g
+constexpr int BIAS_WORDS = 800;
+// SH: the form for shaped scores, which gives a stage of keys for two buffers of biases for either softmax group
+template <int D, bool SH = false> struct Shape {
   static constexpr int HALVES = D / 64;
-  static constexpr int KV_STAGES = D == 64 ? 4 : 5;
-  static constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;  // 112 KB and 256 tensor-memory columns, or 224 KB and 512
+  static constexpr int KV_STAGES = (D == 64 ? 4 : 5) - (SH ? 1 : 0);
+  static constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;  // 109 or 112 KB and 256 tensor-memory columns, or 204 or 224 KB and 512
   static constexpr uint32_t Q_BYTES = HALVES * 128 * 128;     // [128 rows][D] bfloat16
   static constexpr uint32_t KV_BYTES = HALVES * 64 * 128;     // a [64 keys][D] bfloat16 tile
   static constexpr uint32_t TMEM_COLS = D == 64 ? 256u : 512u;  // S: 2 x 64, O: 2 x D
-  static constexpr size_t SMEM_BYTES = (size_t)Q_BYTES + (size_t)KV_STAGES * 2 * KV_BYTES + 2 * 128 * 128 + 256;
+  static constexpr size_t SMEM_BYTES = (size_t)Q_BYTES + (size_t)KV_STAGES * 2 * KV_BYTES + 2 * 128 * 128 + 256 + (SH ? 4 * BIAS_WORDS * 4 : 0);
 };
 constexpr int LOOKAHEAD = 2;                 // tiles in flight behind the one being handed over
 constexpr uint32_t Q_HALF = BM * 128;        // [128 rows][64] bfloat16
@@ -84,8 +93,19 @@ struct TcAttnParams {
 struct TcAttnSinkParams : TcAttnParams {
   const float* sinks;  // [nh] (natural-log units): a number a head whose exponential joins the denominator, without a key or a value
 };
-template <bool SINKS> struct ParamsOf { using type = TcAttnParams; };
-template <> struct ParamsOf<true> { using type = TcAttnSinkParams; };
+// Scores that are more than scaled dot products: a soft cap, a bias by distance and head, first keys that stay visible
+// under a window; sinks too.
+struct TcAttnShapedParams : TcAttnSinkParams {
+  int keep_first;
+  const float* bias;  // [nh][bias_far + 1]
+  int bias_far;
+  float cap_in, cap_out;  // scale / c and c * log2(e)
+};
+// What a kernel is made for: plain scores, sinks, or SHAPED plus which of a bias (1) and a cap (2) it takes.
+enum { PLAIN = 0, SINKS = 1, SHAPED = 4 };
+template <int MODE> struct ParamsOf { using type = TcAttnShapedParams; };
+template <> struct ParamsOf<PLAIN> { using type = TcAttnParams; };
+template <> struct ParamsOf<SINKS> { using type = TcAttnSinkParams; };
 
 // One tile of the softmax for the thread's row.  v: the 64 raw scores (in place: not kept).
 // MASK: some key of the tile may be hidden from some row of the warp.  Returns the tile's sum of
@@ -144,10 +164,58 @@ __device__ __forceinline__ float softmax_tile(uint32_t (&va)[32], uint32_t (&vb)
   return s0 + s1;
 }
 
-template <int D, bool SINKS>
-__global__ void __launch_bounds__(THREADS, Shape<D>::CTAS_PER_SM)
-attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const typename ParamsOf<SINKS>::type p) {
-  constexpr int HALVES = Shape<D>::HALVES, KV_STAGES = Shape<D>::KV_STAGES;
+// tanh(x) = 1 - 2 / (exp(2x) + 1): exact at both ends, absolute error of a few 1e-7 near zero.
+__device__ __forceinline__ float fast_tanh(float x) { return 1.f - __fdividef(2.f, ex2(x * 2.8853900817779268f) + 1.f); }
+
+// The same for shaped scores, which are made in place: s * scale, or with CAP c * tanh(s * scale / c), plus with BIAS the bias of
+// the distance, `brow[-j]` for the tile's key j (a shared-memory row in log2 units).  Keys before `kept` are seen whatever
+// `first` says.
+template <bool BIAS, bool CAP>
+__device__ __forceinline__ float softmax_shaped(uint32_t (&va)[32], uint32_t (&vb)[32], float& m_ref, float& corr, float scale_log2, float cap_in,
+                                                float cap_out, const float* brow, bool mask, int first, int last, int kept, uint32_t p_row, int r7) {
+  float mx = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < 64; ++c) {
+    uint32_t& v = c < 32 ? va[c & 31] : vb[c & 31];
+    const float s = __uint_as_float(v);
+    float x;
+    if (CAP)
+      x = BIAS ? fmaf(cap_out, fast_tanh(s * cap_in), brow[-c]) : cap_out * fast_tanh(s * cap_in);
+    else
+      x = BIAS ? fmaf(s, scale_log2, brow[-c]) : s * scale_log2;
+    if (mask && (c > last || (c < first && c >= kept))) x = -INFINITY;
+    v = __float_as_uint(x);
+    mx = fmaxf(mx, x);
+  }
+  corr = 1.f;
+  if (mx > m_ref + RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY)) {
+    corr = ex2(m_ref - mx);  // 0 the first time
+    m_ref = mx;
+  }
+  const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+  float sum_a = 0.f, sum_b = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = 8 * q + 2 * e;
+      const float e0 = ex2(__uint_as_float(c < 32 ? va[c & 31] : vb[c & 31]) - m_use);
+      const float e1 = ex2(__uint_as_float(c < 32 ? va[(c & 31) + 1] : vb[(c & 31) + 1]) - m_use);
+      sum_a += e0;
+      sum_b += e1;
+      w[e] = pk(e0, e1);
+    }
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p_row + (uint32_t)((q ^ r7) << 4)), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+  }
+  return sum_a + sum_b;
+}
+
+template <int D, int MODE>
+__global__ void __launch_bounds__(THREADS, Shape<D, (MODE >= SHAPED)>::CTAS_PER_SM)
+attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const typename ParamsOf<MODE>::type p) {
+  constexpr bool SH = MODE >= SHAPED, BIAS = SH && (MODE & 1), CAP = SH && (MODE & 2);
+  constexpr int HALVES = Shape<D, SH>::HALVES, KV_STAGES = Shape<D, SH>::KV_STAGES;
   constexpr uint32_t Q_BYTES = Shape<D>::Q_BYTES, KV_BYTES = Shape<D>::KV_BYTES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // no slack for rounding up (two CTAs have to fit an SM): the base must be 1024-byte aligned
@@ -160,6 +228,7 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   const uint32_t q_full = bars, kv_full0 = bars + 8, kv_empty0 = kv_full0 + 8 * KV_STAGES;
   const uint32_t s_full0 = kv_empty0 + 8 * KV_STAGES, p_full0 = s_full0 + 16, pv_done0 = p_full0 + 16;
   const uint32_t tmem_slot = pv_done0 + 16;
+  [[maybe_unused]] float* const bias_s = reinterpret_cast<float*>(smem_raw + (p_s + 2 * P_BYTES + 256 - base));  // [group][2][BIAS_WORDS]
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - base));
 
   pdl_launch();
@@ -188,7 +257,11 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   const int p_first = ctx - q_len + q0;
   const int kv_hi = p_first + n_tok;
   const int kv_lo = live ? (first_key(p_first, p.window) / BN) * BN : 0;
-  const int n_tiles = live ? (kv_hi - kv_lo + BN - 1) / BN : 0;
+  // kept first keys: their tiles come first, then the window's
+  int n_kept = 0;
+  if constexpr (SH) n_kept = live ? min((p.keep_first + BN - 1) / BN, kv_lo / BN) : 0;
+  const int n_tiles = live ? (kv_hi - kv_lo + BN - 1) / BN + n_kept : 0;
+  auto first_of = [&](int t) { return SH && t < n_kept ? t * BN : kv_lo + (t - (SH ? n_kept : 0)) * BN; };  // a tile's first key
 
   if (threadIdx.x == 0) {
     bar_init(q_full, 1);
@@ -232,7 +305,7 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     auto issue_tile = [&](int t) {
       const int s = t % KV_STAGES;
       const uint32_t ks = kv_s + s * 2 * KV_BYTES, vs = ks + KV_BYTES;
-      const int t0 = kv_lo + t * BN;
+      const int t0 = first_of(t);
       long long row[2];  // element offset of the key's row in the cache, or -1
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -274,7 +347,7 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const int s = t % KV_STAGES;
         if (t >= KV_STAGES) ok = __all_sync(0xffffffffu, bar_wait(kv_empty0 + 8 * s, ((t / KV_STAGES) - 1) & 1, p.err));
         if (!ok) break;
-        const int t0 = kv_lo + t * BN;
+        const int t0 = first_of(t);
         const bool ragged = t0 + BN > ctx && (ctx & (p.box_rows - 1)) != 0;
         if (!ragged) {
           // lane j brings box j of the tile (box_rows keys of one page: a K box and a V box)
@@ -417,16 +490,37 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const uint32_t my_s = tmem_s + lane_addr + (uint32_t)(grp * BN), my_o = tmem_o + lane_addr + (uint32_t)(grp * D);
     const uint32_t s_bar = s_full0 + 8 * grp, p_bar = p_full0 + 8 * grp, pv_bar = pv_done0 + 8 * grp;
     float m_ref = -INFINITY, l = 0.f;
-    if constexpr (SINKS) {
-      if (grp == 0 && valid) {  // the sink is where the first group starts: one in the sum at its own maximum
+    if constexpr (MODE != PLAIN) {
+      bool sink = true;
+      if constexpr (SH) sink = p.sinks != nullptr;
+      if (sink && grp == 0 && valid) {  // the sink is where the first group starts: one in the sum at its own maximum
         m_ref = p.sinks[kvh * g + hh] * 1.4426950408889634f;
         l = 1.f;
       }
     }
+    // a head's biases of a tile lie side by side by distance, p - key from -63 of the tile's first query on; heads a stride apart
+    // that puts the lanes of a warp into other banks
+    [[maybe_unused]] const int words = tq + BN - 1, b_stride = BIAS ? (words + 31) / 32 * 32 + (g <= 32 ? 32 / g : 1) % 32 : 0;
     bool ok = true;
     int i = 0;  // index among this group's tiles
-    for (int t = grp; t < n_tiles && ok; t += 2, ++i) {
-      const int key0 = kv_lo + t * BN;
+    int t = grp;
+    for (; t < n_tiles && ok; t += 2, ++i) {
+      const int key0 = first_of(t);
+      [[maybe_unused]] const float* brow = nullptr;
+      if constexpr (BIAS) {
+        float* dst = bias_s + (2 * grp + (i & 1)) * BIAS_WORDS;
+        const int d0 = p_first - key0 - (BN - 1);
+        for (int w = r; w < g * words; w += BM) {
+          const int head = w / words, d = w - head * words;
+          dst[head * b_stride + d] = __ldg(p.bias + (size_t)(kvh * g + head) * (p.bias_far + 1) + min(max(d0 + d, 0), p.bias_far)) * 1.4426950408889634f;
+        }
+        // one barrier a tile: the buffer written here was last read two tiles ago, before the barrier of the last one
+        if (grp == 0)
+          asm volatile("bar.sync 2, %0;" ::"n"(BM) : "memory");
+        else
+          asm volatile("bar.sync 3, %0;" ::"n"(BM) : "memory");
+        brow = dst + hh * b_stride + min(tok, tq - 1) + BN - 1;
+      }
       // (tcgen05.ld and st are warp-wide: the lanes of a warp leave the loop together)
       ok = __all_sync(0xffffffffu, bar_wait(s_bar, i & 1, p.err));
       if (!ok) break;
@@ -441,10 +535,14 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const bool need_mask = (key0 + BN - 1 > pos) || (key0 < lo);
+      bool need_mask = (key0 + BN - 1 > pos) || (key0 < lo);
+      if constexpr (SH) need_mask = need_mask && !(key0 + BN - 1 <= pos && key0 + BN <= p.keep_first);
       const uint32_t p_row = p_s + (uint32_t)grp * P_BYTES + (uint32_t)r * 128u;
       float corr, sum;
-      if (__any_sync(0xffffffffu, need_mask))
+      if constexpr (SH)
+        sum = softmax_shaped<BIAS, CAP>(va, vb, m_ref, corr, p.scale_log2, p.cap_in, p.cap_out, brow, __any_sync(0xffffffffu, need_mask),
+                                        max(lo, key0) - key0, min(pos, key0 + BN - 1) - key0, p.keep_first - key0, p_row, r & 7);
+      else if (__any_sync(0xffffffffu, need_mask))
         sum = softmax_tile<true>(va, vb, m_ref, corr, p.scale_log2, max(lo, key0) - key0, min(pos, key0 + BN - 1) - key0, p_row, r & 7);
       else
         sum = softmax_tile<false>(va, vb, m_ref, corr, p.scale_log2, 0, BN - 1, p_row, r & 7);
@@ -464,6 +562,16 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       fence_async_smem();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       bar_arrive(p_bar);
+    }
+    if constexpr (BIAS) {
+      // a warp whose wait ran out still meets the others of its group at the barriers of the tiles left
+      if (!ok)
+        for (t += 2; t < n_tiles; t += 2) {
+          if (grp == 0)
+            asm volatile("bar.sync 2, %0;" ::"n"(BM) : "memory");
+          else
+            asm volatile("bar.sync 3, %0;" ::"n"(BM) : "memory");
+        }
     }
     if (ok && i > 0) ok = __all_sync(0xffffffffu, bar_wait(pv_bar, (i - 1) & 1, p.err));
     // ---- the two groups' results become one: group 1 hands its maximum and sum over (through its P
@@ -515,11 +623,22 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
 namespace {
 
-template <int D, bool SINKS>
-int launch_tc_attn(const CUtensorMap& mk, const CUtensorMap& mv, const typename ParamsOf<SINKS>::type& p, dim3 grid, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(attn_tcgen05_kernel<D, SINKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<D>::SMEM_BYTES);
+template <int D, int MODE>
+int launch_tc_attn(const CUtensorMap& mk, const CUtensorMap& mv, const typename ParamsOf<MODE>::type& p, dim3 grid, cudaStream_t st) {
+  constexpr size_t smem = Shape<D, (MODE >= SHAPED)>::SMEM_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(attn_tcgen05_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  return launch(attn_tcgen05_kernel<D, SINKS>, grid, dim3(THREADS), Shape<D>::SMEM_BYTES, st, mk, mv, p);
+  return launch(attn_tcgen05_kernel<D, MODE>, grid, dim3(THREADS), smem, st, mk, mv, p);
+}
+
+template <int D>
+int launch_shaped(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnShapedParams& p, dim3 grid, cudaStream_t st) {
+  switch ((p.bias ? 1 : 0) + (p.cap_out > 0.f ? 2 : 0)) {
+    case 0: return launch_tc_attn<D, SHAPED>(mk, mv, p, grid, st);
+    case 1: return launch_tc_attn<D, SHAPED + 1>(mk, mv, p, grid, st);
+    case 2: return launch_tc_attn<D, SHAPED + 2>(mk, mv, p, grid, st);
+    default: return launch_tc_attn<D, SHAPED + 3>(mk, mv, p, grid, st);
+  }
 }
 
 }  // namespace
@@ -531,12 +650,16 @@ KVF_API int kvf_paged_attention_tcgen05_bf16(const void* q, void* out, const voi
                                              int max_q_len, int q_stride, int out_stride, int bt_stride, int nh,
                                              int nkv, int d, int block_size, long long num_blocks, float scale,
                                              int window, const int* work, int n_work, int* err, const float* sinks,
-                                             cudaStream_t st) {
+                                             int keep_first, const float* bias, int bias_far, float softcap, cudaStream_t st) {
   if (B <= 0 || max_q_len <= 0) return 0;
   if ((d != 64 && d != 128) || nkv <= 0 || nh % nkv != 0 || nh / nkv > BM || block_size <= 0 || num_blocks <= 0) return (int)cudaErrorInvalidValue;
   if ((q_stride & 7) || (out_stride & 7) || ((((uintptr_t)q) | ((uintptr_t)out)) & 15)) return (int)cudaErrorInvalidValue;
   if ((unsigned)B > 65535u || (max_q_len + (BM / (nh / nkv)) - 1) / (BM / (nh / nkv)) > 65535) return (int)cudaErrorInvalidValue;
-  TcAttnSinkParams p;
+  if (keep_first < 0 || (keep_first && window <= 0) || softcap < 0.f || (bias && (bias_far < 0 || nh / nkv > 8))) return (int)cudaErrorInvalidValue;
+  TcAttnShapedParams p;
+  p.keep_first = keep_first; p.bias = bias; p.bias_far = bias_far;
+  p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
+  p.cap_out = softcap * 1.4426950408889634f;
   p.q = (const bf16*)q; p.out = (bf16*)out; p.kcache = (const bf16*)kcache; p.vcache = (const bf16*)vcache;
   p.block_tables = block_tables; p.qsl = qsl; p.ctx_lens = ctx_lens; p.err = err;
   p.work = work;
@@ -562,7 +685,9 @@ KVF_API int kvf_paged_attention_tcgen05_bf16(const void* q, void* out, const voi
   const int g = nh / nkv, tq = BM / g;
   if (work && (n_work <= 0 || n_work > 65535)) return (int)cudaErrorInvalidValue;
   const dim3 grid(nkv, work ? n_work : B, work ? 1 : (max_q_len + tq - 1) / tq);
-  if (sinks) return d == 64 ? launch_tc_attn<64, true>(mk, mv, p, grid, st) : launch_tc_attn<128, true>(mk, mv, p, grid, st);
+  if (keep_first || bias || softcap > 0.f) return d == 64 ? launch_shaped<64>(mk, mv, p, grid, st) : launch_shaped<128>(mk, mv, p, grid, st);
+  const TcAttnSinkParams& sunk = p;
+  if (sinks) return d == 64 ? launch_tc_attn<64, SINKS>(mk, mv, sunk, grid, st) : launch_tc_attn<128, SINKS>(mk, mv, sunk, grid, st);
   const TcAttnParams& plain = p;
-  return d == 64 ? launch_tc_attn<64, false>(mk, mv, plain, grid, st) : launch_tc_attn<128, false>(mk, mv, plain, grid, st);
+  return d == 64 ? launch_tc_attn<64, PLAIN>(mk, mv, plain, grid, st) : launch_tc_attn<128, PLAIN>(mk, mv, plain, grid, st);
 }

@@ -30,9 +30,9 @@ _SIGNATURES = {
     "kvf_latent_attention_bf16": "ppppppiiiiiiiiifiiiippp",
     "kvf_latent_attention_tcgen05_bf16": "ppppppiiiiiiiiilfipipp",
     "kvf_paged_attention_decode_biased_bf16": "pppppppiiiiiiiifiiiipppipifpp",
-    "kvf_paged_attention_tcgen05_bf16": "pppppppiiiiiiiiilfipippp",
+    "kvf_paged_attention_tcgen05_bf16": "pppppppiiiiiiiiilfipippipifp",
     "kvf_paged_attention_decode_fused_bf16": "pppppppiiiiiiiifiiiipppp",
-    "kvf_paged_attention_decode_tma_bf16": "pppppppiiiiiiiilfiiiippppiipp",
+    "kvf_paged_attention_decode_tma_bf16": "pppppppiiiiiiiilfiiiippppiipipifp",
     "kvf_gemm_nt_f32": "pppiiiiiip",
     "kvf_gemm_skinny_bf16": "pppiiiiiiiilpp",
     "kvf_set_pdl": "i",
@@ -537,6 +537,11 @@ def tcgen05_attention_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, d
     return dtype == torch.bfloat16 and d in (64, 128) and not decode_form and nh // max(nkv, 1) <= 128
 
 
+def shaped_tcgen05_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, biased: bool) -> bool:
+    """Whether that kernel's form for kept first keys, a bias by distance and capped scores takes the shape."""
+    return tcgen05_attention_supported(dtype, nh, nkv, d, False) and (not biased or nh // max(nkv, 1) <= 8)
+
+
 def tma_decode_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, block_size: int, num_blocks: int) -> bool:
     """Whether the TMA decode kernel (``csrc/attention_decode_tma.cu``) takes this shape."""
     return (
@@ -588,7 +593,8 @@ def paged_attention(
     distance), ``bias`` (added to the scaled scores, by distance and head), ``softcap`` (``c > 0``: a scaled
     score ``s`` becomes ``c * tanh(s / c)``) and ``sinks`` (float ``[nh]``: ``exp(sinks[h])`` joins the softmax's
     denominator of head ``h``; it has no key and no value) are taken by the FP32-pipe kernel and, for bfloat16
-    heads of 64 or 128 with values as wide, by the mma.sync kernels; ``sinks`` without the others also by the tcgen05 and TMA kernels.
+    heads of 64 or 128 with values as wide, by the tcgen05 kernel (many queries; a bias with at most 8 heads a key head), the
+    TMA decode kernel and the mma.sync kernels.
 
     ``q``: rows of ``q_stride`` elements whose first ``nh*d`` are the query heads; ``out``:
     ``[N, nh*d]``.  With ``scratch`` (and every sequence holding one query) the decode form
@@ -624,9 +630,9 @@ def paged_attention(
     if float(softcap) < 0.0:
         raise ValueError("paged_attention: softcap must be positive (0: none)")
     special = vcache is kcache or keep_first > 0 or bias is not None or d > 256 or (dv or d) > 256 or capped
-    # kept first keys and a bias alone, on heads of 64 or 128 in bfloat16 with many queries: the tile form of the mma.sync kernel
+    # kept first keys, a bias and capped scores on heads of 64 or 128 in bfloat16: the tensor cores
     biased_mma = (
-        special and vcache is not kcache and (dv or d) == d and kernel == "auto"
+        special and vcache is not kcache and (dv or d) == d and kernel in ("auto", "tma", "tcgen05")
         and mma_attention_supported(q.dtype, nh, nkv, d, scratch is not None) and (q_stride or q.stride(0)) % 2 == 0 and out.shape[-1] % 2 == 0
         and (scratch is None or len(scratch) > 2)
     )  # fmt: skip
@@ -702,7 +708,17 @@ def paged_attention(
     decode_form = scratch is not None
     use_tc = tcgen05_attention_supported(q.dtype, nh, nkv, d, decode_form) and q_stride % 8 == 0 and out.shape[-1] % 8 == 0 and max_q_len > 1
     use_mma = mma_attention_supported(q.dtype, nh, nkv, d, decode_form)
-    if biased_mma and scratch is not None:
+    # many queries with kept first keys, a bias (of at most 8 heads a key head: a tile's biases lie in shared memory) or capped
+    # scores: the tcgen05 kernel's form for them.  2,048 tokens, 32 heads of 64 under a window of 1,024, with a bias and 64 kept
+    # keys: 76 us, 149 us on the mma.sync tile kernel
+    use_shaped = (
+        biased_mma and use_tc and shaped_tcgen05_supported(q.dtype, nh, nkv, d, bias is not None) and q.data_ptr() % 16 == 0
+        and out.data_ptr() % 16 == 0 and num_seqs <= 65535 and max_q_len <= 65535 * tcgen05_query_tile(nh, nkv)
+    )  # fmt: skip
+    use_tma = tickets is not None and tma_decode_supported(q.dtype, nh, nkv, d, block_size, kcache.shape[0])
+    # decoding with such scores: the TMA kernel's form for them (64 sequences of 32 heads of 64 on 8, contexts of 1,150 to 2,300 under a
+    # window of 1,024, with a bias and 64 kept keys: 36.6 us, 55.8 us on the mma.sync split kernel)
+    if biased_mma and scratch is not None and not use_tma and kernel != "tma":
         name = "kvf_paged_attention_decode_biased_bf16"
         _check(
             _fn(name)(
@@ -713,7 +729,7 @@ def paged_attention(
             name,
         )  # fmt: skip
         return
-    if biased_mma:
+    if biased_mma and scratch is None and not use_shaped and kernel == "auto":
         name = "kvf_paged_attention_mma_biased_bf16"
         _check(
             _fn(name)(
@@ -733,7 +749,7 @@ def paged_attention(
             raise ValueError("the mma.sync attention kernel does not take this shape")
         use_tc = False
     elif kernel == "tcgen05":
-        if not tcgen05_attention_supported(q.dtype, nh, nkv, d, decode_form):
+        if not tcgen05_attention_supported(q.dtype, nh, nkv, d, decode_form) or (biased_mma and not use_shaped):
             raise ValueError("the tcgen05 attention kernel does not take this shape")
         use_tc = True
     if use_tc:
@@ -748,12 +764,11 @@ def paged_attention(
             _fn(name)(
                 _ptr(q), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_tables), _ptr(qsl), _ptr(ctx_lens),
                 num_seqs, max_q_len, q_stride, out.shape[-1], bt_stride, nh, nkv, d, block_size, int(kcache.shape[0]),
-                float(scale), int(window), _ptr(tiles), n_tiles, _ptr(err), _ptr(sinks), _stream(),
+                float(scale), int(window), _ptr(tiles), n_tiles, _ptr(err), _ptr(sinks), int(keep_first), *bias_args, float(softcap), _stream(),
             ),
             name,
         )  # fmt: skip
         return
-    use_tma = tickets is not None and tma_decode_supported(q.dtype, nh, nkv, d, block_size, kcache.shape[0])
     if (kernel == "tma" or single_only) and not use_tma:
         raise ValueError("the TMA decode kernel does not take this shape (or no tickets were given)")
     if use_tma and kernel in ("auto", "tma"):
@@ -762,7 +777,8 @@ def paged_attention(
             _fn(name)(
                 _ptr(q), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_tables), _ptr(qsl), _ptr(ctx_lens),
                 num_seqs, q_stride, out.shape[-1], bt_stride, nh, nkv, d, block_size, int(kcache.shape[0]), float(scale),
-                int(window), split, max_splits, grid_splits, _ptr(pa), _ptr(pm), _ptr(tickets), _ptr(err), int(bool(cluster)) | (2 if single_only else 0), int(wave_target), _ptr(sinks), _stream(),
+                int(window), split, max_splits, grid_splits, _ptr(pa), _ptr(pm), _ptr(tickets), _ptr(err), int(bool(cluster)) | (2 if single_only else 0), int(wave_target), _ptr(sinks),
+                int(keep_first), *bias_args, float(softcap), _stream(),
             ),
             name,
         )  # fmt: skip

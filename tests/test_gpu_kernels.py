@@ -1011,3 +1011,118 @@ def test_latent_attention_routes_by_shape(ops):
     assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
     with pytest.raises(ValueError):
         ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, 40]), i32(ctx), 1, 40, 6, 128, 96, 128**-0.5, kernel="tcgen05")
+
+
+# ------------------------------------------------------------------ shaped scores on tcgen05 (many queries) and by TMA (decoding)
+
+
+def paged_shaped_case(d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts):
+    """Queries, caches on shuffled pages with NaN wherever no key lies, tables, contexts, biases, sinks, and per (request, head) the
+    64-bit result with the bound on what rounding the weights and the result to bfloat16 may change (2^-9 each), times two."""
+    g = torch.Generator().manual_seed(d + nh + window)
+    ctx = [n + s for n, s in zip(lens, starts)]
+    per = [-(-c // block_size) for c in ctx]
+    order = torch.randperm(sum(per) + 2, generator=g).tolist()
+    kc = torch.full((sum(per) + 2, nkv, block_size, d), float("nan"))
+    vc = kc.clone()
+    tables = torch.zeros((len(lens), max(per)), dtype=torch.int32)
+    q = (1.5 * torch.randn((sum(lens), nh * d), generator=g)).bfloat16()
+    rel = 2 * torch.randn((far + 1, nh), generator=g) if far else None
+    sinks = torch.randn(nh, generator=g) if sink else None
+    ref, bound, at, row = [], [], 0, 0
+    for b, (n, c) in enumerate(zip(lens, ctx)):
+        keys, vals = (torch.randn((c, nkv, d), generator=g).bfloat16() for _ in range(2))
+        pages = order[at : at + per[b]]
+        at += per[b]
+        for j in range(c):
+            kc[pages[j // block_size], :, j % block_size], vc[pages[j // block_size], :, j % block_size] = keys[j].float(), vals[j].float()
+        lo, hi = -(-keep // block_size), (max(0, c - n - window + 1) // block_size if window else 0)
+        tables[b, : per[b]] = torch.tensor([-1 if lo <= i < hi else p for i, p in enumerate(pages)], dtype=torch.int32)
+        i, j = torch.arange(c - n, c)[:, None], torch.arange(c)[None]
+        seen = (j <= i) & (((i - j < window) | (j < keep)) if window else True)
+        for h in range(nh):
+            qs = q[row : row + n, h * d : (h + 1) * d].double()
+            s = qs @ keys[:, h // (nh // nkv)].double().T * d**-0.5
+            s = cap * torch.tanh(s / cap) if cap else s
+            s = s + rel[(i - j).clamp(0, far), h].double() if far else s
+            s = s.masked_fill(~seen, -math.inf)
+            if sink:
+                s = torch.cat([s, sinks[h].double().expand(n, 1)], 1)
+            w, v = torch.softmax(s, -1)[:, :c], vals[:, h // (nh // nkv)].double()
+            ref.append((row, h, w @ v))
+            bound.append(2**-8 * (w @ v.abs() + (w @ v).abs()))
+        row += n
+    return q, kc.bfloat16(), vc.bfloat16(), tables, ctx, rel, sinks, ref, bound
+
+
+@pytest.mark.parametrize(
+    "d,nh,nkv,block_size,window,keep,far,cap,sink,lens,starts",
+    [
+        (64, 8, 2, 16, 100, 70, 90, 0.0, False, [33, 1, 130], [300, 200, 0]),  # the bias ends inside the window; a kept tile and a half; a single token
+        (64, 4, 4, 16, 64, 3, 4000, 0.0, True, [200], [77]),  # one head a key head, a table beyond every distance, sinks
+        (64, 6, 2, 32, 0, 0, 50, 5.0, False, [65, 20], [0, 63]),  # 126 of the 128 rows, a bias on capped scores, no window
+        (64, 8, 1, 8, 40, 64, 30, 0.0, False, [90], [140]),  # eight heads a key head, pages that come key by key, kept keys of one tile
+        (128, 8, 2, 16, 130, 200, 128, 3.0, True, [70, 3], [250, 0]),  # heads of 128 with everything at once; kept keys reach into the window
+        (64, 8, 2, 16, 90, 10, 0, 0.0, False, [64, 64], [64, 128]),  # kept keys alone
+        (64, 16, 1, 16, 0, 0, 0, 30.0, True, [150], [10]),  # sixteen heads a key head, capped scores and sinks
+        (128, 2, 1, 48, 1, 0, 7, 0.0, False, [129], [0]),  # a window of the query itself
+    ],
+)
+def test_shaped_scores_of_many_queries_on_tcgen05(ops, d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts):
+    """Unused places of the pages and pages that have come back hold nothing the kernel may read."""
+    q, kc, vc, tables, ctx, rel, sinks, ref, bound = paged_shaped_case(d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    qsl = [0]
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    bias = ops.DistanceBias(dev(rel), i32(list(range(far + 1)))) if far else None
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tq = ops.tcgen05_query_tile(nh, nkv)
+    tiles = sorted([(b, t) for b, n in enumerate(lens) for t in range(0, n, tq)], key=lambda t: -(starts[t[0]] + t[1])) + [(-1, 0)]
+    assert ops.shaped_tcgen05_supported(torch.bfloat16, nh, nkv, d, bias is not None)
+    for work in (None, (i32(tiles).reshape(-1), len(tiles))):
+        out = torch.full((sum(lens), nh * d), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.paged_attention(
+            dev(q), out, dev(kc), dev(vc), dev(tables), i32(qsl), i32(ctx), len(lens), max(lens), nh, nkv, d, d**-0.5,
+            window=window, keep_first=keep, bias=bias, softcap=cap, sinks=dev(sinks) if sink else None, err=err, query_tiles=work,
+        )  # fmt: skip
+        assert int(err.item()) == 0
+        got = out.cpu().double()
+        for (r0, h, o), e in zip(ref, bound):
+            over = (got[r0 : r0 + o.shape[0], h * d : (h + 1) * d] - o).abs() - e
+            assert float(over.max()) <= 0.0, (work is None, r0, h, float(over.max()))
+
+
+@pytest.mark.parametrize(
+    "d,nh,nkv,block_size,window,keep,far,cap,sink,ctx",
+    [
+        (64, 8, 2, 16, 100, 70, 90, 0.0, False, [333, 40, 101, 1]),  # kept keys before the window, inside it, longer than the context
+        (64, 4, 4, 16, 64, 3, 4000, 0.0, True, [277, 64]),  # one head a key head, sinks
+        (64, 6, 2, 32, 0, 0, 50, 5.0, False, [129, 16]),  # three heads a key head, a bias on capped scores
+        (128, 8, 1, 16, 130, 200, 128, 3.0, True, [500, 131, 17]),  # heads of 128 with everything at once
+        (64, 8, 2, 16, 16, 130, 0, 0.0, False, [400, 129]),  # kept keys alone, several ranges of them and ranges of none
+        (64, 16, 2, 48, 0, 0, 0, 30.0, True, [700]),  # capped scores and sinks
+    ],
+)
+def test_shaped_scores_of_a_decode_step_by_tma(ops, d, nh, nkv, block_size, window, keep, far, cap, sink, ctx):
+    """Every form of the ranges' merge: one range, a thread-block cluster, tickets; ranges doubled on the device; and of a mixed
+    batch the single tokens alone."""
+    b = len(ctx)
+    q, kc, vc, tables, _, rel, sinks, ref, bound = paged_shaped_case(d, nh, nkv, block_size, window, keep, far, cap, sink, [1] * b, [c - 1 for c in ctx])
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    bias = ops.DistanceBias(dev(rel), i32(list(range(far + 1)))) if far else None
+    for split, cluster, wave in ((64, True, 0), (64, False, 0), (128, False, 2 * nkv * b), (1024, False, 0)):
+        splits = -(-max(ctx) // split)
+        scratch = (torch.full((b, nh, splits, d), float("nan"), device="cuda"), torch.full((b, nh, splits, 2), float("nan"), device="cuda"), i32([0] * b * nkv))
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        for single in (False, True):
+            out = torch.full((b, nh * d), float("nan"), device="cuda", dtype=torch.bfloat16)
+            ops.paged_attention(
+                dev(q), out, dev(kc), dev(vc), dev(tables), i32(list(range(b + 1))), i32(ctx), b, 1, nh, nkv, d, d**-0.5, window=window, keep_first=keep,
+                bias=bias, softcap=cap, sinks=dev(sinks) if sink else None, err=err, scratch=scratch, max_context=max(ctx), split_size=split,
+                cluster=cluster, wave_target=wave, kernel="tma" if single else "auto", single_only=single,
+            )  # fmt: skip
+            assert int(err.item()) == 0 and int(scratch[2].abs().max()) == 0
+            for (r0, h, o), e in zip(ref, bound):
+                over = (out.cpu().double()[r0, h * d : (h + 1) * d] - o[0]).abs() - e[0]
+                assert float(over.max()) <= 0.0, (split, cluster, r0, h, float(over.max()))
