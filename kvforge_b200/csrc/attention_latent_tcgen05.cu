@@ -4,23 +4,21 @@
 //
 // A CTA serves 128 rows, a row being a (query token, head) pair (128 / nh tokens, every head), and up to 256 value columns: with
 // values of 512 two CTAs share the rows' work, both making the scores.  That costs (d + 256) products a pair of row and key
-// where 2 x (d + 512) / 2 would do, but the accumulator of 128 x 512 alone is all of an SM's tensor memory.  Per tile of 64 keys:
-//   S = Q K^T   tcgen05.mma 128 x 64 x 16, d/16 of them.  What bounds it is shared memory: a product that reads both operands
-//               there takes in 6 KB for 32 cycles of arithmetic, 48 cycles at 128 bytes a cycle.  So the first (up to four) blocks of
-//               64 query numbers lie in tensor memory as the A operand (128 columns), which also leaves room for a second
-//               stage of keys: 80 KB of queries + 2 x 72 KB of keys at d = 576;
-//   softmax     one thread a row, from tensor memory, as in attention_tcgen05.cu (running maximum raised lazily); P takes the place
-//               of S in tensor memory;
+// where 2 x (d + 512) / 2 would do, but the accumulator of 128 x 512 alone is all of an SM's tensor memory.  Per tile of 128 keys:
+//   S = Q K^T   tcgen05.mma 128 x 128 x 16, d/16 of them.  The first (up to four) blocks of 64 query numbers lie in tensor memory
+//               as the A operand (128 columns): 80 KB of queries and 144 KB of keys are what an SM holds;
+//   softmax     two groups of four warps, 64 keys of a row a thread, from tensor memory, as in attention_tcgen05.cu (running maximum
+//               raised lazily; the two halves of a row exchange their maxima); P takes the place of S in tensor memory;
 //   O += P V    P as the A operand from tensor memory, the value tile being the key tile's first dv columns, read as an
-//               MN-major B operand; O stays in tensor memory.
-// S has two buffers: S(t+1) is made while the softmax of tile t runs.  The blocks of a key tile outside the CTA's value
-// columns are free as soon as S is made, the others after P V: each stage has a full and an empty barrier for either part, so
-// that the next tile but one comes in early.  P V has a barrier for the even and one for the odd tiles: a thread that does not
-// wait for every tile's product would mistake the phase before the last for the one it means on a single barrier.  P(t) V(t) has to be over before S(t+2) takes its buffer.
-// Warps: four softmax (thread r owns row r), one loader (TMA boxes of 64 numbers x the keys of a page, 16-byte copies for a last tile
-// that ends inside a page), one issuer.  One CTA an SM.
-// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 240 us against 591 us
-// of the mma.sync kernel, and the same error against 64-bit (the layer around it 717 -> 367 us).
+//               MN-major B operand in blocks of 64 columns, whose chains take turns; O stays in tensor memory.
+// The blocks of a key tile outside the CTA's value columns are free as soon as S is made, the others after P V: either part has a
+// full and an empty barrier, so that the next tile's first part comes in under the softmax and its second under the first's products.
+// Warps: eight softmax (which first bring the queries in), one loader (TMA boxes of 64 numbers x the keys of a page, 16-byte
+// copies for a last tile that ends inside a page), one issuer.  One CTA an SM.
+// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 184 us against 591 us
+// of the mma.sync kernel, and the same error against 64-bit.  What bounds it is that scores, softmax, products and copies of a tile follow one
+// another, for want of room for a second tile: with tiles of 64 keys in two stages and four softmax warps it took 233 us, with tiles of
+// 128 and eight warps 220, and 184 since those eight and not the loader alone bring the queries (147 KB a CTA).
 // Every mbarrier wait is bounded; if one runs out the kernel raises bit 4 of the error flag and winds down.
 #include "tcgen05.cuh"
 
@@ -29,12 +27,12 @@ using namespace kvf::tc;
 
 namespace {
 
-constexpr int BM = 128, BN = 64;
-constexpr int LOADER_WARP = 4, MMA_WARP = 5, THREADS = 192;
+constexpr int BM = 128, BN = 128, HALF = 64;  // rows, keys a tile, keys a softmax group takes of it
+constexpr int SOFTMAX_THREADS = 2 * BM, LOADER_WARP = 8, MMA_WARP = 9, THREADS = 320;
 constexpr int MAX_BLOCKS = 9;                // blocks of 64 numbers of a cache row (d <= 576)
 constexpr int Q_TMEM = 4;                    // blocks of the queries that lie in tensor memory
 constexpr uint32_t Q_BLOCK = BM * 128, K_BLOCK = BN * 128;  // bytes of a [rows][64] block
-constexpr uint32_t COL_O = 0, COL_S = 256, COL_Q = 384;     // tensor-memory columns: O 256, S 2 x 64, Q 4 x 32
+constexpr uint32_t COL_O = 0, COL_S = 256, COL_Q = 384;     // tensor-memory columns: O 256, S 128, Q 4 x 32
 
 struct LatTcParams {
   const bf16* q;
@@ -64,10 +62,9 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       : "memory");
 }
 
-// One tile of the softmax for the thread's row: va, vb the 64 raw scores, w the 64 weights as bfloat16 pairs.  Returns their sum.
+// The maximum of the thread's 64 raw scores, of those from `first` to `last` with MASK.
 template <bool MASK>
-__device__ __forceinline__ float softmax_row(const uint32_t (&va)[32], const uint32_t (&vb)[32], uint32_t (&w)[32], float& m_ref,
-                                             float& corr, float scale_log2, int first, int last) {
+__device__ __forceinline__ float row_max(const uint32_t (&va)[32], const uint32_t (&vb)[32], int first, int last) {
   float mx = -INFINITY;
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
@@ -75,12 +72,11 @@ __device__ __forceinline__ float softmax_row(const uint32_t (&va)[32], const uin
     const float b = (!MASK || (j + 32 >= first && j + 32 <= last)) ? __uint_as_float(vb[j]) : -INFINITY;
     mx = fmaxf(mx, fmaxf(a, b));
   }
-  mx *= scale_log2;  // scale > 0
-  corr = 1.f;
-  if (mx > m_ref + RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY)) {
-    corr = ex2(m_ref - mx);  // 0 the first time
-    m_ref = mx;
-  }
+  return mx;
+}
+// exp2(score * scale - m_ref) of the 64 scores as bfloat16 pairs; returns their sum.
+template <bool MASK>
+__device__ __forceinline__ float weights(const uint32_t (&va)[32], const uint32_t (&vb)[32], uint32_t (&w)[32], float m_ref, float scale_log2, int first, int last) {
   const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
   const uint64_t scale2 = pack2(scale_log2, scale_log2), neg_m2 = pack2(-m_use, -m_use);
   uint64_t sum_a = pack2(0.f, 0.f), sum_b = sum_a;
@@ -109,12 +105,12 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = sm32(smem_raw);
   const uint32_t q_s = base;                                             // [kb - qt] blocks of [128 rows][64]
-  const uint32_t k_s = q_s + (uint32_t)(p.kb - p.qt) * Q_BLOCK;          // per stage [kb] blocks of [64 keys][64]
-  const uint32_t k_stage = (uint32_t)p.kb * K_BLOCK;
-  const uint32_t bars = k_s + 2 * k_stage;
+  const uint32_t k_s = q_s + (uint32_t)(p.kb - p.qt) * Q_BLOCK;          // [kb] blocks of [128 keys][64]
+  const uint32_t xch = k_s + (uint32_t)p.kb * K_BLOCK;                   // [2][2][128] floats: the halves' maxima, of even and odd tiles
+  const uint32_t bars = xch + 4 * BM * 4;
   // part 0 of a key tile: the blocks outside this CTA's value columns; part 1: the others
-  const uint32_t q_full = bars, kf0 = bars + 8, kf1 = bars + 24, ke0 = bars + 40, ke1 = bars + 56, s_full = bars + 72, p_full = bars + 88,
-                 pv_done = bars + 104, drained = bars + 120, tmem_slot = bars + 128;
+  const uint32_t q_full = bars, kf0 = bars + 8, kf1 = bars + 16, ke0 = bars + 24, ke1 = bars + 32, s_full = bars + 40, p_full = bars + 48,
+                 pv_done = bars + 56, drained = bars + 64, tmem_slot = bars + 72;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - base));
 
   pdl_launch();
@@ -141,16 +137,14 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
   const int n_tiles = live ? (kv_hi - kv_lo + BN - 1) / BN : 0;
 
   if (threadIdx.x == 0) {
-    bar_init(q_full, BM + 1);
-    for (int s = 0; s < 2; ++s) {
-      bar_init(kf0 + 8 * s, 1);
-      bar_init(kf1 + 8 * s, 1);
-      bar_init(ke0 + 8 * s, 1);
-      bar_init(ke1 + 8 * s, 1);
-      bar_init(s_full + 8 * s, 1);
-      bar_init(p_full + 8 * s, BM);
-      bar_init(pv_done + 8 * s, 1);
-    }
+    bar_init(q_full, SOFTMAX_THREADS);
+    bar_init(kf0, 1);
+    bar_init(kf1, 1);
+    bar_init(ke0, 1);
+    bar_init(ke1, 1);
+    bar_init(s_full, 1);
+    bar_init(p_full, SOFTMAX_THREADS);
+    bar_init(pv_done, 1);
     bar_init(drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -166,17 +160,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
   pdl_wait();
 
   if (live && warp == LOADER_WARP) {
-    // ---- loader: the queries' blocks that lie in shared memory, then the key tiles
-    const int qc = (p.kb - p.qt) * 8;  // 16-byte chunks of a row
-    for (int idx = lane; idx < BM * qc; idx += 32) {
-      const int r = idx / qc, c = idx - r * qc;
-      const int tok = r / p.nh, hh = r - tok * p.nh;
-      const int at = (p.qt * 8 + c) * 8;
-      const bool valid = tok < n_tok && at < p.d;
-      cpa16(q_s + (uint32_t)(c >> 3) * Q_BLOCK + sw128(r, c & 7),
-            p.q + (valid ? (size_t)(q_begin + q0 + tok) * p.q_stride + (size_t)hh * p.d + at : 0), valid);
-    }
-    cpa_commit();
+    // ---- loader: the key tiles
     const int* bt = p.block_tables + (size_t)b * p.bt_stride;
     auto page_of = [&](int key, int& off) {  // the page of a key (-1: past the context or given back)
       off = 0;
@@ -189,14 +173,11 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
       return bt[key / p.block_size];
     };
     const int boxes = BN / p.box_rows;
+    bool ok = true;
     int last0 = -1, last1 = -1;  // the last tile whose part 0, whose part 1 was asked for
-    bool ok = true, q_handed = false;
     for (int t = 0; t < n_tiles && ok; ++t) {
-      const int s = t & 1;
-      const uint32_t ks = k_s + (uint32_t)s * k_stage;
       const int t0 = kv_lo + t * BN;
       const bool ragged = t0 + BN > ctx && (ctx & (p.box_rows - 1)) != 0;
-      const uint32_t par = ((t >> 1) - 1) & 1;
       if (!ragged) {
         // lane j looks up box j (box_rows keys of one page); then the lanes share out the boxes of the part's blocks
         int off;
@@ -205,22 +186,22 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
         for (int part = 0; part < 2; ++part) {
           const int nb = part ? p.nvb : n0;
           if (nb == 0) continue;
-          if (t >= 2) ok = __all_sync(0xffffffffu, bar_wait((part ? ke1 : ke0) + 8 * s, par, p.err));
+          if (t >= 1) ok = __all_sync(0xffffffffu, bar_wait(part ? ke1 : ke0, (t - 1) & 1, p.err));
           if (!ok) break;
-          const uint32_t bar = (part ? kf1 : kf0) + 8 * s;
+          const uint32_t bar = part ? kf1 : kf0;
           if (lane == 0) bar_expect_tx(bar, (uint32_t)nb * K_BLOCK);
           __syncwarp();
           (part ? last1 : last0) = t;
           for (int i = lane; i < nb * boxes; i += 32) {  // boxes divides 32: a lane keeps its box
             const int j = i / boxes;
             const int kb = part ? vb0 + j : (j < vb0 ? j : j + p.nvb);
-            tma_load_2d(ks + (uint32_t)kb * K_BLOCK + (uint32_t)((lane % boxes) * p.box_rows) * 128u, &map, 64 * kb, row, bar);
+            tma_load_2d(k_s + (uint32_t)kb * K_BLOCK + (uint32_t)((lane % boxes) * p.box_rows) * 128u, &map, 64 * kb, row, bar);
           }
         }
       } else {
         // the sequence's last tile ends inside a page, whose other keys must not be read: key by key, zeros past the context
-        if (t >= 2) {
-          ok = __all_sync(0xffffffffu, (n0 == 0 || bar_wait(ke0 + 8 * s, par, p.err)) && bar_wait(ke1 + 8 * s, par, p.err));
+        if (t >= 1) {
+          ok = __all_sync(0xffffffffu, (n0 == 0 || bar_wait(ke0, (t - 1) & 1, p.err)) && bar_wait(ke1, (t - 1) & 1, p.err));
           if (!ok) break;
         }
         const int chunks = p.kb * 8;
@@ -230,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
           const bf16* src = p.cache + (blk >= 0 ? ((size_t)blk * p.block_size + off) * p.d : 0);
           for (int c = lane; c < chunks; c += 32) {
             const bool valid = blk >= 0 && c * 8 < p.d;
-            cpa16(ks + (uint32_t)(c >> 3) * K_BLOCK + sw128(key, c & 7), src + (valid ? c * 8 : 0), valid);
+            cpa16(k_s + (uint32_t)(c >> 3) * K_BLOCK + sw128(key, c & 7), src + (valid ? c * 8 : 0), valid);
           }
         }
         cpa_commit();
@@ -238,107 +219,101 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
         fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (!q_handed) bar_arrive(q_full);
-          if (n0) bar_arrive(kf0 + 8 * s);
-          bar_arrive(kf1 + 8 * s);
+          if (n0) bar_arrive(kf0);
+          bar_arrive(kf1);
         }
-        q_handed = true;
         if (n0) last0 = t;
         last1 = t;
       }
-      if (ok && !q_handed && (t == 1 || t + 1 == n_tiles)) {  // the first tiles are on their way: now wait for the queries
-        cpa_wait<0>();
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) bar_arrive(q_full);
-        q_handed = true;
-      }
     }
-    cpa_wait<0>();
     // no copy outlives the CTA, whatever made the others leave
-    for (int back = 0; back < 2; ++back) {
-      if (last0 - back >= 0) bar_wait(kf0 + 8 * ((last0 - back) & 1), ((last0 - back) >> 1) & 1, p.err);
-      if (last1 - back >= 0) bar_wait(kf1 + 8 * ((last1 - back) & 1), ((last1 - back) >> 1) & 1, p.err);
-    }
+    if (last0 >= 0) bar_wait(kf0, last0 & 1, p.err);
+    if (last1 >= 0) bar_wait(kf1, last1 & 1, p.err);
   } else if (live && warp == MMA_WARP) {
     if (lane == 0) {
       const uint32_t id_s = idesc(BN, 0), id_o = idesc(64, 1);
-      const uint64_t q_d = sdesc(q_s), k_d = sdesc(k_s);
+      const uint64_t q_d = sdesc(q_s), k_d = sdesc(k_s), v_d = sdesc(k_s + (uint32_t)vb0 * K_BLOCK);
+      const uint32_t s_t = tmem + COL_S, o_t = tmem + COL_O;
       bool ok = bar_wait(q_full, 0, p.err);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      auto issue_s = [&](int t) {
-        const int s = t & 1;
-        const uint32_t dst = tmem + COL_S + (uint32_t)s * BN, par = (t >> 1) & 1;
-        const uint64_t kd = k_d + (uint64_t)(((uint32_t)s * k_stage) >> 4);
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        if (t > 0) ok = bar_wait(pv_done, (t - 1) & 1, p.err);  // S(t) goes where P(t-1) lies
         uint32_t acc = 0;
-        for (int part = 0; part < 2; ++part) {
+        for (int part = 0; part < 2 && ok; ++part) {
           const int nb = part ? p.nvb : n0;
           if (nb == 0) continue;
-          if (!bar_wait((part ? kf1 : kf0) + 8 * s, par, p.err)) return false;
+          ok = bar_wait(part ? kf1 : kf0, t & 1, p.err);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           for (int j = 0; j < nb; ++j) {
             const int kb = part ? vb0 + j : (j < vb0 ? j : j + p.nvb);
-            const uint64_t bd = kd + (uint64_t)((uint32_t)kb * (K_BLOCK >> 4));
+            const uint64_t bd = k_d + (uint64_t)((uint32_t)kb * (K_BLOCK >> 4));
             if (kb < p.qt) {
               const uint32_t a = tmem + COL_Q + (uint32_t)kb * 32u;
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk) {
-                umma_ts(dst, a + 8u * kk, bd + 2 * kk, id_s, acc);
+                umma_ts(s_t, a + 8u * kk, bd + 2 * kk, id_s, acc);
                 acc = 1;
               }
             } else {
               const uint64_t ad = q_d + (uint64_t)((uint32_t)(kb - p.qt) * (Q_BLOCK >> 4));
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk) {
-                umma(dst, ad + 2 * kk, bd + 2 * kk, id_s, acc);
+                umma(s_t, ad + 2 * kk, bd + 2 * kk, id_s, acc);
                 acc = 1;
               }
             }
           }
-          if (part == 0) umma_commit(ke0 + 8 * s);  // what is not a value is free again
+          umma_commit(part ? s_full : ke0);  // S is made; what is not a value is free again
         }
-        umma_commit(s_full + 8 * s);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      if (ok && n_tiles > 1) ok = issue_s(1);
-      for (int t = 0; t < n_tiles && ok; ++t) {
-        const int s = t & 1;
-        ok = bar_wait(p_full + 8 * s, (t >> 1) & 1, p.err);  // P(t) is in tensor memory, O has been rescaled
+        if (ok) ok = bar_wait(p_full, t & 1, p.err);  // P(t) is in tensor memory, O has been rescaled
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = tmem + COL_S + (uint32_t)s * BN;
-        const uint64_t vd = k_d + (uint64_t)(((uint32_t)s * k_stage + (uint32_t)vb0 * K_BLOCK) >> 4);
-        for (int j = 0; j < p.nvb; ++j) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)  // A: 16 keys of P = 8 columns; B: 16 keys = 16 rows of 128 bytes
-            umma_ts(tmem + COL_O + 64u * j, a + 8u * kk, vd + (uint64_t)((uint32_t)j * (K_BLOCK >> 4) + kk * (16 * 128 >> 4)), id_o,
-                    (t > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(pv_done + 8 * s);
-        umma_commit(ke1 + 8 * s);
-        if (t + 2 < n_tiles) {
-          ok = bar_wait(pv_done + 8 * s, (t >> 1) & 1, p.err);  // S(t+2) goes where P(t) lies
-          if (ok) ok = issue_s(t + 2);
-        }
+        for (int kk = 0; kk < BN / 16; ++kk)  // A: 16 keys of P = 8 columns; B: 16 keys = 16 rows of 128 bytes
+          for (int j = 0; j < p.nvb; ++j)
+            umma_ts(o_t + 64u * j, s_t + 8u * kk, v_d + (uint64_t)((uint32_t)j * (K_BLOCK >> 4) + kk * (16 * 128 >> 4)), id_o, (t > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(pv_done);
+        umma_commit(ke1);
       }
       if (!ok) {  // no product outlives the tensor memory
         umma_commit(drained);
         bar_wait(drained, 0, p.err);
       }
     }
-  } else if (live && warp < 4) {
-    // ---- softmax and output: thread r owns row r
-    const int r = threadIdx.x;
+  } else if (live && warp < LOADER_WARP) {
+    // ---- softmax and output: thread r of either group owns row r, group 0 the first 64 keys of a tile, group 1 the others
+    const int grp = warp >> 2, r = threadIdx.x & (BM - 1);
     const int tok = r / p.nh, hh = r - tok * p.nh;
     const bool valid = tok < n_tok;
     const int pos = valid ? p_first + tok : -1;
     const int lo = first_key(pos, p.window);
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t my_s = tmem + lane_addr + COL_S, my_o = tmem + lane_addr + COL_O;
+    float* const mine = reinterpret_cast<float*>(smem_raw + (xch - base)) + grp * BM + r;
+    const float* const theirs = reinterpret_cast<const float*>(smem_raw + (xch - base)) + (grp ^ 1) * BM + r;
     {
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + (valid ? (size_t)(q_begin + q0 + tok) * p.q_stride + (size_t)hh * p.d : 0));
-      for (int blk = 0; blk < p.qt; ++blk) {
+      // the queries: blocks from qt on to shared memory by all 256 threads, then either group writes half of the others to tensor memory
+      const int qc = (p.kb - p.qt) * 8;  // 16-byte chunks of a row
+      const bf16* const rows = p.q + (size_t)(q_begin + q0) * p.q_stride;
+      if (qc) {
+        int rr = (int)threadIdx.x / qc, c = (int)threadIdx.x - rr * qc;
+        const int dr = SOFTMAX_THREADS / qc, dc = SOFTMAX_THREADS - dr * qc;
+        while (rr < BM) {
+          const int tk = rr / p.nh, at = (p.qt * 8 + c) * 8;
+          const bool in = tk < n_tok && at < p.d;
+          cpa16(q_s + (uint32_t)(c >> 3) * Q_BLOCK + sw128(rr, c & 7), rows + (in ? (size_t)tk * p.q_stride + (size_t)(rr - tk * p.nh) * p.d + at : 0), in);
+          rr += dr;
+          c += dc;
+          if (c >= qc) {
+            c -= qc;
+            ++rr;
+          }
+        }
+        cpa_commit();
+      }
+      const uint4* src = reinterpret_cast<const uint4*>(rows + (valid ? (size_t)tok * p.q_stride + (size_t)hh * p.d : 0));
+      for (int blk = grp; blk < p.qt; blk += 2) {
         uint32_t v[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -348,36 +323,44 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
         tmem_st32(tmem + lane_addr + COL_Q + (uint32_t)blk * 32u, v);
       }
       tmem_wait_st();
+      cpa_wait<0>();
+      fence_async_smem();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       bar_arrive(q_full);
     }
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     int t = 0;
-    for (; t < n_tiles && ok; ++t) {
-      const int s = t & 1, key0 = kv_lo + t * BN;
+    for (; t < n_tiles; ++t) {
+      const int key0 = kv_lo + t * BN + grp * HALF;
       // (tcgen05.ld and st are warp-wide: the lanes of a warp leave the loop together)
-      ok = __all_sync(0xffffffffu, bar_wait(s_full + 8 * s, (t >> 1) & 1, p.err));
+      ok = __all_sync(0xffffffffu, bar_wait(s_full, t & 1, p.err));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint32_t va[32], vb[32], w[32];
-      tmem_ld32(my_s + (uint32_t)s * BN, va);
-      tmem_ld32(my_s + (uint32_t)s * BN + 32u, vb);
+      uint32_t va[32], vb[32];
+      tmem_ld32(my_s + (uint32_t)(grp * HALF), va);
+      tmem_ld32(my_s + (uint32_t)(grp * HALF) + 32u, vb);
       tmem_wait(va);
       tmem_wait(vb);
-      const bool need_mask = (key0 + BN - 1 > pos) || (key0 < lo);
-      float corr, sum;
-      if (__any_sync(0xffffffffu, need_mask))
-        sum = softmax_row<true>(va, vb, w, m_ref, corr, p.scale_log2, max(lo, key0) - key0, min(pos, key0 + BN - 1) - key0);
-      else
-        sum = softmax_row<false>(va, vb, w, m_ref, corr, p.scale_log2, 0, BN - 1);
+      const bool mask = __any_sync(0xffffffffu, (key0 + HALF - 1 > pos) || (key0 < lo));
+      const int first = max(lo, key0) - key0, last = min(pos, key0 + HALF - 1) - key0;
+      float mx = mask ? row_max<true>(va, vb, first, last) : row_max<false>(va, vb, 0, HALF - 1);
+      mine[(t & 1) * 2 * BM] = mx;
+      // both halves of every row are in registers: their maxima can be exchanged, and P may take the place of S
+      asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
+      mx = fmaxf(mx, theirs[(t & 1) * 2 * BM]) * p.scale_log2;  // scale > 0
+      float corr = 1.f;
+      if (mx > m_ref + RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY)) {
+        corr = ex2(m_ref - mx);  // 0 the first time
+        m_ref = mx;
+      }
+      uint32_t w[32];
+      const float sum = mask ? weights<true>(va, vb, w, m_ref, p.scale_log2, first, last) : weights<false>(va, vb, w, m_ref, p.scale_log2, 0, HALF - 1);
       l = l * corr + sum;
-      tmem_st32(my_s + (uint32_t)s * BN, w);  // 64 weights = 32 columns, where the thread's scores were
+      tmem_st32(my_s + (uint32_t)(grp * 32), w);  // 64 weights = 32 columns
+      // P V of the tile before is over (S(t) was made after it): either group rescales half of O
       if (t > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
-        ok = __all_sync(0xffffffffu, bar_wait(pv_done + 8 * (s ^ 1), ((t - 1) >> 1) & 1, p.err));  // O holds tiles 0 .. t-1
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int c0 = 0; c0 < 64 * p.nvb; c0 += 32) {
+        for (int c0 = 32 * grp; c0 < 64 * p.nvb; c0 += 64) {
           uint32_t v[32];
           tmem_ld32(my_o + (uint32_t)c0, v);
           tmem_wait(v);
@@ -388,14 +371,21 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
       }
       tmem_wait_st();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      bar_arrive(p_full + 8 * s);
+      bar_arrive(p_full);
     }
-    if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, p.err));
+    // a warp whose wait ran out still meets the others at the barriers of the tiles left
+    if (!ok)
+      for (; t < n_tiles; ++t) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
+    if (ok) ok = __all_sync(0xffffffffu, bar_wait(pv_done, (n_tiles - 1) & 1, p.err));
+    // (the sums take the place that the maxima of the tile before the last had)
+    mine[(n_tiles & 1) * 2 * BM] = l;
+    asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
+    l += theirs[(n_tiles & 1) * 2 * BM];
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inv = l > 0.f ? 1.f / l : 0.f;
       bf16* dst = p.out + (size_t)(q_begin + q0 + (valid ? tok : 0)) * p.out_stride + (size_t)hh * p.dv + vb0 * 64;
-      for (int c0 = 0; c0 < 64 * p.nvb; c0 += 32) {
+      for (int c0 = 32 * grp; c0 < 64 * p.nvb; c0 += 64) {
         uint32_t v[32];
         tmem_ld32(my_o + (uint32_t)c0, v);
         tmem_wait(v);
@@ -453,7 +443,7 @@ KVF_API int kvf_latent_attention_tcgen05_bf16(const void* q, void* out, const vo
   memset(&map, 0, sizeof(map));
   const int rc = cache_map(&map, cache, rows, d, p.box_rows);
   if (rc) return rc;
-  const size_t smem = (size_t)(p.kb - p.qt) * Q_BLOCK + (size_t)2 * p.kb * K_BLOCK + 144;
+  const size_t smem = (size_t)(p.kb - p.qt) * Q_BLOCK + (size_t)p.kb * K_BLOCK + 4 * BM * 4 + 96;
   const cudaError_t e = cudaFuncSetAttribute(latent_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   return launch(latent_tcgen05_kernel, dim3(dv / (64 * p.nvb), work ? n_work : B, work ? 1 : tiles), dim3(THREADS), smem, st, map, p);

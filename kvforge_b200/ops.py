@@ -813,7 +813,7 @@ def latent_attention_supported(dtype: torch.dtype, d: int, dv: int) -> bool:
 
 def latent_tcgen05_supported(dtype: torch.dtype, nh: int, d: int, dv: int, block_size: int) -> bool:
     """Whether the tcgen05 kernel for many queries over such a cache (``csrc/attention_latent_tcgen05.cu``) takes the shape: a row
-    of at most 576 numbers (128 queries of it and two tiles of 64 keys fill an SM's shared memory), pages that come as whole
+    of at most 576 numbers (128 queries of it and a tile of 128 keys fill an SM's shared memory), pages that come as whole
     tensor-map boxes."""
     return dtype == torch.bfloat16 and d % 16 == 0 and dv <= d <= 576 and dv in (64, 128, 256, 512) and 0 < nh <= 128 and block_size % 16 == 0
 
@@ -856,7 +856,7 @@ def latent_attention(
     )  # fmt: skip
     if kernel == "tcgen05" and not takes:
         raise ValueError("latent_attention: the tcgen05 kernel does not take this call")
-    # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 240 us here, 591 us on
+    # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 184 us here, 591 us on
     # the mma.sync kernel; single queries go to its key ranges, which a CTA of 128 rows would leave empty
     if takes and (kernel == "tcgen05" or (kernel == "auto" and max_q_len > 1)):
         tiles, n_tiles = None, 0
