@@ -33,6 +33,18 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // shared library; off unless the host turns it on).
 inline int g_pdl_enabled = 0;
 
+// Shared memory to ask for, for a grid of few CTAs that live long: so much that an SM holds no more of them than the grid has for
+// each SM.  CTAs that are launched under the tail of the kernel before (pdl_launch) go to the SMs that have room
+// first, several to one, and stay there while other SMs idle: the delta rule's 256 CTAs over 2,048 tokens took 860 us behind the
+// kernel that makes their records, 510 with it.
+inline size_t spread_smem(size_t need, long long ctas) {
+  constexpr size_t SM = 228 * 1024, RESERVED = 1024;  // of an SM; what the hardware takes of it for a CTA
+  const long long each = (ctas + 147) / 148;
+  if (each < 1 || each > 32) return need;
+  const size_t room = (SM / (size_t)each - RESERVED) & ~(size_t)127;
+  return need > room ? need : room;
+}
+
 template <typename... KArgs, typename... Args>
 inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};

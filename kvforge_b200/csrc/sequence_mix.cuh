@@ -10,8 +10,9 @@
 //
 // Everything a recurrence reads besides the projections (decays, step sizes, unit norms, the state
 // itself) is float whatever the storage type T is.  Every sum has a fixed order that depends on the
-// sizes alone, so a token's result does not depend on how its sequence was cut into steps or on what
-// else the step holds.
+// sizes alone, so token by token (32-bit storage) a token's result does not depend on how its sequence
+// was cut into steps or on what else the step holds; in bfloat16 a step that holds a sequence of more than
+// four tokens may go four at a time, which shows in the last bits of a float.
 #pragma once
 #include "sequence_common.cuh"
 
@@ -28,6 +29,7 @@ namespace {
 // with k and q made unit vectors per head (x / sqrt(sum x^2 + norm_eps)), q times q_scale,
 // beta = sigmoid(b), g = exp(-exp(A_log[h]) * softplus(a + dt_bias)).
 //
+// (Many tokens a sequence in bfloat16 storage are walked four at a time: delta_groups.cuh.)
 // The walk over a sequence's tokens is a chain: a token's update needs the state the token before
 // left.  What bounds it is the latency of one link, so a link is made short.  A CTA owns a sequence,
 // a head and a tile of columns of S; a column's rows are spread over KS neighbouring lanes, R rows
@@ -74,6 +76,8 @@ struct DeltaParams {
   // the logits of beta (and of a per-head step size) may come as the float slices of a split-K product
   int logit_slices;
   long long logit_slice_stride;
+  // the records of groups of four tokens (delta_groups.cuh), or null: token by token
+  float* groups;
 };
 
 // exp(rate * softplus(x)), rate < 0: exact library functions in 32-bit storage; in bfloat16 storage the fast
@@ -142,6 +146,12 @@ __device__ __forceinline__ void cp_async16(float* smem_dst, const float* gsrc) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
 }
+
+}  // namespace
+
+#include "delta_groups.cuh"
+
+namespace {
 
 // PW producer warps: 4 for walks over many tokens; 1 for steps of a few tokens a sequence (decoding), where a
 // CTA lives for microseconds and what counts is how many of them fit an SM
@@ -389,6 +399,11 @@ template <typename T>
 int dispatch_delta(const DeltaParams& p, int B, int max_q_len, cudaStream_t st) {
   const long long pairs = (long long)p.N * p.H;
   if (pairs <= 0) return 0;
+  if constexpr (sizeof(T) == 2) {
+    // four tokens a link where a sequence brings more than that; 32-bit storage walks token by token, so that its sums
+    // do not depend on how a sequence was cut
+    if (p.groups) return p.per_channel ? dispatch_delta_groups<T, true>(p, B, st) : dispatch_delta_groups<T, false>(p, B, st);
+  }
   int rc = launch(delta_prepare_kernel<T>, dim3((unsigned)((pairs + 3) / 4)), dim3(128), 0, st, p);
   if (rc) return rc;
   const bool few = max_q_len > 0 && max_q_len <= 4;
@@ -434,7 +449,8 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
                                     float* out, int out_stride, const int* qsl, const int* state_slots, int B, int H,  \
                                     int G, int dk, int dv, float q_scale, float norm_eps, int max_q_len, int N,        \
                                     float* kn, float* qn, float* gn, float* sc, int logit_slices,                      \
-                                    long long logit_slice_stride, cudaStream_t st) {                                   \
+                                    long long logit_slice_stride, float* groups, long long groups_floats,              \
+                                    cudaStream_t st) {                                                                 \
     if (B <= 0) return 0;                                                                                              \
     if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || (unsigned)H > 65535u) return (int)cudaErrorInvalidValue;    \
     DeltaParams p;                                                                                                     \
@@ -443,8 +459,14 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
     p.state_stride = state_stride; p.out = out; p.out_stride = out_stride; p.qsl = qsl; p.state_slots = state_slots;   \
     p.H = H; p.G = G; p.dk = dk; p.dv = dv; p.q_scale = q_scale; p.norm_eps = norm_eps; p.chunk = 1; p.buf_floats = 0;  \
     p.kn = kn; p.qn = qn; p.gn = gn; p.sc = sc; p.N = N;                                                               \
-    p.logit_slices = logit_slices; p.logit_slice_stride = logit_slice_stride;                                          \
-    if (!kn || !qn || !sc || (per_channel && !gn)) return (int)cudaErrorInvalidValue;                                  \
+    p.logit_slices = logit_slices; p.logit_slice_stride = logit_slice_stride; p.groups = groups;                       \
+    if (groups) {                                                                                                      \
+      if (sizeof(T) != 2 || dk <= 64 || dk > DG_ROWS || max_q_len <= DG_TOKENS || (((uintptr_t)groups) & 15) ||                        \
+          groups_floats < ((long long)N / DG_TOKENS + B) * H * dg_record(per_channel != 0))                            \
+        return (int)cudaErrorInvalidValue;                                                                             \
+    } else if (!kn || !qn || !sc || (per_channel && !gn)) {                                                            \
+      return (int)cudaErrorInvalidValue;                                                                               \
+    }                                                                                                                  \
     return dispatch_delta<T>(p, B, max_q_len, st);                                                                     \
   }                                                                                                                    \
   KVF_API int kvf_gated_head_norm_##SUF(const float* o, int o_stride, const void* gate, int gate_stride,               \

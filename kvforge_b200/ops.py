@@ -44,7 +44,7 @@ _SIGNATURES = {
     "kvf_causal_conv_{s}": "pippplppiiiiipiip",
     "kvf_conv_set_pdl": "i",
     # libraries "mixers" and "streams"
-    "kvf_gated_delta_{s}": "pppipipippiplpippiiiiiffiippppilp",
+    "kvf_gated_delta_{s}": "pppipipippiplpippiiiiiffiippppilplp",
     "kvf_gated_head_norm_{s}": "pipipfiliipip",
     "kvf_hc_step_{s}": "pppilppppppiiifp",
     "kvf_branch_norm_mean_{s}": "pppppilifppp",
@@ -1270,12 +1270,30 @@ def causal_conv(
     )  # fmt: skip
 
 
+DELTA_GROUP_TOKENS = 4
+
+
+def delta_groups_ok(dtype: torch.dtype, dk: int, max_query_len: int) -> bool:
+    """Whether a step of the delta rule goes four tokens at a time (``csrc/delta_groups.cuh`` has both sides' times)."""
+    return dtype == torch.bfloat16 and 64 < dk <= 128 and max_query_len > DELTA_GROUP_TOKENS
+
+
+def delta_group_record(num_heads: int, per_channel: bool) -> int:
+    """Floats that a group of tokens takes: per head its vectors of 128 numbers and 36 coefficients."""
+    return num_heads * ((13 if per_channel else 8) * 128 + 36)
+
+
+def delta_group_floats(n: int, num_seqs: int, num_heads: int, per_channel: bool) -> int:
+    """Floats of the records of ``n`` tokens in ``num_seqs`` sequences."""
+    return (n // DELTA_GROUP_TOKENS + num_seqs) * delta_group_record(num_heads, per_channel)
+
+
 def gated_delta(
     q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logits: torch.Tensor, step_logits: torch.Tensor,
     a_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, out: torch.Tensor, qsl: torch.Tensor,
     state_slots: torch.Tensor, num_seqs: int, num_heads: int, num_kv_heads: int, dk: int, dv: int, q_scale: float,
     norm_eps: float = 1e-6, max_query_len: int = 0, scratch: tuple[torch.Tensor, ...] | None = None,
-    logit_slices: int = 0, logit_slice_stride: int = 0,
+    logit_slices: int = 0, logit_slice_stride: int = 0, groups: torch.Tensor | None = None,
 ) -> None:  # fmt: skip
     """The gated delta rule over a flat batch, token by token per sequence, on the state
     ``S [heads, dk, dv]`` of each sequence's slot (``csrc/sequence_mix.cuh`` has the equations).
@@ -1288,6 +1306,8 @@ def gated_delta(
     ``scratch``: float buffers ``(kn [N, H*dk], qn [N, H*dk], gn [N, H*dk] or None, sc [N, H*4])`` for what
     a kernel of its own makes of every token before the walk (unit k and q, decays, beta, k.q); without it
     they are allocated here (tests; a step of the engine passes persistent buffers).  Two launches.
+    ``groups``: a float buffer of ``delta_group_floats`` numbers; the step then goes four tokens at a time (``delta_groups_ok``:
+    bfloat16, 64 < dk <= 128, more than four rows of some sequence; ``csrc/delta_groups.cuh``) and needs no ``scratch``.
     ``logit_slices > 1``: ``beta_logits`` (and per-head ``step_logits``) are slice 0 of that many float
     slices of a split-K product, ``logit_slice_stride`` elements apart, summed in slice order."""
     s = _suffix(q.dtype)
@@ -1310,12 +1330,17 @@ def gated_delta(
     sptr, sstride = _state_view(state, h * dk * dv, "delta state")
     _need(qsl, torch.int32, "query_start_loc")
     _need(state_slots, torch.int32, "state_slots")
-    if scratch is None:
+    if groups is not None:
+        _need(groups, torch.float32, "delta groups")
+        if not delta_groups_ok(q.dtype, dk, max_query_len) or groups.numel() < delta_group_floats(n, num_seqs, h, per_channel):
+            raise ValueError("gated_delta: the step does not go in groups, or their buffer is too small")
+        scratch = (None, None, None, None)
+    elif scratch is None:
         mk = lambda w: torch.empty((n, w), dtype=torch.float32, device=q.device)  # noqa: E731
         scratch = (mk(h * dk), mk(h * dk), mk(h * dk) if per_channel else None, mk(h * 4))
     kn, qn, gn, sc = scratch
     for t, w, what in ((kn, h * dk, "kn"), (qn, h * dk, "qn"), (gn, h * dk, "gn"), (sc, h * 4, "sc")):
-        if t is None and what == "gn" and not per_channel:
+        if groups is not None or (t is None and what == "gn" and not per_channel):
             continue
         _need(t, torch.float32, f"scratch {what}")
         if tuple(t.shape) != (n, w):
@@ -1326,7 +1351,8 @@ def gated_delta(
             _ptr(q), _ptr(k), _ptr(v), q.stride(0), _ptr(beta_logits), beta_logits.stride(0), _ptr(step_logits),
             step_logits.stride(0), _ptr(a_log), _ptr(dt_bias), 1 if per_channel else 0, sptr, sstride, _ptr(out),
             out.stride(0), _ptr(qsl), _ptr(state_slots), num_seqs, h, g, dk, dv, float(q_scale), float(norm_eps), int(max_query_len),
-            n, _ptr(kn), _ptr(qn), _ptr(gn) if per_channel else None, _ptr(sc), int(logit_slices), int(logit_slice_stride), _stream(),
+            n, _ptr(kn), _ptr(qn), _ptr(gn) if per_channel else None, _ptr(sc), int(logit_slices), int(logit_slice_stride),
+            _ptr(groups), groups.numel() if groups is not None else 0, _stream(),
         ),
         name,
         2,

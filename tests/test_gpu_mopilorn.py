@@ -389,6 +389,66 @@ def test_gated_delta_rule_through_the_state(dtype, h, g, dk, dv, channel):
     assert float(state[1].abs().max()) == 0 and float(state[:, :5].abs().max()) == 0
 
 
+@pytest.mark.parametrize("rate", [0.0, 3.0, -4.0])  # decays of every size, ones that forget at once, ones that keep all
+@pytest.mark.parametrize(
+    "h,g,dk,dv,channel",
+    [(3, 1, 65, 33, True), (2, 2, 72, 20, False), (2, 1, 96, 130, True), (3, 1, 100, 40, False), (2, 2, 128, 128, True), (2, 1, 128, 128, False), (20, 10, 128, 10, True), (20, 20, 66, 16, False)],
+)
+def test_gated_delta_rule_in_groups_of_four(h, g, dk, dv, channel, rate):
+    """The form that walks four tokens at a time: every remainder of a group, sequences of one token and of none, a padding
+    sequence without a slot, both splits of a head over the lanes, two steps of which the second finds a used state."""
+    from kvforge_b200 import ops
+
+    dev, dt = "cuda", torch.bfloat16
+    gen = torch.Generator().manual_seed(dk + dv)
+    steps = ([37, 1, 0, 6, 4], [5, 11, 0, 1, 130])
+    slots = [2, 5, 1, 0, 4]
+    aw = h * dk if channel else h
+    a_log, dt_bias = rate + 0.5 * torch.randn(h, generator=gen), 0.5 * torch.randn(aw, generator=gen)
+    state = torch.zeros(6, 3 + h * dk * dv, device=dev)
+    seqs = [[] for _ in slots]
+    got = [[] for _ in slots]
+    for k, ls in enumerate(steps):
+        n = sum(ls)
+        qkv, b, a = torch.randn(n, 2 * g * dk + h * dv, generator=gen).to(dt), torch.randn(n, h, generator=gen), torch.randn(n, aw, generator=gen)
+        at = 0
+        for i, m in enumerate(ls):
+            seqs[i].append(tuple(t[at : at + m] for t in (qkv.float(), b, a)))
+            at += m
+        pad = torch.full((3, qkv.shape[1]), float("nan"), dtype=dt)  # rows beyond the last sequence
+        qkv_d, b_d = torch.cat([qkv, pad]).to(dev), torch.cat([b, torch.full((3, h), float("nan"))]).to(dev)
+        a_d = torch.cat([a, torch.full((3, aw), float("nan"))]).to(dev)
+        extra = {}
+        if k == 1 and not channel:
+            parts = torch.randn(3, n + 3, 2 * h, device=dev)
+            parts[0] = torch.cat([b_d, a_d], dim=1) - parts[1] - parts[2]
+            b_d, a_d, extra = parts[0][:, :h], parts[0][:, h:], dict(logit_slices=3, logit_slice_stride=parts.stride(0))
+        qsl, sl = flat_batch(ls + [0], slots + [-1], dev)
+        out = torch.full((n + 3, h * dv), -7.0, device=dev)
+        groups = torch.full((ops.delta_group_floats(n + 3, 6, h, channel),), float("nan"), device=dev)
+        ops.gated_delta(
+            qkv_d[:, : g * dk], qkv_d[:, g * dk : 2 * g * dk], qkv_d[:, 2 * g * dk :], b_d, a_d, a_log.to(dev), dt_bias.to(dev), state[:, 3:],
+            out, qsl, sl, 6, h, g, dk, dv, q_scale=dk**-0.5, max_query_len=max(ls), groups=groups, **extra,
+        )  # fmt: skip
+        assert (out[n:] == -7.0).all()
+        at = 0
+        for i, m in enumerate(ls):
+            got[i].append(out[at : at + m].cpu())
+            at += m
+    for i, parts in enumerate(seqs):
+        qkv, b, a = (torch.cat([p[j] for p in parts]).double() for j in range(3))
+        n = qkv.shape[0]
+        if n == 0:
+            continue
+        q = (plain.unit(qkv[:, : g * dk].view(n, g, dk)) * dk**-0.5).repeat_interleave(h // g, 1)
+        k = plain.unit(qkv[:, g * dk : 2 * g * dk].view(n, g, dk)).repeat_interleave(h // g, 1)
+        decay = torch.exp(-torch.exp(a_log.double()).repeat_interleave(dk if channel else 1) * F.softplus(a + dt_bias.double()))
+        want = plain.delta_rule(q, k, qkv[:, 2 * g * dk :].view(n, h, dv), torch.sigmoid(b), decay.view(n, h, dk) if channel else decay).reshape(n, h * dv)
+        # 32-bit sums of dk terms and of the rounding of the decays that entered the state, as for the walk token by token
+        assert torch.allclose(torch.cat(got[i]).double(), want, atol=5e-5, rtol=5e-4), (i, float((torch.cat(got[i]).double() - want).abs().max()))
+    assert float(state[1].abs().max()) == 0 and float(state[3].abs().max()) == 0 and float(state[:, :3].abs().max()) == 0
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_gated_head_norm_and_branch_mean(dtype):
     from kvforge_b200 import ops
