@@ -10,15 +10,17 @@
 //   softmax     two groups of four warps, 64 keys of a row a thread, from tensor memory, as in attention_tcgen05.cu (running maximum
 //               raised lazily; the two halves of a row exchange their maxima); P takes the place of S in tensor memory;
 //   O += P V    P as the A operand from tensor memory, the value tile being the key tile's first dv columns, read as an
-//               MN-major B operand in blocks of 64 columns, whose chains take turns; O stays in tensor memory.
+//               MN-major B operand of all the CTA's columns at once, blocks of 64 a stride apart (a product of its own for each block
+//               of columns costs the issuing thread some 80 cycles, four of them 24 us of 184); O stays in tensor memory.
 // The blocks of a key tile outside the CTA's value columns are free as soon as S is made, the others after P V: either part has a
 // full and an empty barrier, so that the next tile's first part comes in under the softmax and its second under the first's products.
 // Warps: eight softmax (which first bring the queries in), one loader (TMA boxes of 64 numbers x the keys of a page, 16-byte
 // copies for a last tile that ends inside a page), one issuer.  One CTA an SM.
-// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 184 us against 591 us
+// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 160 us against 591 us
 // of the mma.sync kernel, and the same error against 64-bit.  What bounds it is that scores, softmax, products and copies of a tile follow one
 // another, for want of room for a second tile: with tiles of 64 keys in two stages and four softmax warps it took 233 us, with tiles of
-// 128 and eight warps 220, and 184 since those eight and not the loader alone bring the queries (147 KB a CTA).
+// 128 and eight warps 220, 184 since those eight and not the loader alone bring the queries (147 KB a CTA), and 160 with one product
+// for all value columns (pages of 16 tokens; 156 with pages of 64).
 // Every mbarrier wait is bounded; if one runs out the kernel raises bit 4 of the error flag and winds down.
 #include "tcgen05.cuh"
 
@@ -231,8 +233,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
     if (last1 >= 0) bar_wait(kf1, last1 & 1, p.err);
   } else if (live && warp == MMA_WARP) {
     if (lane == 0) {
-      const uint32_t id_s = idesc(BN, 0), id_o = idesc(64, 1);
-      const uint64_t q_d = sdesc(q_s), k_d = sdesc(k_s), v_d = sdesc(k_s + (uint32_t)vb0 * K_BLOCK);
+      const uint32_t id_s = idesc(BN, 0), id_o = idesc(64 * p.nvb, 1);
+      const uint64_t q_d = sdesc(q_s), k_d = sdesc(k_s), v_d = sdesc_mn(k_s + (uint32_t)vb0 * K_BLOCK, K_BLOCK);
       const uint32_t s_t = tmem + COL_S, o_t = tmem + COL_O;
       bool ok = bar_wait(q_full, 0, p.err);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -270,9 +272,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk)  // A: 16 keys of P = 8 columns; B: 16 keys = 16 rows of 128 bytes
-          for (int j = 0; j < p.nvb; ++j)
-            umma_ts(o_t + 64u * j, s_t + 8u * kk, v_d + (uint64_t)((uint32_t)j * (K_BLOCK >> 4) + kk * (16 * 128 >> 4)), id_o, (t > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < BN / 16; ++kk)  // A: 16 keys of P = 8 columns; B: 16 keys = 16 rows of 128 bytes in each block
+          umma_ts(o_t, s_t + 8u * kk, v_d + (uint64_t)(kk * (16 * 128 >> 4)), id_o, (t > 0 || kk > 0) ? 1u : 0u);
         umma_commit(pv_done);
         umma_commit(ke1);
       }

@@ -73,6 +73,8 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
          ((uint64_t)2 << 61);
 }
+// An MN-major operand of more than 64 numbers across: its [keys][64] blocks lie `stride` bytes apart.
+__device__ __forceinline__ uint64_t sdesc_mn(uint32_t addr, uint32_t stride) { return sdesc(addr) + ((uint64_t)((stride >> 4) - 1) << 16); }
 // kind::f16 instruction descriptor: float accumulator, bfloat16 operands, A K-major, B K-major
 // or MN-major (bit 16), N >> 3 in [17,23), M >> 4 in [24,29).
 __host__ __device__ constexpr uint32_t idesc(int n, int b_mn_major) {
