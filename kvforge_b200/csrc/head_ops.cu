@@ -247,18 +247,32 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(const T* __restrict
 }
 
 // ---------------------------------------------------------------- a logistic gate per head
-// y[n][h][:] *= 1 / (1 + exp(-g[n][h])), in place; g is a column range of a wider row.
-template <typename T>
-__global__ void head_gate_kernel(T* __restrict__ y, const T* __restrict__ g, long long g_stride, long long total, int nh,
-                                 int dv) {
+// y[n][h][:] *= 1 / (1 + exp(-g[n][h])), in place; g is a column range of a wider row.  Bound by reading and writing y once:
+// a thread takes V numbers (16 bytes, where they come so), which share one gate or, with a gate a channel (dv = 1), have V of
+// their own, and a CTA stays with a token, so that finding the head is a 32-bit division.  2,048 tokens of 16 x 128 channels in bfloat16,
+// a gate each: 19.4 us number by number; the layer around it takes 15 us less so.
+template <typename T, int V, bool EACH>
+__global__ void __launch_bounds__(256) head_gate_kernel(T* __restrict__ y, const T* __restrict__ g, long long g_stride, long long n_tokens, int nh, int dv) {
   pdl_launch();
   pdl_wait();
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-    const long long nhid = idx / dv;
-    const long long n = nhid / nh;
-    const int h = (int)(nhid - n * nh);
-    const float z = to_float<T>(g[(size_t)n * g_stride + h]);
-    y[idx] = from_float<T>(to_float<T>(y[idx]) * (1.f / (1.f + expf(-z))));
+  struct alignas(V * sizeof(T)) Vec { T v[V]; };
+  const int per_head = EACH ? 1 : dv / V, per_row = EACH ? nh / V : nh * per_head;
+  for (long long n = blockIdx.x; n < n_tokens; n += gridDim.x) {
+    Vec* row = reinterpret_cast<Vec*>(y + (size_t)n * nh * dv);
+    const T* gates = g + (size_t)n * g_stride;
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < per_row; c += gridDim.y * blockDim.x) {
+      Vec u = row[c];
+      if (EACH) {
+        const Vec z = reinterpret_cast<const Vec*>(gates)[c];
+#pragma unroll
+        for (int e = 0; e < V; ++e) u.v[e] = from_float<T>(to_float<T>(u.v[e]) * (1.f / (1.f + expf(-to_float<T>(z.v[e])))));
+      } else {
+        const float s = 1.f / (1.f + expf(-to_float<T>(gates[c / per_head])));
+#pragma unroll
+        for (int e = 0; e < V; ++e) u.v[e] = from_float<T>(to_float<T>(u.v[e]) * s);
+      }
+      row[c] = u;
+    }
   }
 }
 
@@ -316,10 +330,17 @@ inline unsigned grid_for(long long total, int threads) {
   }                                                                                                                  \
   KVF_API int kvf_head_gate_##SUF(void* y, const void* g, long long g_stride, long long n_tokens, int nh, int dv,    \
                                   cudaStream_t st) {                                                                 \
-    const long long total = n_tokens * nh * dv;                                                                      \
-    if (total <= 0) return 0;                                                                                        \
-    return launch(head_gate_kernel<T>, dim3(grid_for(total, 256)), dim3(256), 0, st, (T*)y, (const T*)g, g_stride,   \
-                  total, nh, dv);                                                                                    \
+    if (n_tokens <= 0 || nh <= 0 || dv <= 0) return 0;                                                               \
+    if ((long long)nh * dv > 0x7fffffffll) return (int)cudaErrorInvalidValue;                                        \
+    constexpr int V = 16 / sizeof(T);                                                                                \
+    const bool each = dv == 1 && nh % V == 0 && g_stride % V == 0 && (((uintptr_t)y | (uintptr_t)g) & 15) == 0;      \
+    const bool wide = each || (dv % V == 0 && ((uintptr_t)y & 15) == 0);                                             \
+    const int chunks = nh * dv / (wide ? V : 1);                                                                     \
+    const long long across = (chunks + 255) / 256;                                                                   \
+    const unsigned gx = (unsigned)(n_tokens < 148 * 64 ? n_tokens : 148 * 64);                                       \
+    const dim3 grid(gx, (unsigned)(across < 64 ? across : 64));                                                      \
+    return launch(each ? head_gate_kernel<T, V, true> : wide ? head_gate_kernel<T, V, false> : head_gate_kernel<T, 1, false>, \
+                  grid, dim3(256), 0, st, (T*)y, (const T*)g, g_stride, n_tokens, nh, dv);                           \
   }
 
 KVF_HEAD_OPS_API(f32, float)

@@ -1126,3 +1126,22 @@ def test_shaped_scores_of_a_decode_step_by_tma(ops, d, nh, nkv, block_size, wind
             for (r0, h, o), e in zip(ref, bound):
                 over = (out.cpu().double()[r0, h * d : (h + 1) * d] - o[0]).abs() - e[0]
                 assert float(over.max()) <= 0.0, (split, cluster, r0, h, float(over.max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,nh,dv", [(1, 1, 8), (3, 5, 7), (5, 3, 24), (700, 16, 192), (9500, 2, 4), (2, 70, 256), (3, 24, 1), (5, 20, 1), (2, 2100, 1)])
+def test_head_gate_widths(ops, dtype, n, nh, dv):
+    """Heads that come as 16-byte words and heads that do not, a gate a channel, rows that start off such a word, more tokens than the
+    grid has rows."""
+    g = torch.Generator().manual_seed(n + dv)
+    y, z = torch.randn(n, nh * dv, generator=g).to(dtype), (3.0 * torch.randn(n, nh + 16 + nh % 2, generator=g)).to(dtype)
+    at = 8 if dv != 7 else 1
+    want = (y.double().view(n, nh, dv) * torch.sigmoid(z[:, at : nh + at].double())[..., None]).view(n, -1)
+    for shift in (0, 1):
+        buf = torch.zeros(n * nh * dv + 2, dtype=dtype, device="cuda")
+        got = buf[shift : shift + n * nh * dv].view(n, -1)
+        got.copy_(y)
+        ops.head_gate(got, z.cuda()[:, at : nh + at], nh, dv)
+        # one rounding of the result, and a few of float on the way
+        tol = (2.0**-8 if dtype == torch.bfloat16 else 2.0**-20) * want.abs() + 1e-30
+        assert ((got.cpu().double() - want).abs() <= tol).all() and float(buf[:shift].abs().sum()) == 0 and float(buf[shift + n * nh * dv :].abs().sum()) == 0
