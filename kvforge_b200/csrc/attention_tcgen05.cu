@@ -58,13 +58,17 @@ constexpr int BIAS_WORDS = 800;
 template <int D, bool SH = false> struct Shape {
   static constexpr int HALVES = D / 64;
   static constexpr int KV_STAGES = (D == 64 ? 4 : 5) - (SH ? 1 : 0);
+  // Tiles in flight behind the one being handed over, without boxes.  The place of tile t + LOOKAHEAD is free when P V of tile
+  // t + LOOKAHEAD - KV_STAGES is done, which the issuer sends out after it has seen the keys two tiles further: those have to be
+  // handed over by then.
+  static constexpr int LOOKAHEAD = KV_STAGES >= 4 ? 2 : 1;
+  static_assert(LOOKAHEAD - KV_STAGES + 2 <= 0, "the loader would wait for what waits for it");
   static constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;  // 109 or 112 KB and 256 tensor-memory columns, or 204 or 224 KB and 512
   static constexpr uint32_t Q_BYTES = HALVES * 128 * 128;     // [128 rows][D] bfloat16
   static constexpr uint32_t KV_BYTES = HALVES * 64 * 128;     // a [64 keys][D] bfloat16 tile
   static constexpr uint32_t TMEM_COLS = D == 64 ? 256u : 512u;  // S: 2 x 64, O: 2 x D
   static constexpr size_t SMEM_BYTES = (size_t)Q_BYTES + (size_t)KV_STAGES * 2 * KV_BYTES + 2 * 128 * 128 + 256 + (SH ? 4 * BIAS_WORDS * 4 : 0);
 };
-constexpr int LOOKAHEAD = 2;                 // tiles in flight behind the one being handed over
 constexpr uint32_t Q_HALF = BM * 128;        // [128 rows][64] bfloat16
 constexpr uint32_t KV_HALF = BN * 128;       // [64 keys][64] bfloat16
 constexpr uint32_t P_BYTES = BM * 128;       // [128 rows][64 keys] bfloat16
@@ -215,7 +219,7 @@ template <int D, int MODE>
 __global__ void __launch_bounds__(THREADS, Shape<D, (MODE >= SHAPED)>::CTAS_PER_SM)
 attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const typename ParamsOf<MODE>::type p) {
   constexpr bool SH = MODE >= SHAPED, BIAS = SH && (MODE & 1), CAP = SH && (MODE & 2);
-  constexpr int HALVES = Shape<D, SH>::HALVES, KV_STAGES = Shape<D, SH>::KV_STAGES;
+  constexpr int HALVES = Shape<D, SH>::HALVES, KV_STAGES = Shape<D, SH>::KV_STAGES, LOOKAHEAD = Shape<D, SH>::LOOKAHEAD;
   constexpr uint32_t Q_BYTES = Shape<D>::Q_BYTES, KV_BYTES = Shape<D>::KV_BYTES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // no slack for rounding up (two CTAs have to fit an SM): the base must be 1024-byte aligned
