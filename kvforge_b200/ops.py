@@ -632,13 +632,16 @@ def paged_attention(
     special = vcache is kcache or keep_first > 0 or bias is not None or d > 256 or (dv or d) > 256 or capped
     # kept first keys, a bias and capped scores on heads of 64 or 128 in bfloat16: the tensor cores
     biased_mma = (
-        special and vcache is not kcache and (dv or d) == d and kernel in ("auto", "tma", "tcgen05")
+        special and vcache is not kcache and (dv or d) == d and kernel in ("auto", "mma", "tma", "tcgen05")
         and mma_attention_supported(q.dtype, nh, nkv, d, scratch is not None) and (q_stride or q.stride(0)) % 2 == 0 and out.shape[-1] % 2 == 0
         and (scratch is None or len(scratch) > 2)
     )  # fmt: skip
     if special and not biased_mma:
         if kernel not in ("auto", "generic"):
-            raise ValueError("only the FP32-pipe attention kernel takes kept first keys, a distance bias, capped scores, sinks, values inside keys or heads wider than 256")
+            raise ValueError(
+                "kept first keys, a distance bias, capped scores and sinks are taken on the tensor cores for bfloat16 heads of 64 or 128 with values as wide; "
+                "they elsewhere, values inside keys and heads wider than 256 by the FP32-pipe attention kernel alone"
+            )
         kernel = "generic"
     check_head_dim(d, MAX_KEY_DIM if special and not biased_mma else 256)
     _need(out, q.dtype, "out")
@@ -718,7 +721,9 @@ def paged_attention(
     use_tma = tickets is not None and tma_decode_supported(q.dtype, nh, nkv, d, block_size, kcache.shape[0])
     # decoding with such scores: the TMA kernel's form for them (64 sequences of 32 heads of 64 on 8, contexts of 1,150 to 2,300 under a
     # window of 1,024, with a bias and 64 kept keys: 36.6 us, 55.8 us on the mma.sync split kernel)
-    if biased_mma and scratch is not None and not use_tma and kernel != "tma":
+    if biased_mma and kernel == "tma" and not use_tma:
+        raise ValueError("the TMA decode kernel does not take this shape (or no tickets were given)")
+    if biased_mma and scratch is not None and (kernel == "mma" or (kernel == "auto" and not use_tma)):
         name = "kvf_paged_attention_decode_biased_bf16"
         _check(
             _fn(name)(
@@ -729,7 +734,7 @@ def paged_attention(
             name,
         )  # fmt: skip
         return
-    if biased_mma and scratch is None and not use_shaped and kernel == "auto":
+    if biased_mma and scratch is None and (kernel == "mma" or (kernel == "auto" and not use_shaped)):
         name = "kvf_paged_attention_mma_biased_bf16"
         _check(
             _fn(name)(

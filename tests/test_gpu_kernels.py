@@ -1145,3 +1145,92 @@ def test_head_gate_widths(ops, dtype, n, nh, dv):
         # one rounding of the result, and a few of float on the way
         tol = (2.0**-8 if dtype == torch.bfloat16 else 2.0**-20) * want.abs() + 1e-30
         assert ((got.cpu().double() - want).abs() <= tol).all() and float(buf[:shift].abs().sum()) == 0 and float(buf[shift + n * nh * dv :].abs().sum()) == 0
+
+
+def run_shaped(ops, d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts, decode=None, **kw):
+    """Runs a case of ``paged_shaped_case`` and returns (output, largest excess over the bound).  ``decode``: (split, cluster)."""
+    q, kc, vc, tables, ctx, rel, sinks, ref, bound = paged_shaped_case(d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    qsl, b = [0], len(lens)
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    if decode is not None:
+        splits = -(-max(ctx) // decode[0])
+        scratch = (torch.full((b, nh, splits, d), float("nan"), device="cuda"), torch.full((b, nh, splits, 2), float("nan"), device="cuda"), i32([0] * b * nkv))
+        kw = dict(kw, scratch=scratch, max_context=max(ctx), split_size=decode[0], cluster=decode[1])
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((sum(lens), nh * d), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.paged_attention(
+        dev(q), out, dev(kc), dev(vc), dev(tables), i32(qsl), i32(ctx), b, max(lens), nh, nkv, d, d**-0.5, window=window, keep_first=keep,
+        bias=ops.DistanceBias(dev(rel), i32(list(range(far + 1)))) if far else None, softcap=cap, sinks=dev(sinks) if sink else None, err=err, **kw,
+    )  # fmt: skip
+    assert int(err.item()) == 0
+    got = out.cpu().double()
+    over = max(float(((got[r0 : r0 + o.shape[0], h * d : (h + 1) * d] - o).abs() - e).max()) for (r0, h, o), e in zip(ref, bound))
+    return out.cpu(), over
+
+
+@pytest.mark.parametrize(
+    "d,nh,nkv,block_size,window,keep,far,cap,sink,lens,starts,takes",
+    [
+        (64, 8, 2, 16, 100, 70, 90, 0.0, False, [33, 1, 130], [300, 200, 0], True),
+        (128, 8, 2, 16, 130, 200, 128, 3.0, True, [70, 3], [250, 0], True),
+        (64, 16, 1, 16, 0, 0, 0, 30.0, True, [150], [10], True),  # sixteen heads a key head, without a bias
+        (64, 16, 1, 16, 60, 20, 40, 0.0, False, [70], [100], False),  # with one: more than a tile's biases have room for
+        (128, 9, 1, 8, 0, 0, 50, 5.0, True, [40, 5], [0, 70], False),
+    ],
+)
+def test_shaped_scores_of_many_queries_by_either_kernel(ops, d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts, takes):
+    """The mma.sync tile kernel, which stays for what the tcgen05 kernel's form does not take; and which of them "auto" is."""
+    case = (d, nh, nkv, block_size, window, keep, far, cap, sink, lens, starts)
+    auto, over = run_shaped(ops, *case)
+    assert over <= 0.0, over
+    tiles, over = run_shaped(ops, *case, kernel="mma")
+    assert over <= 0.0, over
+    if takes:
+        assert torch.equal(auto, run_shaped(ops, *case, kernel="tcgen05")[0]) and not torch.equal(auto, tiles)
+    else:
+        assert torch.equal(auto, tiles)
+        with pytest.raises(ValueError):
+            run_shaped(ops, *case, kernel="tcgen05")
+    with pytest.raises(ValueError):
+        run_shaped(ops, *case, kernel="tma")
+
+
+@pytest.mark.parametrize(
+    "d,nh,nkv,block_size,window,keep,far,cap,sink,ctx,takes",
+    [
+        (64, 8, 2, 16, 100, 70, 90, 0.0, False, [333, 40, 101, 1], True),
+        (128, 8, 1, 16, 130, 200, 128, 3.0, True, [500, 131, 17], True),
+        (64, 16, 1, 16, 60, 20, 40, 0.0, False, [300, 7], False),  # more than eight heads a key head
+        (64, 8, 2, 8, 0, 0, 50, 5.0, False, [200, 65], False),  # pages that are no multiple of sixteen
+    ],
+)
+def test_shaped_scores_of_a_decode_step_by_either_kernel(ops, d, nh, nkv, block_size, window, keep, far, cap, sink, ctx, takes):
+    case = (d, nh, nkv, block_size, window, keep, far, cap, sink, [1] * len(ctx), [c - 1 for c in ctx])
+    for split in (64, 1024):
+        auto, over = run_shaped(ops, *case, decode=(split, False))
+        assert over <= 0.0, (split, over)
+        ranges, over = run_shaped(ops, *case, decode=(split, False), kernel="mma")
+        assert over <= 0.0, (split, over)
+        if takes:
+            assert torch.equal(auto, run_shaped(ops, *case, decode=(split, False), kernel="tma")[0])
+            assert split == 64 or not torch.equal(auto, ranges)  # (ranges of 64 keys: both give a warp sixteen)
+        else:
+            assert torch.equal(auto, ranges)
+            with pytest.raises(ValueError):
+                run_shaped(ops, *case, decode=(split, False), kernel="tma")
+        with pytest.raises(ValueError):
+            run_shaped(ops, *case, decode=(split, False), kernel="tcgen05")
+
+
+def test_latent_attention_of_many_queries_is_the_tcgen05_kernel_s(ops):
+    """"auto" takes the tcgen05 kernel where that takes the shape, with and without a list of tiles."""
+    q, cache, tables, ctx, ref, bound = paged_latent_case([150, 3], [20, 500], 16, 576, 512, 16, 0, 2)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    outs = {}
+    for kernel in ("auto", "tcgen05", "mma"):
+        out = outs[kernel] = torch.empty((153, 16 * 512), device="cuda", dtype=torch.bfloat16)
+        ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, 150, 153]), i32(ctx), 2, 150, 16, 576, 512, 576**-0.5, kernel=kernel)
+        assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
+    assert torch.equal(outs["auto"], outs["tcgen05"]) and not torch.equal(outs["auto"], outs["mma"])
