@@ -588,7 +588,8 @@ int run_dec(const void* q, void* out, const void* kcache, const void* vcache,
             int split_size, int max_splits, int grid_splits, float* part_acc, float* part_ml, int* tickets, int* err,
             int flags, int wave_target, const float* sinks, int keep_first, const float* bias, int bias_far, float softcap, cudaStream_t st) {
   if (B <= 0) return 0;
-  if (keep_first < 0 || (keep_first && window <= 0) || softcap < 0.f || (bias && bias_far < 0)) return (int)cudaErrorInvalidValue;
+  if (keep_first < 0 || softcap < 0.f || (bias && bias_far < 0)) return (int)cudaErrorInvalidValue;
+  if (window <= 0) keep_first = 0;  // without a window every key before the query is seen, or every one of its chunk
   const int cluster = flags & 1;
   if ((d != 64 && d != 128) || nkv <= 0 || nh <= 0 || nh % nkv != 0 || nh / nkv > 8) return (int)cudaErrorInvalidValue;
   if (block_size <= 0 || block_size % UNIT != 0 || num_blocks <= 0) return (int)cudaErrorInvalidValue;

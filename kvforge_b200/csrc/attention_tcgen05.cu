@@ -659,7 +659,8 @@ KVF_API int kvf_paged_attention_tcgen05_bf16(const void* q, void* out, const voi
   if ((d != 64 && d != 128) || nkv <= 0 || nh % nkv != 0 || nh / nkv > BM || block_size <= 0 || num_blocks <= 0) return (int)cudaErrorInvalidValue;
   if ((q_stride & 7) || (out_stride & 7) || ((((uintptr_t)q) | ((uintptr_t)out)) & 15)) return (int)cudaErrorInvalidValue;
   if ((unsigned)B > 65535u || (max_q_len + (BM / (nh / nkv)) - 1) / (BM / (nh / nkv)) > 65535) return (int)cudaErrorInvalidValue;
-  if (keep_first < 0 || (keep_first && window <= 0) || softcap < 0.f || (bias && (bias_far < 0 || nh / nkv > 8))) return (int)cudaErrorInvalidValue;
+  if (keep_first < 0 || softcap < 0.f || (bias && (bias_far < 0 || nh / nkv > 8))) return (int)cudaErrorInvalidValue;
+  if (window <= 0) keep_first = 0;  // without a window every key before the query is seen, or every one of its chunk
   TcAttnShapedParams p;
   p.keep_first = keep_first; p.bias = bias; p.bias_far = bias_far;
   p.cap_in = softcap > 0.f ? scale / softcap : 0.f;

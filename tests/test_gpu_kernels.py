@@ -1234,3 +1234,17 @@ def test_latent_attention_of_many_queries_is_the_tcgen05_kernel_s(ops):
         ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, 150, 153]), i32(ctx), 2, 150, 16, 576, 512, 576**-0.5, kernel=kernel)
         assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
     assert torch.equal(outs["auto"], outs["tcgen05"]) and not torch.equal(outs["auto"], outs["mma"])
+
+
+@pytest.mark.parametrize("d,nh,nkv,block_size", [(64, 8, 2, 16), (128, 4, 1, 16), (64, 9, 1, 8), (48, 4, 2, 16)])
+@pytest.mark.parametrize("far,cap", [(0, 0.0), (30, 0.0), (0, 5.0)])
+def test_kept_keys_without_a_window_change_nothing(ops, d, nh, nkv, block_size, far, cap):
+    """Every key before a query is seen anyway: by the tensor-core kernels and, with heads of 48, on the FP32 pipes."""
+    for lens, starts, decode in (([70, 3], [90, 0], None), ([1, 1], [300, 20], (64, False)), ([1, 1], [300, 20], (512, True))):
+        outs = []
+        for keep in (0, 70):
+            out, over = run_shaped(ops, d, nh, nkv, block_size, 0, keep, far, cap, False, lens, starts, decode=decode)
+            assert over <= 0.0, (lens, keep, over)
+            outs.append(out)
+        plain_elsewhere = d == 64 and nh == 9 or d == 48  # without kept keys other kernels take plain scores there
+        assert torch.equal(*outs) or (plain_elsewhere and not far and not cap)
