@@ -590,8 +590,10 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       const float m_all = fmaxf(m_ref, other.x);
       const float w0 = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - m_all), w1 = (other.x == -INFINITY) ? 0.f : ex2(other.x - m_all);
       const float l_all = l * w0 + other.y * w1;
-      const float f0 = l_all > 0.f ? w0 / l_all : 0.f, f1 = l_all > 0.f ? w1 / l_all : 0.f;
-      const bool use1 = __any_sync(0xffffffffu, other.y > 0.f);  // group 1 saw a tile (else its accumulator was never written)
+      // a sum that is no number (a key that is none, an infinite score) shows in the result
+      const float f0 = l_all != 0.f ? w0 / l_all : 0.f, f1 = l_all != 0.f ? w1 / l_all : 0.f;
+      const bool seen1 = other.y != 0.f;                   // this row saw a key of group 1
+      const bool use1 = __any_sync(0xffffffffu, seen1);  // group 1 saw a tile (else its accumulator was never written)
       bf16* dst = p.out + (size_t)(q_begin + q0 + (valid ? tok : 0)) * p.out_stride + (size_t)(kvh * g + hh) * D;
 #pragma unroll
       for (int c0 = 0; c0 < D; c0 += 32) {
@@ -608,7 +610,7 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             f[e] = __uint_as_float(v[j + e]) * f0;
-            if (use1 && f1 != 0.f) f[e] += __uint_as_float(u[j + e]) * f1;
+            if (use1 && seen1) f[e] += __uint_as_float(u[j + e]) * f1;
           }
           if (valid)
             *reinterpret_cast<uint4*>(dst + c0 + j) = make_uint4(pk(f[0], f[1]), pk(f[2], f[3]), pk(f[4], f[5]), pk(f[6], f[7]));

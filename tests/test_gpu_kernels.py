@@ -1248,3 +1248,28 @@ def test_kept_keys_without_a_window_change_nothing(ops, d, nh, nkv, block_size, 
             outs.append(out)
         plain_elsewhere = d == 64 and nh == 9 or d == 48  # without kept keys other kernels take plain scores there
         assert torch.equal(*outs) or (plain_elsewhere and not far and not cap)
+
+
+@pytest.mark.parametrize("shape", [(64, 8, 2, 16), (64, 4, 2, 8), (128, 4, 1, 16)])
+@pytest.mark.parametrize("far,cap,window,keep", [(0, 0.0, 0, 0), (30, 0.0, 0, 0), (0, 5.0, 0, 0), (20, 3.0, 90, 70)])
+@pytest.mark.parametrize("bad", [5, 70, 133, 199])  # in either of the tiles that two groups of warps take in turn, and in the last
+def test_what_is_no_number_shows_in_the_rows_that_see_it(ops, shape, far, cap, window, keep, bad):
+    """One key that is NaN: every head of every query that sees it is NaN, the others are what they were."""
+    d, nh, nkv, bs = shape
+    q, kc, vc, tables, ctx, rel, sinks, ref, bound = paged_shaped_case(d, nh, nkv, bs, window, keep, far, cap, False, [200], [0])
+    kc[int(tables[0, bad // bs]), :, bad % bs, 3] = float("nan")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    bias = ops.DistanceBias(dev(rel), i32(list(range(far + 1)))) if far else None
+    for kernel in ("auto", "mma"):
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        out = torch.zeros((200, nh * d), device="cuda", dtype=torch.bfloat16)
+        ops.paged_attention(
+            dev(q), out, dev(kc), dev(vc), dev(tables), i32([0, 200]), i32([200]), 1, 200, nh, nkv, d, d**-0.5, window=window, keep_first=keep,
+            bias=bias, softcap=cap, err=err, kernel=kernel,
+        )  # fmt: skip
+        assert int(err.item()) == 0
+        got, i = out.cpu().double(), torch.arange(200)
+        sees = (i >= bad) & ((i - bad < window) | (bad < keep) if window else True)
+        assert torch.isnan(got[sees]).all() and not torch.isnan(got[~sees]).any(), kernel
+        for (r0, h, o), e in zip(ref, bound):
+            assert float(((got[:, h * d : (h + 1) * d] - o).abs() - e)[~sees].max()) <= 0.0, (kernel, h)
