@@ -451,7 +451,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           L = L * f + ex2(sk - mm);
         }
         p.out[(size_t)(q_begin + q_len - 1) * p.out_stride + (size_t)(kvh * g + r) * D + dcol] =
-            __float2bfloat16_rn(L > 0.f ? acc / L : 0.f);
+            __float2bfloat16_rn(L != 0.f ? acc / L : 0.f);  // (a sum that is no number shows in the result)
         continue;
       }
       const size_t slot = slot0 + (size_t)r * p.max_splits;
@@ -493,7 +493,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         L += w * ld_cluster(theirs + (D + 1) * 4);
       }
       p.out[(size_t)(q_begin + q_len - 1) * p.out_stride + (size_t)(kvh * g + r) * D + dcol] =
-          __float2bfloat16_rn(L > 0.f ? acc / L : 0.f);
+          __float2bfloat16_rn(L != 0.f ? acc / L : 0.f);
     }
     cluster_barrier();  // nobody leaves while its shared memory may still be read
     return;

@@ -1273,3 +1273,29 @@ def test_what_is_no_number_shows_in_the_rows_that_see_it(ops, shape, far, cap, w
         assert torch.isnan(got[sees]).all() and not torch.isnan(got[~sees]).any(), kernel
         for (r0, h, o), e in zip(ref, bound):
             assert float(((got[:, h * d : (h + 1) * d] - o).abs() - e)[~sees].max()) <= 0.0, (kernel, h)
+
+
+@pytest.mark.parametrize("d,nh,nkv", [(64, 8, 2), (128, 8, 1)])
+@pytest.mark.parametrize("far,cap", [(0, 0.0), (30, 0.0), (0, 5.0)])
+def test_what_is_no_number_shows_in_a_decode_step(ops, d, nh, nkv, far, cap):
+    """A NaN key in one of three sequences: as the only range of its sequence, among the ranges of a cluster, among ranges that
+    merge by tickets, and on the mma.sync kernel."""
+    ctx = [40, 200, 130]
+    q, kc, vc, tables, _, rel, sinks, ref, bound = paged_shaped_case(d, nh, nkv, 16, 0, 0, far, cap, False, [1] * 3, [c - 1 for c in ctx])
+    kc[int(tables[1, 150 // 16]), :, 150 % 16, 3] = float("nan")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    bias = ops.DistanceBias(dev(rel), i32(list(range(far + 1)))) if far else None
+    for split, cluster, kernel in ((64, True, "tma"), (64, False, "tma"), (256, False, "tma"), (64, False, "mma")):
+        ns = -(-200 // split)
+        scratch = (torch.zeros((3, nh, ns, d), device="cuda"), torch.zeros((3, nh, ns, 2), device="cuda"), i32([0] * 3 * nkv))
+        out, err = torch.zeros((3, nh * d), device="cuda", dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.paged_attention(
+            dev(q), out, dev(kc), dev(vc), dev(tables), i32([0, 1, 2, 3]), i32(ctx), 3, 1, nh, nkv, d, d**-0.5, bias=bias, softcap=cap, err=err,
+            scratch=scratch, max_context=200, split_size=split, cluster=cluster, kernel=kernel,
+        )  # fmt: skip
+        assert int(err.item()) == 0 and int(scratch[2].abs().max()) == 0
+        got = out.cpu().double()
+        assert torch.isnan(got[1]).all(), (split, cluster, kernel)
+        for (r0, h, o), e in zip(ref, bound):
+            if r0 != 1:
+                assert float(((got[r0, h * d : (h + 1) * d] - o[0]).abs() - e[0]).max()) <= 0.0, (split, cluster, kernel, r0, h)
