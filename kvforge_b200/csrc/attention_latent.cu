@@ -344,15 +344,17 @@ __global__ void __launch_bounds__(WARPS * 32 * MT) latent_attn_kernel(const LatP
 }
 
 // Merge the partial results of the key ranges of one (sequence, head), in range order.  What bounds it is the latency of a
-// range's loads: the ranges' factors are made once in shared memory, a thread per range, and a thread's four columns of eight
-// ranges are asked for at once (64 sequences, 16 heads of 512 values, 18 ranges, 38 MB: 48.6 us when every thread made every
-// factor and took its columns one by one, 29.7 us so).
-__global__ void __launch_bounds__(128) latent_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
+// range's loads: the ranges' factors are made once in shared memory, a thread per range and 256 ranges at a time, and a thread's
+// four columns of eight ranges are asked for at once (64 sequences, 16 heads of 512 values, 18 ranges, 38 MB: 48.6 us when every
+// thread made every factor and took its columns one by one, 29.7 us so).
+constexpr int MERGE_THREADS = 128, MERGE_RANGES = 256;
+__global__ void __launch_bounds__(MERGE_THREADS) latent_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
                                       const int* __restrict__ qsl, const int* __restrict__ ctx_lens, int nh, int dv, int out_stride,
                                       int split_size, int max_splits) {
   pdl_launch();
   pdl_wait();
-  extern __shared__ float factors[];  // [max_splits] exp(m - M), zero for a range that saw nothing; then [max_splits] times its sum
+  __shared__ float factors[MERGE_RANGES];  // exp(m - M), zero for a range that saw nothing
+  __shared__ float sums[MERGE_RANGES];     // times its sum
   __shared__ float red[32];
   const int b = blockIdx.y, head = blockIdx.x;
   const int q_begin = qsl[b], q_len = qsl[b + 1] - q_begin;
@@ -363,32 +365,32 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __rest
   float M = -INFINITY;
   for (int s = threadIdx.x; s < ns; s += blockDim.x) M = fmaxf(M, part_ml[(base + s) * 2]);
   M = block_max(M, red);
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-    const float ms = part_ml[(base + s) * 2], w = ms != -INFINITY ? expf(ms - M) : 0.f;
-    factors[s] = w;
-    factors[max_splits + s] = ms != -INFINITY ? w * part_ml[(base + s) * 2 + 1] : 0.f;
-  }
-  __syncthreads();
-  float L = 0.f;
-#pragma unroll 4
-  for (int s = 0; s < ns; ++s) L += factors[max_splits + s];
-  const float inv = L > 0.f ? 1.f / L : 0.f;
-  bf16* o = out + (size_t)(q_begin + q_len - 1) * out_stride + (size_t)head * dv;
+  const int j = threadIdx.x * 4;  // this thread's columns (dv is a multiple of 32 and at most 512)
   const bool wide = (((uintptr_t)part_acc) & 15) == 0;
-  for (int j = threadIdx.x * 4; j < dv; j += blockDim.x * 4) {
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* col = part_acc + base * dv + j;  // dv is a multiple of 32
-    for (int s0 = 0; s0 < ns; s0 += 8) {
+  const float* col = part_acc + base * dv + j;
+  float L = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int c0 = 0; c0 < ns; c0 += MERGE_RANGES) {
+    const int nc = min(MERGE_RANGES, ns - c0);
+    if (c0) __syncthreads();  // the factors before have been read
+    for (int s = threadIdx.x; s < nc; s += blockDim.x) {
+      const float ms = part_ml[(base + c0 + s) * 2], w = ms != -INFINITY ? expf(ms - M) : 0.f;
+      factors[s] = w;
+      sums[s] = ms != -INFINITY ? w * part_ml[(base + c0 + s) * 2 + 1] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int s = 0; s < nc; ++s) L += sums[s];
+    for (int s0 = 0; j < dv && s0 < nc; s0 += 8) {
       float4 x[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        if (s0 + i < ns) {
-          const float* src = col + (size_t)(s0 + i) * dv;
+        if (s0 + i < nc) {
+          const float* src = col + (size_t)(c0 + s0 + i) * dv;
           x[i] = wide ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
         }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float w = s0 + i < ns ? factors[s0 + i] : 0.f;
+        const float w = s0 + i < nc ? factors[s0 + i] : 0.f;
         if (w == 0.f) continue;  // (a range that saw nothing has left its partial results as they were)
         a[0] = fmaf(w, x[i].x, a[0]);
         a[1] = fmaf(w, x[i].y, a[1]);
@@ -396,9 +398,12 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __rest
         a[3] = fmaf(w, x[i].w, a[3]);
       }
     }
-    *reinterpret_cast<uint32_t*>(o + j) = pack2(a[0] * inv, a[1] * inv);
-    *reinterpret_cast<uint32_t*>(o + j + 2) = pack2(a[2] * inv, a[3] * inv);
   }
+  if (j >= dv) return;
+  const float inv = L > 0.f ? 1.f / L : 0.f;
+  bf16* o = out + (size_t)(q_begin + q_len - 1) * out_stride + (size_t)head * dv + j;
+  *reinterpret_cast<uint32_t*>(o) = pack2(a[0] * inv, a[1] * inv);
+  *reinterpret_cast<uint32_t*>(o + 2) = pack2(a[2] * inv, a[3] * inv);
 }
 
 template <int NTW, int MT>
@@ -423,12 +428,8 @@ int launch_latent(LatParams p, int B, int max_q_len, int grid_splits, cudaStream
     }
     int rc = launch(kern, dim3(grid_splits, B, p.chunks), dim3(WARPS * 32), smem, st, p);
     if (rc) return rc;
-    const size_t factors = (size_t)2 * p.max_splits * sizeof(float);
-    if (factors > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(latent_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)factors);
-      if (e != cudaSuccess) return (int)e;
-    }
-    return launch(latent_combine_kernel, dim3(p.nh, B), dim3(128), factors, st, (const float*)p.part_acc, (const float*)p.part_ml, p.out,
+    static_assert(NTW * 32 <= 4 * MERGE_THREADS, "four columns a thread of the merge");
+    return launch(latent_combine_kernel, dim3(p.nh, B), dim3(MERGE_THREADS), 0, st, (const float*)p.part_acc, (const float*)p.part_ml, p.out,
                   p.qsl, p.ctx_lens, p.nh, p.dv, p.out_stride, p.split_size, p.max_splits);
   }
   // 64 or 32 rows a CTA (16 or 8 warps) where some sequence brings enough tokens to fill them

@@ -1299,3 +1299,19 @@ def test_what_is_no_number_shows_in_a_decode_step(ops, d, nh, nkv, far, cap):
         for (r0, h, o), e in zip(ref, bound):
             if r0 != 1:
                 assert float(((got[r0, h * d : (h + 1) * d] - o[0]).abs() - e[0]).max()) <= 0.0, (split, cluster, kernel, r0, h)
+
+
+@pytest.mark.parametrize("ranges", [1, 8, 255, 256, 257, 3000, 6140, 30000])
+def test_latent_decode_merges_any_number_of_ranges(ops, ranges):
+    """Scratch of up to 30,000 ranges of 32 keys, and contexts that use all of the first few hundred and their edges."""
+    nh, d, dv, bs = 3, 64, 64, 16
+    used = min(ranges, 600)
+    ctx = [used * 32, max(1, used * 32 - 17), 1]
+    q, cache, tables, ctx, ref, bound = paged_latent_case([1] * 3, [c - 1 for c in ctx], nh, d, dv, bs, 0, ranges)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    scratch = (torch.full((3, nh, ranges, dv), float("nan"), device="cuda"), torch.full((3, nh, ranges, 2), float("nan"), device="cuda"))
+    out = torch.full((3, nh * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention(
+        dev(q), out, dev(cache), dev(tables), i32([0, 1, 2, 3]), i32(ctx), 3, 1, nh, d, dv, d**-0.5, scratch=scratch, max_context=max(ctx), split_size=32,
+    )  # fmt: skip
+    assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
