@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) latent_combine_kernel(const flo
                                       int split_size, int max_splits) {
   pdl_launch();
   pdl_wait();
-  __shared__ float factors[MERGE_RANGES];  // exp(m - M), zero for a range that saw nothing
+  __shared__ float factors[MERGE_RANGES];  // exp(m - M), below zero for a range that saw nothing
   __shared__ float sums[MERGE_RANGES];     // times its sum
   __shared__ float red[32];
   const int b = blockIdx.y, head = blockIdx.x;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) latent_combine_kernel(const flo
     const int nc = min(MERGE_RANGES, ns - c0);
     if (c0) __syncthreads();  // the factors before have been read
     for (int s = threadIdx.x; s < nc; s += blockDim.x) {
-      const float ms = part_ml[(base + c0 + s) * 2], w = ms != -INFINITY ? expf(ms - M) : 0.f;
+      const float ms = part_ml[(base + c0 + s) * 2], w = ms != -INFINITY ? expf(ms - M) : -1.f;
       factors[s] = w;
       sums[s] = ms != -INFINITY ? w * part_ml[(base + c0 + s) * 2 + 1] : 0.f;
     }
@@ -390,8 +390,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) latent_combine_kernel(const flo
         }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float w = s0 + i < nc ? factors[s0 + i] : 0.f;
-        if (w == 0.f) continue;  // (a range that saw nothing has left its partial results as they were)
+        const float w = s0 + i < nc ? factors[s0 + i] : -1.f;
+        if (w < 0.f) continue;  // (a range that saw nothing has left its partial results as they were; one whose factor is zero counts: NaN stays NaN)
         a[0] = fmaf(w, x[i].x, a[0]);
         a[1] = fmaf(w, x[i].y, a[1]);
         a[2] = fmaf(w, x[i].z, a[2]);

@@ -1315,3 +1315,21 @@ def test_latent_decode_merges_any_number_of_ranges(ops, ranges):
         dev(q), out, dev(cache), dev(tables), i32([0, 1, 2, 3]), i32(ctx), 3, 1, nh, d, dv, d**-0.5, scratch=scratch, max_context=max(ctx), split_size=32,
     )  # fmt: skip
     assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
+
+
+def test_latent_decode_shows_what_is_no_number_in_any_range(ops):
+    """A NaN key in a range whose scores lie so far below the others' that its factor in the merge is zero."""
+    nh, d, dv = 2, 64, 64
+    q, cache, tables, ctx, ref, bound = paged_latent_case([1, 1], [199, 199], nh, d, dv, 16, 0, 5)
+    q = torch.ones_like(q)
+    for b in range(2):
+        for j in range(200):
+            cache[int(tables[b, j // 16]), 0, j % 16] = 20.0 if j >= 64 else -20.0  # scores of 160 and -160
+    cache[int(tables[1, 2]), 0, 5, 3] = float("nan")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    scratch = (torch.zeros((2, nh, 4, dv), device="cuda"), torch.zeros((2, nh, 4, 2), device="cuda"))
+    out = torch.zeros((2, nh * dv), device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention(
+        dev(q), out, dev(cache), dev(tables), i32([0, 1, 2]), i32(ctx), 2, 1, nh, d, dv, d**-0.5, scratch=scratch, max_context=200, split_size=64,
+    )  # fmt: skip
+    assert (out[0] == 20.0).all() and torch.isnan(out[1]).all()
