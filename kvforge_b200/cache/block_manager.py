@@ -69,17 +69,14 @@ class _Pool:
         # the same tables as int32 arrays (with room to grow), so that a step copies a table instead of converting a list
         self.arrays: dict[str, np.ndarray] = {}
 
-    def put(self, seq_id: str, i: int, b: int) -> None:
-        """Entry ``i`` of a request's table, at most one past its end."""
+    def sync(self, seq_id: str, first: int) -> None:
+        """Entries of the array from ``first`` on become the list's."""
         table, array = self.tables[seq_id], self.arrays[seq_id]
-        if i == len(table):
-            table.append(b)
-            if i == len(array):
-                array = np.resize(array, 2 * i + 8)
-                self.arrays[seq_id] = array
-        else:
-            table[i] = b
-        array[i] = b
+        if len(table) > len(array):
+            grown = np.empty(2 * len(table) + 8, dtype=np.int32)
+            grown[:first] = array[:first]
+            array = self.arrays[seq_id] = grown
+        array[first : len(table)] = table[first:]
 
     def pop(self) -> int:
         if not self.free:
@@ -87,6 +84,18 @@ class _Pool:
         b = self.free.pop()
         self.held[b] = True
         return b
+
+    def take(self, n: int) -> list[int]:
+        """``n`` pages, those that ``pop`` would give one after another."""
+        if n > len(self.free):
+            raise NoFreeBlocksError("KV cache exhausted")
+        if n <= 0:
+            return []
+        pages = self.free[: -n - 1 : -1]
+        del self.free[-n:]
+        for b in pages:
+            self.held[b] = True
+        return pages
 
     def release(self, b: int) -> None:
         if b < 0 or b >= self.num_blocks or not self.held[b]:
@@ -227,8 +236,8 @@ class BlockManager:
                 raise NoFreeBlocksError(f"cannot allocate {need} blocks for {seq_id}")
             plan.append(need)
         for pool, need in zip(self._pools, plan):
-            pool.tables[seq_id] = [pool.pop() for _ in range(need)]
-            pool.arrays[seq_id] = np.array(pool.tables[seq_id], dtype=np.int32)
+            pages = pool.tables[seq_id] = pool.take(need)
+            pool.arrays[seq_id] = np.array(pages, dtype=np.int32)
         self._num_tokens[seq_id] = num_tokens
         return 0
 
@@ -251,21 +260,31 @@ class BlockManager:
         want = self.blocks_needed(total_tokens)
         for pool in self._pools:
             table = pool.tables[seq_id]
+            changed = len(table)  # the first entry that changes
             if pool.spec.kind == "full":
-                while len(table) < want:
-                    pool.put(seq_id, len(table), pool.pop())
+                if changed < want:
+                    table += pool.take(want - changed)
+                    pool.sync(seq_id, changed)
                 continue
             first = self._first_live_block(pool, write_start)
             kept = min(self._kept_blocks(pool), first)
             for i in range(kept, min(first, len(table))):
                 if table[i] >= 0:
                     pool.release(table[i])
-                    pool.put(seq_id, i, RELEASED)
-            while len(table) < want:
-                pool.put(seq_id, len(table), RELEASED if kept <= len(table) < first else pool.pop())
+                    table[i] = RELEASED
+                    if i < changed:
+                        changed = i
+            if changed < want:
+                table += pool.take(min(kept, want) - len(table))
+                table += [RELEASED] * (min(first, want) - len(table))
+                table += pool.take(want - len(table))
             for i in [*range(min(kept, want)), *range(first, want)]:
                 if table[i] < 0:
-                    pool.put(seq_id, i, pool.pop())
+                    table[i] = pool.pop()
+                    if i < changed:
+                        changed = i
+            if changed < len(table):
+                pool.sync(seq_id, changed)
         self._num_tokens[seq_id] = max(self._num_tokens[seq_id], total_tokens)
         return []
 

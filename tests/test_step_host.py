@@ -168,3 +168,71 @@ def test_a_step_of_single_tokens_is_laid_out_as_its_tables_say():
             bm.allocate("gone", 1, 1)
             bm.append_slots("gone", 250, 249)
             runner._fill([BatchItem("gone", [1], 20, "last")], lay)
+
+
+def test_pages_taken_at_once_are_those_taken_one_by_one():
+    """Tables of full, window and chunk groups under random growth, and their arrays, against a manager that takes every page by
+    itself and keeps lists alone."""
+    import numpy as np
+    import pytest
+
+    from kvforge_b200.cache.block_manager import RELEASED, BlockManager, GroupSpec, NoFreeBlocksError
+
+    class OneByOne:
+        def __init__(self, n):
+            self.free, self.tables = list(range(n - 1, -1, -1)), {}
+
+        def allocate(self, seq, pages):
+            self.tables[seq] = [self.free.pop() for _ in range(pages)]
+
+        def append(self, seq, want, first, kept):
+            table = self.tables[seq]
+            for i in range(kept, min(first, len(table))):
+                if table[i] >= 0:
+                    self.free.append(table[i])
+                    table[i] = RELEASED
+            while len(table) < want:
+                table.append(RELEASED if kept <= len(table) < first else self.free.pop())
+            for i in [*range(min(kept, want)), *range(first, want)]:
+                if table[i] < 0:
+                    table[i] = self.free.pop()
+
+        def release(self, seq):
+            self.free += [b for b in reversed(self.tables.pop(seq)) if b >= 0]
+
+    rng = random.Random(3)
+    for case in range(10):
+        bs = rng.choice([1, 4, 16])
+        specs = [GroupSpec(), GroupSpec("window", 40, rng.choice([0, 9])), GroupSpec("chunk", 48)]
+        bm, plain = BlockManager(900, bs, 0.0, specs), [OneByOne(900) for _ in specs]
+        at = {}
+        for step in range(200):
+            seq = f"r{rng.randrange(5)}"
+            if seq not in at:
+                n, scheduled = rng.randint(1, 60), rng.choice([1, 7, 30])
+                bm.allocate(seq, n, scheduled)
+                for g, p in enumerate(plain):
+                    p.allocate(seq, -(-(n if g == 0 else min(n, scheduled)) // bs))
+                at[seq] = 0
+            elif at[seq] > 120 or rng.random() < 0.1:
+                bm.free(seq)
+                for p in plain:
+                    p.release(seq)
+                del at[seq]
+            else:
+                start = max(0, at[seq] - rng.choice([0, 0, 0, 13]))  # sometimes back: pages that came back are taken anew
+                end = start + rng.choice([1, 1, 5, 33])
+                bm.append_slots(seq, end, start)
+                for g, (p, spec) in enumerate(zip(plain, specs)):
+                    first = 0 if g == 0 else max(0, start - 39) // bs if g == 1 else (start - start % 48) // bs
+                    p.append(seq, -(-end // bs), first, min(-(-spec.keep_first // bs), first) if g else 0)
+                at[seq] = end
+            bm.check_invariants()
+            for g, p in enumerate(plain):
+                for s in at:
+                    assert bm.get_block_table(s, g) == p.tables[s] and np.array_equal(bm.table_array(s, g), p.tables[s]), (case, step, g, s)
+    pool = BlockManager(5, 4)._pools[0]
+    assert pool.take(0) == [] and pool.take(-2) == [] and pool.take(3) == [0, 1, 2] and pool.pop() == 3
+    with pytest.raises(NoFreeBlocksError):
+        pool.take(2)
+    assert pool.take(1) == [4] and pool.held == [True] * 5
