@@ -139,6 +139,14 @@ class GatedDeltaRule(Mixer):
         self.a_log, self.dt_bias, self.norm_w = W["A_log"], W["dt_bias"], W["norm"]
         del dev, dt
 
+    def _walk_rows(self, num_seqs: int) -> tuple[bool, int]:
+        """(whether the walk token by token only sees steps of a few tokens a sequence, rows that its buffers are made for):
+        where longer steps go in groups, the step's token budget would be memory that nothing uses."""
+        rt = self.rt
+        if not ops.delta_groups_ok(rt.dtype, self.dk, ops.DELTA_GROUP_TOKENS + 1):
+            return False, rt.max_tokens
+        return True, min(rt.max_tokens, ops.DELTA_GROUP_TOKENS * max(rt.max_seqs, num_seqs))
+
     def forward(self, ctx, x: torch.Tensor, cache):
         rt = self.rt
         n = x.shape[0]
@@ -186,10 +194,9 @@ class GatedDeltaRule(Mixer):
             record = ops.delta_group_record(H, self.decay == "channel")
             groups = rt.buf("delta.groups", n // per + ctx.num_seqs, record, f32, cap=rt.max_tokens // per + max(rt.max_seqs, ctx.num_seqs))
         else:
-            scratch = (
-                rt.buf("delta.kn", n, H * dk, f32), rt.buf("delta.qn", n, H * dk, f32),
-                rt.buf("delta.gn", n, H * dk, f32) if self.decay == "channel" else None, rt.buf("delta.sc", n, H * 4, f32),
-            )  # fmt: skip
+            few, cap = self._walk_rows(ctx.num_seqs)
+            buf = lambda what, w: rt.buf(f"delta.{'few_' if few else ''}{what}", n, w, f32, cap=cap)  # noqa: E731
+            scratch = (buf("kn", H * dk), buf("qn", H * dk), buf("gn", H * dk) if self.decay == "channel" else None, buf("sc", H * 4))
         ops.gated_delta(
             qkv[:, : self.c_q], qkv[:, self.c_q : 2 * self.c_q], qkv[:, 2 * self.c_q :], small[:, :H], step, self.a_log, self.dt_bias,
             cache.state[:, self.conv_floats :], read, ctx.query_start_loc, ctx.state_slots, ctx.num_seqs, H, self.G, dk, dv,

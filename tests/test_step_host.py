@@ -236,3 +236,24 @@ def test_pages_taken_at_once_are_those_taken_one_by_one():
     with pytest.raises(NoFreeBlocksError):
         pool.take(2)
     assert pool.take(1) == [4] and pool.held == [True] * 5
+
+
+def test_buffers_of_the_delta_rule_s_walk_hold_what_the_walk_may_see():
+    """Where steps of more than four tokens a sequence go in groups, the walk's buffers are made for four tokens a sequence."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from kvforge_b200 import PRESETS
+    from kvforge_b200.engine.core import spec_from_config
+    from kvforge_b200.parts.base import PartSpec, build_part
+
+    spec = next(p for s in spec_from_config(PRESETS["mopilorn-1b"]).layers for p in [s.block.params["mixer"]] if p.kind == "gated_delta_rule")
+    for dtype, dk, budget, seqs, want in (
+        (torch.bfloat16, 128, 2048, 64, (True, 256)), (torch.bfloat16, 128, 2048, 1000, (True, 2048)), (torch.bfloat16, 65, 512, 3, (True, 12)),
+        (torch.bfloat16, 64, 2048, 64, (False, 2048)), (torch.bfloat16, 256, 2048, 64, (False, 2048)), (torch.float32, 128, 2048, 64, (False, 2048)),
+    ):  # fmt: skip
+        part = build_part("mixer", PartSpec(spec.kind, {**spec.params, "head_dim": dk}), "")
+        part.rt = SimpleNamespace(dtype=dtype, max_tokens=budget, max_seqs=seqs)
+        assert part._walk_rows(1) == want, (dtype, dk)
+        assert part._walk_rows(2000) == (want[0], budget)
