@@ -252,15 +252,15 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(const T* __restrict
 // their own, and a CTA stays with a token, so that finding the head is a 32-bit division.  2,048 tokens of 16 x 128 channels in bfloat16,
 // a gate each: 19.4 us number by number; the layer around it takes 15 us less so.
 template <typename T, int V, bool EACH>
-__global__ void __launch_bounds__(256) head_gate_kernel(T* __restrict__ y, const T* __restrict__ g, long long g_stride, long long n_tokens, int nh, int dv) {
+__global__ void __launch_bounds__(256) head_gate_kernel(T* __restrict__ y, long long y_stride, const T* __restrict__ g, long long g_stride, long long n_tokens, int nh, int dv) {
   pdl_launch();
   pdl_wait();
   struct alignas(V * sizeof(T)) Vec { T v[V]; };
-  const int per_head = EACH ? 1 : dv / V, per_row = EACH ? nh / V : nh * per_head;
+  const unsigned per_head = EACH ? 1 : dv / V, per_row = EACH ? nh / V : nh * per_head;
   for (long long n = blockIdx.x; n < n_tokens; n += gridDim.x) {
-    Vec* row = reinterpret_cast<Vec*>(y + (size_t)n * nh * dv);
+    Vec* row = reinterpret_cast<Vec*>(y + (size_t)n * y_stride);
     const T* gates = g + (size_t)n * g_stride;
-    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < per_row; c += gridDim.y * blockDim.x) {
+    for (unsigned c = blockIdx.y * blockDim.x + threadIdx.x; c < per_row; c += gridDim.y * blockDim.x) {
       Vec u = row[c];
       if (EACH) {
         const Vec z = reinterpret_cast<const Vec*>(gates)[c];
@@ -331,16 +331,21 @@ inline unsigned grid_for(long long total, int threads) {
   KVF_API int kvf_head_gate_##SUF(void* y, const void* g, long long g_stride, long long n_tokens, int nh, int dv,    \
                                   cudaStream_t st) {                                                                 \
     if (n_tokens <= 0 || nh <= 0 || dv <= 0) return 0;                                                               \
-    if ((long long)nh * dv > 0x7fffffffll) return (int)cudaErrorInvalidValue;                                        \
     constexpr int V = 16 / sizeof(T);                                                                                \
     const bool each = dv == 1 && nh % V == 0 && g_stride % V == 0 && (((uintptr_t)y | (uintptr_t)g) & 15) == 0;      \
     const bool wide = each || (dv % V == 0 && ((uintptr_t)y & 15) == 0);                                             \
-    const int chunks = nh * dv / (wide ? V : 1);                                                                     \
-    const long long across = (chunks + 255) / 256;                                                                   \
     const unsigned gx = (unsigned)(n_tokens < 148 * 64 ? n_tokens : 148 * 64);                                       \
-    const dim3 grid(gx, (unsigned)(across < 64 ? across : 64));                                                      \
-    return launch(each ? head_gate_kernel<T, V, true> : wide ? head_gate_kernel<T, V, false> : head_gate_kernel<T, 1, false>, \
-                  grid, dim3(256), 0, st, (T*)y, (const T*)g, g_stride, n_tokens, nh, dv);                           \
+    /* so many heads at a time that places in a row are 32-bit numbers (a multiple of V where dv = 1) */             \
+    const int most = dv < (1 << 30) ? (1 << 30) / dv : 1;                                                            \
+    for (long long h0 = 0; h0 < nh; h0 += most) {                                                                    \
+      const int heads = (int)(nh - h0 < most ? nh - h0 : most);                                                      \
+      const long long across = ((long long)heads * dv / (wide ? V : 1) + 255) / 256;                                 \
+      const dim3 grid(gx, (unsigned)(across < 64 ? across : 64));                                                    \
+      const int rc = launch(each ? head_gate_kernel<T, V, true> : wide ? head_gate_kernel<T, V, false> : head_gate_kernel<T, 1, false>,\
+                            grid, dim3(256), 0, st, (T*)y + h0 * dv, (long long)nh * dv, (const T*)g + h0, g_stride, n_tokens, heads, dv);\
+      if (rc) return rc;                                                                                             \
+    }                                                                                                                \
+    return 0;                                                                                                        \
   }
 
 KVF_HEAD_OPS_API(f32, float)

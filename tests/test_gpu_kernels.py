@@ -1333,3 +1333,12 @@ def test_latent_decode_shows_what_is_no_number_in_any_range(ops):
         dev(q), out, dev(cache), dev(tables), i32([0, 1, 2]), i32(ctx), 2, 1, nh, d, dv, d**-0.5, scratch=scratch, max_context=200, split_size=64,
     )  # fmt: skip
     assert (out[0] == 20.0).all() and torch.isnan(out[1]).all()
+
+
+def test_head_gate_of_rows_beyond_32_bits(ops):
+    y = torch.ones((1, 2 * (2**30 + 8)), dtype=torch.bfloat16, device="cuda")
+    z = torch.tensor([[0.0, 2.0]], dtype=torch.bfloat16, device="cuda")
+    ops.head_gate(y, z, 2, 2**30 + 8)
+    for h, want in ((0, 0.5), (1, torch.sigmoid(torch.tensor(2.0)).bfloat16().item())):
+        half = y[0, h * (2**30 + 8) : (h + 1) * (2**30 + 8)]
+        assert float(half.min()) == float(half.max()) == want
