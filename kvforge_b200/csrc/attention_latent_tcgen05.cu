@@ -15,7 +15,7 @@
 // The blocks of a key tile outside the CTA's value columns are free as soon as S is made, the others after P V: either part has a
 // full and an empty barrier, so that the next tile's first part comes in under the softmax and its second under the first's products.
 // Warps: eight softmax (which first bring the queries in), one loader (TMA boxes of 64 numbers x the keys of a page, 16-byte
-// copies for a last tile that ends inside a page), one issuer.  One CTA an SM.
+// copies for the page that the context ends in), one issuer.  One CTA an SM.
 // 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 160 us against 591 us
 // of the mma.sync kernel, and the same error against 64-bit.  What bounds it is that scores, softmax, products and copies of a tile follow one
 // another, for want of room for a second tile: with tiles of 64 keys in two stages and four softmax warps it took 233 us, with tiles of
@@ -201,21 +201,36 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
           }
         }
       } else {
-        // the sequence's last tile ends inside a page, whose other keys must not be read: key by key, zeros past the context
+        // the sequence's last tile ends inside a page, whose other keys must not be read: that page's box comes key by key, with
+        // zeros past the context, the others as above
         if (t >= 1) {
           ok = __all_sync(0xffffffffu, (n0 == 0 || bar_wait(ke0, (t - 1) & 1, p.err)) && bar_wait(ke1, (t - 1) & 1, p.err));
           if (!ok) break;
         }
-        const int chunks = p.kb * 8;
-        for (int key = 0; key < BN; ++key) {
-          int off;
-          const int blk = page_of(t0 + key, off);
-          const bf16* src = p.cache + (blk >= 0 ? ((size_t)blk * p.block_size + off) * p.d : 0);
-          for (int c = lane; c < chunks; c += 32) {
-            const bool valid = blk >= 0 && c * 8 < p.d;
-            cpa16(k_s + (uint32_t)(c >> 3) * K_BLOCK + sw128(key, c & 7), src + (valid ? c * 8 : 0), valid);
-          }
+        int off;
+        const int blk = page_of(t0 + p.box_rows * (lane % boxes), off);
+        const int row = blk >= 0 ? blk * p.block_size + off : p.total_rows;
+        const int cut = (ctx - t0) / p.box_rows;  // the box that the context ends in
+        const uint32_t others = (uint32_t)((boxes - 1) * p.box_rows) * 128u;
+        if (lane == 0) {
+          if (n0) bar_more_tx(kf0, (uint32_t)n0 * others);
+          bar_more_tx(kf1, (uint32_t)p.nvb * others);
         }
+        __syncwarp();
+        for (int i = lane; i < p.kb * boxes; i += 32) {  // boxes divides 32: a lane keeps its box
+          const int kb = i / boxes;
+          if (lane % boxes != cut)
+            tma_load_2d(k_s + (uint32_t)kb * K_BLOCK + (uint32_t)((lane % boxes) * p.box_rows) * 128u, &map, 64 * kb, row, kb >= vb0 && kb < vb0 + p.nvb ? kf1 : kf0);
+        }
+        int cut_off;
+        const int cut_blk = page_of(t0 + cut * p.box_rows, cut_off);
+        const bf16* const src = p.cache + (cut_blk >= 0 ? ((size_t)cut_blk * p.block_size + cut_off) * p.d : 0);
+        const int keys = cut_blk >= 0 ? ctx - t0 - cut * p.box_rows : 0, chunks = p.kb * 8;
+        for (int key = 0; key < p.box_rows; ++key)
+          for (int c = lane; c < chunks; c += 32) {
+            const bool valid = key < keys && c * 8 < p.d;
+            cpa16(k_s + (uint32_t)(c >> 3) * K_BLOCK + sw128(cut * p.box_rows + key, c & 7), src + (valid ? (size_t)key * p.d + c * 8 : 0), valid);
+          }
         cpa_commit();
         cpa_wait<0>();
         fence_async_smem();

@@ -1342,3 +1342,19 @@ def test_head_gate_of_rows_beyond_32_bits(ops):
     for h, want in ((0, 0.5), (1, torch.sigmoid(torch.tensor(2.0)).bfloat16().item())):
         half = y[0, h * (2**30 + 8) : (h + 1) * (2**30 + 8)]
         assert float(half.min()) == float(half.max()) == want
+
+
+@pytest.mark.parametrize("nh,d,dv,block_size", [(16, 576, 512, 16), (16, 576, 512, 64), (4, 208, 128, 48), (5, 64, 64, 32)])
+@pytest.mark.parametrize("ctx", [1, 15, 17, 63, 65, 100, 127, 129, 143, 255, 257, 300])
+def test_latent_attention_of_contexts_that_end_anywhere(ops, nh, d, dv, block_size, ctx):
+    """The last tile's boxes: whole ones, the one that the context ends in, and those past it, whose places hold NaN."""
+    n = min(ctx, 40)
+    q, cache, tables, ctxs, ref, bound = paged_latent_case([n, 1], [ctx - n, ctx - 1], nh, d, dv, block_size, 0, ctx + d)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((n + 1, nh * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention(
+        dev(q), out, dev(cache), dev(tables), i32([0, n, n + 1]), i32(ctxs), 2, n, nh, d, dv, d**-0.5, kernel="tcgen05", err=err,
+    )  # fmt: skip
+    assert int(err.item()) == 0
+    assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
