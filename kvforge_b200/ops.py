@@ -713,7 +713,7 @@ def paged_attention(
     use_mma = mma_attention_supported(q.dtype, nh, nkv, d, decode_form)
     # many queries with kept first keys, a bias (of at most 8 heads a key head: a tile's biases lie in shared memory) or capped
     # scores: the tcgen05 kernel's form for them.  2,048 tokens, 32 heads of 64 under a window of 1,024, with a bias and 64 kept
-    # keys: 76 us, 149 us on the mma.sync tile kernel
+    # keys: 77 us, 149 us on the mma.sync tile kernel
     use_shaped = (
         biased_mma and use_tc and shaped_tcgen05_supported(q.dtype, nh, nkv, d, bias is not None) and q.data_ptr() % 16 == 0
         and out.data_ptr() % 16 == 0 and num_seqs <= 65535 and max_q_len <= 65535 * tcgen05_query_tile(nh, nkv)

@@ -1358,3 +1358,20 @@ def test_latent_attention_of_contexts_that_end_anywhere(ops, nh, d, dv, block_si
     )  # fmt: skip
     assert int(err.item()) == 0
     assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
+
+
+def off_by(out, ref, d):
+    """Relative error of ``run_shaped``'s output against the 64-bit results of its case."""
+    got = out.double()
+    num = sum(float((got[r0 : r0 + o.shape[0], h * d : (h + 1) * d] - o).square().sum()) for r0, h, o in ref)
+    return math.sqrt(num / sum(float(o.square().sum()) for _, _, o in ref))
+
+
+@pytest.mark.parametrize("d,nh,nkv,far,cap,sink", [(64, 8, 2, 200, 0.0, False), (64, 8, 2, 0, 30.0, False), (128, 8, 2, 100, 20.0, True)])
+def test_shaped_scores_on_tcgen05_are_no_further_off(ops, d, nh, nkv, far, cap, sink):
+    """Against 64 bits, as far off as the mma.sync kernel: both round the same weights to bfloat16, with the largest one exact.
+    4,000 rows: the ratio of two such errors varies by 1 / sqrt(2 x 4,000), so 4 % are more than three times that."""
+    case = (d, nh, nkv, 16, 0, 0, far, cap, sink, [130, 370], [400, 0])
+    ref = paged_shaped_case(*case)[7]
+    errors = [off_by(run_shaped(ops, *case, kernel=kernel)[0], ref, d) for kernel in ("tcgen05", "mma")]
+    assert errors[0] <= 1.04 * errors[1], errors
