@@ -720,7 +720,7 @@ def paged_attention(
     )  # fmt: skip
     use_tma = tickets is not None and tma_decode_supported(q.dtype, nh, nkv, d, block_size, kcache.shape[0])
     # decoding with such scores: the TMA kernel's form for them (64 sequences of 32 heads of 64 on 8, contexts of 1,150 to 2,300 under a
-    # window of 1,024, with a bias and 64 kept keys: 36.6 us, 55.8 us on the mma.sync split kernel)
+    # window of 1,024, with a bias and 64 kept keys: 37.3 us, 55.8 us on the mma.sync split kernel)
     if biased_mma and kernel == "tma" and not use_tma:
         raise ValueError("the TMA decode kernel does not take this shape (or no tickets were given)")
     if biased_mma and scratch is not None and (kernel == "mma" or (kernel == "auto" and not use_tma)):
