@@ -7,8 +7,8 @@
 // where 2 x (d + 512) / 2 would do, but the accumulator of 128 x 512 alone is all of an SM's tensor memory.  Per tile of 128 keys:
 //   S = Q K^T   tcgen05.mma 128 x 128 x 16, d/16 of them.  The first (up to four) blocks of 64 query numbers lie in tensor memory
 //               as the A operand (128 columns): 80 KB of queries and 144 KB of keys are what an SM holds;
-//   softmax     two groups of four warps, 64 keys of a row a thread, from tensor memory, as in attention_tcgen05.cu (running maximum
-//               raised lazily; the two halves of a row exchange their maxima); P takes the place of S in tensor memory;
+//   softmax     two groups of four warps, 64 keys of a row a thread, from tensor memory, as in attention_tcgen05.cu (the two
+//               halves of a row exchange their maxima); P takes the place of S in tensor memory;
 //   O += P V    P as the A operand from tensor memory, the value tile being the key tile's first dv columns, read as an
 //               MN-major B operand of all the CTA's columns at once, blocks of 64 a stride apart (a product of its own for each block
 //               of columns costs the issuing thread some 80 cycles, four of them 24 us of 184); O stays in tensor memory.
@@ -16,11 +16,11 @@
 // full and an empty barrier, so that the next tile's first part comes in under the softmax and its second under the first's products.
 // Warps: eight softmax (which first bring the queries in), one loader (TMA boxes of 64 numbers x the keys of a page, 16-byte
 // copies for the page that the context ends in), one issuer.  One CTA an SM.
-// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 160 us against 591 us
+// 2,048 tokens, 16 heads, d = 576, dv = 512 (73 GFLOP without what the two halves repeat, 46 us at the tensor peak): 161 us against 587 us
 // of the mma.sync kernel, and the same error against 64-bit.  What bounds it is that scores, softmax, products and copies of a tile follow one
 // another, for want of room for a second tile: with tiles of 64 keys in two stages and four softmax warps it took 233 us, with tiles of
-// 128 and eight warps 220, 184 since those eight and not the loader alone bring the queries (147 KB a CTA), and 160 with one product
-// for all value columns (pages of 16 tokens; 156 with pages of 64).
+// 128 and eight warps 220, 184 since those eight and not the loader alone bring the queries (147 KB a CTA), and 153 with one product
+// for all value columns (pages of 16 tokens); the exact maximum (below) costs 8 of the 161.
 // Every mbarrier wait is bounded; if one runs out the kernel raises bit 4 of the error flag and winds down.
 #include "tcgen05.cuh"
 
@@ -76,7 +76,8 @@ __device__ __forceinline__ float row_max(const uint32_t (&va)[32], const uint32_
   }
   return mx;
 }
-// exp2(score * scale - m_ref) of the 64 scores as bfloat16 pairs; returns their sum.
+// exp2(score * scale - m_ref) of the 64 scores as bfloat16 pairs; returns the (float) sum of what was stored, so that the
+// division cancels a part of the rounding: a weight's error counts by how far its value lies from the result.
 template <bool MASK>
 __device__ __forceinline__ float weights(const uint32_t (&va)[32], const uint32_t (&vb)[32], uint32_t (&w)[32], float m_ref, float scale_log2, int first, int last) {
   const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
@@ -92,11 +93,13 @@ __device__ __forceinline__ float weights(const uint32_t (&va)[32], const uint32_
       if (c < first || c > last) e0 = 0.f;
       if (c + 1 < first || c + 1 > last) e1 = 0.f;
     }
+    const uint32_t both = pk(e0, e1);
+    w[c >> 1] = both;
+    const uint64_t rounded = pack2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u));
     if (c & 2)
-      sum_b = add2(sum_b, pack2(e0, e1));
+      sum_b = add2(sum_b, rounded);
     else
-      sum_a = add2(sum_a, pack2(e0, e1));
-    w[c >> 1] = pk(e0, e1);
+      sum_a = add2(sum_a, rounded);
   }
   float s0, s1;
   unpack2(add2(sum_a, sum_b), s0, s1);
@@ -366,7 +369,10 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
       asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
       mx = fmaxf(mx, theirs[(t & 1) * 2 * BM]) * p.scale_log2;  // scale > 0
       float corr = 1.f;
-      if (mx > m_ref + RESCALE_STEP || (m_ref == -INFINITY && mx > -INFINITY)) {
+      // Followed exactly, so that the largest weight is one, which no rounding changes (rises of less than a factor of 2^8 left
+      // alone and the weights summed before they are rounded: results are 1.01 to 1.24 times as far off against 64 bits as on the
+      // mma.sync kernel, with both 0.995 to 1.004; 2,048 tokens 153 us and 161).
+      if (mx > m_ref) {
         corr = ex2(m_ref - mx);  // 0 the first time
         m_ref = mx;
       }

@@ -861,7 +861,7 @@ def latent_attention(
     )  # fmt: skip
     if kernel == "tcgen05" and not takes:
         raise ValueError("latent_attention: the tcgen05 kernel does not take this call")
-    # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 160 us here, 591 us on
+    # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 161 us here, 587 us on
     # the mma.sync kernel; single queries go to its key ranges, which a CTA of 128 rows would leave empty
     if takes and (kernel == "tcgen05" or (kernel == "auto" and max_q_len > 1)):
         tiles, n_tiles = None, 0

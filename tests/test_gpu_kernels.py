@@ -1385,3 +1385,20 @@ def test_shaped_scores_of_a_decode_step_by_tma_are_no_further_off(ops, d, nh, nk
     ref = paged_shaped_case(*case)[7]
     errors = [off_by(run_shaped(ops, *case, decode=(256, False), kernel=kernel)[0], ref, d) for kernel in ("tma", "mma")]
     assert errors[0] <= 1.02 * errors[1], errors
+
+
+@pytest.mark.parametrize("nh,d,dv,lens,starts", [(16, 576, 512, [150, 100], [0, 300]), (8, 320, 256, [300], [200])])
+@pytest.mark.parametrize("sharp", [1.0, 3.0])
+def test_latent_attention_on_tcgen05_is_no_further_off(ops, nh, d, dv, lens, starts, sharp):
+    """Against 64 bits, as far off as the mma.sync kernel.  2,400 and more rows: the ratio of two such errors varies by
+    1 / sqrt(2 x 2,400), so 5 % are more than three times that."""
+    q, cache, tables, ctx, ref, bound = paged_latent_case(lens, starts, nh, d, dv, 16, 0, 3, sharp)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    qsl, errors = [0], []
+    for n in lens:
+        qsl.append(qsl[-1] + n)
+    for kernel in ("tcgen05", "mma"):
+        out = torch.empty((sum(lens), nh * dv), device="cuda", dtype=torch.bfloat16)
+        ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32(qsl), i32(ctx), len(lens), max(lens), nh, d, dv, d**-0.5, kernel=kernel)
+        errors.append(float((out.cpu().double() - ref).norm() / ref.norm()))
+    assert errors[0] <= 1.05 * errors[1], errors
