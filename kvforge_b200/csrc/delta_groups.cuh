@@ -10,7 +10,7 @@
 //   A_ij = k_i^T (g_{j+1} .. g_i) k_j  (j < i)      B_ij = q_i^T (g_{j+1} .. g_i) k_j  (j <= i)
 //   u_i = beta_i (v_i - a_i - sum_{j<i} A_ij u_j)    o_i = p_i + sum_{j<=i} B_ij u_j
 //   S   = c_4 S0 + sum_j ((g_{j+1} .. g_4) k_j) u_j
-// which is the rule with the terms in another order, all of it 32-bit.  One link now serves four tokens: eight dot products side
+// which is the rule with the terms in another order, all of it 32-bit or more.  One link now serves four tokens: eight dot products side
 // by side, one shuffle tree of eight values that halves what a lane holds at every level, a triangle of six multiply-adds, one
 // write.  The multiply-adds of the state are 13 a number and group where the walk has 16, and pairs of rows share a packed
 // instruction.
@@ -21,9 +21,9 @@
 // column, R rows each in registers; records come through a ring in shared memory by cp.async, one barrier a group.
 // Groups start at a step's first token of the sequence; a last group is filled up with tokens of zero keys and beta.
 //
-// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 631 us by the walk, 513 here (both kernels), 24 heads
-// over 1,500 923 and 464, 8 heads with a decay a head 449 and 349; 61 sequences of which one brings 40 tokens 165 and 92.  Against
-// 64-bit the outputs are off by 1.3e-7 of their norm either way (1.28 and 1.31).  A group is some 430 instructions a warp on its
+// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 630 us by the walk, 535 here (both kernels), 24 heads
+// over 1,500 920 and 487, 8 heads with a decay a head 449 and 352; 61 sequences of which one brings 40 tokens 165 and 92.  Against
+// 64-bit the outputs are off by 1.28e-7 of their norm by the walk, 1.20e-7 here.  A group is some 430 instructions a warp on its
 // way to the next state, and the latency of the shuffles and of the triangle between them.  Heads of at most 64 rows and of
 // more than 128 keep the walk: 4 x 64 over 700 tokens 148 us by the walk and 160 here, 3 x 32 over 131 35 and 57, 2 x 256 over 333 91
 // and 92: a narrow head's link is short already, a wide one's 16 rows a lane are all instructions.
@@ -76,6 +76,16 @@ __device__ __forceinline__ void dg_load4(const bf16* src, int left, bool wide, f
   }
 }
 
+__device__ __forceinline__ double dg_warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The norms and the products of decays are made in double, so that an entry of a record is rounded once: a walk token by token
+// rounds a decayed state where a record holds decayed keys, and with float factors (one rounding more a token of the
+// group) outputs were 0.2 to 7 % further off against 64 bits than the walk's.  Outputs are 0.89 to 1.01 of the walk's error so, the
+// state's between 0.95 and 1.07, 1.00 on average; 16 heads with a decay a channel over 2,048 tokens 513 us with float factors, 535 so.
 template <bool CH>
 __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaParams p, int nseq) {
   pdl_launch();
@@ -134,13 +144,14 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
 #pragma unroll
   for (int i = 0; i < DG_TOKENS; ++i) gh[i] = CH ? 1.f : __shfl_sync(0xffffffffu, gl, i);
   // sums over the rows: |k|^2, |q|^2 and the decayed products of every pair (a decay a head: the plain products)
-  float sk[DG_TOKENS] = {}, sq[DG_TOKENS] = {}, pa[6] = {}, pb[10] = {};
+  double sk[DG_TOKENS] = {}, sq[DG_TOKENS] = {};
+  float pa[6] = {}, pb[10] = {};
 #pragma unroll
   for (int e = 0; e < 4; ++e)
 #pragma unroll
     for (int j = 0; j < DG_TOKENS; ++j) {
-      sk[j] = fmaf(k[j][e], k[j][e], sk[j]);
-      sq[j] = fmaf(q[j][e], q[j][e], sq[j]);
+      sk[j] = fma((double)k[j][e], (double)k[j][e], sk[j]);
+      sq[j] = fma((double)q[j][e], (double)q[j][e], sq[j]);
       float kd = k[j][e];  // (g_{j+1} .. g_i) k_j
       pb[j * (j + 1) / 2 + j] = fmaf(q[j][e], kd, pb[j * (j + 1) / 2 + j]);
 #pragma unroll
@@ -152,13 +163,13 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
     }
 #pragma unroll
   for (int i = 0; i < DG_TOKENS; ++i) {
-    sk[i] = 1.f / sqrtf(warp_sum(sk[i]) + p.norm_eps);
-    sq[i] = p.q_scale / sqrtf(warp_sum(sq[i]) + p.norm_eps);
+    sk[i] = 1.0 / sqrt(dg_warp_sum(sk[i]) + p.norm_eps);
+    sq[i] = p.q_scale / sqrt(dg_warp_sum(sq[i]) + p.norm_eps);
   }
   float* rec = p.groups + ((size_t)(dg_base(first, b) + grp) * p.H + h) * dg_record(CH);
-  float cp[DG_TOKENS], cs[DG_TOKENS];  // a decay a head: g_1 .. g_i and g_{j+1} .. g_4
+  double cp[DG_TOKENS], cs[DG_TOKENS];  // a decay a head: g_1 .. g_i and g_{j+1} .. g_4
   cp[0] = gh[0];
-  cs[DG_TOKENS - 1] = 1.f;
+  cs[DG_TOKENS - 1] = 1.0;
 #pragma unroll
   for (int i = 1; i < DG_TOKENS; ++i) {
     cp[i] = cp[i - 1] * gh[i];
@@ -168,12 +179,12 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
   for (int i = 0; i < DG_TOKENS; ++i) {
 #pragma unroll
     for (int j = 0; j <= i; ++j) {
-      float d = 1.f;
+      double d = 1.0;
       if (!CH)
 #pragma unroll
         for (int e = j + 1; e <= i; ++e) d *= gh[e];
-      pb[i * (i + 1) / 2 + j] = warp_sum(pb[i * (i + 1) / 2 + j]) * (sq[i] * sk[j]) * d;
-      if (j < i) pa[i * (i - 1) / 2 + j] = warp_sum(pa[i * (i - 1) / 2 + j]) * (sk[i] * sk[j]) * d;
+      pb[i * (i + 1) / 2 + j] = (float)(warp_sum(pb[i * (i + 1) / 2 + j]) * (sq[i] * sk[j]) * d);
+      if (j < i) pa[i * (i - 1) / 2 + j] = (float)(warp_sum(pa[i * (i - 1) / 2 + j]) * (sk[i] * sk[j]) * d);
     }
   }
   float* co = rec + (CH ? 13 : 8) * DG_ROWS;
@@ -185,20 +196,20 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) co[12 + 4 * i + j] = j <= i ? pb[i * (i + 1) / 2 + (j <= i ? j : 0)] : 0.f;
-      co[28 + i] = cp[i];
-      co[32 + i] = cs[i];
+      co[28 + i] = (float)cp[i];
+      co[32 + i] = (float)cs[i];
     }
   }
   auto put = [&](int which, const float (&f)[4]) { *reinterpret_cast<float4*>(rec + which * DG_ROWS + r) = make_float4(f[0], f[1], f[2], f[3]); };
-  float cc[4] = {1.f, 1.f, 1.f, 1.f}, ss[4] = {1.f, 1.f, 1.f, 1.f};
+  double cc[4] = {1.0, 1.0, 1.0, 1.0}, ss[4] = {1.0, 1.0, 1.0, 1.0};
 #pragma unroll
   for (int i = 0; i < DG_TOKENS; ++i) {
     float fk[4], fq[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (CH) cc[e] *= g[i][e];
-      fk[e] = cc[e] * (k[i][e] * sk[i]);
-      fq[e] = cc[e] * (q[i][e] * sq[i]);
+      fk[e] = (float)(cc[e] * (k[i][e] * sk[i]));
+      fq[e] = (float)(cc[e] * (q[i][e] * sq[i]));
     }
     put(i, fk);
     put(DG_TOKENS + i, fq);
@@ -207,13 +218,16 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
       float fs[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        fs[e] = ss[e] * (k[j][e] * sk[j]);
+        fs[e] = (float)(ss[e] * (k[j][e] * sk[j]));
         ss[e] *= g[j][e];
       }
       put(2 * DG_TOKENS + j, fs);
     }
   }
-  if (CH) put(3 * DG_TOKENS, cc);
+  if (CH) {
+    const float c4[4] = {(float)cc[0], (float)cc[1], (float)cc[2], (float)cc[3]};
+    put(3 * DG_TOKENS, c4);
+  }
 }
 
 // ---- the walk over the groups
@@ -416,6 +430,7 @@ int dispatch_delta_groups(const DeltaParams& p, int B, cudaStream_t st) {
   const dim3 grid((unsigned)((warps + 3) / 4));
   const int rc = launch(delta_group_prepare_kernel<CH>, grid, dim3(128), 0, st, p, B);
   if (rc) return rc;
+  // (Figures here are those with float factors in the records; double ones add some 4 % to either side.)
   // What counts for a few long sequences is a short link (16 lanes a column: 16 heads of 128 x 128 over 2,048 tokens 513 us against
   // 506, 24 heads over 1,500 464 against 538, 8 x 256 tokens of 16 heads 348 against 388; with a decay a head 349 against 465 for
   // 8 heads); once every SM has more than a dozen CTAs to work off it is the number of instructions (8 lanes: 50 x 40 tokens of 16

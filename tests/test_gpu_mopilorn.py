@@ -547,3 +547,38 @@ def test_general_rotation_and_cache_write(dtype, interleaved, rot):
         assert torch.allclose(kc[sl // bs, :, sl % bs].float().cpu().double(), turned[i, nh:], atol=tol, rtol=tol)
         assert torch.equal(vc[sl // bs, :, sl % bs].float().cpu(), v[i])
     assert float(kc.float().abs().sum(-1).gt(0).sum()) == 12 * nkv
+
+
+@pytest.mark.parametrize("h,dk,dv,channel", [(6, 128, 128, True), (6, 128, 128, False), (5, 100, 96, True)])
+def test_gated_delta_rule_in_groups_is_no_further_off(h, dk, dv, channel):
+    """Against 64 bits, the form four tokens at a time and the walk token by token: outputs over 600 tokens of three sequences.  Records
+    with one rounding an entry are 5 to 11 % nearer than the walk, with a rounding a factor 1 to 7 % further off."""
+    from kvforge_b200 import ops
+
+    gen = torch.Generator().manual_seed(dk)
+    lens, dev, dt = [300, 200, 100], "cuda", torch.bfloat16
+    n, aw = sum(lens), h * dk if channel else h
+    qkv, b, a = torch.randn(n, 2 * h * dk + h * dv, generator=gen).to(dt), torch.randn(n, h, generator=gen), torch.randn(n, aw, generator=gen)
+    a_log, dt_bias = 0.5 * torch.randn(h, generator=gen), 0.5 * torch.randn(aw, generator=gen)
+    decay = torch.exp(-torch.exp(a_log.double()).repeat_interleave(dk if channel else 1) * F.softplus(a.double() + dt_bias.double()))
+    want, at = [], 0
+    for m in lens:
+        row = slice(at, at + m)
+        q = plain.unit(qkv[row, : h * dk].double().view(m, h, dk)) * dk**-0.5
+        k = plain.unit(qkv[row, h * dk : 2 * h * dk].double().view(m, h, dk))
+        g = decay[row].view(m, h, dk) if channel else decay[row]
+        want.append(plain.delta_rule(q, k, qkv[row, 2 * h * dk :].double().view(m, h, dv), torch.sigmoid(b[row].double()), g).reshape(m, -1))
+        at += m
+    want = torch.cat(want)
+    qsl, sl = flat_batch(lens, [0, 1, 2], dev)
+    errors = []
+    for grouped in (True, False):
+        state, out = torch.zeros(3, h * dk * dv, device=dev), torch.empty(n, h * dv, device=dev)
+        groups = torch.empty(ops.delta_group_floats(n, 3, h, channel), device=dev) if grouped else None
+        x = qkv.to(dev)
+        ops.gated_delta(
+            x[:, : h * dk], x[:, h * dk : 2 * h * dk], x[:, 2 * h * dk :], b.to(dev), a.to(dev), a_log.to(dev), dt_bias.to(dev), state, out, qsl, sl,
+            3, h, h, dk, dv, q_scale=dk**-0.5, max_query_len=max(lens), groups=groups,
+        )  # fmt: skip
+        errors.append(float((out.cpu().double() - want).norm() / want.norm()))
+    assert errors[0] <= errors[1], errors
