@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
   const int n_tok = live ? min(p.tq, q_len - q0) : 0;
   const int p_first = ctx - q_len + q0;
   const int kv_hi = p_first + n_tok;
-  const int kv_lo = live ? (first_key(p_first, p.window) / BN) * BN : 0;
+  const int seen_lo = live ? first_key(p_first, p.window) : 0, kv_lo = (seen_lo / BN) * BN;
   const int n_tiles = live ? (kv_hi - kv_lo + BN - 1) / BN : 0;
 
   if (threadIdx.x == 0) {
@@ -289,9 +289,12 @@ __global__ void __launch_bounds__(THREADS, 1) latent_tcgen05_kernel(const __grid
         if (ok) ok = bar_wait(p_full, t & 1, p.err);  // P(t) is in tensor memory, O has been rescaled
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // Only the keys that some row of the CTA may see: a weight of zero times a value that is no number is none, and a tile
+        // reaches up to 127 keys beyond the last query (and before the first one's window).
+        const int key0 = kv_lo + t * BN, kk_lo = max(0, seen_lo - key0) / 16, kk_hi = min(BN, kv_hi - key0 + 15) / 16;
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // A: 16 keys of P = 8 columns; B: 16 keys = 16 rows of 128 bytes in each block
-          umma_ts(o_t, s_t + 8u * kk, v_d + (uint64_t)(kk * (16 * 128 >> 4)), id_o, (t > 0 || kk > 0) ? 1u : 0u);
+          if (kk >= kk_lo && kk < kk_hi) umma_ts(o_t, s_t + 8u * kk, v_d + (uint64_t)(kk * (16 * 128 >> 4)), id_o, (t > 0 || kk > kk_lo) ? 1u : 0u);
         umma_commit(pv_done);
         umma_commit(ke1);
       }

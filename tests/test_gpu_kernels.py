@@ -1402,3 +1402,28 @@ def test_latent_attention_on_tcgen05_is_no_further_off(ops, nh, d, dv, lens, sta
         ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32(qsl), i32(ctx), len(lens), max(lens), nh, d, dv, d**-0.5, kernel=kernel)
         errors.append(float((out.cpu().double() - ref).norm() / ref.norm()))
     assert errors[0] <= 1.05 * errors[1], errors
+
+
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("bad", [3, 64, 140, 200, 243])
+def test_latent_attention_keeps_what_is_no_number_near(ops, window, bad):
+    """A NaN row of the cache: every query that sees it is NaN; of the others only those whose tile of eight queries reaches into
+    the sixteen keys around it may be."""
+    nh, d, dv, n = 16, 192, 128, 250
+    q, cache, tables, ctx, ref, bound = paged_latent_case([n], [0], nh, d, dv, 16, window, bad)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    page = int(tables[0, bad // 16])
+    cache[page if page >= 0 else -1, 0, bad % 16] = float("nan")
+    for kernel in ("tcgen05", "mma"):
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        out = torch.zeros((n, nh * dv), device="cuda", dtype=torch.bfloat16)
+        ops.latent_attention(dev(q), out, dev(cache), dev(tables), i32([0, n]), i32(ctx), 1, n, nh, d, dv, d**-0.5, window=window, kernel=kernel, err=err)
+        assert int(err.item()) == 0
+        got, i = out.cpu().double(), torch.arange(n)
+        sees = (i >= bad) & (i - bad < (window or n))
+        first = i // 8 * 8
+        near = (first + 7 >= bad // 16 * 16) & (first - (window or n) + 1 <= bad // 16 * 16 + 15)
+        assert torch.isnan(got[sees]).all(), kernel
+        if kernel == "tcgen05" and bool((~near).any()):
+            assert not torch.isnan(got[~near]).any()
+            assert float(((got - ref).abs() - bound)[~near].max()) <= 0.0
