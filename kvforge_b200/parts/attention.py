@@ -366,7 +366,10 @@ class PagedAttention(Mixer):
         shape = (self.nh, self.nkv, self.d, self.scale)
         # bfloat16: the decode kernel may lengthen its key ranges from the step's longest context (the merge
         # order then follows the batch, within rounding); 32-bit keeps one order whatever the batch
-        wave = ops.attention_wave_target(ctx.num_seqs, self.nkv, self.d) if q.dtype == torch.bfloat16 else 0
+        # ... Shaped scores keep the launch's ranges: of each warp's weights the largest is exactly one, and with fewer ranges fewer
+        # are (4 and 8 sequences at 4,000 keys: 2 to 8 % further off against 64 bits, 1.0 to 1.25 times as fast; 64 sequences 2 % slower)
+        shaped = self.bias is not None or self.keep_first > 0 or bool(self.softcap)
+        wave = ops.attention_wave_target(ctx.num_seqs, self.nkv, self.d) if q.dtype == torch.bfloat16 and not shaped else 0
         if ctx.all_single_query:
             scratch, bound, split = self._scratch(ctx)
         tiles = ctx.query_tiles.get(self._query_tile)

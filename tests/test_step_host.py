@@ -257,3 +257,37 @@ def test_buffers_of_the_delta_rule_s_walk_hold_what_the_walk_may_see():
         part.rt = SimpleNamespace(dtype=dtype, max_tokens=budget, max_seqs=seqs)
         assert part._walk_rows(1) == want, (dtype, dk)
         assert part._walk_rows(2000) == (want[0], budget)
+
+
+def test_shaped_scores_keep_the_ranges_of_the_launch(monkeypatch):
+    """The decode kernel may lengthen its ranges for plain scores in bfloat16 alone, in steps of single tokens and in mixed ones."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from kvforge_b200 import ops
+    from kvforge_b200.parts.attention import PagedAttention
+
+    calls = []
+    monkeypatch.setattr(ops, "paged_attention", lambda *a, **kw: calls.append(kw))
+    for dtype, shape, lengthens in (
+        (torch.bfloat16, {}, True), (torch.bfloat16, {"sinks": object()}, True), (torch.float32, {}, False),
+        (torch.bfloat16, {"bias": object()}, False), (torch.bfloat16, {"keep_first": 4}, False), (torch.bfloat16, {"softcap": 30.0}, False),
+    ):  # fmt: skip
+        part = object.__new__(PagedAttention)
+        for k, v in dict(window=64, chunk=None, dv=64, keep_first=0, bias=None, softcap=0.0, sinks=None, nh=8, nkv=2, d=64, scale=0.1, _query_tile=32).items():
+            setattr(part, k, shape.get(k, v))
+        part.rt = SimpleNamespace(err=None, capturing=False)
+        part._scratch = lambda ctx: ((), 100, 64)
+        q, cache = torch.zeros(8, 512, dtype=dtype), SimpleNamespace(k=torch.zeros(4, 2, 16, 64), v=None, group=0)
+        tiles = SimpleNamespace(num_single=3, multi=None, multi_count=1, tiles=None, count=4)
+        for single in (True, False):
+            calls.clear()
+            ctx = SimpleNamespace(
+                block_tables=[None], query_start_loc=None, context_lens=None, num_seqs=4, max_query_len=1 if single else 9, block_size=16,
+                all_single_query=single, query_tiles={} if single else {32: tiles},
+            )  # fmt: skip
+            part.attend(ctx, q, 512, None, cache)
+            ranges = [kw for kw in calls if kw.get("scratch") is not None]
+            assert len(ranges) == (1 if single or dtype == torch.bfloat16 else 0)
+            assert all((kw["wave_target"] > 0) == lengthens for kw in ranges), shape
