@@ -823,6 +823,9 @@ def latent_tcgen05_supported(dtype: torch.dtype, nh: int, d: int, dv: int, block
     return dtype == torch.bfloat16 and d % 16 == 0 and dv <= d <= 576 and dv in (64, 128, 256, 512) and 0 < nh <= 128 and block_size % 16 == 0
 
 
+LATENT_SHORT_CONTEXT = 64  # keys up to which the mma.sync kernel stays for many queries
+
+
 def latent_query_tile(nh: int) -> int:
     """Query tokens of one sequence that a CTA of that kernel takes."""
     return 128 // nh
@@ -839,8 +842,8 @@ def latent_attention(
     ``out [N, nh*dv]``, bfloat16, on the tensor cores.  With ``scratch`` (partial results ``[B, nh, splits, dv]`` and
     their maxima and sums ``[B, nh, splits, 2]``, float) and one query a sequence the decode form runs: ranges of
     ``split_size`` keys in parallel, then a merge.  Without it and with more than one query in some sequence the tcgen05
-    kernel runs where it takes the shape (``kernel``: ``"mma"`` or ``"tcgen05"`` force one; ``err`` and ``query_tiles``, tiles of
-    ``latent_query_tile`` queries, as in ``paged_attention``)."""
+    kernel runs where it takes the shape, unless ``max_context`` says that no context is longer than 64 keys (``kernel``: ``"mma"`` or
+    ``"tcgen05"`` force one; ``err`` and ``query_tiles``, tiles of ``latent_query_tile`` queries, as in ``paged_attention``)."""
     if kernel not in ("auto", "mma", "tcgen05"):
         raise ValueError("latent_attention: kernel is 'auto', 'mma' or 'tcgen05'")
     if not latent_attention_supported(q.dtype, d, dv):
@@ -862,8 +865,13 @@ def latent_attention(
     if kernel == "tcgen05" and not takes:
         raise ValueError("latent_attention: the tcgen05 kernel does not take this call")
     # more than one query in some sequence: 2,048 tokens of one sequence (16 heads, rows of 576, values of 512) 161 us here, 587 us on
-    # the mma.sync kernel; single queries go to its key ranges, which a CTA of 128 rows would leave empty
-    if takes and (kernel == "tcgen05" or (kernel == "auto" and max_q_len > 1)):
+    # the mma.sync kernel; single queries go to its key ranges, which a CTA of 128 rows would leave empty.  A CTA's start (tensor
+    # memory, its 128 queries, one tile of 128 keys) takes 8 to 15 us whatever the context.  Contexts of 2, 40, 64, 80, 128 and 200 keys,
+    # the prompt of one sequence, us on tcgen05 / mma.sync: 16 heads of 576: 13.3 / 8.7, 16.6 / 15.2, 15.1 / 15.3, 15.1 / 18.8,
+    # 15.2 / 22.9, 23.9 / 34.3; 8 of 320: 11.2 / 6.0, 12.8 / 10.7, 12.3 / 10.8, 12.2 / 13.5, 12.2 / 16.6, 19.0 / 24.9; 8 and 40
+    # sequences cross at the same place (8 x 40 tokens of 32 heads 32.1 / 25.5, 8 x 64 29.4 / 29.5, 8 x 128 57.2 / 69.1)
+    short = max_context is not None and max_context <= LATENT_SHORT_CONTEXT
+    if takes and (kernel == "tcgen05" or (kernel == "auto" and max_q_len > 1 and not short)):
         tiles, n_tiles = None, 0
         if query_tiles is not None:
             tiles, n_tiles = query_tiles

@@ -177,7 +177,8 @@ class LatentAttention(Mixer):
             tiles = ctx.query_tiles.get(self._query_tile)
             ops.latent_attention(
                 qa, o_lat, cache.k, ctx.block_tables[cache.group], ctx.query_start_loc, ctx.context_lens, ctx.num_seqs, ctx.max_query_len,
-                h, d, r, self.scale, window=int(self.window or 0), scratch=scratch, max_context=bound, split_size=split, err=rt.err,
+                h, d, r, self.scale, window=int(self.window or 0), scratch=scratch, max_context=bound if scratch is not None else ctx.max_context_len,
+                split_size=split, err=rt.err,
                 query_tiles=(tiles.tiles, tiles.count) if tiles is not None else None,
             )  # fmt: skip
         else:

@@ -1427,3 +1427,18 @@ def test_latent_attention_keeps_what_is_no_number_near(ops, window, bad):
         if kernel == "tcgen05" and bool((~near).any()):
             assert not torch.isnan(got[~near]).any()
             assert float(((got - ref).abs() - bound)[~near].max()) <= 0.0
+
+
+@pytest.mark.parametrize("longest", [64, 65])
+def test_latent_attention_of_short_contexts_stays_with_mma(ops, longest):
+    q, cache, tables, ctx, ref, bound = paged_latent_case([longest, 3], [0, 20], 16, 576, 512, 16, 0, 2)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    outs = {}
+    for kernel, known in (("auto", longest), ("auto", None), ("tcgen05", longest), ("mma", None)):
+        out = outs[kernel, known] = torch.empty((longest + 3, 16 * 512), device="cuda", dtype=torch.bfloat16)
+        ops.latent_attention(
+            dev(q), out, dev(cache), dev(tables), i32([0, longest, longest + 3]), i32(ctx), 2, longest, 16, 576, 512, 576**-0.5, kernel=kernel, max_context=known,
+        )  # fmt: skip
+        assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
+    assert torch.equal(outs["auto", None], outs["tcgen05", longest]) and not torch.equal(outs["auto", None], outs["mma", None])
+    assert torch.equal(outs["auto", longest], outs["mma", None] if longest == 64 else outs["auto", None])
