@@ -542,6 +542,33 @@ def shaped_tcgen05_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, bias
     return tcgen05_attention_supported(dtype, nh, nkv, d, False) and (not biased or nh // max(nkv, 1) <= 8)
 
 
+def shaped_tcgen05_pays(d: int, g: int, nkv: int, num_seqs: int, num_tokens: int, max_q_len: int, keys: int, biased: bool) -> bool:
+    """Whether the tcgen05 kernel's form for shaped scores is the faster one for a step whose queries see at most ``keys`` keys;
+    ``g`` heads a key head.  A CTA of it takes 128 rows, has a start of 7 to 9 us and walks two tiles of 64 keys at a time; one of
+    the mma.sync kernel takes 64 rows, starts in 2 to 8 us and walks one, and twice as many run side by side.  So that one wins
+    where contexts are short, and where sequences bring so few tokens that the other's rows stay empty over more than one wave.
+
+    Microseconds a wave, fitted to five shapes (heads of 64 and 128, 1 to 8 heads a key head, with and without a bias) at 2 to
+    384 keys, 1 to 40 sequences and 2 tokens to whole prompts, both kernels timed (620 steps): the choice is never more than 9 %
+    slower than mma.sync alone, and 0.5 % on average slower than the better of the two.  Examples, tcgen05 / mma.sync, with a bias, 32
+    heads of 64 on 8: 64 tokens 10.0 / 8.2, 128 10.6 / 11.2, 256 15.1 / 17.6; 40 sequences of 2 tokens behind 190 29.2 / 20.4, of 32
+    tokens behind 160 28.2 / 31.4."""
+    wide, full = d > 64, max_q_len * g >= 16
+    pairs = -(-keys // 128)
+
+    def waves(rows: int, resident: int) -> int:
+        tile = max(1, rows // g)
+        return -(-nkv * min(num_seqs * -(-max_q_len // tile), num_tokens // tile + num_seqs) // (148 * resident))
+
+    if wide:
+        per_tile = (7.5, 5.2) if biased and full else (2.0, 9.0) if biased else (3.2, 6.6) if full else (2.5, 6.4)
+    else:
+        per_tile = (5.2, 3.0) if biased and full else (2.4, 5.8) if biased else (4.0, 2.65) if full else (2.5, 4.0)
+    tcgen05 = waves(128, 1 if wide else 2) * (8.8 + 4.8 * pairs if wide else 6.8 + 4.0 * pairs)
+    mma = waves(64, 2 if wide else 4) * (per_tile[0] + per_tile[1] * keys / 64)
+    return tcgen05 <= 1.02 * mma
+
+
 def tma_decode_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, block_size: int, num_blocks: int) -> bool:
     """Whether the TMA decode kernel (``csrc/attention_decode_tma.cu``) takes this shape."""
     return (
@@ -599,7 +626,8 @@ def paged_attention(
     ``q``: rows of ``q_stride`` elements whose first ``nh*d`` are the query heads; ``out``:
     ``[N, nh*d]``.  With ``scratch`` (and every sequence holding one query) the decode form
     runs: key ranges of ``split_size`` in parallel, then a merge; ``max_context`` bounds the
-    contexts.  ``kernel``: ``"auto"`` takes, for bfloat16, the tcgen05 kernel (many queries, head
+    contexts.  Without ``scratch`` it is optional: the longest context, from which "auto" chooses the
+    kernel of shaped scores (``shaped_tcgen05_pays``).  ``kernel``: ``"auto"`` takes, for bfloat16, the tcgen05 kernel (many queries, head
     size 64) or the mma.sync kernel (decode form; head size 128) and the FP32-pipe kernel
     elsewhere; ``"generic"``, ``"mma"``, ``"tma"`` and ``"tcgen05"`` force one (tests).  ``err``: the
     device error flag (a bounded wait inside a kernel raises it).  ``cluster``: the TMA decode kernel
@@ -718,6 +746,9 @@ def paged_attention(
         biased_mma and use_tc and shaped_tcgen05_supported(q.dtype, nh, nkv, d, bias is not None) and q.data_ptr() % 16 == 0
         and out.data_ptr() % 16 == 0 and num_seqs <= 65535 and max_q_len <= 65535 * tcgen05_query_tile(nh, nkv)
     )  # fmt: skip
+    if use_shaped and kernel == "auto" and max_context is not None and scratch is None:
+        span = abs(window) + TC_ATTN_ROWS + keep_first if window else max_context
+        use_shaped = shaped_tcgen05_pays(d, nh // nkv, nkv, num_seqs, q.shape[0], max_q_len, min(max_context, span), bias is not None)
     use_tma = tickets is not None and tma_decode_supported(q.dtype, nh, nkv, d, block_size, kcache.shape[0])
     # decoding with such scores: the TMA kernel's form for them (64 sequences of 32 heads of 64 on 8, contexts of 1,150 to 2,300 under a
     # window of 1,024, with a bias and 64 kept keys: 37.3 us, 55.8 us on the mma.sync split kernel)

@@ -392,6 +392,8 @@ class PagedAttention(Mixer):
             elif tiles.multi_count > 0:
                 ops.paged_attention(*args, ctx.max_query_len, *shape, query_tiles=(tiles.multi, tiles.multi_count), **common)
             return
+        if scratch is None and not ctx.context_bound:
+            bound = ctx.max_context_len  # (a captured step is made for longer contexts and more tiles than it may have)
         ops.paged_attention(
             *args, ctx.max_query_len, *shape, scratch=scratch, max_context=bound, split_size=split,
             cluster=ctx.num_seqs * self.nkv <= CLUSTER_MERGE_MAX_PAIRS, wave_target=wave if scratch is not None else 0,

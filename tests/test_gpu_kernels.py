@@ -1442,3 +1442,14 @@ def test_latent_attention_of_short_contexts_stays_with_mma(ops, longest):
         assert float(((out.cpu().double() - ref).abs() - bound).max()) <= 0.0
     assert torch.equal(outs["auto", None], outs["tcgen05", longest]) and not torch.equal(outs["auto", None], outs["mma", None])
     assert torch.equal(outs["auto", longest], outs["mma", None] if longest == 64 else outs["auto", None])
+
+
+@pytest.mark.parametrize("n,longest", [(3, 3), (40, 60), (200, 300)])
+def test_shaped_scores_of_short_contexts_choose_their_kernel(ops, n, longest):
+    case = (64, 8, 2, 16, 0, 0, 50, 5.0, False, [n, 1], [longest - n, 0])
+    auto, over = run_shaped(ops, *case, max_context=longest)
+    assert over <= 0.0, over
+    pays = ops.shaped_tcgen05_pays(64, 4, 2, 2, n + 1, n, longest, True)
+    assert pays == (longest == 300)
+    assert torch.equal(auto, run_shaped(ops, *case, kernel="tcgen05" if pays else "mma")[0])
+    assert torch.equal(run_shaped(ops, *case, kernel="tcgen05", max_context=longest)[0], run_shaped(ops, *case)[0])

@@ -285,9 +285,31 @@ def test_shaped_scores_keep_the_ranges_of_the_launch(monkeypatch):
             calls.clear()
             ctx = SimpleNamespace(
                 block_tables=[None], query_start_loc=None, context_lens=None, num_seqs=4, max_query_len=1 if single else 9, block_size=16,
-                all_single_query=single, query_tiles={} if single else {32: tiles},
+                all_single_query=single, query_tiles={} if single else {32: tiles}, context_bound=0, max_context_len=50,
             )  # fmt: skip
             part.attend(ctx, q, 512, None, cache)
             ranges = [kw for kw in calls if kw.get("scratch") is not None]
             assert len(ranges) == (1 if single or dtype == torch.bfloat16 else 0)
             assert all((kw["wave_target"] > 0) == lengthens for kw in ranges), shape
+
+
+def test_kernel_of_shaped_scores_by_the_times_of_both():
+    """Steps of many sequences, few tokens, short and long contexts: (head size, heads a key head, key heads, sequences, tokens each,
+    longest context, with a bias, us on the mma.sync kernel, us on the tcgen05 kernel), as timed.  The chosen kernel takes at most
+    a tenth more than the mma.sync kernel and at most a fifth more than the better of the two."""
+    from kvforge_b200 import ops
+
+    timed = [
+        (64, 4, 8, 1, 2, 2, True, 5.5, 9.8), (64, 4, 8, 1, 64, 64, True, 8.2, 10.0), (64, 4, 8, 1, 128, 128, True, 11.2, 10.6),
+        (64, 4, 8, 1, 256, 256, True, 17.6, 15.1), (64, 4, 8, 40, 2, 384, True, 38.3, 39.9), (64, 4, 8, 40, 32, 192, True, 31.4, 28.2),
+        (64, 4, 8, 40, 40, 40, True, 19.8, 28.3), (64, 4, 8, 8, 192, 192, True, 28.4, 23.7), (64, 4, 8, 4, 2, 256, True, 25.7, 15.8),
+        (64, 8, 4, 8, 32, 256, True, 18.3, 15.4), (64, 8, 4, 1, 32, 192, True, 14.7, 14.3), (64, 8, 4, 8, 2, 80, True, 9.6, 11.2),
+        (64, 1, 16, 20, 32, 80, False, 10.9, 21.0), (64, 1, 16, 40, 32, 384, False, 43.5, 60.4), (64, 1, 16, 4, 384, 384, False, 25.0, 19.8),
+        (128, 3, 8, 20, 2, 80, False, 14.1, 25.8), (128, 3, 8, 40, 32, 64, False, 28.5, 33.4), (128, 3, 8, 4, 384, 384, False, 88.7, 47.6),
+        (128, 3, 8, 4, 2, 192, False, 21.6, 17.5), (128, 4, 4, 1, 2, 256, True, 35.9, 20.6), (128, 4, 4, 4, 32, 128, True, 17.7, 13.6),
+        (128, 4, 4, 20, 40, 40, True, 12.0, 23.6), (128, 4, 4, 20, 2, 384, True, 56.5, 24.8), (64, 4, 8, 1, 2048, 2048, True, 148.9, 76.2),
+    ]  # fmt: skip
+    for d, g, nkv, seqs, n, keys, biased, mma, tcgen05 in timed:
+        took = tcgen05 if ops.shaped_tcgen05_pays(d, g, nkv, seqs, seqs * n, n, keys, biased) else mma
+        assert took <= 1.1 * mma and took <= 1.2 * min(mma, tcgen05), (d, g, seqs, n, keys, took)
+    assert ops.shaped_tcgen05_pays(64, 4, 8, 2, 2048, 1536, 2048, True) and ops.shaped_tcgen05_pays(64, 128, 1, 1, 40, 40, 4096, False)
