@@ -21,9 +21,9 @@
 // column, R rows each in registers; records come through a ring in shared memory by cp.async, one barrier a group.
 // Groups start at a step's first token of the sequence; a last group is filled up with tokens of zero keys and beta.
 //
-// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 630 us by the walk, 535 here (both kernels), 24 heads
-// over 1,500 920 and 487, 8 heads with a decay a head 449 and 352; 61 sequences of which one brings 40 tokens 165 and 92.  Against
-// 64-bit the outputs are off by 1.28e-7 of their norm by the walk, 1.20e-7 here.  A group is some 430 instructions a warp on its
+// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 630 us by the walk, 605 here (both kernels), 24 heads
+// over 1,500 920 and 521, 8 heads with a decay a head 449 and 353; 61 sequences of which one brings 40 tokens 165 and 93.  Against
+// 64-bit the outputs are off by 1.28e-7 of their norm by the walk, 1.16e-7 here.  A group is some 430 instructions a warp on its
 // way to the next state, and the latency of the shuffles and of the triangle between them.  Heads of at most 64 rows and of
 // more than 128 keep the walk: 4 x 64 over 700 tokens 148 us by the walk and 160 here, 3 x 32 over 131 35 and 57, 2 x 256 over 333 91
 // and 92: a narrow head's link is short already, a wide one's 16 rows a lane are all instructions.
@@ -84,8 +84,10 @@ __device__ __forceinline__ double dg_warp_sum(double v) {
 
 // The norms and the products of decays are made in double, so that an entry of a record is rounded once: a walk token by token
 // rounds a decayed state where a record holds decayed keys, and with float factors (one rounding more a token of the
-// group) outputs were 0.2 to 7 % further off against 64 bits than the walk's.  Outputs are 0.89 to 1.01 of the walk's error so, the
-// state's between 0.95 and 1.07, 1.00 on average; 16 heads with a decay a channel over 2,048 tokens 513 us with float factors, 535 so.
+// group) outputs were 0.2 to 7 % further off against 64 bits than the walk's, the state up to 14 %.  With what is taken from a value
+// summed first (below) outputs are 0.82 to 1.02 of the walk's error, the state 0.86 to 1.00 (six seeds each of five shapes and three
+// rates of decay; where a state hardly decays both sides are off by the decays' own rounding).  16 heads with a decay a channel over
+// 2,048 tokens: 513 us with float factors, 535 with double ones, 605 with the other order too; with a decay a head 440, 447 and 450.
 template <bool CH>
 __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaParams p, int nseq) {
   pdl_launch();
@@ -348,11 +350,13 @@ __global__ void __launch_bounds__(DG_THREADS) delta_groups_kernel(const DeltaPar
       a[0] *= cc.x; a[1] *= cc.y; a[2] *= cc.z; a[3] *= cc.w;
     }
     float u[DG_TOKENS];
-    u[0] = beta.x * (to_float<T>(vv[0]) - a[0]);
-    const float r1 = to_float<T>(vv[1]) - a[1], r2 = fmaf(-A0.y, u[0], to_float<T>(vv[2]) - a[2]), r3 = fmaf(-A0.w, u[0], to_float<T>(vv[3]) - a[3]);
-    u[1] = beta.y * fmaf(-A0.x, u[0], r1);
-    u[2] = beta.z * fmaf(-A0.z, u[1], r2);
-    u[3] = beta.w * fmaf(-A1.y, u[2], fmaf(-A1.x, u[1], r3));
+    // what is taken from a value is summed first: the sums are small beside it, and so is what they are rounded by
+    const float v0 = beta.x * to_float<T>(vv[0]), v1 = beta.y * to_float<T>(vv[1]), v2 = beta.z * to_float<T>(vv[2]), v3 = beta.w * to_float<T>(vv[3]);
+    u[0] = fmaf(-beta.x, a[0], v0);
+    const float a2 = fmaf(A0.y, u[0], a[2]), a3 = fmaf(A0.w, u[0], a[3]);
+    u[1] = fmaf(-beta.y, fmaf(A0.x, u[0], a[1]), v1);
+    u[2] = fmaf(-beta.z, fmaf(A0.z, u[1], a2), v2);
+    u[3] = fmaf(-beta.w, fmaf(A1.y, u[2], fmaf(A1.x, u[1], a3)), v3);
     // the write: sums over the rows of different lanes and pairs, so the tokens go outside
     uint64_t uu[DG_TOKENS];
     uu[0] = dg_pack(u[0] * cs.x, u[0] * cs.x);
@@ -430,7 +434,7 @@ int dispatch_delta_groups(const DeltaParams& p, int B, cudaStream_t st) {
   const dim3 grid((unsigned)((warps + 3) / 4));
   const int rc = launch(delta_group_prepare_kernel<CH>, grid, dim3(128), 0, st, p, B);
   if (rc) return rc;
-  // (Figures here are those with float factors in the records; double ones add some 4 % to either side.)
+  // (Figures here are from before the records' factors were double and the order of the sums below.)
   // What counts for a few long sequences is a short link (16 lanes a column: 16 heads of 128 x 128 over 2,048 tokens 513 us against
   // 506, 24 heads over 1,500 464 against 538, 8 x 256 tokens of 16 heads 348 against 388; with a decay a head 349 against 465 for
   // 8 heads); once every SM has more than a dozen CTAs to work off it is the number of instructions (8 lanes: 50 x 40 tokens of 16
