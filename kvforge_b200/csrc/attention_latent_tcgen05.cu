@@ -3,8 +3,9 @@
 // attention_latent.cu.
 //
 // A CTA serves 128 rows, a row being a (query token, head) pair (128 / nh tokens, every head), and up to 256 value columns: with
-// values of 512 two CTAs share the rows' work, both making the scores.  That costs (d + 256) products a pair of row and key
-// where 2 x (d + 512) / 2 would do, but the accumulator of 128 x 512 alone is all of an SM's tensor memory.  Per tile of 128 keys:
+// values of 512 two CTAs share the rows' work, both making the scores.  That costs 2 x (d + 256) products a pair of row and key where
+// d + 512 would do (1,664 and 1,088 for d = 576), but the accumulator of 128 x 512 alone is all of an SM's tensor memory.  Per tile
+// of 128 keys:
 //   S = Q K^T   tcgen05.mma 128 x 128 x 16, d/16 of them.  The first (up to four) blocks of 64 query numbers lie in tensor memory
 //               as the A operand (128 columns): 80 KB of queries and 144 KB of keys are what an SM holds;
 //   softmax     two groups of four warps, 64 keys of a row a thread, from tensor memory, as in attention_tcgen05.cu (the two

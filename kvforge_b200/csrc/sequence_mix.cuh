@@ -11,8 +11,10 @@
 // Everything a recurrence reads besides the projections (decays, step sizes, unit norms, the state
 // itself) is float whatever the storage type T is.  Every sum has a fixed order that depends on the
 // sizes alone, so token by token (32-bit storage) a token's result does not depend on how its sequence
-// was cut into steps or on what else the step holds; in bfloat16 a step that holds a sequence of more than
-// four tokens may go four at a time, which shows in the last bits of a float.
+// was cut into steps or on what else the step holds.  In bfloat16 a step goes four tokens at a time when the
+// longest run of tokens it is launched for has more than four, in groups from the step's first token of a sequence on;
+// a captured step of many tokens is launched for runs of all of them, so it always does.  The last bits of
+// a float, in outputs and states, then follow the cut, the step's other sequences and whether it was captured.
 #pragma once
 #include "sequence_common.cuh"
 
