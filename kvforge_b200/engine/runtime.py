@@ -45,7 +45,7 @@ class Runtime:
         return self._side
 
     def buf(self, name: str, rows: int, cols: int, dtype: torch.dtype | None = None, cap: int | None = None) -> torch.Tensor:
-        """A ``[rows, cols]`` view of the persistent buffer ``name`` (contents undefined).
+        """A ``[rows, cols]`` view of the persistent buffer ``name`` (contents undefined: zeros, or what earlier steps left).
         It is made for ``cap`` rows (default: the token budget of a step) and grows if more
         are asked for."""
         dtype = dtype or self.dtype
@@ -58,7 +58,9 @@ class Runtime:
                 cap = 1 << max(4, (max(rows, 1) - 1).bit_length())
             else:
                 cap = max(rows, self.max_tokens if cap is None else cap)
-            t = torch.empty((cap, cols), dtype=dtype, device=self.device)
+            # zeros once: kernels leave rows alone that belong to no sequence, and a part that mixes the rows of a padded step
+            # (with weights of zero) must not meet what the memory held before
+            t = torch.zeros((cap, cols), dtype=dtype, device=self.device)
             self._buffers[key] = t
         return t[:rows]
 

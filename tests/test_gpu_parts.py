@@ -387,6 +387,14 @@ def test_a_toy_mixer_with_state_is_registered_built_and_stepped(tmp_path):
         unregister_architecture("ToyStateForCausalLM")
 
 
+def test_rows_of_padding_are_numbers_whatever_the_memory_held(tmp_path):
+    """The same with free memory full of NaN: a padded step's rows that belong to no sequence are multiplied by zero in the toy mixer."""
+    for size in (1 << 9, 1 << 12, 1 << 15, 1 << 18, 1 << 21, 1 << 24):
+        junk = [torch.full((size,), float("nan"), device="cuda") for _ in range(12)]
+        del junk
+    test_a_toy_mixer_with_state_is_registered_built_and_stepped(tmp_path)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_the_toy_mixers_state_survives_graphs_chunked_prefill_and_preemption_in_the_engine(tmp_path, dtype):
     """The same toy model through ``InferenceEngine`` with CUDA graphs: prompts cut into portions
