@@ -21,8 +21,8 @@
 // column, R rows each in registers; records come through a ring in shared memory by cp.async, one barrier a group.
 // Groups start at a step's first token of the sequence; a last group is filled up with tokens of zero keys and beta.
 //
-// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 630 us by the walk, 605 here (both kernels), 24 heads
-// over 1,500 920 and 521, 8 heads with a decay a head 449 and 353; 61 sequences of which one brings 40 tokens 165 and 93.  Against
+// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 630 us by the walk, 530 here (both kernels), 24 heads
+// over 1,500 920 and 498, 8 heads with a decay a head 449 and 351; 61 sequences of which one brings 40 tokens 165 and 89.  Against
 // 64-bit the outputs are off by 1.28e-7 of their norm by the walk, 1.16e-7 here.  A group is some 430 instructions a warp on its
 // way to the next state, and the latency of the shuffles and of the triangle between them.  Heads of at most 64 rows and of
 // more than 128 keep the walk: 4 x 64 over 700 tokens 148 us by the walk and 160 here, 3 x 32 over 131 35 and 57, 2 x 256 over 333 91
@@ -87,7 +87,7 @@ __device__ __forceinline__ double dg_warp_sum(double v) {
 // group) outputs were 0.2 to 7 % further off against 64 bits than the walk's, the state up to 14 %.  With what is taken from a value
 // summed first (below) outputs are 0.82 to 1.02 of the walk's error, the state 0.86 to 1.00 (six seeds each of five shapes and three
 // rates of decay; where a state hardly decays both sides are off by the decays' own rounding).  16 heads with a decay a channel over
-// 2,048 tokens: 513 us with float factors, 535 with double ones, 605 with the other order too; with a decay a head 440, 447 and 450.
+// 2,048 tokens: 513 us with float factors, 530 so; with a decay a head 440 and 448.
 template <bool CH>
 __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaParams p, int nseq) {
   pdl_launch();
@@ -233,8 +233,12 @@ __global__ void __launch_bounds__(128) delta_group_prepare_kernel(const DeltaPar
 }
 
 // ---- the walk over the groups
+// Four CTAs an SM: 124 to 128 registers a thread.  Without a bound the compiler takes 90 to 168 and, where it takes 90, puts the
+// record's reads where the chain waits for them (16 heads of 128 with a decay a channel over 2,048 tokens 605 us, with it 530; 8 heads
+// 438 and 363; 8 sequences of 256 tokens and 8 heads with a decay a head 211 and 166); a bound of one or two gives 136 to 186 and is
+// 355 for those 8 heads, but 394 instead of 331 for 50 x 40 tokens, whose CTAs want to share an SM.
 template <typename T, int KS, int R, bool CH>
-__global__ void __launch_bounds__(DG_THREADS) delta_groups_kernel(const DeltaParams p) {
+__global__ void __launch_bounds__(DG_THREADS, 4) delta_groups_kernel(const DeltaParams p) {
   pdl_launch();
   pdl_wait();
   static_assert(KS * R == DG_ROWS && KS >= 8, "eight sums a column are shared out over the lanes");
