@@ -12,8 +12,8 @@
 // itself) is float whatever the storage type T is.  Every sum has a fixed order that depends on the
 // sizes alone, so token by token (32-bit storage) a token's result does not depend on how its sequence
 // was cut into steps or on what else the step holds.  In bfloat16 a step goes four tokens at a time when the
-// longest run of tokens it is launched for has more than four, in groups from the step's first token of a sequence on;
-// a captured step of many tokens is launched for runs of all of them, so it always does.  The last bits of
+// longest run of tokens it is launched for has more than four, and sixty-four at a time when its sequences are long, in groups or
+// chunks from the step's first token of a sequence on; a captured step of many tokens is launched for runs of all of them.  The last bits of
 // a float, in outputs and states, then follow the cut, the step's other sequences and whether it was captured.
 #pragma once
 #include "sequence_common.cuh"
@@ -31,7 +31,7 @@ namespace {
 // with k and q made unit vectors per head (x / sqrt(sum x^2 + norm_eps)), q times q_scale,
 // beta = sigmoid(b), g = exp(-exp(A_log[h]) * softplus(a + dt_bias)).
 //
-// (Many tokens a sequence in bfloat16 storage are walked four at a time: delta_groups.cuh.)
+// (Many tokens a sequence in bfloat16 storage go four or sixty-four at a time: delta_groups.cuh, delta_chunks.cuh.)
 // The walk over a sequence's tokens is a chain: a token's update needs the state the token before
 // left.  What bounds it is the latency of one link, so a link is made short.  A CTA owns a sequence,
 // a head and a tile of columns of S; a column's rows are spread over KS neighbouring lanes, R rows
@@ -80,6 +80,8 @@ struct DeltaParams {
   long long logit_slice_stride;
   // the records of groups of four tokens (delta_groups.cuh), or null: token by token
   float* groups;
+  // the records of chunks of sixty-four tokens (delta_chunks.cuh), or null
+  float* chunks;
 };
 
 // exp(rate * softplus(x)), rate < 0: exact library functions in 32-bit storage; in bfloat16 storage the fast
@@ -152,6 +154,7 @@ __device__ __forceinline__ void cp_async16(float* smem_dst, const float* gsrc) {
 }  // namespace
 
 #include "delta_groups.cuh"
+#include "delta_chunks.cuh"
 
 namespace {
 
@@ -404,6 +407,7 @@ int dispatch_delta(const DeltaParams& p, int B, int max_q_len, cudaStream_t st) 
   if constexpr (sizeof(T) == 2) {
     // four tokens a link where a sequence brings more than that; 32-bit storage walks token by token, so that its sums
     // do not depend on how a sequence was cut
+    if (p.chunks) return p.per_channel ? dispatch_delta_chunks<true>(p, B, st) : dispatch_delta_chunks<false>(p, B, st);
     if (p.groups) return p.per_channel ? dispatch_delta_groups<T, true>(p, B, st) : dispatch_delta_groups<T, false>(p, B, st);
   }
   int rc = launch(delta_prepare_kernel<T>, dim3((unsigned)((pairs + 3) / 4)), dim3(128), 0, st, p);
@@ -452,6 +456,7 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
                                     int G, int dk, int dv, float q_scale, float norm_eps, int max_q_len, int N,        \
                                     float* kn, float* qn, float* gn, float* sc, int logit_slices,                      \
                                     long long logit_slice_stride, float* groups, long long groups_floats,              \
+                                    float* chunks, long long chunks_floats,                                            \
                                     cudaStream_t st) {                                                                 \
     if (B <= 0) return 0;                                                                                              \
     if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || (unsigned)H > 65535u) return (int)cudaErrorInvalidValue;    \
@@ -462,7 +467,12 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
     p.H = H; p.G = G; p.dk = dk; p.dv = dv; p.q_scale = q_scale; p.norm_eps = norm_eps; p.chunk = 1; p.buf_floats = 0;  \
     p.kn = kn; p.qn = qn; p.gn = gn; p.sc = sc; p.N = N;                                                               \
     p.logit_slices = logit_slices; p.logit_slice_stride = logit_slice_stride; p.groups = groups;                       \
-    if (groups) {                                                                                                      \
+    p.chunks = chunks;                                                                                                 \
+    if (chunks) {                                                                                                      \
+      if (sizeof(T) != 2 || groups || dk <= 64 || dk > DC_ROWS || (dv & 3) || (out_stride & 3) ||                      \
+          ((((uintptr_t)chunks) | ((uintptr_t)out)) & 15) || chunks_floats < ((long long)N / DC_T + B) * H * dc_record(dv)) \
+        return (int)cudaErrorInvalidValue;                                                                             \
+    } else if (groups) {                                                                                                      \
       if (sizeof(T) != 2 || dk <= 64 || dk > DG_ROWS || max_q_len <= DG_TOKENS || (((uintptr_t)groups) & 15) ||                        \
           groups_floats < ((long long)N / DG_TOKENS + B) * H * dg_record(per_channel != 0))                            \
         return (int)cudaErrorInvalidValue;                                                                             \

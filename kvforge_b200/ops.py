@@ -44,7 +44,7 @@ _SIGNATURES = {
     "kvf_causal_conv_{s}": "pippplppiiiiipiip",
     "kvf_conv_set_pdl": "i",
     # libraries "mixers" and "streams"
-    "kvf_gated_delta_{s}": "pppipipippiplpippiiiiiffiippppilplp",
+    "kvf_gated_delta_{s}": "pppipipippiplpippiiiiiffiippppilplplp",
     "kvf_gated_head_norm_{s}": "pipipfiliipip",
     "kvf_hc_step_{s}": "pppilppppppiiifp",
     "kvf_branch_norm_mean_{s}": "pppppilifppp",
@@ -1332,12 +1332,35 @@ def delta_group_floats(n: int, num_seqs: int, num_heads: int, per_channel: bool)
     return (n // DELTA_GROUP_TOKENS + num_seqs) * delta_group_record(num_heads, per_channel)
 
 
+DELTA_CHUNK_TOKENS = 64
+
+
+def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, per_channel: bool, n: int, num_seqs: int, max_query_len: int) -> bool:
+    """Whether a step of the delta rule goes sixty-four tokens at a time rather than four.  A chunk costs about the same however
+    few of its tokens there are, so the step needs long sequences and few short ones beside them.  Groups of four and chunks, us,
+    16 heads of 128 x 128 with a decay a channel: one sequence of 256 tokens 71 and 68, of 512 133 and 84, of 2,048 525 and 276; 8 of
+    256 386 and 291; 1,000 and 8 single tokens 373 and 301, 400 and 20 219 and 323; 30 of 64 307 and 362.  8 heads with a decay a head:
+    one of 256 55 and 69, of 384 75 and 75, of 1,024 181 and 108."""
+    few = 256 if per_channel else 384
+    return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= 384 and n >= 96 * num_seqs
+
+
+def delta_chunk_record(num_heads: int, dv: int) -> int:
+    """Floats that a chunk of tokens takes: per head 28,800 and the columns of 64 tokens and of a state."""
+    return num_heads * (28800 + (DELTA_CHUNK_TOKENS + 128) * dv)
+
+
+def delta_chunk_floats(n: int, num_seqs: int, num_heads: int, dv: int) -> int:
+    """Floats of the records of ``n`` tokens in ``num_seqs`` sequences."""
+    return (n // DELTA_CHUNK_TOKENS + num_seqs) * delta_chunk_record(num_heads, dv)
+
+
 def gated_delta(
     q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logits: torch.Tensor, step_logits: torch.Tensor,
     a_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, out: torch.Tensor, qsl: torch.Tensor,
     state_slots: torch.Tensor, num_seqs: int, num_heads: int, num_kv_heads: int, dk: int, dv: int, q_scale: float,
     norm_eps: float = 1e-6, max_query_len: int = 0, scratch: tuple[torch.Tensor, ...] | None = None,
-    logit_slices: int = 0, logit_slice_stride: int = 0, groups: torch.Tensor | None = None,
+    logit_slices: int = 0, logit_slice_stride: int = 0, groups: torch.Tensor | None = None, chunks: torch.Tensor | None = None,
 ) -> None:  # fmt: skip
     """The gated delta rule over a flat batch, token by token per sequence, on the state
     ``S [heads, dk, dv]`` of each sequence's slot (``csrc/sequence_mix.cuh`` has the equations).
@@ -1352,6 +1375,9 @@ def gated_delta(
     they are allocated here (tests; a step of the engine passes persistent buffers).  Two launches.
     ``groups``: a float buffer of ``delta_group_floats`` numbers; the step then goes four tokens at a time (``delta_groups_ok``:
     bfloat16, 64 < dk <= 128, more than four rows of some sequence; ``csrc/delta_groups.cuh``) and needs no ``scratch``.
+    ``chunks``: a float buffer of ``delta_chunk_floats`` numbers on a 16-byte boundary; the step then goes sixty-four tokens at a time
+    (bfloat16, 64 < dk <= 128, dv and the rows of ``out`` multiples of four numbers; ``csrc/delta_chunks.cuh``; ``delta_chunks_ok`` says
+    when that is the faster form) and needs neither ``groups`` nor ``scratch``.  Three launches.
     ``logit_slices > 1``: ``beta_logits`` (and per-head ``step_logits``) are slice 0 of that many float
     slices of a split-K product, ``logit_slice_stride`` elements apart, summed in slice order."""
     s = _suffix(q.dtype)
@@ -1374,7 +1400,13 @@ def gated_delta(
     sptr, sstride = _state_view(state, h * dk * dv, "delta state")
     _need(qsl, torch.int32, "query_start_loc")
     _need(state_slots, torch.int32, "state_slots")
-    if groups is not None:
+    if chunks is not None:
+        _need(chunks, torch.float32, "delta chunks")
+        fits = q.dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and out.stride(0) % 4 == 0 and (out.data_ptr() | chunks.data_ptr()) % 16 == 0
+        if not fits or groups is not None or chunks.numel() < delta_chunk_floats(n, num_seqs, h, dv):
+            raise ValueError("gated_delta: the step does not go in chunks, or their buffer is too small")
+        scratch = (None, None, None, None)
+    elif groups is not None:
         _need(groups, torch.float32, "delta groups")
         if not delta_groups_ok(q.dtype, dk, max_query_len) or groups.numel() < delta_group_floats(n, num_seqs, h, per_channel):
             raise ValueError("gated_delta: the step does not go in groups, or their buffer is too small")
@@ -1384,7 +1416,7 @@ def gated_delta(
         scratch = (mk(h * dk), mk(h * dk), mk(h * dk) if per_channel else None, mk(h * 4))
     kn, qn, gn, sc = scratch
     for t, w, what in ((kn, h * dk, "kn"), (qn, h * dk, "qn"), (gn, h * dk, "gn"), (sc, h * 4, "sc")):
-        if groups is not None or (t is None and what == "gn" and not per_channel):
+        if groups is not None or chunks is not None or (t is None and what == "gn" and not per_channel):
             continue
         _need(t, torch.float32, f"scratch {what}")
         if tuple(t.shape) != (n, w):
@@ -1396,10 +1428,10 @@ def gated_delta(
             step_logits.stride(0), _ptr(a_log), _ptr(dt_bias), 1 if per_channel else 0, sptr, sstride, _ptr(out),
             out.stride(0), _ptr(qsl), _ptr(state_slots), num_seqs, h, g, dk, dv, float(q_scale), float(norm_eps), int(max_query_len),
             n, _ptr(kn), _ptr(qn), _ptr(gn) if per_channel else None, _ptr(sc), int(logit_slices), int(logit_slice_stride),
-            _ptr(groups), groups.numel() if groups is not None else 0, _stream(),
+            _ptr(groups), groups.numel() if groups is not None else 0, _ptr(chunks), chunks.numel() if chunks is not None else 0, _stream(),
         ),
         name,
-        2,
+        2 if chunks is None else 3,
     )  # fmt: skip
 
 

@@ -187,9 +187,14 @@ class GatedDeltaRule(Mixer):
             gate = main[:, self.off_gate : self.off_gate + self.c_v]
         read = rt.buf("delta.read", n, self.c_v, torch.float32)
         f32 = torch.float32
-        scratch = groups = None
-        if ops.delta_groups_ok(rt.dtype, dk, ctx.max_query_len):
-            # many tokens in bfloat16: four at a time, from records of the groups
+        scratch = groups = chunks = None
+        if ops.delta_chunks_ok(rt.dtype, dk, dv, self.decay == "channel", n, ctx.num_seqs, ctx.max_query_len):
+            # many tokens a sequence in bfloat16: sixty-four at a time, from records of the chunks
+            per = ops.DELTA_CHUNK_TOKENS
+            record = ops.delta_chunk_record(H, dv)
+            chunks = rt.buf("delta.chunks", n // per + ctx.num_seqs, record, f32, cap=rt.max_tokens // per + max(rt.max_seqs, ctx.num_seqs))
+        elif ops.delta_groups_ok(rt.dtype, dk, ctx.max_query_len):
+            # a few tokens a sequence: four at a time, from records of the groups
             per = ops.DELTA_GROUP_TOKENS
             record = ops.delta_group_record(H, self.decay == "channel")
             groups = rt.buf("delta.groups", n // per + ctx.num_seqs, record, f32, cap=rt.max_tokens // per + max(rt.max_seqs, ctx.num_seqs))
@@ -201,7 +206,7 @@ class GatedDeltaRule(Mixer):
             qkv[:, : self.c_q], qkv[:, self.c_q : 2 * self.c_q], qkv[:, 2 * self.c_q :], small[:, :H], step, self.a_log, self.dt_bias,
             cache.state[:, self.conv_floats :], read, ctx.query_start_loc, ctx.state_slots, ctx.num_seqs, H, self.G, dk, dv,
             q_scale=dk**-0.5, norm_eps=1e-6, max_query_len=ctx.max_query_len, scratch=scratch,
-            logit_slices=slices if slices > 1 else 0, logit_slice_stride=slice_stride, groups=groups,
+            logit_slices=slices if slices > 1 else 0, logit_slice_stride=slice_stride, groups=groups, chunks=chunks,
         )  # fmt: skip
         y = rt.buf("delta.y", n, self.c_v)
         ops.gated_head_norm(read, gate, self.norm_w, self.eps, y, H, dv, activation=self.gate)

@@ -449,6 +449,87 @@ def test_gated_delta_rule_in_groups_of_four(h, g, dk, dv, channel, rate):
     assert float(state[1].abs().max()) == 0 and float(state[3].abs().max()) == 0 and float(state[:, :3].abs().max()) == 0
 
 
+@pytest.mark.parametrize("rate", [-4.0, 0.0, 3.0])
+@pytest.mark.parametrize("h,g,dk,dv,channel", [(2, 2, 128, 128, True), (2, 1, 128, 32, False), (3, 1, 65, 36, True), (2, 1, 100, 4, False), (1, 1, 96, 260, True)])
+def test_gated_delta_rule_in_chunks(h, g, dk, dv, channel, rate):
+    """The form that takes sixty-four tokens at a time: chunks of 1, 15 .. 17, 63 and 64 tokens, every block boundary, both widths of
+    the chain's tiles, sequences of one token and of none, a padding sequence without a slot, two steps of which the second finds a
+    used state; what a token brings that is no number reaches no earlier token and no other sequence."""
+    from kvforge_b200 import ops
+
+    dev, dt = "cuda", torch.bfloat16
+    gen = torch.Generator().manual_seed(dk + dv)
+    steps = ([65, 1, 0, 17, 64], [15, 130, 0, 63, 16])
+    slots = [2, 5, 1, 0, 4]
+    aw = h * dk if channel else h
+    a_log, dt_bias = rate + 0.5 * torch.randn(h, generator=gen), 0.5 * torch.randn(aw, generator=gen)
+    state = torch.zeros(6, 4 + h * dk * dv, device=dev)
+    seqs, got = [[] for _ in slots], [[] for _ in slots]
+    for k, ls in enumerate(steps):
+        n = sum(ls)
+        qkv, b, a = torch.randn(n, 2 * g * dk + h * dv, generator=gen).to(dt), torch.randn(n, h, generator=gen), torch.randn(n, aw, generator=gen)
+        at = 0
+        for i, m in enumerate(ls):
+            seqs[i].append(tuple(t[at : at + m] for t in (qkv.float(), b, a)))
+            at += m
+        pad = lambda t: torch.cat([t, torch.full((3, t.shape[1]), float("nan"), dtype=t.dtype)]).to(dev)  # noqa: E731  rows beyond the last sequence
+        qsl, sl = flat_batch(ls + [0], slots + [-1], dev)
+        chunks = torch.full((ops.delta_chunk_floats(n + 3, 6, h, dv),), float("nan"), device=dev)
+
+        def run(x, to, out):
+            ops.gated_delta(
+                x[:, : g * dk], x[:, g * dk : 2 * g * dk], x[:, 2 * g * dk :], pad(b), pad(a), a_log.to(dev), dt_bias.to(dev), to[:, 4:], out, qsl, sl, 6,
+                h, g, dk, dv, q_scale=dk**-0.5, max_query_len=max(ls), chunks=chunks,
+            )  # fmt: skip
+
+        bad, at = pad(qkv), sum(ls[:3]) + 5  # a token of the fourth sequence
+        bad[at, g * dk :] = float("nan")
+        clean, spoilt, before = torch.full((n + 3, h * dv), -7.0, device=dev), torch.full((n + 3, h * dv), -7.0, device=dev), state.clone()
+        run(bad, before, spoilt)
+        run(pad(qkv), state, clean)
+        others = [t for t in range(n) if t < at or t >= sum(ls[:4])]
+        assert torch.equal(spoilt[others], clean[others]) and spoilt[at : sum(ls[:4])].isnan().all()
+        assert (clean[n:] == -7.0).all() and torch.equal(before[[1, 2, 3, 4, 5]], state[[1, 2, 3, 4, 5]])
+        at = 0
+        for i, m in enumerate(ls):
+            got[i].append(clean[at : at + m].cpu())
+            at += m
+    for i, parts in enumerate(seqs):
+        qkv, b, a = (torch.cat([p[j] for p in parts]).double() for j in range(3))
+        n = qkv.shape[0]
+        if n == 0:
+            continue
+        q = (plain.unit(qkv[:, : g * dk].view(n, g, dk)) * dk**-0.5).repeat_interleave(h // g, 1)
+        k = plain.unit(qkv[:, g * dk : 2 * g * dk].view(n, g, dk)).repeat_interleave(h // g, 1)
+        decay = torch.exp(-torch.exp(a_log.double()).repeat_interleave(dk if channel else 1) * F.softplus(a + dt_bias.double()))
+        want = plain.delta_rule(q, k, qkv[:, 2 * g * dk :].view(n, h, dv), torch.sigmoid(b), decay.view(n, h, dk) if channel else decay).reshape(n, h * dv)
+        # 32-bit sums and the rounding of the decays, as for the walk token by token
+        assert torch.allclose(torch.cat(got[i]).double(), want, atol=5e-5, rtol=5e-4), (i, float((torch.cat(got[i]).double() - want).abs().max()))
+    assert float(state[1].abs().max()) == 0 and float(state[3].abs().max()) == 0 and float(state[:, :4].abs().max()) == 0
+
+
+def test_delta_chunks_refuse_what_they_do_not_take():
+    from kvforge_b200 import ops
+
+    dev, h, dk, dv, n = "cuda", 2, 128, 32, 70
+    x = torch.zeros(n, 2 * h * dk + h * dv, device=dev, dtype=torch.bfloat16)
+    b, state, out = torch.zeros(n, h, device=dev), torch.zeros(1, h * dk * dv, device=dev), torch.zeros(n, h * dv, device=dev)
+    qsl, sl = flat_batch([n], [0], dev)
+
+    def run(width, chunks, to=out):
+        y = x[:, : 2 * h * width + h * dv]
+        ops.gated_delta(
+            y[:, : h * width], y[:, h * width : 2 * h * width], y[:, 2 * h * width :], b, b, b[0].contiguous(), b[0].contiguous(),
+            state[:, : h * width * dv], to, qsl, sl, 1, h, h, width, dv, q_scale=1.0, max_query_len=n, chunks=chunks,
+        )  # fmt: skip
+
+    room = torch.zeros(ops.delta_chunk_floats(n, 1, h, dv) + 4, device=dev)
+    run(dk, room)
+    for width, chunks in ((64, room), (dk, room[:-5]), (dk, room[1:])):
+        with pytest.raises(ValueError):
+            run(width, chunks)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_gated_head_norm_and_branch_mean(dtype):
     from kvforge_b200 import ops
