@@ -5,12 +5,14 @@
 //   y_t = S_t^T C_t + D_h x_t
 //
 //   prepare   : a CTA per token: step sizes and decays, d x, B and C as floats.  Nothing here depends on the state.
-//   walk      : decay_walk with one decay a token and head, or for many tokens decay_chunks.
+//   walk      : decay_walk with one decay a token and head, or for many tokens chunks: state_space_tcgen05.cuh in bfloat16 where it
+//               takes the sizes, else decay_chunks.
 //   wide_norm : what follows a recurrence: the read-out (plus D x), gated before or after a norm over wide parts of the
 //               row (one part, or several equal ones), times a weight.
 //
 // Everything is float whatever the storage type T of projections and results.
 #include "decay_chunks.cuh"
+#include "state_space_tcgen05.cuh"
 
 using namespace kvf;
 
@@ -80,6 +82,22 @@ __global__ void __launch_bounds__(256) state_space_prepare_kernel(const T* __res
       Run<float, V>::store(cn + n * gn + (c - inner - gn), f);
     }
   }
+}
+
+// The logarithms of the decays and the step sizes alone.
+template <typename T>
+__global__ void __launch_bounds__(256) state_space_steps_kernel(const T* __restrict__ dt, long long lddt, const float* __restrict__ dt_bias,
+                                                                 const float* __restrict__ a_log, long long n_tokens, int H,
+                                                                 float* __restrict__ decay, float* __restrict__ step) {
+  pdl_launch();
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_tokens * H) return;
+  const long long n = i / H;
+  const int h = (int)(i - n * H);
+  const float d = softplus_exact(to_float<T>(dt[n * lddt + h]) + dt_bias[h]);
+  step[i] = d;
+  decay[i] = -expf(a_log[h]) * d;
 }
 
 // ---------------------------------------------------------------- wide norm and gate
@@ -191,13 +209,40 @@ int wide_norm_gate(const WideNormParams& p, long long n_tokens, cudaStream_t st)
                                     const float* a_log, float* state, long long state_stride, float* out,               \
                                     long long out_stride, const int* qsl, const int* state_slots, int B,                \
                                     long long n_tokens, int H, int G, int ns, int dv, float* decay, float* cn,          \
-                                    float* bn, float* vn, int max_q_len, float* raw, cudaStream_t st) {                             \
+                                    float* bn, float* vn, int max_q_len, float* raw, int* err, cudaStream_t st) {       \
     if (B <= 0 || n_tokens <= 0) return 0;                                                                              \
     if (H <= 0 || G <= 0 || H % G || ns <= 0 || ns > 512 || dv <= 0 || (unsigned)B > 65535u || (unsigned)H > 65535u ||  \
         n_tokens > 0x7fffffffLL)                                                                                        \
       return (int)cudaErrorInvalidValue;                                                                                \
     const int gn = G * ns;                                                                                              \
     auto al = [](const void* q, size_t b) { return ((uintptr_t)q % b) == 0; };                                          \
+    const long long inner = (long long)H * dv;                                                                          \
+    if (raw && sizeof(T) == 2 && ns <= 128 && ns % 8 == 0 && dv % 8 == 0 && ldx % 8 == 0 && al(x, 16) && al(vn, 16) &&  \
+        inner * n_tokens >= n_tokens * H + 4 + n_tokens * G * ssm::TOKENS && (unsigned)G <= 65535u &&                        \
+        state_stride % 4 == 0 && out_stride % 4 == 0 && al(state, 16) && al(out, 16)) {                                 \
+      /* the step sizes and the scores lie where the other form keeps its values */                                     \
+      const long long pairs = n_tokens * H;                                                                             \
+      float* const scores = vn + (pairs + 3) / 4 * 4;                                                                   \
+      const size_t ssm_smem = (size_t)2 * 64 * (ssm::N_MAX + 4) * sizeof(float);                                        \
+      if ((dv + 63) / 64 > 65535) return (int)cudaErrorInvalidValue;                                                    \
+      cudaError_t e = cudaFuncSetAttribute(ssm::chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,             \
+                                           (int)ssm::SMEM);                                                             \
+      if (e == cudaSuccess)                                                                                             \
+        e = cudaFuncSetAttribute(ssm::scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm_smem);       \
+      if (e != cudaSuccess) return (int)e;                                                                              \
+      int rc = launch(state_space_steps_kernel<T>, dim3((unsigned)((pairs + 255) / 256)), dim3(256), (size_t)0, st,     \
+                      (const T*)dt, lddt, dt_bias, a_log, n_tokens, H, decay, vn);                                      \
+      if (rc) return rc;                                                                                                \
+      rc = launch(ssm::scores_kernel, dim3((unsigned)(n_tokens / ssm::TOKENS + B), 3, G), dim3(256), ssm_smem, st,           \
+                  (const bf16*)x, ldx, inner, inner + gn, qsl, B, G, ns, scores);                                       \
+      if (rc) return rc;                                                                                                \
+      ssm::Params p{(const bf16*)x, ldx,         decay, vn, scores, state, state_stride, out, out_stride,               \
+                    qsl,            state_slots, err,   H,  G,      ns,    dv,           0};                            \
+      CUtensorMap map;                                                                                                  \
+      memset(&map, 0, sizeof(map));                                                                                     \
+      if (ns == ssm::N_MAX && dv % ssm::DV == 0) p.use_tma = ssm::rows_map(&map, x, ldx, inner + 2 * gn, n_tokens) == 0; \
+      return launch(ssm::chunks_kernel, dim3((dv + 63) / 64, H, B), dim3(ssm::THREADS), ssm::SMEM, st, map, p);         \
+    }                                                                                                                   \
     const bool vec = dv % 4 == 0 && gn % 4 == 0 && ldx % 4 == 0 && al(x, 4 * sizeof(T)) && al(vn, 16) && al(bn, 16) &&  \
                      al(cn, 16);                                                                                        \
     int rc = launch(vec ? state_space_prepare_kernel<T, 4> : state_space_prepare_kernel<T, 1>,                          \

@@ -81,7 +81,7 @@ _SIGNATURES = {
     "kvf_retention_gate_{s}": "plplfiliiplp",
     "kvf_tanh_norm_{s}": "pppilfppppplip",
     "kvf_decay_set_pdl": "i",
-    "kvf_state_space_{s}": "plplppplplppiliiiippppipp",
+    "kvf_state_space_{s}": "plplppplplppiliiiippppippp",
     "kvf_wide_norm_gate_{s}": "plpplipliipffliiplp",
     # library "joint"
     "kvf_joint_norm_cache_{s}": "plpilipppiifppiifpppiiiiiilpp",
@@ -2358,11 +2358,25 @@ def retention_gate(o: torch.Tensor, gate: torch.Tensor | None, eps: float, out: 
 STATE_SPACE_MAX_STATE = RETENTION_MAX_KEY_DIM  # the same walk
 
 
+def state_space_tensor_cores(dtype: torch.dtype, num_heads: int, groups: int, n_state: int, dv: int) -> bool:
+    """Whether the chunked form of ``state_space`` runs on the tensor cores (``csrc/state_space_tcgen05.cuh``) for rows of ``x`` on
+    16-byte boundaries: bfloat16, a state of at most 128 rows, and room for the scores and step sizes where the FP32 form keeps its
+    values."""
+    return dtype == torch.bfloat16 and n_state <= 128 and n_state % 8 == 0 and dv % 8 == 0 and num_heads * dv >= num_heads + 128 * groups + 4
+
+
+def state_space_chunks_pay(n: int, num_seqs: int, max_query_len: int) -> bool:
+    """Whether that form is faster than the walk: a chunk of 128 tokens costs the same however few of its tokens there are.  Walk and
+    chunks, us, 64 heads of 128 x 64: one sequence of 64 tokens 25 and 34, of 128 41 and 28, of 2,048 520 and 122; 8 of 64 87 and 88, 8 of
+    128 154 and 64, 8 of 256 299 and 88; 400 and 20 single tokens 161 and 195."""
+    return max_query_len >= 128 and n >= 64 * num_seqs
+
+
 def state_space(
     x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor, out: torch.Tensor,
     qsl: torch.Tensor, state_slots: torch.Tensor, num_seqs: int, num_heads: int, groups: int, n_state: int, dv: int,
     scratch: tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor] | None = None, max_query_len: int = 0,
-    raw: torch.Tensor | None = None,
+    raw: torch.Tensor | None = None, err: torch.Tensor | None = None,
 ) -> None:  # fmt: skip
     """A state space per head whose step size follows the token, over a flat batch, on the float state ``S [heads, n_state,
     dv]`` of each sequence's slot: ``d = softplus(dt + dt_bias)``, ``S <- exp(-exp(a_log) d) S + B (d x)^T``, ``out = S^T C``
@@ -2370,7 +2384,9 @@ def state_space(
     [groups*n_state] | C [groups*n_state]`` after their convolution; head ``h`` takes group ``h // (H / groups)``; ``dt``
     holds rows of ``H`` logits.  ``scratch``: float buffers ``(decay [N, H], cn [N, G*n_state], bn [N, G*n_state], vn
     [N, H*dv])``; without it they are allocated here.  ``max_query_len`` as in ``retention``.  With ``raw`` (float
-    scratch ``[N, groups*64]``) the chunked form runs.  Two launches, three in the chunked form."""
+    scratch ``[N, groups*64]``) the chunked form runs, in bfloat16 on the tensor cores
+    where ``csrc/state_space_tcgen05.cuh`` takes the sizes (a bounded wait that runs out then raises bit 4 of the device flag ``err``).
+    Two launches, three in the chunked form."""
     s = _suffix(x.dtype)
     _rows2d(x, None, "x")
     _rows2d(dt, x.dtype, "dt")
@@ -2404,7 +2420,7 @@ def state_space(
         _fn(name, DECAY_LIB)(
             _ptr(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), sptr, sstride, _ptr(out), out.stride(0), _ptr(qsl),
             _ptr(state_slots), int(num_seqs), n, h, g, int(n_state), int(dv), _ptr(decay), _ptr(cn), _ptr(bn), _ptr(vn), int(max_query_len),
-            _ptr(raw), _stream(),
+            _ptr(raw), _ptr(err), _stream(),
         ),
         name,
         3 if raw is not None else 2,

@@ -91,13 +91,17 @@ class StateSpace(Mixer):
         f32 = torch.float32
         read = rt.buf("ssm.read", n, self.inner, f32)
         scratch = (rt.buf("ssm.decay", n, H, f32), rt.buf("ssm.cn", n, gn, f32), rt.buf("ssm.bn", n, gn, f32), rt.buf("ssm.vn", n, self.inner, f32))
-        # many tokens of few sequences in bfloat16: chunk by chunk; 32-bit: token by token, the same bits however a sequence is cut
+        # many tokens of a sequence in bfloat16: chunk by chunk; 32-bit: token by token, the same bits however a sequence is cut
         state, raw = cache.state[:, self.conv_floats :], None
-        if rt.dtype == torch.bfloat16 and ops.chunks_pay(ctx.num_seqs, ctx.max_query_len) and ops.chunks_ok(self.N, dv, state):
+        if ops.state_space_tensor_cores(rt.dtype, H, self.G, self.N, dv):
+            chunks = ops.state_space_chunks_pay(n, ctx.num_seqs, ctx.max_query_len)
+        else:
+            chunks = rt.dtype == torch.bfloat16 and ops.chunks_pay(ctx.num_seqs, ctx.max_query_len)
+        if chunks and ops.chunks_ok(self.N, dv, state):
             raw = rt.buf("ssm.raw", n, self.G * ops.CHUNK_TOKENS, f32)
         ops.state_space(
             xbc, y[:, self.dt_off : self.dt_off + H], self.dt_bias, self.a_log, state, read, ctx.query_start_loc,
-            ctx.state_slots, ctx.num_seqs, H, self.G, self.N, dv, scratch, max_query_len=ctx.max_query_len, raw=raw,
+            ctx.state_slots, ctx.num_seqs, H, self.G, self.N, dv, scratch, max_query_len=ctx.max_query_len, raw=raw, err=rt.err,
         )  # fmt: skip
         out = rt.buf("ssm.out", n, self.inner)
         ops.wide_norm_gate(

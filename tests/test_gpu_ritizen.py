@@ -459,6 +459,64 @@ def test_lightning_attention_through_the_state(dtype, heads, dk, dv, t):
     two_requests(part, rt, x, ref, x2, ref2, cache, dtype)
 
 
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("heads,groups,dk,dv", [(4, 1, 128, 64), (2, 1, 128, 128), (24, 1, 16, 8), (3, 1, 72, 136), (8, 2, 128, 72)])
+def test_state_space_chunks_on_the_tensor_cores(heads, groups, dk, dv, positive):
+    """The chunked form in bfloat16 against 64 bits: chunks of 128 tokens that are full (boxes) or not (copies), every edge of a block
+    of 32, states carried at places that are no chunk's edge, decays from hardly any to ones that leave nothing, sequences without
+    tokens or slot, and a token that is no number: it reaches no other sequence and nothing before its half chunk."""
+    from kvforge_b200 import ops
+
+    assert ops.state_space_tensor_cores(torch.bfloat16, heads, groups, dk, dv)
+    g = torch.Generator().manual_seed(heads + dk)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    steps = [[257, 1, 31, 0, 128, 65], [129, 130, 33, 0, 64, 300]]
+    slots = [5, 0, 3, 6, -1, 2]
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    a_log, bias = r(heads) - 2.0, r(heads)
+    state = torch.zeros(7, heads * dk * dv + 4, device="cuda")
+    seqs, got = [[] for _ in slots], [[] for _ in slots]
+    inner = heads * dv
+    for lens in steps:
+        n = sum(lens)
+        x = r(n, inner + 2 * groups * dk)
+        x = (torch.nn.functional.silu(x) if positive else x).bfloat16()
+        dt = (2.0 * r(n, heads)).bfloat16()
+        dt[::37] += 12.0
+        starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        outs = []
+        for spoil in (True, False):
+            y, to = x.clone(), state if not spoil else state.clone()
+            bad = 100  # a token of the first sequence
+            if spoil:
+                y[bad] = float("nan")
+            out, raw = torch.full((n, inner), -7.0, device="cuda"), torch.empty(n, groups * ops.CHUNK_TOKENS, device="cuda")
+            err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            ops.state_space(y.cuda(), dt.cuda(), bias.cuda(), a_log.cuda(), to[:, 4:], out, i32(starts), i32(slots), len(lens), heads, groups, dk, dv,
+                            max_query_len=max(lens), raw=raw, err=err)  # fmt: skip
+            assert int(err) == 0
+            outs.append((out.cpu(), to.cpu()))
+        (spoilt, spoilt_state), (clean, after) = outs
+        keep = [t for t in range(n) if t < 64 or t >= starts[1]]
+        assert torch.equal(spoilt[keep], clean[keep]) and spoilt[bad : starts[1]].isnan().any(dim=1).all()
+        assert torch.equal(spoilt_state[[0, 1, 2, 3, 4, 6]], after[[0, 1, 2, 3, 4, 6]])
+        assert bool((clean[starts[4] : starts[5]] == -7.0).all())  # a sequence without a slot
+        for i in range(len(lens)):
+            rows = slice(starts[i], starts[i + 1])
+            seqs[i].append((x[rows].double(), dt[rows].double()))
+            got[i].append(clean[rows])
+    for i, parts in enumerate(seqs):
+        if slots[i] < 0 or sum(p[0].shape[0] for p in parts) == 0:
+            continue
+        x, dt = (torch.cat([p[j] for p in parts]) for j in range(2))
+        m = x.shape[0]
+        v, k, q = x[:, :inner].view(m, heads, dv), x[:, inner : inner + groups * dk].view(m, groups, dk), x[:, inner + groups * dk :].view(m, groups, dk)
+        ref = plain.state_space_walk(v, k, q, plain.softplus(dt + bias.double()), a_log.double(), torch.zeros(heads, dtype=torch.float64)).reshape(m, inner)
+        # 32-bit sums of up to 128 terms over scores of as many, each 2^-24 a term at the most: some 1e-7 of the norm, and four times that
+        assert float((torch.cat(got[i]).double() - ref).norm() / ref.norm()) < 5e-7, i
+    assert float(state[[1, 4]].abs().max()) == 0.0 and float(state[:, :4].abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("per_token", [False, True])
 @pytest.mark.parametrize("heads,groups,dk,dv", [(4, 4, 16, 24), (6, 2, 20, 12), (3, 1, 4, 4), (2, 2, 128, 100), (8, 1, 128, 64), (5, 5, 100, 36), (40, 2, 64, 128)])
 def test_recurrences_chunk_by_chunk(per_token, heads, groups, dk, dv):
