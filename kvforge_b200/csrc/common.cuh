@@ -45,6 +45,19 @@ inline size_t spread_smem(size_t need, long long ctas) {
   return need > room ? need : room;
 }
 
+// True in one lane of a converged warp.  A thread chosen so, and not by its lane's number, is known to the compiler to be alone: what
+// it hands to the tensor core and the copy engine (descriptors, addresses) then stays in uniform registers (eight tcgen05.mma of 128 x 96 x
+// 16 between two waits: 95 cycles each behind `lane == 0`, 67 behind this).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 template <typename... KArgs, typename... Args>
 inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};

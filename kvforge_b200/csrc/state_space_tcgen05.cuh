@@ -354,7 +354,7 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
     if (last >= 0) bar_wait(full0 + 8 * (last & 1), (last >> 1) & 1, p.err);
     if (last >= 1) bar_wait(full0 + 8 * ((last - 1) & 1), ((last - 1) >> 1) & 1, p.err);
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       const uint32_t k16 = (16 * 128) >> 4;  // 16 rows of a tile whose rows are walked
       const uint64_t td = sdesc(terms);

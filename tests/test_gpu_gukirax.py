@@ -6,6 +6,7 @@ captured graphs; and greedy generation through the engine's entry point."""
 from __future__ import annotations
 
 import json
+import math
 import subprocess
 import sys
 from pathlib import Path
@@ -304,6 +305,63 @@ def test_attention_whose_heads_talk(dtype, nh, nkv, d, dv, rot, t, bs):
     for cuts in ([(0, t)], [(0, 17), (17, 19), (19, 20), (20, 21), (21, 34), (34, 35), (35, 36), (36, t - 3), (t - 3, t - 2), (t - 2, t)]):
         got = step_mixer(part, rt, x, bs, table, cuts, cache)
         assert rel_rows(got, ref) < part_tol(dtype), cuts
+
+
+@pytest.mark.parametrize(
+    "nh,nkv,d,bs,window,sink",
+    [(32, 8, 64, 16, 0, True), (12, 4, 64, 48, 0, True), (8, 8, 64, 32, 50, True), (6, 1, 64, 64, 0, False), (8, 2, 128, 16, 0, True), (16, 4, 128, 64, 130, False), (3, 3, 128, 32, 0, True)],
+)
+def test_long_queries_on_the_tensor_cores(nh, nkv, d, bs, window, sink):
+    """The tcgen05 kernel for many queries against 64 bits: contexts and portions around its tiles of 96 or 64 keys and of 128 rows, a
+    single token and no token beside them, a context that ends inside a page (what lies behind it is no number), every page size's
+    boxes, tiles from a list and from the grid; what it does not take is refused."""
+    from kvforge_b200 import ops
+
+    g = torch.Generator().manual_seed(nh + d + bs)
+    lens, past = [97, 1, 0, 130, 64, 33], [0, 95, 0, 7, 300, 64]
+    n, tot = sum(lens), [a + b for a, b in zip(lens, past)]
+    per = [-(-t // bs) for t in tot]
+    order = torch.randperm(sum(per), generator=g).tolist()
+    k, v = (torch.randn(sum(per), nkv, bs, d, generator=g) for _ in range(2))
+    k = (k / k.pow(2).mean(-1, keepdim=True).sqrt()).bfloat16()
+    v, q = v.bfloat16(), torch.randn(n, nh * d, generator=g).bfloat16()
+    talk, sinks = torch.eye(nh) + 0.2 * torch.randn(nh, nh, generator=g), torch.randn(nh, generator=g)
+    tables, at, want = torch.zeros(len(lens), max(per), dtype=torch.int32), 0, torch.zeros(n, nh, d, dtype=torch.float64)
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    for i, m in enumerate(per):
+        tables[i, :m] = torch.tensor(order[at : at + m], dtype=torch.int32)
+        at += m
+        if not lens[i]:
+            continue
+        keys, vals = (t[tables[i, :m].long()].transpose(1, 2).reshape(-1, nkv, d)[: tot[i]].double().repeat_interleave(nh // nkv, 1) for t in (k, v))
+        s = torch.einsum("thd,jhd->htj", q[starts[i] : starts[i + 1]].double().view(-1, nh, d), keys) * d**-0.5
+        s = torch.einsum("ab,btj->atj", talk.double(), s)
+        pos, j = torch.arange(past[i], tot[i])[:, None], torch.arange(tot[i])[None]
+        s = s.masked_fill((j > pos) | (j <= pos - window if window else j < 0), -math.inf)
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(nh, s.shape[1], 1)], dim=2)
+        want[starts[i] : starts[i + 1]] = torch.einsum("htj,jhd->thd", torch.softmax(s, -1)[..., : tot[i]], vals)
+        for t in (k, v):  # what lies behind the context in its last page
+            t[tables[i, m - 1].long(), :, (tot[i] - 1) % bs + 1 :] = math.nan
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    tq = ops.talking_query_tile(nh, nkv)
+    tiles = [(b, x) for b, m in enumerate(lens) for x in range(0, m, tq)] + [(-1, 0)]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for listed in (True, False):
+        out = torch.full((n, nh * d), math.nan, device="cuda", dtype=torch.bfloat16)
+
+        def run(**kw):
+            ops.talking_attention(
+                q.cuda(), out, k.cuda(), v.cuda(), tables.cuda(), i32(starts), i32(tot), len(lens), max(lens), nh, nkv, d, d, d**-0.5, talk.cuda(),
+                sinks.cuda() if sink else None, window=window, kernel="tcgen05", err=err, query_tiles=(i32(tiles).reshape(-1), len(tiles)) if listed else None, **kw,
+            )  # fmt: skip
+
+        run()
+        assert int(err) == 0
+        # the result's rounding (2^-9 of a number) and that of two bfloat16 terms of queries and weights (2^-17 of a score)
+        assert float((out.cpu().double().view(n, nh, d) - want).norm() / want.norm()) < 2.5e-3 and rel_rows(out.cpu().view(n, nh, d), want) < 1e-2
+    with pytest.raises(ValueError):
+        run(q_stride=nh * d + 4)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
