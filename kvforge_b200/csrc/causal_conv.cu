@@ -52,6 +52,9 @@ __device__ __forceinline__ void load_floats(const float* p, float* f) {
 // taps are known at compile time and a thread keeps its weights in registers.  Each output is one chain of
 // fused multiply-adds over the taps, oldest first, whichever form runs.
 constexpr int CONV_ROWS = 4;  // rows of a tile when a step has many
+// Rows of a tile when its sequences are long too: the weights, as many bytes as four rows of inputs and outputs, are then read once for
+// sixteen.  2,048 tokens of one sequence, 6,144 channels and four taps: 23.8 us with tiles of four rows, 14.5 with these (50 MB).
+constexpr int CONV_LONG = 16;
 
 template <typename T, int VEC, int TAPS>
 __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w,
@@ -113,6 +116,60 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ 
         VecIO<T, VEC>::store(out + (size_t)(n0 + rr) * out_stride + c, acc);
       }
       return;
+    }
+  }
+  if constexpr (TAPS > 0 && VEC * sizeof(T) == 16) {
+    if (rows == CONV_LONG) {
+      const int n0 = blockIdx.x * CONV_LONG;
+      const int b0 = n0 < N ? seq_of_row(qsl, B, n0) : -1;
+      if (b0 < 0) return;
+      const int first = qsl[b0], end = qsl[b0 + 1];
+      if (n0 + CONV_LONG <= end && n0 + CONV_LONG <= N) {
+        // four rows at a time, the next four on their way (as they are stored: a conversion would wait for them)
+        const T* const src = x + (size_t)n0 * x_stride + c;
+        uint4 ahead[CONV_ROWS];
+        auto ask = [&](int r0) {
+#pragma unroll
+          for (int i = 0; i < CONV_ROWS; ++i) ahead[i] = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + i) * x_stride);
+        };
+        ask(0);
+        const int slot = state_slots[b0];
+        const float* st = slot >= 0 ? state + (size_t)slot * state_stride : nullptr;
+        float u[TAPS - 1 + CONV_ROWS][VEC];  // the inputs before these rows, then theirs
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i) {
+          const int t = n0 - first - (TAPS - 1) + i;
+          if (t >= 0) {
+            VecIO<T, VEC>::load(x + (size_t)(first + t) * x_stride + c, u[i]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) u[i][e] = st ? st[(size_t)(TAPS - 1 + t) * C + c + e] : 0.f;
+          }
+        }
+#pragma unroll
+        for (int r0 = 0; r0 < CONV_LONG; r0 += CONV_ROWS) {
+#pragma unroll
+          for (int i = 0; i < CONV_ROWS; ++i) VecIO<T, VEC>::load(reinterpret_cast<const T*>(&ahead[i]), u[TAPS - 1 + i]);
+          if (r0 + CONV_ROWS < CONV_LONG) ask(r0 + CONV_ROWS);
+#pragma unroll
+          for (int rr = 0; rr < CONV_ROWS; ++rr) {
+            float acc[VEC];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+              acc[e] = cb[e];
+#pragma unroll
+              for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wr[e][j], u[rr + j][e], acc[e]);
+              if (act == 1) acc[e] = silu_of<T>(acc[e]);
+            }
+            VecIO<T, VEC>::store(out + (size_t)(n0 + r0 + rr) * out_stride + c, acc);
+          }
+#pragma unroll
+          for (int i = 0; i < TAPS - 1; ++i)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) u[i][e] = u[i + CONV_ROWS][e];
+        }
+        return;
+      }
     }
   }
   for (int rr = 0; rr < rows; ++rr) {
@@ -229,7 +286,7 @@ int launch_conv_few(const T* x, int x_stride, const float* w, const float* bias,
 template <typename T, int VEC>
 int launch_conv(const T* x, int x_stride, const float* w, const float* bias, const float* state, long long state_stride, const int* qsl,
                 const int* state_slots, int N, int B, int C, int taps, int act, T* out, int out_stride, cudaStream_t st) {
-  const int rows = N >= 1024 ? CONV_ROWS : 1;
+  const int rows = N < 1024 ? 1 : taps <= 4 && VEC * sizeof(T) == 16 && N >= 64 * (long long)B ? CONV_LONG : CONV_ROWS;
   const int per_cta = 128 * VEC;
   dim3 grid((N + rows - 1) / rows, (C + per_cta - 1) / per_cta);
   if (grid.y > 65535u) return (int)cudaErrorInvalidValue;

@@ -307,6 +307,34 @@ def test_attention_whose_heads_talk(dtype, nh, nkv, d, dv, rot, t, bs):
         assert rel_rows(got, ref) < part_tol(dtype), cuts
 
 
+@pytest.mark.parametrize("nh,nkv,d,dv,rot,norm", [(4, 2, 64, 64, 32, True), (3, 1, 128, 64, 128, True), (5, 5, 32, 32, 16, False), (2, 1, 16, 8, 0, True), (6, 2, 256, 256, 64, True)])
+def test_heads_of_many_tokens_as_of_few(nh, nkv, d, dv, rot, norm):
+    """Steps of many tokens take eight numbers a thread, steps of few a warp a head: the same rows by either, a token without a slot
+    and one beyond the pool among them."""
+    from kvforge_b200 import ops
+
+    n, bs = 170, 16
+    g = torch.Generator().manual_seed(d + rot)
+    wide = nh * d + nkv * d + 8
+    x = torch.randn(n, wide, generator=g).bfloat16().cuda()
+    pos = torch.randint(0, 5000, (n,), generator=g, dtype=torch.int32).cuda()
+    inv = (10000.0 ** (-torch.arange(rot // 2) / max(1, rot // 2))).float().cuda()
+    slots = torch.randperm(12 * bs, generator=g)[:n].int()
+    slots[7], slots[100] = -1, 12 * bs
+    slots = slots.cuda()
+    results = []
+    for cut in (n, 100):  # one step, or steps too small for it
+        y, k, v = x.clone(), torch.zeros(12, nkv, bs, d, dtype=torch.bfloat16, device="cuda"), torch.zeros(12, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        for a in range(0, n, cut):
+            r = slice(a, min(n, a + cut))
+            ops.qk_prepare(y[r], pos[r].contiguous(), inv, 1e-5 if norm else None, slots[r].contiguous(), k, v, nh, nkv, d, dv, nh * d, nh * d, d, bs, err)
+        assert int(err) == 2
+        results.append((y.float(), k.float(), v.float()))
+    for a, b in zip(*results):  # sums in another order: a number may round the other way
+        assert bool(((a - b).abs() <= 2**-7 * b.abs()).all()) and float((a != b).float().mean()) < 0.01
+
+
 @pytest.mark.parametrize(
     "nh,nkv,d,bs,window,sink",
     [(32, 8, 64, 16, 0, True), (12, 4, 64, 48, 0, True), (8, 8, 64, 32, 50, True), (6, 1, 64, 64, 0, False), (8, 2, 128, 16, 0, True), (16, 4, 128, 64, 130, False), (3, 3, 128, 32, 0, True)],

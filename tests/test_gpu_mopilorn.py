@@ -389,6 +389,32 @@ def test_gated_delta_rule_through_the_state(dtype, h, g, dk, dv, channel):
     assert float(state[1].abs().max()) == 0 and float(state[:, :5].abs().max()) == 0
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("taps,lens", [(4, [1024]), (3, [700, 1, 333]), (2, [15, 1010]), (4, [17, 1007, 3, 40])])
+def test_convolution_of_long_sequences_has_the_bits_of_short_steps(taps, lens, dtype):
+    """Tiles of sixteen rows, and what lies across a sequence's border, against the same rows one step after another of fewer rows than
+    such tiles take."""
+    from kvforge_b200 import ops
+
+    dev, dt, c = "cuda", DT[dtype], 48
+    gen = torch.Generator().manual_seed(taps)
+    x, w, bias = torch.randn(sum(lens), c, generator=gen).to(dev, dt), torch.randn(taps, c, generator=gen).to(dev), torch.randn(c, generator=gen).to(dev)
+    slots = list(range(len(lens)))
+    start = torch.randn(len(lens), (taps - 1) * c, generator=gen).to(dev)
+    results = []
+    for step in (max(lens), 300):
+        state, out = start.clone(), torch.empty_like(x)
+        for a in range(0, max(lens), step):
+            part = [max(0, min(m, a + step) - a) for m in lens]
+            rows = torch.tensor([sum(lens[:i]) + a + j for i, m in enumerate(part) for j in range(m)], device=dev)
+            qsl, sl = flat_batch(part, slots, dev)
+            y = torch.empty(len(rows), c, device=dev, dtype=dt)
+            ops.causal_conv(x[rows].contiguous(), w, state, qsl, sl, len(lens), y, activation="silu", max_query_len=max(part), bias=bias)
+            out[rows] = y
+        results.append((out, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 @pytest.mark.parametrize("rate", [0.0, 3.0, -4.0])  # decays of every size, ones that forget at once, ones that keep all
 @pytest.mark.parametrize(
     "h,g,dk,dv,channel",

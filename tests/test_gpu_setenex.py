@@ -408,3 +408,37 @@ def test_small_parts():
     row = torch.randn(40)
     ops.add_row(resid, row.cuda())
     assert torch.equal(resid.cpu(), table[[3, 0, 8, 3]] * 2.5 + row)
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("nh,nkv,dk,dv,rot,weights,mixed", [(4, 2, 64, 64, 64, True, True), (3, 1, 128, 64, 32, True, False), (2, 2, 32, 32, 0, False, True), (5, 1, 16, 8, 16, False, False), (2, 1, 256, 256, 128, True, True)])
+def test_normed_heads_of_many_tokens_as_of_few(nh, nkv, dk, dv, rot, weights, mixed, split):
+    """Steps of many tokens take eight numbers a thread, steps of few a warp a head: the same rows by either, a token without a slot
+    and one beyond the pool among them."""
+    from kvforge_b200 import ops
+
+    n, bs = 170, 16
+    g = torch.Generator().manual_seed(dk + rot)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    x = r(n, (nh + nkv) * dk + nkv * dv).bfloat16()
+    pos = torch.randint(0, 5000, (n,), generator=g, dtype=torch.int32).cuda()
+    inv = (10000.0 ** (-torch.arange(rot // 2) / max(1, rot // 2))).float().cuda() if rot else None
+    q_w, k_w = (1 + 0.1 * r(dk), 1 + 0.1 * r(dk)) if weights else (None, None)
+    first, lam = (r(n, nkv * dv).bfloat16(), torch.full((1,), 0.3, device="cuda")) if mixed else (None, None)
+    slots = torch.randperm(12 * bs, generator=g)[:n].int()
+    slots[7], slots[100] = -1, 12 * bs
+    slots = slots.cuda()
+    results = []
+    for cut in (n, 100):  # one step, or steps too small for it
+        y, k, v = x.clone(), torch.zeros(12, nkv, bs, dk, dtype=torch.bfloat16, device="cuda"), torch.zeros(12, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
+        keep, err = torch.zeros(n, nkv * dv, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        for a in range(0, n, cut):
+            rows = slice(a, min(n, a + cut))
+            ops.head_norm_cache(
+                y[rows], pos[rows].contiguous(), q_w, k_w, 1e-5, inv, slots[rows].contiguous(), k, v, nh, nkv, dk, dv, bs, err, interleaved=not split,
+                v_keep=keep[rows], v_first=first[rows] if mixed else None, v_lambda=lam, magnitude=1.25 if rot else 1.0,
+            )  # fmt: skip
+        assert int(err) == 2
+        results.append((y.float(), k.float(), v.float(), keep.float()))
+    for a, b in zip(*results):  # sums in another order: a number may round the other way
+        assert bool(((a - b).abs() <= 2**-7 * b.abs()).all()) and float((a != b).float().mean()) < 0.01
