@@ -17,10 +17,9 @@
 //            issues the products; two bring the next chunk in and make its exponentials.  Per chunk: the update, C S, the weights times
 //            x, all with M = 128 and N = 64, 24 products each (of 55 cycles: 2.1 us a chunk).
 //
-// 64 heads of 128 x 64, one sequence of 2,048 tokens: 122 us with the two kernels before it (steps 2, scores 8, chunks 109) against 327 of
-// the FP32 form (decay_chunks.cuh) and 520 of the walk; 96 heads 125 and 636.  A chunk takes 6.8 us, a chain of update, split of the
-// state, C S, weights times x and read-out; the products alone are 2.3 (weights from tensor memory run at half the rate here that
-// they have by themselves, for a reason not found).  Against 64 bits outputs are off by 0.70e-7 to 1.14e-7 of their norm (FP32 form
+// 64 heads of 128 x 64, one sequence of 2,048 tokens: 119 us with the two kernels before it (steps 2, scores 8, chunks 106) against 327 of
+// the FP32 form (decay_chunks.cuh) and 520 of the walk; 96 heads 122 and 636.  A chunk takes 6.6 us, a chain of update, split of the
+// state, C S, weights times x and read-out; the products alone are 2.3.  Against 64 bits outputs are off by 0.70e-7 to 1.14e-7 of their norm (FP32 form
 // 0.82e-7 to 1.72e-7), states by 0.44e-7 to 1.03e-7 (0.47e-7 to 1.79e-7), over three rates of decay, x of normal noise and behind
 // silu; with x, B and C all positive and hardly a decay the state is 1.3 times as far off as there, the outputs 0.8 times.
 //
@@ -280,8 +279,56 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
     };
     bool ok = true;
     int last = -1;
+    float next_l[4], next_d[4];
+    auto ask = [&](int c) {
+      const int t0 = c * TOKENS, n = min(TOKENS, q_len - t0);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = 4 * lane + e;
+        const size_t row = (size_t)(q_begin + t0 + min(t, n - 1)) * p.H + h;
+        const float l = p.log_decay[row], d = p.step[row];
+        next_l[e] = t < n ? l : 0.f;
+        next_d[e] = t < n ? d : 0.f;
+      }
+    };
+    ask(0);
     for (int c = 0; c < chunks && ok; ++c) {
       const int s = c & 1, t0 = c * TOKENS, n = min(TOKENS, q_len - t0);
+      // ---- the factors, tokens 4 lane .. + 3: made before the stage is free, from numbers asked for a chunk ago
+      double g[4], r[4];  // the sums up to each token; at the start of blocks 0 .. 3
+      float d[4], w[4], al[4], eg[4], bd[3][4];
+      double sum = 0.0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        d[e] = next_d[e];
+        sum += (double)next_l[e];
+        g[e] = sum;
+      }
+      if (c + 1 < chunks) ask(c + 1);
+      double incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      double before = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane == 0) before = 0.0;
+      r[0] = 0.0;
+      r[1] = __shfl_sync(0xffffffffu, incl, 7);
+      r[2] = __shfl_sync(0xffffffffu, incl, 15);
+      r[3] = __shfl_sync(0xffffffffu, incl, 23);
+      const double total = __shfl_sync(0xffffffffu, incl, 31);
+      const int blk = lane >> 3;
+      const double start = blk == 0 ? r[0] : blk == 1 ? r[1] : blk == 2 ? r[2] : r[3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        g[e] += before;
+        eg[e] = expf((float)g[e]);
+        w[e] = expf((float)(total - g[e]));
+        al[e] = expf((float)(g[e] - start));
+#pragma unroll
+        for (int I = 1; I < 4; ++I) bd[I - 1][e] = expf((float)fmin(0.0, r[I] - g[e])) * d[e];  // (of the tokens before block I)
+      }
       if (c >= 2) ok = warp_wait(empty0 + 8 * s, ((c >> 1) - 1) & 1, p.err);
       if (!ok) break;
       const uint32_t at = base + s * STAGE, bar = full0 + 8 * s;
@@ -296,54 +343,23 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
         tile(at + 4 * HALF, xo, min(DV, p.dv - c0), 1, t0, n);
         cpa_commit();
       }
-      {
-        Factors& f = factors[s];
-        double g[4], r[4];  // tokens 4 lane .. + 3; the sums at the start of block 0 .. 3
-        float d[4];
-        double sum = 0.0;
+      Factors& f = factors[s];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = 4 * lane + e;
-          const size_t row = (size_t)(q_begin + t0 + (t < n ? t : 0)) * p.H + h;
-          const float l = t < n ? p.log_decay[row] : 0.f;
-          d[e] = t < n ? p.step[row] : 0.f;
-          sum += (double)l;
-          g[e] = sum;
-        }
-        double incl = sum;
+      for (int e = 0; e < 4; ++e) {
+        const int t = 4 * lane + e;
+        const double g2 = g[e] * 1.4426950408889634;
+        f.gh[t] = (float)g2;
+        f.gl[t] = (float)(g2 - (double)(float)g2);
+        f.d[t] = d[e];
+        f.eg[t] = eg[e];
+        f.wd[t] = w[e] * d[e];
+        f.wr[t] = fmaf(w[e], d[e], -w[e] * d[e]);
+        f.al[t] = al[e];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double up = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += up;
-        }
-        double before = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) before = 0.0;
-        r[0] = 0.0;
-        r[1] = __shfl_sync(0xffffffffu, incl, 7);
-        r[2] = __shfl_sync(0xffffffffu, incl, 15);
-        r[3] = __shfl_sync(0xffffffffu, incl, 23);
-        const double total = __shfl_sync(0xffffffffu, incl, 31);
-        const int blk = lane >> 3;
-        const double start = blk == 0 ? r[0] : blk == 1 ? r[1] : blk == 2 ? r[2] : r[3];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = 4 * lane + e;
-          g[e] += before;
-          const double g2 = g[e] * 1.4426950408889634;
-          f.gh[t] = (float)g2;
-          f.gl[t] = (float)(g2 - (double)(float)g2);
-          f.d[t] = d[e];
-          f.eg[t] = expf((float)g[e]);
-          const float w = expf((float)(total - g[e]));
-          f.wd[t] = w * d[e];
-          f.wr[t] = fmaf(w, d[e], -w * d[e]);
-          f.al[t] = expf((float)(g[e] - start));
-#pragma unroll
-          for (int I = 1; I < 4; ++I)
-            if (blk < I) f.bd[I - 1][t] = expf((float)(r[I] - g[e])) * d[e];
-        }
-        if (lane == 0) f.keep = expf((float)total);
+        for (int I = 1; I < 4; ++I)
+          if (blk < I) f.bd[I - 1][t] = bd[I - 1][e];
       }
+      if (lane == 0) f.keep = expf((float)total);
       cpa_wait<0>();
       fence_async_smem();
       __syncwarp();
@@ -370,10 +386,9 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          umma(tmem + COL_L, bt + kk * k16, td + ((2 * HALF) >> 4) + kk * k16, ID_UPDATE, kk > 0);
-          umma(tmem + COL_L, bt + kk * k16, td + (HALF >> 4) + kk * k16, ID_UPDATE, 1u);
-          umma(tmem + COL_U + DV * (kk >> 2), bt + kk * k16, td + kk * k16, ID_UPDATE, (kk & 3) != 0);
+        for (int i = 0; i < 24; ++i) {  // (one sum after another: products that take turns at two sums wait for one another)
+          const int kk = i & 7, term = 2 - (i >> 3);
+          umma(tmem + (term ? COL_L : COL_U + DV * (kk >> 2)), bt + kk * k16, td + ((term * HALF) >> 4) + kk * k16, ID_UPDATE, term ? i > 0 : (kk & 3) != 0);
         }
         umma_commit(update_done);
         // C S: the state's terms take the place of the scaled x's
@@ -381,11 +396,10 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t ck = cd + (((kk >> 2) * HALF) >> 4) + 2 * (kk & 3);
-          umma(tmem + COL_L, ck, td + ((2 * HALF) >> 4) + kk * k16, ID_OUT, kk > 0);
-          umma(tmem + COL_L, ck, td + (HALF >> 4) + kk * k16, ID_OUT, 1u);
-          umma(tmem + COL_R + DV * (kk >> 2), ck, td + kk * k16, ID_OUT, (kk & 3) != 0);
+        for (int i = 0; i < 24; ++i) {
+          const int kk = i & 7, term = 2 - (i >> 3);
+          umma(tmem + (term ? COL_L : COL_R + DV * (kk >> 2)), cd + (((kk >> 2) * HALF) >> 4) + 2 * (kk & 3), td + ((term * HALF) >> 4) + kk * k16, ID_OUT,
+               term ? i > 0 : (kk & 3) != 0);
         }
         umma_commit(read_done);
         // the weights times x, where the update was
