@@ -16,10 +16,12 @@
 // take the product of the very decays between the two tokens; between blocks J < I it is (decays from the start of I up to i) x (of
 // the blocks between) x (from j to the end of J), all factors at most one.
 //
-// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 276 us (prepare 124, chain 105, read 45) against 525 by
-// groups of four; 24 heads over 1,500 tokens 309 and 498, 8 heads with a decay a head over 2,048 196 and 351.  All three kernels are bound
+// 16 heads of 128 x 128 with a decay a channel, one sequence of 2,048 tokens: 269 us (prepare 124, chain 98, read 45) against 525 by
+// groups of four; 24 heads over 1,500 tokens 292 and 498, 8 heads with a decay a head over 2,048 187 and 351.  All three kernels are bound
 // by what shared memory hands to registers, 4 bytes a lane and cycle: the broadcast of A in the solve (a word a multiply-add), 8 x 4 and
-// 4 x 4 register tiles elsewhere.  A link of the chain is 3.3 us (6,200 cycles, of which 3,600 are its reads of W, S, K and u).
+// 4 x 4 register tiles elsewhere.  A link of the chain is 3.1 us (of some 5,800 cycles 3,600 are
+// its reads of W, S, K and u; with the rows of W S shared out over the warps instead of its tokens, and so with sums that go through
+// shared memory and two barriers more, 3.3 us).
 // Against 64 bits the outputs are off by 1.10e-7 of their norm there (groups 1.16e-7, walk 1.28e-7), the states by 0.89e-7 (0.91e-7,
 // 0.96e-7); over three rates of decay and three seeds each outputs are 0.86 to 1.01 of the groups' error and at most the walk's.  That
 // takes sums of A and B ended in double, and beta x kept whole in the solve (without them 1.06).
@@ -416,7 +418,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_prepare_kernel(cons
 }
 
 // ---- the chain
-template <int DVT> constexpr size_t dc_chain_smem() { return (size_t)(2 * (2 * 8192 + DC_T * DVT + DC_ROWS) + DC_ROWS * DVT + 8 * DC_T * DVT) * 4; }
+template <int DVT> constexpr size_t dc_chain_smem() { return (size_t)(2 * (2 * 8192 + DC_T * DVT + DC_ROWS) + DC_ROWS * DVT) * 4; }
 
 template <int DVT>
 __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const DeltaParams p) {
@@ -426,7 +428,6 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
   constexpr int NQ = DVT / 16, STAGE = 2 * 8192 + DC_T * DVT + DC_ROWS;
   extern __shared__ __align__(16) float sm[];
   float* const S = sm + 2 * STAGE;            // [128][DVT]
-  float* const part = S + DC_ROWS * DVT;      // [8][DVT][64] the warps' sums of W S
   const int b = blockIdx.y, h = blockIdx.z, c0 = blockIdx.x * DVT;
   const int first = p.qsl[b], q_len = p.qsl[b + 1] - first;
   const int slot = p.state_slots[b];
@@ -435,14 +436,15 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
   const int chunks = (q_len + DC_T - 1) / DC_T;
   const size_t step = (size_t)p.H * dc_record(dv);
   float* const rec0 = p.chunks + ((size_t)dc_base(first, b) * p.H + h) * dc_record(dv);
-  // place of a 16-byte word of columns in a row of u: odd tokens' words lie elsewhere, so that two tokens' reads do not collide
+  // place of a 16-byte word of columns in a row of u or S: odd rows' words lie elsewhere, so that two rows' reads do not collide
+  // (as those of W^T do)
   auto word = [](int t, int q) { return DVT == 32 ? q ^ ((t & 1) << 2) : q; };
   auto load = [&](int c) {
     if (c < chunks) {
       const float* rec = rec0 + (size_t)c * step;
       float* dst = sm + (c & 1) * STAGE;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) cp_async16(dst + 4 * (tid + 256 * i), rec + 4 * (tid + 256 * i));  // W^T, then K
+      for (int i = 0; i < 16; ++i) cp_async16(dst + 4 * ((i < 8 ? tid ^ ((tid >> 4) & 1) : tid) + 256 * i), rec + 4 * (tid + 256 * i));  // W^T, then K
       float* ud = dst + 2 * 8192;
 #pragma unroll
       for (int i = 0; i < NQ; ++i) {
@@ -462,14 +464,12 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
   // a warp owns rows 16 warp .. + 15 of S throughout
   for (int idx = lane; idx < 16 * DVT; idx += 32) {
     const int r = 16 * warp + idx / DVT, c = idx % DVT;
-    S[r * DVT + c] = r < dk && c0 + c < dv ? sg[(size_t)r * dv + c] : 0.f;
+    S[r * DVT + 4 * word(r, c >> 2) + (c & 3)] = r < dk && c0 + c < dv ? sg[(size_t)r * dv + c] : 0.f;
   }
-  __syncwarp();
   for (int c = 0; c < chunks; ++c) {
-    __syncthreads();  // the other stage has been read
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the stage is there, S is whole and the other stage has been read
     load(c + 1);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
     const float* const W = sm + (c & 1) * STAGE;
     const float* const Kh = W + 8192;
     float* const U = sm + (c & 1) * STAGE + 2 * 8192;
@@ -479,22 +479,23 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
     for (int i = 0; i < DVT / 8; ++i) {  // S0 for the read-out
       const int idx = lane + 32 * i, r = 16 * warp + idx / (DVT / 4), q = idx % (DVT / 4);
       if (c0 + 4 * q < dv)
-        *reinterpret_cast<float4*>(rec + DC_U + (size_t)(DC_T + r) * dv + c0 + 4 * q) = *reinterpret_cast<const float4*>(S + r * DVT + 4 * q);
+        *reinterpret_cast<float4*>(rec + DC_U + (size_t)(DC_T + r) * dv + c0 + 4 * q) = *reinterpret_cast<const float4*>(S + r * DVT + 4 * word(r, q));
     }
-    {  // W S over the warp's rows: tokens 4 tg .. + 3 and 32 + 4 tg .. + 3, columns 4 cg .. + 3 (and 16 on)
-      const int tg = lane & 7, cg = lane >> 3;
+    {  // u = U - W S for tokens 8 warp .. + 7: rows kg, kg + 8 .. of S, columns 4 cg .. + 3 (and 16 on); then the eight kg are summed
+      const int cg = lane & 3, kg = lane >> 2;
       uint64_t acc[4][4 * NQ];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4 * NQ; ++j) acc[i][j] = 0ull;
+      const float* const wp = W + kg * DC_T + 8 * warp;
+      const int odd = kg & 1;
 #pragma unroll
       for (int kk = 0; kk < 16; ++kk) {
-        const int k = 16 * warp + kk;
-        const ulonglong2 w0 = dc_pairs(W + k * DC_T + 4 * tg), w1 = dc_pairs(W + k * DC_T + 32 + 4 * tg);
+        const ulonglong2 w0 = dc_pairs(wp + 8 * kk * DC_T + 4 * odd), w1 = dc_pairs(wp + 8 * kk * DC_T + 4 - 4 * odd);
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-          const float4 s4 = *reinterpret_cast<const float4*>(S + k * DVT + 16 * q + 4 * cg);
+          const float4 s4 = *reinterpret_cast<const float4*>(S + (kg + 8 * kk) * DVT + 4 * word(kg, 4 * q + cg));
           const uint64_t s[4] = {dc_both(s4.x), dc_both(s4.y), dc_both(s4.z), dc_both(s4.w)};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -505,31 +506,30 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
           }
         }
       }
-      float* const mine = part + warp * DC_T * DVT;
+      // a lane keeps half of what it has at each of three exchanges: the last is one token's four columns
+      const int t = 8 * warp + kg;
 #pragma unroll
-      for (int j = 0; j < 4 * NQ; ++j) {
-        float* const row = mine + (16 * (j / 4) + 4 * cg + (j & 3)) * DC_T + 4 * tg;
-        *reinterpret_cast<ulonglong2*>(row) = make_ulonglong2(acc[0][j], acc[1][j]);
-        *reinterpret_cast<ulonglong2*>(row + 32) = make_ulonglong2(acc[2][j], acc[3][j]);
+      for (int q = 0; q < NQ; ++q) {
+        float s[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint64_t two[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint64_t keep = (kg & 4) ? acc[2 + i][4 * q + j] : acc[i][4 * q + j], give = (kg & 4) ? acc[i][4 * q + j] : acc[2 + i][4 * q + j];
+            two[i] = dc_add(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+          }
+          const uint64_t keep = (kg & 2) ? two[1] : two[0], give = (kg & 2) ? two[0] : two[1];
+          float lo, hi;
+          dc_split(dc_add(keep, __shfl_xor_sync(0xffffffffu, give, 8)), lo, hi);
+          s[j] = (odd ? hi : lo) + __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 4);
+        }
+        float4* const at = reinterpret_cast<float4*>(U + t * DVT + 4 * word(t, 4 * q + cg));
+        float4 u = *at;
+        u.x -= s[0]; u.y -= s[1]; u.z -= s[2]; u.w -= s[3];
+        *at = u;
+        if (c0 + 16 * q + 4 * cg < dv) *reinterpret_cast<float4*>(rec + DC_U + (size_t)t * dv + c0 + 16 * q + 4 * cg) = u;
       }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NQ; ++i) {  // u = U - sum over the warps
-      const int t = tid & 63, q = (tid >> 6) + 4 * i;
-      float s[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float y[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) y[w] = part[(w * DVT + 4 * q + e) * DC_T + t];
-        s[e] = ((y[0] + y[1]) + (y[2] + y[3])) + ((y[4] + y[5]) + (y[6] + y[7]));
-      }
-      float4* const at = reinterpret_cast<float4*>(U + t * DVT + 4 * word(t, q));
-      float4 u = *at;
-      u.x -= s[0]; u.y -= s[1]; u.z -= s[2]; u.w -= s[3];
-      *at = u;
-      if (c0 + 4 * q < dv) *reinterpret_cast<float4*>(rec + DC_U + (size_t)t * dv + c0 + 4 * q) = u;
     }
     __syncthreads();
     {  // S <- c S + K^T u on the warp's rows: every other token, rows 4 rg .. + 3, columns 4 cg .. + 3 (and 16 on)
@@ -570,22 +570,21 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_chain_kernel(const 
             v[j][2 * i] = k0 + __shfl_xor_sync(0xffffffffu, g0, 1);
             v[j][2 * i + 1] = k1 + __shfl_xor_sync(0xffffffffu, g1, 1);
           }
-        float* const at = S + (16 * warp + 4 * rg) * DVT + 16 * q + 4 * cg + 2 * th;
+        float* const at = S + (16 * warp + 4 * rg) * DVT + 2 * th;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          float2* const s2 = reinterpret_cast<float2*>(at + r * DVT);
+          float2* const s2 = reinterpret_cast<float2*>(at + r * DVT + 4 * word(r, 4 * q + cg));
           const float cr = r == 0 ? c4.x : r == 1 ? c4.y : r == 2 ? c4.z : c4.w;
           const float2 old = *s2;
           *s2 = make_float2(fmaf(cr, old.x, v[0][r]), fmaf(cr, old.y, v[1][r]));
         }
       }
-      __syncwarp();
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
   for (int idx = lane; idx < 16 * DVT; idx += 32) {
     const int r = 16 * warp + idx / DVT, c = idx % DVT;
-    if (r < dk && c0 + c < dv) sg[(size_t)r * dv + c] = S[r * DVT + c];
+    if (r < dk && c0 + c < dv) sg[(size_t)r * dv + c] = S[r * DVT + 4 * word(r, c >> 2) + (c & 3)];
   }
 }
 

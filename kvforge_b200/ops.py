@@ -1339,8 +1339,8 @@ DELTA_CHUNK_TOKENS = 64
 def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, per_channel: bool, n: int, num_seqs: int, max_query_len: int) -> bool:
     """Whether a step of the delta rule goes sixty-four tokens at a time rather than four.  A chunk costs about the same however
     few of its tokens there are, so the step needs long sequences and few short ones beside them.  Groups of four and chunks, us,
-    16 heads of 128 x 128 with a decay a channel: one sequence of 256 tokens 71 and 68, of 512 133 and 84, of 2,048 525 and 276; 8 of
-    256 386 and 291; 1,000 and 8 single tokens 373 and 301, 400 and 20 219 and 323; 30 of 64 307 and 362.  8 heads with a decay a head:
+    16 heads of 128 x 128 with a decay a channel: one sequence of 256 tokens 71 and 68, of 512 133 and 84, of 2,048 525 and 269; 8 of
+    256 386 and 282; 1,000 and 8 single tokens 373 and 301, 400 and 20 219 and 323; 30 of 64 307 and 362.  8 heads with a decay a head:
     one of 256 55 and 69, of 384 75 and 75, of 1,024 181 and 108."""
     few = 256 if per_channel else 384
     return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= 384 and n >= 96 * num_seqs
