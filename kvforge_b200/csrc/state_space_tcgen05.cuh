@@ -80,11 +80,10 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate)
       : "memory");
 }
-// A whole warp waits, or arrives once.
+// A whole warp waits (every lane sees the phase over itself: a shuffle of one lane's wait would hand on the answer, but not the order
+// of what was written before it), or arrives once.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* err) {
-  bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = bar_wait(bar, parity, err);
-  return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+  return __all_sync(0xffffffffu, bar_wait(bar, parity, err));
 }
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
   __syncwarp();

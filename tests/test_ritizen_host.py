@@ -221,3 +221,14 @@ def test_plain_model_sees_its_chunk_and_carries_its_states():
     assert [j for j in range(17) if moved(j)] == [12, 13, 14, 15, 16]
     config["layers"][0]["mixer"]["right_scale"] = 0.5
     assert all(moved(j) for j in range(17))
+
+
+def test_every_lane_that_goes_on_behind_a_barrier_has_waited_itself():
+    """One lane's wait handed on by a shuffle tells the others that a phase is over, not what was written before it."""
+    import re
+
+    from kvforge_b200.native import CSRC
+
+    for path in sorted(CSRC.glob("*.cu*")):
+        for body in re.findall(r"\n[^\n]*\bbool \w*wait\w*\([^\n]*\{\n(.*?)\n\}", path.read_text(), flags=re.S):
+            assert "__shfl" not in body and "threadIdx" not in body, path.name
