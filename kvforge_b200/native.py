@@ -48,7 +48,7 @@ LIBRARIES: dict[str, tuple[list[str], list[str]]] = {
     # layers whose sublayer results are gated and normed before they join the residual stream, heads that are
     # rotated and then normed; attention whose heads talk before the softmax; libraries of their own for the same reason
     "gated": (["gated_ops.cu"], []),
-    "talking": (["attention_talking_f32.cu", "attention_talking_bf16.cu", "attention_talking_mma.cu", "attention_talking_tcgen05.cu"], []),
+    "talking": (["attention_talking_f32.cu", "attention_talking_bf16.cu", "attention_talking_mma.cu"], []),
     # recurrent mixers with one decay a head or a token and head, the norm and gate after them, a norm without statistics;
     # a library of its own for the same reason
     "decay": (["retention.cu", "state_space.cu", "tanh_norm.cu"], []),

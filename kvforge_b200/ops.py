@@ -74,7 +74,6 @@ _SIGNATURES = {
     "kvf_talking_attention_{s}": "pppppppppiiiiiiiiiifiiiippp",
     "kvf_talking_attention_mma_bf16": "pppppppppiiiiiiiiiifiiiippp",
     "kvf_talking_mma_ok": "iiiiii",
-    "kvf_talking_attention_tcgen05_bf16": "pppppppppiiiiiiiiilfipipp",
     "kvf_talking_set_pdl": "i",
     "kvf_gated_set_pdl": "i",
     # library "decay"
@@ -2115,41 +2114,18 @@ def talking_mma_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, dv: int
     return _talking_mma_known[key]
 
 
-def talking_tcgen05_supported(dtype: torch.dtype, nh: int, nkv: int, d: int, dv: int, block_size: int) -> bool:
-    """Whether the tcgen05 kernel for many queries (``csrc/attention_talking_tcgen05.cu``) takes the shape: bfloat16, heads of 64 or 128
-    with values as wide as keys, at most 512 numbers in a token's keys, pages of a multiple of 16 tokens."""
-    return dtype == torch.bfloat16 and d == dv and d in (64, 128) and nkv * d <= 512 and nh // nkv <= 128 and block_size % 16 == 0
-
-
-def talking_query_tile(nh: int, nkv: int) -> int:
-    """Queries of one sequence that a CTA of that kernel serves."""
-    return max(1, 128 // max(1, nh // nkv))
-
-
-# Contexts of at most so many keys are a tile of the mma.sync kernel or two, without the long queries of the tcgen05 kernel before
-# them: a prompt of 16, 64, 128, 256, 2,048 tokens, us on mma.sync / tcgen05, 32 heads of 64 on 8: 15 / 17, 17 / 17, 25 / 19, 43 / 21,
-# 390 / 147; 16 tokens behind 1,000 156 / 43, 32 x 2 behind 500 70 / 58, 30 single tokens behind 1,000 beside a prompt of 200 219 / 86;
-# 16 heads of 128 on 4: 16 tokens 15 / 16, 256 39 / 23, 1,024 135 / 55.
-TALKING_SHORT_CONTEXT = 64
-
-
 def talking_attention(
     q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, block_tables: torch.Tensor,
     query_start_loc: torch.Tensor, context_lens: torch.Tensor, num_seqs: int, max_query_len: int, nh: int, nkv: int, d: int, dv: int,
     scale: float, talk: torch.Tensor | None, sink: torch.Tensor | None, q_stride: int | None = None, window: int = 0,
-    scratch: tuple | None = None, max_context: int | None = None, split_size: int = 256, kernel: str = "auto",
-    err: torch.Tensor | None = None, query_tiles: tuple[torch.Tensor, int] | None = None,
+    scratch: tuple | None = None, max_context: int | None = None, split_size: int = 256,
 ) -> None:  # fmt: skip
     """Causal attention over the paged cache whose heads' scores are mixed before the softmax
     (``s'_h = sum_g talk[h, g] s_g``, ``talk`` float ``[nh, nh]`` or ``None``) and whose softmax may have a sink
     (``sink`` float ``[nh]``: ``exp(sink_h)`` joins the denominator, with no key and no value).  ``q`` rows hold
     ``nh`` heads of ``d`` (row stride ``q_stride``), ``out [N, nh * dv]``; ``scratch``: the decode form (every
     sequence one query; key ranges of ``split_size`` in parallel, then a merge) with ``(part_acc, part_ml, _)``
-    as ``attention_scratch_shapes`` gives them.  Without it and with more than one query in some sequence the tcgen05 kernel runs where it
-    takes the shape, unless ``max_context`` says that the contexts are short (``kernel``: ``"auto"``; ``"mma"`` and ``"tcgen05"`` force one; ``err`` and
-    ``query_tiles``, tiles of ``talking_query_tile`` queries, as in ``paged_attention``)."""
-    if kernel not in ("auto", "mma", "tcgen05"):
-        raise ValueError("talking_attention: kernel is 'auto', 'mma' or 'tcgen05'")
+    as ``attention_scratch_shapes`` gives them."""
     s = _suffix(q.dtype)
     _need(q, None, "q", contiguous=False)
     _need(out, q.dtype, "out")
@@ -2167,34 +2143,6 @@ def talking_attention(
             _need(t, torch.float32, what)
             if tuple(t.shape) != shape:
                 raise ValueError(f"talking_attention: {what} must be {shape}")
-    stride = int(q_stride or q.stride(0))
-    takes = (
-        talking_tcgen05_supported(q.dtype, nh, nkv, d, dv, int(block_size)) and scratch is None and talk is not None and window >= 0
-        and float(scale) > 0.0 and stride % 8 == 0 and out.stride(0) % 8 == 0
-        and (q.data_ptr() | out.data_ptr() | kcache.data_ptr() | vcache.data_ptr()) % 16 == 0
-        and kcache.shape[0] * nkv * block_size < 2**31 - 64
-        and (0 < query_tiles[1] <= 65535 if query_tiles is not None else num_seqs <= 65535 and max_query_len <= 65535 * talking_query_tile(nh, nkv))
-    )  # fmt: skip
-    short = max_context is not None and 0 < max_context <= TALKING_SHORT_CONTEXT
-    if kernel == "tcgen05" and not takes:
-        raise ValueError("talking_attention: the tcgen05 kernel does not take this call")
-    if takes and (kernel == "tcgen05" or (kernel == "auto" and max_query_len > 1 and not short)):
-        tiles, n_tiles = None, 0
-        if query_tiles is not None:
-            tiles, n_tiles = query_tiles
-            _need(tiles, torch.int32, "query tiles")
-            if tiles.numel() < 2 * n_tiles:
-                raise ValueError("talking_attention: the list holds fewer query tiles than it says")
-        name = "kvf_talking_attention_tcgen05_bf16"
-        _check(
-            _fn(name, TALKING_LIB)(
-                _ptr(q), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_tables), _ptr(query_start_loc), _ptr(context_lens), _ptr(talk), _ptr(sink),
-                int(num_seqs), int(max_query_len), stride, out.stride(0), block_tables.stride(0), nh, nkv, d, int(block_size), int(kcache.shape[0]),
-                float(scale), int(window), _ptr(tiles), n_tiles, _ptr(err), _stream(),
-            ),
-            name,
-        )  # fmt: skip
-        return
     acc = ml = None
     split = max_splits = grid_splits = 0
     if scratch is not None:
@@ -2211,7 +2159,7 @@ def talking_attention(
     _check(
         _fn(name, TALKING_LIB)(
             _ptr(q), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_tables), _ptr(query_start_loc), _ptr(context_lens), _ptr(talk), _ptr(sink),
-            int(num_seqs), int(max_query_len), stride, out.stride(0), block_tables.stride(0), nh, nkv, d, dv, block_size,
+            int(num_seqs), int(max_query_len), int(q_stride or q.stride(0)), out.stride(0), block_tables.stride(0), nh, nkv, d, dv, block_size,
             float(scale), int(window), split, max_splits, grid_splits, _ptr(acc), _ptr(ml), _stream(),
         ),
         name,

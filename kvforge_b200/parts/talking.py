@@ -120,10 +120,6 @@ class TalkingAttention(Mixer):
         table = self.position.table() if self.position is not None else None
         if table is not None and getattr(self.position, "pairs_interleaved", False):
             raise ValueError("attention whose heads talk turns split pairs")
-        self._query_tile = None
-        if rt.dtype == torch.bfloat16 and self.talks and self.dv == self.d and self.d in (64, 128) and self.nkv * self.d <= 512:
-            self._query_tile = ops.talking_query_tile(self.nh, self.nkv)
-            rt.query_tile_sizes.add(self._query_tile)
         self.inv_freq = table if table is not None else torch.empty(0, dtype=torch.float32, device=rt.device)
 
     def forward(self, ctx, x: torch.Tensor, cache):
@@ -148,11 +144,9 @@ class TalkingAttention(Mixer):
         if ctx.all_single_query:
             (acc, ml, _), bound, split = decode_scratch(rt, ctx, self.nh, self.nkv, self.d, self.dv, None, TALKING_RANGE)
             scratch = (acc, ml)
-        tiles = ctx.query_tiles.get(self._query_tile)
         ops.talking_attention(
             y, out, cache.k, cache.v, ctx.block_tables[cache.group], ctx.query_start_loc, ctx.context_lens, ctx.num_seqs, ctx.max_query_len,
-            self.nh, self.nkv, self.d, self.dv, self.scale, self.talk, self.sink, q_stride=self.in_dim, scratch=scratch,
-            max_context=bound if scratch is not None else ctx.max_context_len,
-            split_size=split, err=rt.err, query_tiles=(tiles.tiles, tiles.count) if tiles is not None else None,
+            self.nh, self.nkv, self.d, self.dv, self.scale, self.talk, self.sink, q_stride=self.in_dim, scratch=scratch, max_context=bound,
+            split_size=split,
         )  # fmt: skip
         return project(rt, "attn.proj", out, self.w_o, ctx)

@@ -339,10 +339,9 @@ def test_heads_of_many_tokens_as_of_few(nh, nkv, d, dv, rot, norm):
     "nh,nkv,d,bs,window,sink",
     [(32, 8, 64, 16, 0, True), (12, 4, 64, 48, 0, True), (8, 8, 64, 32, 50, True), (6, 1, 64, 64, 0, False), (8, 2, 128, 16, 0, True), (16, 4, 128, 64, 130, False), (3, 3, 128, 32, 0, True)],
 )
-def test_long_queries_on_the_tensor_cores(nh, nkv, d, bs, window, sink):
-    """The tcgen05 kernel for many queries against 64 bits: contexts and portions around its tiles of 96 or 64 keys and of 128 rows, a
-    single token and no token beside them, a context that ends inside a page (what lies behind it is no number), every page size's
-    boxes, tiles from a list and from the grid; what it does not take is refused."""
+def test_many_queries_of_heads_that_talk(nh, nkv, d, bs, window, sink):
+    """Steps of many queries against 64 bits: contexts and portions around tiles of 32, 64 and 96 keys, a single token and no token
+    beside them, a context that ends inside a page (what lies behind it is no number), pages of several sizes, windows."""
     from kvforge_b200 import ops
 
     g = torch.Generator().manual_seed(nh + d + bs)
@@ -372,24 +371,45 @@ def test_long_queries_on_the_tensor_cores(nh, nkv, d, bs, window, sink):
         for t in (k, v):  # what lies behind the context in its last page
             t[tables[i, m - 1].long(), :, (tot[i] - 1) % bs + 1 :] = math.nan
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
-    tq = ops.talking_query_tile(nh, nkv)
-    tiles = [(b, x) for b, m in enumerate(lens) for x in range(0, m, tq)] + [(-1, 0)]
-    err = torch.zeros(1, dtype=torch.int32, device="cuda")
-    for listed in (True, False):
-        out = torch.full((n, nh * d), math.nan, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((n, nh * d), math.nan, device="cuda", dtype=torch.bfloat16)
+    ops.talking_attention(
+        q.cuda(), out, k.cuda(), v.cuda(), tables.cuda(), i32(starts), i32(tot), len(lens), max(lens), nh, nkv, d, d, d**-0.5, talk.cuda(),
+        sinks.cuda() if sink else None, window=window,
+    )  # fmt: skip
+    # the result's rounding: at most 2^-9 of a number, 1.66e-3 of the norm; the weights' two bfloat16 terms add 2^-17
+    assert float((out.cpu().double().view(n, nh, d) - want).norm() / want.norm()) < 1.75e-3 and rel_rows(out.cpu().view(n, nh, d), want) < 1e-2
 
-        def run(**kw):
-            ops.talking_attention(
-                q.cuda(), out, k.cuda(), v.cuda(), tables.cuda(), i32(starts), i32(tot), len(lens), max(lens), nh, nkv, d, d, d**-0.5, talk.cuda(),
-                sinks.cuda() if sink else None, window=window, kernel="tcgen05", err=err, query_tiles=(i32(tiles).reshape(-1), len(tiles)) if listed else None, **kw,
-            )  # fmt: skip
 
-        run()
-        assert int(err) == 0
-        # the result's rounding (2^-9 of a number) and that of two bfloat16 terms of queries and weights (2^-17 of a score)
-        assert float((out.cpu().double().view(n, nh, d) - want).norm() / want.norm()) < 2.5e-3 and rel_rows(out.cpu().view(n, nh, d), want) < 1e-2
-    with pytest.raises(ValueError):
-        run(q_stride=nh * d + 4)
+@pytest.mark.parametrize("nh,nkv,d,n", [(32, 8, 64, 4096), (16, 4, 128, 12288), (6, 1, 64, 32768)])
+def test_mixed_scores_keep_the_bits_of_a_float(nh, nkv, d, n):
+    """Every token sees itself and the token before it, with values of one and minus one: the result is tanh of half the difference
+    of two scores of some 2,000, and shows a score's error where that difference is near zero."""
+    from kvforge_b200 import ops
+
+    bs, size = 16, 2000.0
+    g = torch.Generator().manual_seed(nh + d)
+    k, q = torch.randn(n, nkv, d, generator=g).bfloat16(), torch.randn(n, nh, d, generator=g).bfloat16()
+    talk = torch.eye(nh) + 0.2 * torch.randn(nh, nh, generator=g)
+    sign = 1.0 - 2.0 * (torch.arange(n) % 2)
+    pages = lambda t: t.view(n // bs, bs, nkv, d).transpose(1, 2).contiguous().cuda()  # noqa: E731
+    kd = k.double().repeat_interleave(nh // nkv, 1)
+    before = torch.cat([torch.zeros_like(kd[:1]), kd[:-1]])
+    diff = (torch.einsum("thd,thd->th", q.double(), kd) - torch.einsum("thd,thd->th", q.double(), before)) @ talk.double().T
+    scale = size / float(diff[1:].pow(2).mean().sqrt()) * 2**0.5
+    diff = scale * diff[1:]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    out = torch.empty(n, nh * d, device="cuda", dtype=torch.bfloat16)
+    ops.talking_attention(
+        q.view(n, -1).cuda(), out, pages(k), pages(sign[:, None, None].expand(n, nkv, d).bfloat16().contiguous()), i32(list(range(n // bs)))[None].contiguous(),
+        i32([0, n]), i32([n]), 1, n, nh, nkv, d, d, scale, talk.cuda(), None, window=2,
+    )  # fmt: skip
+    got = out.cpu().double().view(n, nh, d)[1:, :, 0] * sign[1:, None]
+    near = diff.abs() < 1.0
+    assert int(near.sum()) >= 20
+    off = 2.0 * torch.atanh(got[near].clamp(-0.999, 0.999)) - diff[near]
+    # a result of at most tanh(1/2) rounded by 2^-9 of itself moves the difference by at most 2.3e-3; two scores of 2,000, each with an
+    # error of some 2^-23 of itself, by 0.4e-3
+    assert float(off.pow(2).mean().sqrt()) < 2.7e-3, float(off.pow(2).mean().sqrt())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
