@@ -1333,6 +1333,7 @@ def delta_group_floats(n: int, num_seqs: int, num_heads: int, per_channel: bool)
 
 
 DELTA_CHUNK_TOKENS = 64
+DELTA_CHUNK_MEAN = 96  # tokens a sequence that a step in chunks has at least, on the average
 
 
 def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, per_channel: bool, n: int, num_seqs: int, max_query_len: int) -> bool:
@@ -1342,12 +1343,17 @@ def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, per_channel: bool, n: 
     256 386 and 282; 1,000 and 8 single tokens 373 and 301, 400 and 20 219 and 323; 30 of 64 307 and 362.  8 heads with a decay a head:
     one of 256 55 and 69, of 384 75 and 75, of 1,024 181 and 108."""
     few = 256 if per_channel else 384
-    return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= 384 and n >= 96 * num_seqs
+    return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= 384 and n >= DELTA_CHUNK_MEAN * num_seqs
 
 
 def delta_chunk_record(num_heads: int, dv: int) -> int:
     """Floats that a chunk of tokens takes: per head 28,800 and the columns of 64 tokens and of a state."""
     return num_heads * (28800 + (DELTA_CHUNK_TOKENS + 128) * dv)
+
+
+def delta_chunk_records(max_tokens: int) -> int:
+    """The most records that a step of at most ``max_tokens`` tokens has under ``delta_chunks_ok``."""
+    return max_tokens // DELTA_CHUNK_TOKENS + max_tokens // DELTA_CHUNK_MEAN
 
 
 def delta_chunk_floats(n: int, num_seqs: int, num_heads: int, dv: int) -> int:

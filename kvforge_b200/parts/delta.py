@@ -147,6 +147,12 @@ class GatedDeltaRule(Mixer):
             return False, rt.max_tokens
         return True, min(rt.max_tokens, ops.DELTA_GROUP_TOKENS * max(rt.max_seqs, num_seqs))
 
+    def _chunks(self, n: int, num_seqs: int) -> torch.Tensor:
+        """The records of a step's chunks.  They are large (16 heads of 128 x 128: 3.4 MB each), so their buffer is made for the sequences
+        that the rule lets a step of the token budget have, not for every request slot."""
+        record = ops.delta_chunk_record(self.H, self.dv)
+        return self.rt.buf("delta.chunks", n // ops.DELTA_CHUNK_TOKENS + num_seqs, record, torch.float32, cap=ops.delta_chunk_records(self.rt.max_tokens))
+
     def forward(self, ctx, x: torch.Tensor, cache):
         rt = self.rt
         n = x.shape[0]
@@ -190,9 +196,7 @@ class GatedDeltaRule(Mixer):
         scratch = groups = chunks = None
         if ops.delta_chunks_ok(rt.dtype, dk, dv, self.decay == "channel", n, ctx.num_seqs, ctx.max_query_len):
             # many tokens a sequence in bfloat16: sixty-four at a time, from records of the chunks
-            per = ops.DELTA_CHUNK_TOKENS
-            record = ops.delta_chunk_record(H, dv)
-            chunks = rt.buf("delta.chunks", n // per + ctx.num_seqs, record, f32, cap=rt.max_tokens // per + max(rt.max_seqs, ctx.num_seqs))
+            chunks = self._chunks(n, ctx.num_seqs)
         elif ops.delta_groups_ok(rt.dtype, dk, ctx.max_query_len):
             # a few tokens a sequence: four at a time, from records of the groups
             per = ops.DELTA_GROUP_TOKENS

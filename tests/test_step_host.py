@@ -259,6 +259,33 @@ def test_buffers_of_the_delta_rule_s_walk_hold_what_the_walk_may_see():
         assert part._walk_rows(2000) == (want[0], budget)
 
 
+def test_buffer_of_the_delta_rule_s_chunks_follows_the_rule_and_not_the_request_slots():
+    from types import SimpleNamespace
+
+    import torch
+
+    from kvforge_b200 import PRESETS, ops
+    from kvforge_b200.engine.core import spec_from_config
+    from kvforge_b200.parts.base import build_part
+
+    for model in ("mopilorn-1b", "mopilorn-3b"):
+        for layer in spec_from_config(PRESETS[model]).layers:
+            if layer.block.params["mixer"].kind != "gated_delta_rule":
+                continue
+            part, asked = build_part("mixer", layer.block.params["mixer"], ""), []
+            for budget, slots in ((2048, 256), (2048, 1), (700, 64), (400, 8)):
+                part.rt = SimpleNamespace(max_tokens=budget, max_seqs=slots, buf=lambda name, rows, cols, dtype, cap: asked.append((rows, cols, cap)))
+                widest = 0
+                for n in range(1, budget + 1):
+                    for seqs in range(1, slots + 1):
+                        if ops.delta_chunks_ok(torch.bfloat16, part.dk, part.dv, part.decay == "channel", n, seqs, n):
+                            if n in (384, 1000, budget):
+                                part._chunks(n, seqs)
+                                assert asked[-1][0] <= asked[-1][2] and asked[-1][0] * asked[-1][1] == ops.delta_chunk_floats(n, seqs, part.H, part.dv)
+                            widest = max(widest, n // ops.DELTA_CHUNK_TOKENS + seqs)
+                assert widest <= asked[-1][2] <= budget // 64 + budget // 96  # no record that no step can use, whatever the slots
+
+
 def test_shaped_scores_keep_the_ranges_of_the_launch(monkeypatch):
     """The decode kernel may lengthen its ranges for plain scores in bfloat16 alone, in steps of single tokens and in mixed ones."""
     from types import SimpleNamespace
