@@ -401,8 +401,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_prepare_kernel(cons
         float lo, hi;
         dc_split(s[j >> 1], lo, hi);
         // beta x is kept whole: a chunk's u is rounded once more than a group's, when the chain takes W S from it
-        const float xv = __uint_as_float(x[jq & 3][e] << shift), bx = bj * xv;
-        u[e] = bx + fmaf(-bj, (j & 1) ? hi : lo, fmaf(bj, xv, -bx));
+        const float xv = __uint_as_float(x[jq & 3][e] << shift), bx = bj * xv, rest = fmaf(bj, xv, -bx);
+        u[e] = bx + fmaf(-bj, (j & 1) ? hi : lo, rest == rest ? rest : 0.f);  // (an infinite value has no rest)
         const uint64_t uu = dc_both(u[e]);
 #pragma unroll
         for (int iq = (j + 1) / 4; iq < 16; ++iq) {

@@ -534,6 +534,36 @@ def test_gated_delta_rule_in_chunks(h, g, dk, dv, channel, rate):
     assert float(state[1].abs().max()) == 0 and float(state[3].abs().max()) == 0 and float(state[:, :4].abs().max()) == 0
 
 
+@pytest.mark.parametrize("channel", [True, False])
+def test_an_infinite_value_is_infinite_in_its_own_token_s_read_out(channel):
+    """In chunks as token by token: of the token that brings it the column's read-out is infinite (and no number in the tokens after,
+    whose state holds infinities of either sign); tokens before it and other columns are what they are without it."""
+    from kvforge_b200 import ops
+
+    dev, h, dk, dv, n = "cuda", 2, 128, 32, 200
+    gen = torch.Generator().manual_seed(7)
+    aw = h * dk if channel else h
+    qkv, b, a = torch.randn(n, 2 * h * dk + h * dv, generator=gen).bfloat16().to(dev), torch.randn(n, h, generator=gen).to(dev), torch.randn(n, aw, generator=gen).to(dev)
+    a_log, dt_bias = torch.zeros(h, device=dev), torch.zeros(aw, device=dev)
+    qsl, sl = flat_batch([n], [0], dev)
+
+    def run(x, **kw):
+        out, state = torch.empty(n, h * dv, device=dev), torch.zeros(1, h * dk * dv, device=dev)
+        ops.gated_delta(x[:, : h * dk], x[:, h * dk : 2 * h * dk], x[:, 2 * h * dk :], b, a, a_log, dt_bias, state, out, qsl, sl, 1, h, h, dk, dv, q_scale=1.0, max_query_len=n, **kw)
+        return out
+
+    chunks = lambda: torch.full((ops.delta_chunk_floats(n, 1, h, dv),), float("nan"), device=dev)  # noqa: E731
+    clean = run(qkv, chunks=chunks())
+    for t, col in ((0, 0), (15, 3), (16, 5), (63, 40), (64, 33), (130, 20), (199, 63)):
+        bad = qkv.clone()
+        bad[t, 2 * h * dk + col] = -float("inf")
+        got, walk = run(bad, chunks=chunks()), run(bad)
+        others = [c for c in range(h * dv) if c != col]
+        assert torch.equal(got[:t], clean[:t]) and torch.equal(got[:, others], clean[:, others])
+        assert bool(got[t, col].isinf()) and got[t, col] == walk[t, col], (t, col)
+        assert not bool(got[t:, col].isfinite().any())
+
+
 def test_delta_chunks_refuse_what_they_do_not_take():
     from kvforge_b200 import ops
 
