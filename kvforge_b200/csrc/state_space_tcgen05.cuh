@@ -50,7 +50,7 @@ struct Factors {
   float bd[3][96];                  // e^(r of block I + 1 - g_s) d_s for the tokens before that block
   float keep, pad[3];               // e^(g_n)
 };
-constexpr size_t SMEM = 2 * (size_t)STAGE + 3 * (size_t)HALF + 2 * sizeof(Factors) + 128;
+constexpr size_t SMEM = 2 * (size_t)STAGE + 3 * (size_t)HALF + 2 * sizeof(Factors) + 160;
 
 struct Params {
   const bf16* x;  // rows of x [H*dv] | B [G*N] | C [G*N]
@@ -234,6 +234,8 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
   const uint32_t bars = terms + 3 * HALF + 2 * (uint32_t)sizeof(Factors);
   const uint32_t full0 = bars, empty0 = bars + 16, read_done = bars + 40, update_done = bars + 48, out_done = bars + 56,
                  x_ready = bars + 64, p_ready = bars + 72, s_ready = bars + 80, r_free = bars + 88, drained = bars + 96, tmem_slot = bars + 104;
+  // a bit for every token of a chunk (of even and odd chunks) whose x is an infinity or no number in some of the CTA's columns
+  uint32_t* const odd_x = reinterpret_cast<uint32_t*>(smem_raw + (bars - base) + 112);
   pdl_launch();
   pdl_wait();
   const int b = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * DV;
@@ -246,6 +248,7 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int chunks = (q_len + TOKENS - 1) / TOKENS;
   if (tid == 0) {
+    for (int i = 0; i < 8; ++i) odd_x[i] = 0u;
     for (int s = 0; s < 2; ++s) {
       bar_init(full0 + 8 * s, 1);
       bar_init(empty0 + 8 * s, 1 + MMA_WARP);
@@ -441,14 +444,25 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
       fence_async_smem();
     };
     // The scaled x of a chunk, for the update; its place is free once the chunk before's C S, which read the state there, is over.
+    // What is infinite or no number is taken out of x itself: the weights of later tokens are zeros, and zero times it would reach the
+    // tokens before it.  The read-out adds it to its own token and those after.
     auto scale_x = [&](int c) {
       const int s = c & 1;
       if (!warp_wait(full0 + 8 * s, (c >> 1) & 1, p.err)) return false;
       float x[16], v[16];
       const float w = factors[s].wd[r], rest = factors[s].wr[r];
-      const unsigned char* const row = smem_raw + s * STAGE + 4 * HALF;
+      unsigned char* const row = smem_raw + s * STAGE + 4 * HALF;
       bf16x8_to_float(*reinterpret_cast<const uint4*>(row + sw128(r, 2 * q4)), x);
       bf16x8_to_float(*reinterpret_cast<const uint4*>(row + sw128(r, 2 * q4 + 1)), x + 8);
+      float odd = 0.f;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) odd = fmaf(x[j], 0.f, odd);
+      if (odd != odd) {
+        atomicOr(odd_x + 4 * s + (r >> 5), 1u << (r & 31));
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (x[j] * 0.f != 0.f) *reinterpret_cast<unsigned short*>(row + sw128(r, 2 * q4 + (j >> 3)) + 2 * (j & 7)) = 0;
+      }
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = x[j] * w;
       put_row(v, [&](int j) { return fmaf(x[j], rest, fmaf(x[j], w, -x[j] * w)); });
@@ -512,7 +526,8 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
       }  // (the others are zeros)
     };
     bool ok = scale_x(0);
-    int met = 0;  // barriers of all the warps that work
+    asm volatile("bar.sync 1, %0;" ::"n"(MMA_WARP * 32) : "memory");  // (the odd tokens of the first chunk are known to all)
+    int met = 0;  // barriers of all the warps that work, of the chunks' read-outs
     float v[32];
     ask(0, v);
     for (int c = 0; c < chunks && ok; ++c) {
@@ -563,9 +578,22 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
       wait16(b);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       warp_arrive(r_free);
-      if (blk >= 2)  // tokens of the first half take nothing of the second's, not even zero times it
 #pragma unroll
-        for (int j = 0; j < 16; ++j) o[j] += __uint_as_float(b[j]);
+      for (int j = 0; j < 16; ++j) o[j] += __uint_as_float(b[j]);
+      const uint4 odd = *reinterpret_cast<const uint4*>(odd_x + 4 * ph);
+      if (odd.x | odd.y | odd.z | odd.w) {
+#pragma unroll 1
+        for (int s = 0; s <= r; ++s) {
+          if (!(odd_x[4 * ph + (s >> 5)] >> (s & 31) & 1u)) continue;
+          const float wt = raw[(size_t)(c * TOKENS + s) * p.G * TOKENS] * (ex2((f.gh[r] - f.gh[s]) + (f.gl[r] - f.gl[s])) * f.d[s]);
+          const bf16* const xs = p.x + (size_t)(q_begin + c * TOKENS + s) * p.ldx + (size_t)h * p.dv + c0 + 16 * q4;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float x = c0 + 16 * q4 + j < p.dv ? __bfloat162float(xs[j]) : 0.f;
+            if (x * 0.f != 0.f) o[j] = fmaf(wt, x, o[j]);
+          }
+        }
+      }
       // By way of B's place, which the update has read: a warp then writes whole rows (straight from the registers a warp's 16 bytes a
       // row go to 32 rows at a time, which kept the path to memory busy for 3,000 cycles).
       unsigned char* const rows = smem_raw + ph * STAGE + 2 * HALF;
@@ -574,6 +602,7 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
         *reinterpret_cast<float4*>(rows + r * 256 + (((4 * q4 + q) ^ (r & 7)) << 4)) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
       asm volatile("bar.sync 1, %0;" ::"n"(MMA_WARP * 32) : "memory");
       ++met;
+      if (tid < 4) odd_x[4 * ph + tid] = 0u;  // (before the chunk after the next's scaled x, which waits for this warp)
       const int n = min(TOKENS, q_len - c * TOKENS);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {

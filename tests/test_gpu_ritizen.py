@@ -6,6 +6,7 @@ generation through the engine's entry point."""
 from __future__ import annotations
 
 import json
+import math
 import subprocess
 import sys
 from pathlib import Path
@@ -464,7 +465,7 @@ def test_lightning_attention_through_the_state(dtype, heads, dk, dv, t):
 def test_state_space_chunks_on_the_tensor_cores(heads, groups, dk, dv, positive):
     """The chunked form in bfloat16 against 64 bits: chunks of 128 tokens that are full (boxes) or not (copies), every edge of a block
     of 32, states carried at places that are no chunk's edge, decays from hardly any to ones that leave nothing, sequences without
-    tokens or slot, and a token that is no number: it reaches no other sequence and nothing before its half chunk."""
+    tokens or slot, and a token that is no number: it reaches no other sequence and nothing before it."""
     from kvforge_b200 import ops
 
     assert ops.state_space_tensor_cores(torch.bfloat16, heads, groups, dk, dv)
@@ -497,7 +498,7 @@ def test_state_space_chunks_on_the_tensor_cores(heads, groups, dk, dv, positive)
             assert int(err) == 0
             outs.append((out.cpu(), to.cpu()))
         (spoilt, spoilt_state), (clean, after) = outs
-        keep = [t for t in range(n) if t < 64 or t >= starts[1]]
+        keep = [t for t in range(n) if t < bad or t >= starts[1]]
         assert torch.equal(spoilt[keep], clean[keep]) and spoilt[bad : starts[1]].isnan().any(dim=1).all()
         assert torch.equal(spoilt_state[[0, 1, 2, 3, 4, 6]], after[[0, 1, 2, 3, 4, 6]])
         assert bool((clean[starts[4] : starts[5]] == -7.0).all())  # a sequence without a slot
@@ -515,6 +516,44 @@ def test_state_space_chunks_on_the_tensor_cores(heads, groups, dk, dv, positive)
         # 32-bit sums of up to 128 terms over scores of as many, each 2^-24 a term at the most: some 1e-7 of the norm, and four times that
         assert float((torch.cat(got[i]).double() - ref).norm() / ref.norm()) < 5e-7, i
     assert float(state[[1, 4]].abs().max()) == 0.0 and float(state[:, :4].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("what", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("heads,groups,dk,dv", [(4, 1, 128, 64), (6, 2, 128, 128), (3, 1, 72, 136)])
+def test_state_space_chunks_keep_odd_values_from_the_tokens_before(heads, groups, dk, dv, what):
+    """An x that is infinite or no number, at the edges of blocks of 32 tokens and of chunks: tokens before it and other columns have the
+    bits that they have without it, its own read-out is the like of it, and it shows in every token after."""
+    from kvforge_b200 import ops
+
+    assert ops.state_space_tensor_cores(torch.bfloat16, heads, groups, dk, dv)
+    g = torch.Generator().manual_seed(dk + dv)
+    n, inner = 300, heads * dv
+    x, dt = torch.randn(n, inner + 2 * groups * dk, generator=g).bfloat16().cuda(), torch.randn(n, heads, generator=g).bfloat16().cuda()
+    bias, a_log = torch.zeros(heads, device="cuda"), torch.full((heads,), -4.0, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def run(y):
+        out, state = torch.empty(n, inner, device="cuda"), torch.zeros(1, heads * dk * dv, device="cuda")
+        raw, err = torch.empty(n, groups * ops.CHUNK_TOKENS, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.state_space(y, dt, bias, a_log, state, out, i32([0, n]), i32([0]), 1, heads, groups, dk, dv, max_query_len=n, raw=raw, err=err)
+        assert int(err) == 0
+        return out, state.view(heads, dk, dv)
+
+    clean, after = run(x)
+    assert bool(clean.isfinite().all())
+    b, c = (x[:, inner + i * groups * dk : inner + (i + 1) * groups * dk].double().view(n, groups, dk) for i in range(2))
+    score = (b * c).sum(-1).repeat_interleave(heads // groups, 1)
+    for t, col in ((0, 0), (1, dv - 1), (31, 5), (32, dv + 17), (63, 40), (64, 8), (100, inner - 1), (127, 15), (128, 16), (255, 31), (256, 3), (299, 7)):
+        y = x.clone()
+        y[t, col] = what
+        got, state = run(y)
+        others = [i for i in range(inner) if i != col]
+        assert torch.equal(got[:t], clean[:t]) and torch.equal(got[:, others], clean[:, others]), (t, col)
+        own = float(got[t, col])
+        assert math.isnan(own) if math.isnan(what) else own == math.copysign(1.0, float(score[t, col // dv])) * what, (t, col, own)
+        assert not bool(got[t:, col].isfinite().any()) and not bool(state[col // dv, :, col % dv].isfinite().any())
+        state[col // dv, :, col % dv] = after[col // dv, :, col % dv]
+        assert torch.equal(state, after)
 
 
 @pytest.mark.parametrize("per_token", [False, True])
