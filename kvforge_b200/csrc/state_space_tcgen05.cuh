@@ -8,20 +8,25 @@
 // Every product of the second kernel has one operand that is a bfloat16 number as it is stored (B, C, x); the other (the state, the
 // scores with their decays, the scaled x) is a float that goes in as three bfloat16 terms, whose sum is that float exactly.  Products of
 // bfloat16 numbers are exact in float, so these are float products; sums in tensor memory are cut, not rounded, so no accumulator takes
-// more than 64 terms of a sum (its low terms first) and the parts are added in float.
+// more than 64 terms of a sum (32 of the update's; its low terms first) and the parts are added in float.
 //
-//   scores : C_t . B_s of every chunk, once for the heads that share B and C, on the FP32 pipes: a sum of 128 in one accumulator in
-//            tensor memory is off by 1.2e-7 to 1.7e-7 of its norm, here by 0.3e-7 (a chain of multiply-adds 0.7e-7 to 0.9e-7).
+//   scores : C_t . B_s of every chunk, once for the heads that share B and C, on the FP32 pipes, sixteen numbers at a time, what they
+//            give added in double: a sum of 128 in one accumulator in tensor memory is off by 1.2e-7 to 1.7e-7 of its norm.
 //   chunks : a CTA owns (sequence, head, 64 columns) and goes through the sequence's chunks.  Warps 0 .. 15 do what is between the
 //            products: row r of the chunk (or of the state, which stays in registers) and a quarter of the columns a thread; a warp
-//            issues the products; two bring the next chunk in and make its exponentials.  Per chunk: the update, C S, the weights times
+//            issues the products; one brings the next chunk in and makes its exponentials.  Per chunk: the update, C S, the weights times
 //            x, all with M = 128 and N = 64, 24 products each (of 55 cycles: 2.1 us a chunk).
 //
-// 64 heads of 128 x 64, one sequence of 2,048 tokens: 119 us with the two kernels before it (steps 2, scores 8, chunks 106) against 327 of
-// the FP32 form (decay_chunks.cuh) and 520 of the walk; 96 heads 122 and 636.  A chunk takes 6.6 us, a chain of update, split of the
-// state, C S, weights times x and read-out; the products alone are 2.3.  Against 64 bits outputs are off by 0.70e-7 to 1.14e-7 of their norm (FP32 form
-// 0.82e-7 to 1.72e-7), states by 0.44e-7 to 1.03e-7 (0.47e-7 to 1.79e-7), over three rates of decay, x of normal noise and behind
-// silu; with x, B and C all positive and hardly a decay the state is 1.3 times as far off as there, the outputs 0.8 times.
+// 64 heads of 128 x 64, one sequence of 2,048 tokens: 115 us with the two kernels before it, against 327 of the FP32 form (decay_chunks.cuh)
+// and 516 of the walk; 96 heads 117 and 751; 8 sequences of 128 61 and 150.  A chunk takes 6.6 us, a chain of update, split of the state, C
+// S, weights times x and read-out; the products alone are 2.3.
+// Against 64 bits, in 1e-7 of the norm, this form / the FP32 form / the walk, averages over 16 heads and six seeds, x, B and C behind silu:
+//   a_log about  0 : outputs 0.66 / 0.99 / 0.78, states 0.65 / 0.65 / 0.66      -2 : 0.67 / 0.90 / 1.26, 0.75 / 0.85 / 1.35
+//                1 : outputs 0.63 / 0.97 / 0.73, states 0.56 / 0.57 / 0.58      -6 : 0.57 / 0.85 / 16.5, 0.59 / 0.94 / 22.2
+// and as much nearer for normal ones (0: 0.69 / 1.04 / 1.00, 0.65 / 0.66 / 0.67).  With all of x, B and C positive and decays that leave
+// only the last tokens (0 and 1) the state is further off, 0.64 / 0.56 / 0.61 and 0.61 / 0.53 / 0.55: there the tensor core cuts every
+// term of a sum downwards.  It takes the sums of the scores in double (with floats 0.11 more for outputs at 0), 2^x to a unit in the last
+// place (0.06), sums of 32 tokens for the update, and the three factors below.
 //
 // Between blocks of 32 tokens a decay is the product of the decays to and from a block's start; inside one it is the exponential of a
 // difference of sums of two floats each (every exponent is at most zero).
@@ -39,9 +44,11 @@ constexpr int MMA_WARP = 16, LOADER_WARP = 17, THREADS = 576;
 constexpr uint32_t HALF = TOKENS * 128;            // bytes of a [128][64] tile
 constexpr uint32_t STAGE = 5 * HALF;          // C (two halves), B (two halves), x
 constexpr uint32_t COL_P = 0, COL_R = 192, COL_U = 320, COL_L = 448;  // weights, C S, the update and then the weights times x, low terms of C S and of the update
-// Tensor memory cuts what does not fit a float towards zero, half a unit in the last place a sum on average; this much of a sum is given
-// back through its low terms, which can hold it (and 2^-24 of the weights, whose low and high terms share a sum).
-constexpr float CUT = 0x1.4p-25f;
+// Tensor memory cuts what does not fit a float towards zero.  So much of a sum is given back, through its low terms: what C S (sums of four
+// products), the update (of two) and the weights times x (of four, whose low and high terms share a sum) lose on the average of x, B
+// and C of either sign and behind silu, a_log from -6 to 1 (0 and 2^-24 for the update: its state at 0 0.68 and 0.67; 0 and 2^-24 for the
+// weights: outputs 0.1 to 0.2 and 0.0 to 0.1 further off).  A sum whose terms are all positive loses up to 1.04e-7 of itself, others 0.65e-7.
+constexpr float CUT = 0x1.4p-25f, CUT_U = 0x1.4p-25f, CUT_P = 0x1.8p-25f;
 // what a chunk's logarithms become
 struct Factors {
   float gh[TOKENS], gl[TOKENS];               // g_t in log2 units, as a float and the rest
@@ -89,16 +96,19 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) bar_arrive(bar);
 }
-// Two floats' next bfloat16 term; what is left of them once `share` of it is taken away stays.
-__device__ __forceinline__ uint32_t take(float& a, float& b, float share = 1.f) {
+// Two floats' next bfloat16 term; what is left of them stays, and `more` times the term with it.
+__device__ __forceinline__ uint32_t take(float& a, float& b, float more = 0.f) {
   const uint32_t w = pk(a, b);
-  unpack2(fma2(pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), pack2(-share, -share), pack2(a, b)), a, b);
+  const uint64_t t = pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  uint64_t rest = fma2(t, pack2(-1.f, -1.f), pack2(a, b));
+  if (more != 0.f) rest = fma2(t, pack2(more, more), rest);
+  unpack2(rest, a, b);
   return w;
 }
 // N floats as three bfloat16 terms, in pairs.  An infinity is its first term, with nothing left of it.  more(j): what number j has
 // beyond its float.
 template <int N, typename Put, typename More>
-__device__ __forceinline__ void put_terms(float (&v)[N], float share, Put put, More more) {
+__device__ __forceinline__ void put_terms(float (&v)[N], float share, Put put, More more) {  // (`share` of the first term on top)
   uint32_t w[N / 2];
 #pragma unroll
   for (int j = 0; j < N / 2; ++j) w[j] = take(v[2 * j], v[2 * j + 1], share);
@@ -119,6 +129,26 @@ __device__ __forceinline__ void put_terms(float (&v)[N], float share, Put put, M
 #pragma unroll
   for (int j = 0; j < N / 2; ++j) w[j] = pk(v[2 * j], v[2 * j + 1]);
   put(2, w);
+}
+// 2^(hi + lo) of two numbers of at most zero (|lo| far below one), to 0.6 units in the last place: 2^f over [-1/2, 1/2] is one and f times a
+// polynomial of degree five through the Chebyshev points.  (With ex2.approx of the rounded hi + lo the outputs are off by a tenth more.)
+__device__ __forceinline__ void exp2_pair(uint64_t hi, uint64_t lo, float& a, float& b) {
+  constexpr float ROUND = 12582912.f;  // 1.5 x 2^23: the sum's last bits are the nearest whole number
+  const uint64_t minus = pack2(-1.f, -1.f), t = add2(hi, pack2(ROUND, ROUND)), n = add2(t, pack2(-ROUND, -ROUND));
+  const uint64_t f = add2(fma2(n, minus, hi), lo);
+  uint64_t q = pack2(0x1.44400400p-13f, 0x1.44400400p-13f);
+  q = fma2(q, f, pack2(0x1.5f089600p-10f, 0x1.5f089600p-10f));
+  q = fma2(q, f, pack2(0x1.3b2a1c00p-7f, 0x1.3b2a1c00p-7f));
+  q = fma2(q, f, pack2(0x1.c6af6c00p-5f, 0x1.c6af6c00p-5f));
+  q = fma2(q, f, pack2(0x1.ebfbe000p-3f, 0x1.ebfbe000p-3f));
+  q = fma2(q, f, pack2(0x1.62e43000p-1f, 0x1.62e43000p-1f));
+  q = fma2(q, f, pack2(1.f, 1.f));
+  float x0, x1, t0, t1;
+  unpack2(q, a, b);
+  unpack2(t, t0, t1);
+  unpack2(hi, x0, x1);
+  a = x0 < -126.f ? 0.f : a * __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
+  b = x1 < -126.f ? 0.f : b * __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
 }
 __device__ __forceinline__ void put4(uint32_t at, const uint32_t* w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
@@ -186,7 +216,7 @@ static __global__ void __launch_bounds__(256) scores_kernel(const bf16* __restri
   }
   __syncthreads();
   const int tg = threadIdx.x & 15, sg = threadIdx.x >> 4;  // rows tg + 16 i of C, sg + 16 j of B
-  float sum[4][4] = {};
+  double sum[4][4] = {};
   for (int k0 = 0; k0 < ns; k0 += 16) {  // eight terms an accumulator: even and odd numbers of sixteen
     uint64_t acc[4][4];
 #pragma unroll
@@ -213,7 +243,7 @@ static __global__ void __launch_bounds__(256) scores_kernel(const bf16* __restri
       for (int j = 0; j < 4; ++j) {
         float lo, hi;
         unpack2(acc[i][j], lo, hi);
-        sum[i][j] += lo + hi;
+        sum[i][j] += (double)lo + (double)hi;
       }
   }
 #pragma unroll
@@ -222,7 +252,7 @@ static __global__ void __launch_bounds__(256) scores_kernel(const bf16* __restri
     if (s >= n) continue;
     float* const dst = raw + ((size_t)(first + s) * G + grp) * TOKENS + t0 + tg;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) dst[16 * i] = sum[i][j];
+    for (int i = 0; i < 4; ++i) dst[16 * i] = (float)sum[i][j];
   }
 }
 
@@ -390,7 +420,8 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
 #pragma unroll
         for (int i = 0; i < 24; ++i) {  // (one sum after another: products that take turns at two sums wait for one another)
           const int kk = i & 7, term = 2 - (i >> 3);
-          umma(tmem + (term ? COL_L : COL_U + DV * (kk >> 2)), bt + kk * k16, td + ((term * HALF) >> 4) + kk * k16, ID_UPDATE, term ? i > 0 : (kk & 3) != 0);
+          umma(tmem + (term ? COL_L : (kk < 4 ? COL_U : COL_R) + DV * ((kk >> 1) & 1)), bt + kk * k16, td + ((term * HALF) >> 4) + kk * k16, ID_UPDATE,
+               term ? i > 0 : (kk & 1) != 0);
         }
         umma_commit(update_done);
         // C S: the state's terms take the place of the scaled x's
@@ -437,7 +468,7 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
     float* const og = p.out + (size_t)q_begin * p.out_stride + (size_t)h * p.dv + c0;
     const float* const raw = p.raw + ((size_t)q_begin * p.G + h / (p.H / p.G)) * TOKENS + r;
     auto put_row = [&](float (&v)[16], auto more) {  // the thread's 16 numbers of row r, in three tiles
-      put_terms(v, 1.f, [&](int term, const uint32_t(&w)[8]) {
+      put_terms(v, 0.f, [&](int term, const uint32_t(&w)[8]) {
         put4(terms + term * HALF + sw128(r, 2 * q4), w);
         put4(terms + term * HALF + sw128(r, 2 * q4 + 1), w + 4);
       }, more);
@@ -511,17 +542,17 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
           v[j + 3] *= al * b4.w;
         }
       } else if (q4 == blk) {
-        const float gh = f.gh[r], gl = f.gl[r];
+        const uint64_t gh = pack2(f.gh[r], f.gh[r]), gl = pack2(f.gl[r], f.gl[r]), minus = pack2(-1.f, -1.f);
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const float4 h4 = *reinterpret_cast<const float4*>(f.gh + 32 * q4 + j), l4 = *reinterpret_cast<const float4*>(f.gl + 32 * q4 + j),
-                       d4 = *reinterpret_cast<const float4*>(f.d + 32 * q4 + j);
-          const float e0 = ex2((gh - h4.x) + (gl - l4.x)) * d4.x, e1 = ex2((gh - h4.y) + (gl - l4.y)) * d4.y;
-          const float e2 = ex2((gh - h4.z) + (gl - l4.z)) * d4.z, e3 = ex2((gh - h4.w) + (gl - l4.w)) * d4.w;
-          v[j] = j <= lane ? v[j] * e0 : 0.f;
-          v[j + 1] = j + 1 <= lane ? v[j + 1] * e1 : 0.f;
-          v[j + 2] = j + 2 <= lane ? v[j + 2] * e2 : 0.f;
-          v[j + 3] = j + 3 <= lane ? v[j + 3] * e3 : 0.f;
+        for (int j = 0; j < 32; j += 2) {
+          const uint64_t h2 = *reinterpret_cast<const uint64_t*>(f.gh + 32 * q4 + j), l2 = *reinterpret_cast<const uint64_t*>(f.gl + 32 * q4 + j);
+          const float2 d2 = *reinterpret_cast<const float2*>(f.d + 32 * q4 + j);
+          const uint64_t x = fma2(h2, minus, gh);  // what rounding takes from the difference goes to its low part (sums only fall)
+          const uint64_t rest = fma2(add2(h2, fma2(gh, minus, x)), minus, fma2(l2, minus, gl));
+          float e0, e1;
+          exp2_pair(x, rest, e0, e1);
+          v[j] = j <= lane ? v[j] * (e0 * d2.x) : 0.f;
+          v[j + 1] = j + 1 <= lane ? v[j + 1] * (e1 * d2.y) : 0.f;
         }
       }  // (the others are zeros)
     };
@@ -544,15 +575,27 @@ static __global__ void __launch_bounds__(THREADS, 1) chunks_kernel(const __grid_
         for (int j = 0; j < 16; ++j) y[j] = S[j];
         put_row(y, [](int) { return 0.f; });
         const float keep = f.keep;
-        sums(COL_U, b, [&](int j, float x) { S[j] = fmaf(keep, S[j], x); });
+        ld16(mine + COL_U + 16 * q4, b);
+        wait16(b);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) S[j] = with(b[j], S[j]);
+        for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(b[j]);
+#pragma unroll
+        for (uint32_t col : {COL_U + DV, COL_R, COL_R + DV}) {
+          ld16(mine + col + 16 * q4, b);
+          wait16(b);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) y[j] += __uint_as_float(b[j]);
+        }
+        ld16(mine + COL_L + 16 * q4, b);
+        wait16(b);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) S[j] = fmaf(keep, S[j], y[j] + fmaf(y[j], CUT_U, __uint_as_float(b[j])));
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         warp_arrive(s_ready);  // (C S's low terms lie where the update's did)
       }
       // ---- the weights, under C S (the products with those of the chunk before are over)
       weigh(f, v);
-      put_terms(v, 1.f - 0x1p-24f, [&](int term, const uint32_t(&w)[16]) { st16(mine + COL_P + 64 * term + 16 * q4, w); }, [](int) { return 0.f; });
+      put_terms(v, CUT_P, [&](int term, const uint32_t(&w)[16]) { st16(mine + COL_P + 64 * term + 16 * q4, w); }, [](int) { return 0.f; });
       tmem_wait_st();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       warp_arrive(p_ready);

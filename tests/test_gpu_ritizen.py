@@ -556,6 +556,46 @@ def test_state_space_chunks_keep_odd_values_from_the_tokens_before(heads, groups
         assert torch.equal(state, after)
 
 
+@pytest.mark.parametrize("kind,rate,slack", [("silu", 0.0, 1.03), ("silu", -2.0, 1.0), ("silu", -6.0, 1.0), ("normal", 0.0, 1.03), ("normal", -6.0, 1.0), ("positive", 0.0, 1.2), ("positive", -6.0, 1.0)])
+def test_state_space_chunks_are_no_further_off(kind, rate, slack):
+    """Against 64 bits, the tensor-core form, the FP32 form (which rows off 16-byte boundaries take) and the walk token by token: outputs
+    and states of two sequences, four seeds.  Sums made in tensor memory are cut: the state has a few per cent of slack where nothing but
+    the last tokens counts, a fifth where all its terms are positive besides."""
+    from kvforge_b200 import ops
+
+    heads, dk, dv, lens, dev = 16, 128, 64, [384, 200], "cuda"
+    n, inner = sum(lens), heads * dv
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+    sums = {form: torch.zeros(2, dtype=torch.float64) for form in ("tensor", "pipes", "walk")}
+    for seed in range(4):
+        g = torch.Generator(device=dev).manual_seed(seed)
+        r = lambda *s: torch.randn(*s, generator=g, device=dev)  # noqa: E731
+        x = r(n, inner + 2 * dk)
+        x = (torch.nn.functional.silu(x) if kind == "silu" else x.abs() if kind == "positive" else x).bfloat16()
+        dt, bias, a_log = r(n, heads).bfloat16(), 0.5 * r(heads), rate + 0.5 * r(heads)
+        step = torch.nn.functional.softplus(dt.double() + bias.double(), threshold=200.0)
+        decay = torch.exp(-torch.exp(a_log.double()) * step)
+        v, k, q = x[:, :inner].double().view(n, heads, dv) * step[:, :, None], x[:, inner : inner + dk].double(), x[:, inner + dk :].double()
+        want, last, at = torch.empty(n, heads, dv, dtype=torch.float64, device=dev), [], 0
+        for m in lens:
+            s = torch.zeros(heads, dk, dv, dtype=torch.float64, device=dev)
+            for t in range(at, at + m):
+                s = s * decay[t][:, None, None] + k[t][None, :, None] * v[t][:, None]
+                want[t] = torch.einsum("n,hnv->hv", q[t], s)
+            last.append(s)
+            at += m
+        want, last = want.view(n, inner), torch.stack(last).view(2, -1)
+        for form in sums:
+            rows = torch.zeros(n, x.shape[1] + 4, dtype=x.dtype, device=dev)[:, : x.shape[1]] if form == "pipes" else torch.empty_like(x)
+            rows.copy_(x)
+            out, state = torch.empty(n, inner, device=dev), torch.zeros(2, heads * dk * dv, device=dev)
+            raw = None if form == "walk" else torch.empty(n, ops.CHUNK_TOKENS, device=dev)
+            ops.state_space(rows, dt, bias, a_log, state, out, i32([0, lens[0], n]), i32([0, 1]), 2, heads, 1, dk, dv, max_query_len=max(lens), raw=raw)
+            sums[form] += torch.stack([(out - want).norm() / want.norm(), (state - last).norm() / last.norm()]).cpu() / 4
+    best = torch.minimum(sums["pipes"], sums["walk"])
+    assert float(sums["tensor"][0]) <= float(best[0]) and float(sums["tensor"][1]) <= slack * float(best[1]), sums
+
+
 @pytest.mark.parametrize("per_token", [False, True])
 @pytest.mark.parametrize("heads,groups,dk,dv", [(4, 4, 16, 24), (6, 2, 20, 12), (3, 1, 4, 4), (2, 2, 128, 100), (8, 1, 128, 64), (5, 5, 100, 36), (40, 2, 64, 128)])
 def test_recurrences_chunk_by_chunk(per_token, heads, groups, dk, dv):
