@@ -53,7 +53,9 @@ __device__ __forceinline__ void load_floats(const float* p, float* f) {
 // fused multiply-adds over the taps, oldest first, whichever form runs.
 constexpr int CONV_ROWS = 4;  // rows of a tile when a step has many
 // Rows of a tile when its sequences are long too: the weights, as many bytes as four rows of inputs and outputs, are then read once for
-// sixteen.  2,048 tokens of one sequence, 6,144 channels and four taps: 23.8 us with tiles of four rows, 14.5 with these (50 MB).
+// sixteen.  2,048 tokens of one sequence, 6,144 channels and four taps: 22.5 us with tiles of four rows, 16.1 with these (50 MB).  Such
+// tiles begin with their sequences: one that lay in two did its rows one by one (31 sequences of 66 tokens: 30.8 with such tiles, 27.8
+// in fours; these 18.6 and 28.0).
 constexpr int CONV_LONG = 16;
 
 template <typename T, int VEC, int TAPS>
@@ -118,60 +120,6 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ 
       return;
     }
   }
-  if constexpr (TAPS > 0 && VEC * sizeof(T) == 16) {
-    if (rows == CONV_LONG) {
-      const int n0 = blockIdx.x * CONV_LONG;
-      const int b0 = n0 < N ? seq_of_row(qsl, B, n0) : -1;
-      if (b0 < 0) return;
-      const int first = qsl[b0], end = qsl[b0 + 1];
-      if (n0 + CONV_LONG <= end && n0 + CONV_LONG <= N) {
-        // four rows at a time, the next four on their way (as they are stored: a conversion would wait for them)
-        const T* const src = x + (size_t)n0 * x_stride + c;
-        uint4 ahead[CONV_ROWS];
-        auto ask = [&](int r0) {
-#pragma unroll
-          for (int i = 0; i < CONV_ROWS; ++i) ahead[i] = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + i) * x_stride);
-        };
-        ask(0);
-        const int slot = state_slots[b0];
-        const float* st = slot >= 0 ? state + (size_t)slot * state_stride : nullptr;
-        float u[TAPS - 1 + CONV_ROWS][VEC];  // the inputs before these rows, then theirs
-#pragma unroll
-        for (int i = 0; i < TAPS - 1; ++i) {
-          const int t = n0 - first - (TAPS - 1) + i;
-          if (t >= 0) {
-            VecIO<T, VEC>::load(x + (size_t)(first + t) * x_stride + c, u[i]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) u[i][e] = st ? st[(size_t)(TAPS - 1 + t) * C + c + e] : 0.f;
-          }
-        }
-#pragma unroll
-        for (int r0 = 0; r0 < CONV_LONG; r0 += CONV_ROWS) {
-#pragma unroll
-          for (int i = 0; i < CONV_ROWS; ++i) VecIO<T, VEC>::load(reinterpret_cast<const T*>(&ahead[i]), u[TAPS - 1 + i]);
-          if (r0 + CONV_ROWS < CONV_LONG) ask(r0 + CONV_ROWS);
-#pragma unroll
-          for (int rr = 0; rr < CONV_ROWS; ++rr) {
-            float acc[VEC];
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-              acc[e] = cb[e];
-#pragma unroll
-              for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wr[e][j], u[rr + j][e], acc[e]);
-              if (act == 1) acc[e] = silu_of<T>(acc[e]);
-            }
-            VecIO<T, VEC>::store(out + (size_t)(n0 + r0 + rr) * out_stride + c, acc);
-          }
-#pragma unroll
-          for (int i = 0; i < TAPS - 1; ++i)
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) u[i][e] = u[i + CONV_ROWS][e];
-        }
-        return;
-      }
-    }
-  }
   for (int rr = 0; rr < rows; ++rr) {
     const int n = blockIdx.x * rows + rr;
     if (n >= N) return;
@@ -203,6 +151,81 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ 
       for (int e = 0; e < VEC; ++e) acc[e] = silu_of<T>(acc[e]);
     }
     VecIO<T, VEC>::store(out + (size_t)n * out_stride + c, acc);
+  }
+}
+
+// Tiles of CONV_LONG rows, which begin with their sequences; a sequence has at most rows / 16 + 1 of them.
+template <typename T, int VEC, int TAPS>
+__global__ void __launch_bounds__(128) causal_conv_long_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w,
+                                                               const float* __restrict__ bias, const float* __restrict__ state,
+                                                               long long state_stride, const int* __restrict__ qsl,
+                                                               const int* __restrict__ state_slots, int N, int B, int C, int act,
+                                                               T* __restrict__ out, int out_stride) {
+  pdl_launch();
+  pdl_wait();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+  if (c >= C) return;
+  float cb[VEC], wr[VEC][TAPS];
+  load_floats<VEC>(bias ? bias + c : nullptr, cb);
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j) {
+    float t[VEC];
+    load_floats<VEC>(w + (size_t)j * C + c, t);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) wr[e][j] = t[e];
+  }
+  const int tile = blockIdx.x;
+  int b = 0, hi = B - 1;  // the last sequence whose tiles begin at or before this one
+  while (b < hi) {
+    const int mid = (b + hi + 1) >> 1;
+    if (qsl[mid] / CONV_LONG + mid <= tile) b = mid; else hi = mid - 1;
+  }
+  const int first = qsl[b], end = min(qsl[b + 1], N), n0 = first + (tile - (first / CONV_LONG + b)) * CONV_LONG;
+  if (n0 >= end) return;
+  // four rows at a time, the next four on their way (as they are stored: a conversion would wait for them)
+  const T* const src = x + (size_t)n0 * x_stride + c;
+  uint4 ahead[CONV_ROWS];
+  auto ask = [&](int r0) {
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i)
+      ahead[i] = n0 + r0 + i < end ? *reinterpret_cast<const uint4*>(src + (size_t)(r0 + i) * x_stride) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  ask(0);
+  const int slot = state_slots[b];
+  const float* st = slot >= 0 ? state + (size_t)slot * state_stride : nullptr;
+  float u[TAPS - 1 + CONV_ROWS][VEC];  // the inputs before these rows, then theirs
+#pragma unroll
+  for (int i = 0; i < TAPS - 1; ++i) {
+    const int t = n0 - first - (TAPS - 1) + i;
+    if (t >= 0) {
+      VecIO<T, VEC>::load(x + (size_t)(first + t) * x_stride + c, u[i]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) u[i][e] = st ? st[(size_t)(TAPS - 1 + t) * C + c + e] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int r0 = 0; r0 < CONV_LONG; r0 += CONV_ROWS) {
+    if (n0 + r0 >= end) return;
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i) VecIO<T, VEC>::load(reinterpret_cast<const T*>(&ahead[i]), u[TAPS - 1 + i]);
+    if (r0 + CONV_ROWS < CONV_LONG) ask(r0 + CONV_ROWS);
+#pragma unroll
+    for (int rr = 0; rr < CONV_ROWS; ++rr) {
+      float acc[VEC];
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        acc[e] = cb[e];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wr[e][j], u[rr + j][e], acc[e]);
+        if (act == 1) acc[e] = silu_of<T>(acc[e]);
+      }
+      if (n0 + r0 + rr < end) VecIO<T, VEC>::store(out + (size_t)(n0 + r0 + rr) * out_stride + c, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < TAPS - 1; ++i)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) u[i][e] = u[i + CONV_ROWS][e];
   }
 }
 
@@ -286,10 +309,19 @@ int launch_conv_few(const T* x, int x_stride, const float* w, const float* bias,
 template <typename T, int VEC>
 int launch_conv(const T* x, int x_stride, const float* w, const float* bias, const float* state, long long state_stride, const int* qsl,
                 const int* state_slots, int N, int B, int C, int taps, int act, T* out, int out_stride, cudaStream_t st) {
-  const int rows = N < 1024 ? 1 : taps <= 4 && VEC * sizeof(T) == 16 && N >= 64 * (long long)B ? CONV_LONG : CONV_ROWS;
-  const int per_cta = 128 * VEC;
-  dim3 grid((N + rows - 1) / rows, (C + per_cta - 1) / per_cta);
-  if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
+  const int per_cta = 128 * VEC, columns = (C + per_cta - 1) / per_cta;
+  const int rows = N < 1024 ? 1 : CONV_ROWS;
+  if (columns > 65535) return (int)cudaErrorInvalidValue;
+  if constexpr (VEC * sizeof(T) == 16) {
+    // tiles of sixteen rows where every SM has one: 2,048 channels, tiles of four and of sixteen, us: 1,024 tokens 7.0 and 8.1, 2,048
+    // tokens 10.2 and 8.8, 32 sequences of 64 11.4 and 10.7; 3,072 channels, 1,024 tokens 9.2 and 8.6
+    if (N >= 1024 && taps >= 2 && taps <= 4 && N >= 64 * (long long)B && (long long)(N / CONV_LONG) * columns >= 148) {
+      const dim3 tiles(N / CONV_LONG + B, columns);
+      auto kernel = taps == 2 ? causal_conv_long_kernel<T, VEC, 2> : taps == 3 ? causal_conv_long_kernel<T, VEC, 3> : causal_conv_long_kernel<T, VEC, 4>;
+      return launch(kernel, tiles, dim3(128), (size_t)0, st, x, x_stride, w, bias, state, state_stride, qsl, state_slots, N, B, C, act, out, out_stride);
+    }
+  }
+  dim3 grid((N + rows - 1) / rows, columns);
 #define KVF_CONV_CASE(TP)                                                                                             \
   launch(causal_conv_kernel<T, VEC, TP>, dim3(grid), dim3(128), (size_t)(0), st, x, x_stride, w, bias, state, state_stride, qsl, state_slots, N, B, C, \
                                                         taps, act, out, out_stride, rows)

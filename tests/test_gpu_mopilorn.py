@@ -390,19 +390,19 @@ def test_gated_delta_rule_through_the_state(dtype, h, g, dk, dv, channel):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("taps,lens", [(4, [1024]), (3, [700, 1, 333]), (2, [15, 1010]), (4, [17, 1007, 3, 40])])
+@pytest.mark.parametrize("taps,lens", [(4, [1024]), (3, [700, 1, 333]), (2, [15, 1010]), (4, [17, 1007, 3, 40]), (1, [1030]), (4, [67, 70, 65, 66, 71, 129, 61, 58, 90, 70, 66, 90, 63, 70]), (3, [64] * 16), (2, [69] * 15)])
 def test_convolution_of_long_sequences_has_the_bits_of_short_steps(taps, lens, dtype):
     """Tiles of sixteen rows, and what lies across a sequence's border, against the same rows one step after another of fewer rows than
     such tiles take."""
     from kvforge_b200 import ops
 
-    dev, dt, c = "cuda", DT[dtype], 48
+    dev, dt, c = "cuda", DT[dtype], 2056  # so many that sixteen rows a tile still give every SM one
     gen = torch.Generator().manual_seed(taps)
     x, w, bias = torch.randn(sum(lens), c, generator=gen).to(dev, dt), torch.randn(taps, c, generator=gen).to(dev), torch.randn(c, generator=gen).to(dev)
     slots = list(range(len(lens)))
     start = torch.randn(len(lens), (taps - 1) * c, generator=gen).to(dev)
     results = []
-    for step in (max(lens), 300):
+    for step in (max(lens), min(300, max(lens) // 3)):
         state, out = start.clone(), torch.empty_like(x)
         for a in range(0, max(lens), step):
             part = [max(0, min(m, a + step) - a) for m in lens]
