@@ -549,7 +549,7 @@ KVF_API int kvf_gated_set_pdl(int enabled) {
     if (n_tokens <= 0) return 0;                                                                                      \
     if (d <= 0 || d > 32 * PREP_EPL || dv <= 0 || dv > v_step || rot < 0 || rot > d || (rot & 1) || nh < 0 || nkv < 0) \
       return (int)cudaErrorInvalidValue;                                                                              \
-    if (sizeof(T) == 2 && n_tokens >= HEAD_VEC_TOKENS && head_vec_ok(d, rot, true) && dv % 8 == 0 && row_stride % 8 == 0 && \
+    if (sizeof(T) == 2 && n_tokens >= HEAD_VEC_PREPARE && head_vec_ok(d, rot, true) && dv % 8 == 0 && row_stride % 8 == 0 && \
         k_off % 8 == 0 && v_off % 8 == 0 && v_step % 8 == 0 && aligned16({x, kcache, vcache}))                        \
       return launch(qk_prepare_vec_kernel, dim3(n_tokens), dim3(HEAD_VEC_THREADS), (size_t)rot * sizeof(float), st,   \
                     (bf16*)x, row_stride, k_off, v_off, v_step, positions, inv_freq, rot, norm, eps, slots,           \

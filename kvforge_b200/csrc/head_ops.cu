@@ -377,7 +377,7 @@ inline unsigned grid_for(long long total, int threads) {
     if ((v_first && !v_lambda) || count <= 0 || count > dk) return (int)cudaErrorInvalidValue;                       \
     if ((row_stride & 1) || ((((uintptr_t)qkv) | ((uintptr_t)kcache)) & (2 * sizeof(T) - 1)))                       \
       return (int)cudaErrorInvalidValue;                                                                             \
-    if (sizeof(T) == 2 && n_tokens >= HEAD_VEC_TOKENS && head_vec_ok(dk, rot, split_pairs != 0) && dv % 8 == 0 &&    \
+    if (sizeof(T) == 2 && n_tokens >= HEAD_VEC_NORM && head_vec_ok(dk, rot, split_pairs != 0) && dv % 8 == 0 &&    \
         row_stride % 8 == 0 && aligned16({qkv, kcache, vcache, v_keep, v_first}))                                    \
       return launch(head_norm_vec_kernel, dim3(n_tokens), dim3(HEAD_VEC_THREADS), (size_t)rot * sizeof(float), st,   \
                     (bf16*)qkv, row_stride, positions, q_w, k_w, eps, inv_freq, rot, split_pairs, slots,             \

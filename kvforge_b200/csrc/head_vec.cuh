@@ -8,9 +8,13 @@
 namespace kvf {
 
 constexpr int HEAD_VEC_THREADS = 128;
-// Steps of fewer tokens stay with a warp a head: a CTA a token leaves too few warps in flight then (8 tokens, 40 heads of 64: 13.6 us
-// against 20.0).
-constexpr int HEAD_VEC_TOKENS = 128;
+// Steps of fewer tokens stay with a warp a head: a CTA a token leaves too few warps in flight there.  A warp a head and this form, us:
+//   rotation and head norm (qk_prepare)  32 query heads on 8 of 64: 128 tokens 4.0 and 4.6, 192 5.6 and 4.7, 256 6.3 and 4.7, 2,048 33 and 11
+//                                        24 on 8 of 128: 128 4.6 and 5.4, 192 5.5 and 5.7, 256 7.3 and 5.7, 2,048 35 and 15
+//   head norm with rotation and cache write  32 on 8 of 64: 128 3.9 and 5.0, 256 5.8 and 5.2, 384 7.1 and 5.4, 2,048 21 and 12
+//                                        24 on 8 of 128: 128 4.0 and 6.0, 256 5.9 and 6.4, 384 7.8 and 7.0, 2,048 22 and 18
+//                                        8 on 2 of 128: 256 3.7 and 4.4, 384 4.5 and 4.6, 512 4.8 and 4.9, 1,024 7.8 and 5.8
+constexpr int HEAD_VEC_PREPARE = 256, HEAD_VEC_NORM = 384;
 
 __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
   uint4 u;

@@ -313,18 +313,18 @@ def test_heads_of_many_tokens_as_of_few(nh, nkv, d, dv, rot, norm):
     and one beyond the pool among them."""
     from kvforge_b200 import ops
 
-    n, bs = 170, 16
+    n, bs = 430, 16
     g = torch.Generator().manual_seed(d + rot)
     wide = nh * d + nkv * d + 8
     x = torch.randn(n, wide, generator=g).bfloat16().cuda()
     pos = torch.randint(0, 5000, (n,), generator=g, dtype=torch.int32).cuda()
     inv = (10000.0 ** (-torch.arange(rot // 2) / max(1, rot // 2))).float().cuda()
-    slots = torch.randperm(12 * bs, generator=g)[:n].int()
-    slots[7], slots[100] = -1, 12 * bs
+    slots = torch.randperm(30 * bs, generator=g)[:n].int()
+    slots[7], slots[100] = -1, 30 * bs
     slots = slots.cuda()
     results = []
     for cut in (n, 100):  # one step, or steps too small for it
-        y, k, v = x.clone(), torch.zeros(12, nkv, bs, d, dtype=torch.bfloat16, device="cuda"), torch.zeros(12, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
+        y, k, v = x.clone(), torch.zeros(30, nkv, bs, d, dtype=torch.bfloat16, device="cuda"), torch.zeros(30, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
         err = torch.zeros(1, dtype=torch.int32, device="cuda")
         for a in range(0, n, cut):
             r = slice(a, min(n, a + cut))

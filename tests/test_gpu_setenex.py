@@ -417,7 +417,7 @@ def test_normed_heads_of_many_tokens_as_of_few(nh, nkv, dk, dv, rot, weights, mi
     and one beyond the pool among them."""
     from kvforge_b200 import ops
 
-    n, bs = 170, 16
+    n, bs = 430, 16
     g = torch.Generator().manual_seed(dk + rot)
     r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
     x = r(n, (nh + nkv) * dk + nkv * dv).bfloat16()
@@ -425,12 +425,12 @@ def test_normed_heads_of_many_tokens_as_of_few(nh, nkv, dk, dv, rot, weights, mi
     inv = (10000.0 ** (-torch.arange(rot // 2) / max(1, rot // 2))).float().cuda() if rot else None
     q_w, k_w = (1 + 0.1 * r(dk), 1 + 0.1 * r(dk)) if weights else (None, None)
     first, lam = (r(n, nkv * dv).bfloat16(), torch.full((1,), 0.3, device="cuda")) if mixed else (None, None)
-    slots = torch.randperm(12 * bs, generator=g)[:n].int()
-    slots[7], slots[100] = -1, 12 * bs
+    slots = torch.randperm(30 * bs, generator=g)[:n].int()
+    slots[7], slots[100] = -1, 30 * bs
     slots = slots.cuda()
     results = []
     for cut in (n, 100):  # one step, or steps too small for it
-        y, k, v = x.clone(), torch.zeros(12, nkv, bs, dk, dtype=torch.bfloat16, device="cuda"), torch.zeros(12, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
+        y, k, v = x.clone(), torch.zeros(30, nkv, bs, dk, dtype=torch.bfloat16, device="cuda"), torch.zeros(30, nkv, bs, dv, dtype=torch.bfloat16, device="cuda")
         keep, err = torch.zeros(n, nkv * dv, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
         for a in range(0, n, cut):
             rows = slice(a, min(n, a + cut))
