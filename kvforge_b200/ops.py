@@ -1336,14 +1336,17 @@ DELTA_CHUNK_TOKENS = 64
 DELTA_CHUNK_MEAN = 96  # tokens a sequence that a step in chunks has at least, on the average
 
 
-def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, per_channel: bool, n: int, num_seqs: int, max_query_len: int) -> bool:
+def delta_chunks_ok(dtype: torch.dtype, dk: int, dv: int, num_heads: int, per_channel: bool, n: int, num_seqs: int, max_query_len: int) -> bool:
     """Whether a step of the delta rule goes sixty-four tokens at a time rather than four.  A chunk costs about the same however
-    few of its tokens there are, so the step needs long sequences and few short ones beside them.  Groups of four and chunks, us,
-    16 heads of 128 x 128 with a decay a channel: one sequence of 256 tokens 71 and 68, of 512 133 and 84, of 2,048 525 and 269; 8 of
-    256 386 and 282; 1,000 and 8 single tokens 373 and 301, 400 and 20 219 and 323; 30 of 64 307 and 362.  8 heads with a decay a head:
-    one of 256 55 and 69, of 384 75 and 75, of 1,024 181 and 108."""
-    few = 256 if per_channel else 384
-    return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= 384 and n >= DELTA_CHUNK_MEAN * num_seqs
+    few of its tokens there are, so the step needs long sequences and few short ones beside them, the fewer the more heads fill the SMs.
+    Groups of four and chunks, us, heads of 128 x 128, a decay a channel (a head): one sequence of 256 tokens with 8 heads 53 and 61 (50
+    and 61), 16 heads 68 and 61 (63 and 61), 32 heads 108 and 79 (87 and 79); of 384 with 4 heads 73 and 67 (71 and 67); of 2,048 with 16
+    heads 523 and 263 (444 and 266); two of 256 with 4 heads 53 and 61, 8 heads 68 and 66 (62 and 66), 16 heads 109 and 80 (87 and 80); 500
+    and 3 single tokens with 16 heads 188 and 127 (151 and 125), 32 heads 213 and 241 (173 and 251); 1,000 and 8 single tokens with 24
+    heads 407 and 345 (324 and 347)."""
+    few = 256 if num_heads * n >= 4096 and (per_channel or num_heads >= 16) else 384
+    mean = max(DELTA_CHUNK_MEAN, (4 if per_channel else 5) * num_heads)
+    return dtype == torch.bfloat16 and 64 < dk <= 128 and dv % 4 == 0 and max_query_len >= few and n >= mean * num_seqs
 
 
 def delta_chunk_record(num_heads: int, dv: int) -> int:

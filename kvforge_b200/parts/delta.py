@@ -194,7 +194,7 @@ class GatedDeltaRule(Mixer):
         read = rt.buf("delta.read", n, self.c_v, torch.float32)
         f32 = torch.float32
         scratch = groups = chunks = None
-        if ops.delta_chunks_ok(rt.dtype, dk, dv, self.decay == "channel", n, ctx.num_seqs, ctx.max_query_len):
+        if ops.delta_chunks_ok(rt.dtype, dk, dv, H, self.decay == "channel", n, ctx.num_seqs, ctx.max_query_len):
             # many tokens a sequence in bfloat16: sixty-four at a time, from records of the chunks
             chunks = self._chunks(n, ctx.num_seqs)
         elif ops.delta_groups_ok(rt.dtype, dk, ctx.max_query_len):

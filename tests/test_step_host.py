@@ -278,12 +278,28 @@ def test_buffer_of_the_delta_rule_s_chunks_follows_the_rule_and_not_the_request_
                 widest = 0
                 for n in range(1, budget + 1):
                     for seqs in range(1, slots + 1):
-                        if ops.delta_chunks_ok(torch.bfloat16, part.dk, part.dv, part.decay == "channel", n, seqs, n):
+                        if ops.delta_chunks_ok(torch.bfloat16, part.dk, part.dv, part.H, part.decay == "channel", n, seqs, n):
                             if n in (384, 1000, budget):
                                 part._chunks(n, seqs)
                                 assert asked[-1][0] <= asked[-1][2] and asked[-1][0] * asked[-1][1] == ops.delta_chunk_floats(n, seqs, part.H, part.dv)
                             widest = max(widest, n // ops.DELTA_CHUNK_TOKENS + seqs)
                 assert widest <= asked[-1][2] <= budget // 64 + budget // 96  # no record that no step can use, whatever the slots
+
+
+def test_steps_that_go_in_chunks_are_those_measured_faster():
+    """Groups of four against chunks of sixty-four, heads of 128 x 128: (heads, a decay a channel, lengths, chunks are faster)."""
+    import torch
+
+    from kvforge_b200 import ops
+
+    for heads, channel, lens, faster in (
+        (4, True, [256] * 2, False), (8, True, [256], False), (8, True, [256] * 2, True), (16, True, [256], True), (32, True, [256], True), (4, True, [384], True),
+        (16, True, [1000] + [1] * 8, True), (16, True, [400] + [1] * 20, False), (32, True, [500] + [1] * 3, False), (24, True, [500] + [1] * 3, True), (16, True, [64] * 30, False),
+        (8, False, [256], False), (8, False, [256] * 2, False), (16, False, [256] * 2, True), (32, False, [256], True), (4, False, [384], True), (8, False, [64] * 30, False),
+        (24, False, [1000] + [1] * 8, False), (32, False, [500] + [1] * 3, False), (16, False, [700] + [100] * 6, True), (24, False, [500] * 4, True),
+    ):  # fmt: skip
+        assert ops.delta_chunks_ok(torch.bfloat16, 128, 128, heads, channel, sum(lens), len(lens), max(lens)) == faster, (heads, channel, lens)
+    assert not ops.delta_chunks_ok(torch.float32, 128, 128, 16, True, 2048, 1, 2048) and not ops.delta_chunks_ok(torch.bfloat16, 64, 128, 16, True, 2048, 1, 2048)
 
 
 def test_shaped_scores_keep_the_ranges_of_the_launch(monkeypatch):
