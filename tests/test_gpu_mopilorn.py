@@ -476,7 +476,7 @@ def test_gated_delta_rule_in_groups_of_four(h, g, dk, dv, channel, rate):
 
 
 @pytest.mark.parametrize("rate", [-4.0, 0.0, 3.0])
-@pytest.mark.parametrize("h,g,dk,dv,channel", [(2, 2, 128, 128, True), (2, 1, 128, 32, False), (3, 1, 65, 36, True), (2, 1, 100, 4, False), (1, 1, 96, 260, True)])
+@pytest.mark.parametrize("h,g,dk,dv,channel", [(2, 2, 128, 128, True), (2, 1, 128, 32, False), (3, 1, 65, 36, True), (2, 1, 100, 4, False), (1, 1, 96, 260, True), (4, 2, 128, 128, False), (3, 3, 96, 132, True)])
 def test_gated_delta_rule_in_chunks(h, g, dk, dv, channel, rate):
     """The form that takes sixty-four tokens at a time: chunks of 1, 15 .. 17, 63 and 64 tokens, every block boundary, both widths of
     the chain's tiles, sequences of one token and of none, a padding sequence without a slot, two steps of which the second finds a
@@ -487,6 +487,7 @@ def test_gated_delta_rule_in_chunks(h, g, dk, dv, channel, rate):
     gen = torch.Generator().manual_seed(dk + dv)
     steps = ([65, 1, 0, 17, 64], [15, 130, 0, 63, 16])
     slots = [2, 5, 1, 0, 4]
+    assert (6 * h * -(-dv // 16) > 148) == ((h, dv) in ((4, 128), (3, 132)))  # tiles of 32 columns where there are more of 16 than SMs
     aw = h * dk if channel else h
     a_log, dt_bias = rate + 0.5 * torch.randn(h, generator=gen), 0.5 * torch.randn(aw, generator=gen)
     state = torch.zeros(6, 4 + h * dk * dv, device=dev)
@@ -726,6 +727,89 @@ def test_gated_delta_rule_in_groups_is_no_further_off(h, dk, dv, channel):
         )  # fmt: skip
         errors.append((float((out.cpu().double() - want).norm() / want.norm()), float((state.cpu().double().reshape(-1) - last).norm() / last.norm())))
     assert errors[0][0] <= errors[1][0] and errors[0][1] <= 1.1 * errors[1][1], errors
+
+
+@pytest.mark.parametrize("rate", [-4.0, 0.0, 2.0])
+@pytest.mark.parametrize("h,dk,dv,channel", [(8, 128, 128, True), (8, 128, 64, False), (6, 100, 36, True)])
+def test_gated_delta_rule_in_chunks_is_no_further_off(h, dk, dv, channel, rate):
+    """Against 64 bits, sixty-four tokens at a time, four at a time and the walk: outputs and states of three sequences, three seeds.
+    Averages over heads and seeds vary by one or two per cent for outputs and by a few for states."""
+    from kvforge_b200 import ops
+
+    lens, dev, dt = [384, 200, 100], "cuda", torch.bfloat16
+    n, aw = sum(lens), h * dk if channel else h
+    qsl, sl = flat_batch(lens, [0, 1, 2], dev)
+    errors = {form: torch.zeros(2, dtype=torch.float64) for form in ("chunks", "groups", "walk")}
+    for seed in range(3):
+        gen = torch.Generator(device=dev).manual_seed(seed)
+        r = lambda *shape: torch.randn(*shape, generator=gen, device=dev)  # noqa: E731
+        qkv, b, a, a_log, dt_bias = r(n, 2 * h * dk + h * dv).to(dt), r(n, h), r(n, aw), rate + 0.5 * r(h), 0.5 * r(aw)
+        decay = torch.exp(-torch.exp(a_log.double()).repeat_interleave(dk if channel else 1) * F.softplus(a.double() + dt_bias.double(), threshold=200.0))
+        decay = decay.view(n, h, dk) if channel else decay[:, :, None].expand(n, h, dk)
+        q, k = (plain.unit(qkv[:, i * h * dk : (i + 1) * h * dk].double().view(n, h, dk)) for i in range(2))
+        v, beta = qkv[:, 2 * h * dk :].double().view(n, h, dv), torch.sigmoid(b.double())
+        want, last, at = torch.empty(n, h, dv, dtype=torch.float64, device=dev), [], 0
+        for m in lens:
+            s = torch.zeros(h, dk, dv, dtype=torch.float64, device=dev)
+            for t in range(at, at + m):
+                s = s * decay[t][:, :, None]
+                s = s + k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], s)))[:, None]
+                want[t] = torch.einsum("hd,hdv->hv", q[t] * dk**-0.5, s)
+            last.append(s.reshape(-1))
+            at += m
+        want, last = want.view(n, -1), torch.stack(last)
+        for form in errors:
+            state, out = torch.zeros(3, h * dk * dv, device=dev), torch.empty(n, h * dv, device=dev)
+            size = {"chunks": lambda: ops.delta_chunk_floats(n, 3, h, dv), "groups": lambda: ops.delta_group_floats(n, 3, h, channel)}.get(form)
+            extra = {form: torch.empty(size(), device=dev)} if size else {}
+            ops.gated_delta(
+                qkv[:, : h * dk], qkv[:, h * dk : 2 * h * dk], qkv[:, 2 * h * dk :], b, a, a_log, dt_bias, state, out, qsl, sl,
+                3, h, h, dk, dv, q_scale=dk**-0.5, max_query_len=max(lens), **extra,
+            )  # fmt: skip
+            errors[form] += torch.stack([(out - want).norm() / want.norm(), (state - last).norm() / last.norm()]).cpu() / 3
+    best = torch.minimum(errors["groups"], errors["walk"])
+    assert float(errors["chunks"][0]) <= 1.03 * float(best[0]) and float(errors["chunks"][1]) <= 1.1 * float(best[1]), errors
+
+
+def test_long_runs_go_in_chunks_eager_and_as_captured_graphs(tmp_path, monkeypatch):
+    """Whole models whose steps bring hundreds of tokens a sequence, heads of 64 < dk <= 128 in bfloat16: prompts, portions behind them
+    on the state that they left and single tokens after, run eagerly and as graphs, are the plain implementation's within rounding, and
+    the long steps do go sixty-four tokens at a time."""
+    from kvforge_b200 import ops
+    from mopilorn_cases import attention, delta, layer
+
+    config = {
+        "architecture": "Mopilorn", "vocab": 131, "width": 64, "norm": {"eps": 1e-6},
+        "layers": [
+            layer("channel_delta", delta(2, 1, 72, 16, 2), 80),
+            layer("parallel", {"left": attention(2, 2, 16, 16, 3, 40), "right": delta(2, 2, 128, 24, 3)}, 64),
+        ],
+    }  # fmt: skip
+    w = random_tensors(config, (4, 4), seed=32)
+    folder = write_folder(tmp_path / "long", config, w)
+    reqs = {f"r{i}": tokens(131, 806, 80 + i) for i in range(2)}
+    ref = {rid: plain_logits(config, w, t) for rid, t in reqs.items()}
+    scale = float(torch.cat(list(ref.values())).pow(2).mean().sqrt())
+    cuts, steps = [(400, 390), (400, 400)] + [(1, 1)] * 6 + [(0, 10)], []
+    at = dict.fromkeys(reqs, 0)
+    for cut in cuts:
+        entries, end = [], []
+        for rid, k in zip(reqs, cut):
+            if k:
+                entries.append({"id": rid, "tokens": reqs[rid][at[rid] : at[rid] + k], "want": [k - 1]})
+                at[rid] += k
+                if at[rid] == 806:
+                    end.append(rid)
+        steps.append({"step": len(steps), "entries": entries, "end": end})
+    assert set(at.values()) == {806}
+    took, real = [], ops.gated_delta
+    monkeypatch.setattr(ops, "gated_delta", lambda *a, **kw: (took.append((a[0].shape[0], kw.get("chunks") is not None)), real(*a, **kw))[1])
+    for graphs in (False, True):
+        took.clear()
+        outs, runner = run_trace(folder, "bfloat16", steps, 16, max_live=2, cuda_graphs=graphs)
+        check(steps, outs, ref, scale, TOL["bfloat16"])
+        assert {form for n, form in took if n >= 700} == {True} and not any(form for n, form in took if n < 384)
+        assert not graphs or any(key[0] >= 700 and not key[-1] for key in runner.core.runner._graphs)
 
 
 def test_short_runs_eager_and_as_captured_graphs(tmp_path):
