@@ -56,15 +56,6 @@ struct LatTcParams {
   float scale_log2;
 };
 
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t id, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate)
-      : "memory");
-}
-
 // The maximum of the thread's 64 raw scores, of those from `first` to `last` with MASK.
 template <bool MASK>
 __device__ __forceinline__ float row_max(const uint32_t (&va)[32], const uint32_t (&vb)[32], int first, int last) {

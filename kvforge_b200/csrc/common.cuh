@@ -46,8 +46,8 @@ inline size_t spread_smem(size_t need, long long ctas) {
 }
 
 // True in one lane of a converged warp.  A thread chosen so, and not by its lane's number, is known to the compiler to be alone: what
-// it hands to the tensor core and the copy engine (descriptors, addresses) then stays in uniform registers (eight tcgen05.mma of 128 x 96 x
-// 16 between two waits: 95 cycles each behind `lane == 0`, 67 behind this).
+// it hands to the tensor core and the copy engine (descriptors, addresses) then stays in uniform registers (the state space's chunks, 64
+// heads and 2,048 tokens: 118.4 us behind `lane == 0`, 114.6 behind this).
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(

@@ -79,14 +79,6 @@ struct Params {
 // A x B with A either K-major or (bit 15) M-major, B K-major or (bit 16) N-major
 constexpr uint32_t ID_OUT = idesc(DV, 1), ID_UPDATE = idesc(DV, 1) | (1u << 15);
 
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t id, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate)
-      : "memory");
-}
 // A whole warp waits (every lane sees the phase over itself: a shuffle of one lane's wait would hand on the answer, but not the order
 // of what was written before it), or arrives once.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* err) {

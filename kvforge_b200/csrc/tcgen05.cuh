@@ -93,6 +93,15 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, ui
       ::"r"(tmem_d), "l"(a), "l"(b), "r"(id), "r"(accumulate)
       : "memory");
 }
+// The same with A in tensor memory.
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t id, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate)
+      : "memory");
+}
 // The same with the accumulate flag known when compiling (no predicate to set up at run time).
 template <int ACC>
 __device__ __forceinline__ void umma_c(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id) {
