@@ -1,5 +1,7 @@
 // The short causal convolution over time per channel that mixers with a running state put between their projections
 // and the recurrence.
+#include <type_traits>
+
 #include "sequence_common.cuh"
 
 using namespace kvf;
@@ -53,9 +55,9 @@ __device__ __forceinline__ void load_floats(const float* p, float* f) {
 // fused multiply-adds over the taps, oldest first, whichever form runs.
 constexpr int CONV_ROWS = 4;  // rows of a tile when a step has many
 // Rows of a tile when its sequences are long too: the weights, as many bytes as four rows of inputs and outputs, are then read once for
-// sixteen.  2,048 tokens of one sequence, 6,144 channels and four taps: 22.5 us with tiles of four rows, 16.1 with these (50 MB).  Such
-// tiles begin with their sequences: one that lay in two did its rows one by one (31 sequences of 66 tokens: 30.8 with such tiles, 27.8
-// in fours; these 18.6 and 28.0).
+// sixteen.  2,048 tokens of one sequence, 6,144 channels and four taps: 22.5 us with tiles of four rows, 14.3 with these (50 MB).  Such
+// tiles begin with their sequences: one that lay in two did its rows one by one (31 sequences of 66 tokens: 30.7 with such tiles, 28.0 in
+// fours, 17.1 with these).
 constexpr int CONV_LONG = 16;
 
 template <typename T, int VEC, int TAPS>
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const T* __restrict__ 
 
 // Tiles of CONV_LONG rows, which begin with their sequences; a sequence has at most rows / 16 + 1 of them.
 template <typename T, int VEC, int TAPS>
-__global__ void __launch_bounds__(128) causal_conv_long_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w,
+__global__ void __launch_bounds__(128, 4) causal_conv_long_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w,
                                                                const float* __restrict__ bias, const float* __restrict__ state,
                                                                long long state_stride, const int* __restrict__ qsl,
                                                                const int* __restrict__ state_slots, int N, int B, int C, int act,
@@ -182,51 +184,58 @@ __global__ void __launch_bounds__(128) causal_conv_long_kernel(const T* __restri
   }
   const int first = qsl[b], end = min(qsl[b + 1], N), n0 = first + (tile - (first / CONV_LONG + b)) * CONV_LONG;
   if (n0 >= end) return;
-  // four rows at a time, the next four on their way (as they are stored: a conversion would wait for them)
-  const T* const src = x + (size_t)n0 * x_stride + c;
-  uint4 ahead[CONV_ROWS];
-  auto ask = [&](int r0) {
-#pragma unroll
-    for (int i = 0; i < CONV_ROWS; ++i)
-      ahead[i] = n0 + r0 + i < end ? *reinterpret_cast<const uint4*>(src + (size_t)(r0 + i) * x_stride) : make_uint4(0u, 0u, 0u, 0u);
-  };
-  ask(0);
   const int slot = state_slots[b];
   const float* st = slot >= 0 ? state + (size_t)slot * state_stride : nullptr;
-  float u[TAPS - 1 + CONV_ROWS][VEC];  // the inputs before these rows, then theirs
+  const T* const src = x + (size_t)n0 * x_stride + c;
+  // four rows at a time, the next four on their way (as they are stored: a conversion would wait for them)
+  auto rows = [&](auto whole) {
+    constexpr bool WHOLE = decltype(whole)::value;
+    uint4 ahead[CONV_ROWS];
+    auto ask = [&](int r0) {
 #pragma unroll
-  for (int i = 0; i < TAPS - 1; ++i) {
-    const int t = n0 - first - (TAPS - 1) + i;
-    if (t >= 0) {
-      VecIO<T, VEC>::load(x + (size_t)(first + t) * x_stride + c, u[i]);
-    } else {
+      for (int i = 0; i < CONV_ROWS; ++i)
+        ahead[i] = WHOLE || n0 + r0 + i < end ? *reinterpret_cast<const uint4*>(src + (size_t)(r0 + i) * x_stride) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    ask(0);
+    float u[TAPS - 1 + CONV_ROWS][VEC];  // the inputs before these rows, then theirs
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) u[i][e] = st ? st[(size_t)(TAPS - 1 + t) * C + c + e] : 0.f;
-    }
-  }
+    for (int i = 0; i < TAPS - 1; ++i) {
+      const int t = n0 - first - (TAPS - 1) + i;
+      if (t >= 0) {
+        VecIO<T, VEC>::load(x + (size_t)(first + t) * x_stride + c, u[i]);
+      } else {
 #pragma unroll
-  for (int r0 = 0; r0 < CONV_LONG; r0 += CONV_ROWS) {
-    if (n0 + r0 >= end) return;
-#pragma unroll
-    for (int i = 0; i < CONV_ROWS; ++i) VecIO<T, VEC>::load(reinterpret_cast<const T*>(&ahead[i]), u[TAPS - 1 + i]);
-    if (r0 + CONV_ROWS < CONV_LONG) ask(r0 + CONV_ROWS);
-#pragma unroll
-    for (int rr = 0; rr < CONV_ROWS; ++rr) {
-      float acc[VEC];
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) {
-        acc[e] = cb[e];
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wr[e][j], u[rr + j][e], acc[e]);
-        if (act == 1) acc[e] = silu_of<T>(acc[e]);
+        for (int e = 0; e < VEC; ++e) u[i][e] = st ? st[(size_t)(TAPS - 1 + t) * C + c + e] : 0.f;
       }
-      if (n0 + r0 + rr < end) VecIO<T, VEC>::store(out + (size_t)(n0 + r0 + rr) * out_stride + c, acc);
     }
+#pragma unroll(WHOLE ? CONV_LONG / CONV_ROWS : 1)
+    for (int r0 = 0; r0 < CONV_LONG; r0 += CONV_ROWS) {
+      if (!WHOLE && n0 + r0 >= end) return;
 #pragma unroll
-    for (int i = 0; i < TAPS - 1; ++i)
+      for (int i = 0; i < CONV_ROWS; ++i) VecIO<T, VEC>::load(reinterpret_cast<const T*>(&ahead[i]), u[TAPS - 1 + i]);
+      if (r0 + CONV_ROWS < CONV_LONG) ask(r0 + CONV_ROWS);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) u[i][e] = u[i + CONV_ROWS][e];
-  }
+      for (int rr = 0; rr < CONV_ROWS; ++rr) {
+        float acc[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          acc[e] = cb[e];
+#pragma unroll
+          for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wr[e][j], u[rr + j][e], acc[e]);
+          if (act == 1) acc[e] = silu_of<T>(acc[e]);
+        }
+        if (WHOLE || n0 + r0 + rr < end) VecIO<T, VEC>::store(out + (size_t)(n0 + r0 + rr) * out_stride + c, acc);
+      }
+#pragma unroll
+      for (int i = 0; i < TAPS - 1; ++i)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) u[i][e] = u[i + CONV_ROWS][e];
+    }
+  };
+  if (n0 + CONV_LONG <= end)
+    rows(std::true_type());
+  else
+    rows(std::false_type());
 }
 
 // Steps in which no sequence brings more than CONV_FEW rows (decoding): a thread owns VEC channels of ALL rows of
