@@ -24,7 +24,8 @@
 // shared memory and two barriers more, 3.3 us).
 // Against 64 bits the outputs are off by 1.10e-7 of their norm there (groups 1.16e-7, walk 1.28e-7), the states by 0.89e-7 (0.91e-7,
 // 0.96e-7); over three rates of decay and three seeds each outputs are 0.86 to 1.01 of the groups' error and at most the walk's.  That
-// takes sums of A and B ended in double, and beta x kept whole in the solve (without them 1.06).
+// takes sums of A and B inside a block ended in double (those between blocks end in float), and beta x kept whole in the solve (without
+// them 1.06).
 #pragma once
 
 namespace {

@@ -46,8 +46,9 @@ constexpr uint32_t STAGE = 5 * HALF;          // C (two halves), B (two halves),
 constexpr uint32_t COL_P = 0, COL_R = 192, COL_U = 320, COL_L = 448;  // weights, C S, the update and then the weights times x, low terms of C S and of the update
 // Tensor memory cuts what does not fit a float towards zero.  So much of a sum is given back, through its low terms: what C S (sums of four
 // products), the update (of two) and the weights times x (of four, whose low and high terms share a sum) lose on the average of x, B
-// and C of either sign and behind silu, a_log from -6 to 1 (0 and 2^-24 for the update: its state at 0 0.68 and 0.67; 0 and 2^-24 for the
-// weights: outputs 0.1 to 0.2 and 0.0 to 0.1 further off).  A sum whose terms are all positive loses up to 1.04e-7 of itself, others 0.65e-7.
+// and C of either sign and behind silu, a_log from -6 to 1.  With nothing given back to the update the state at 0 behind silu is off
+// by 0.68, with six fifths of its share by 0.67; with a third less of the weights' share outputs are up to 0.07 further off, with a
+// third more between 0.03 nearer and 0.03 further.  A sum whose terms are all positive loses up to 1.04e-7 of itself, others 0.65e-7.
 constexpr float CUT = 0x1.4p-25f, CUT_U = 0x1.4p-25f, CUT_P = 0x1.8p-25f;
 // what a chunk's logarithms become
 struct Factors {

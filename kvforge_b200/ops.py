@@ -2376,8 +2376,9 @@ def state_space_tensor_cores(dtype: torch.dtype, num_heads: int, groups: int, n_
 
 def state_space_chunks_pay(n: int, num_seqs: int, max_query_len: int) -> bool:
     """Whether that form is faster than the walk: a chunk of 128 tokens costs the same however few of its tokens there are.  Walk and
-    chunks, us, 64 heads of 128 x 64: one sequence of 64 tokens 25 and 34, of 128 41 and 28, of 2,048 520 and 122; 8 of 64 87 and 88, 8 of
-    128 154 and 64, 8 of 256 299 and 88; 400 and 20 single tokens 161 and 195."""
+    chunks, us, 64 heads of 128 x 64: one sequence of 64 tokens 23 and 27, of 128 38 and 24, of 2,048 515 and 115; 8 of 64 82 and 75, 8 of
+    128 150 and 61, 8 of 256 296 and 86; 130 and a single token 41 and 34, 400 and 5 152 and 74, 400 and 20 157 and 171.  32 heads of 64 x
+    64: one of 128 27 and 23, 8 of 128 46 and 39."""
     return max_query_len >= 128 and n >= 64 * num_seqs
 
 
