@@ -17,7 +17,7 @@ import torch
 
 import plain_ritizen as plain
 import traces
-from ritizen_cases import CASES, attention, lightning, mamba2, parallel, plain_logits, random_config, random_tensors, row_error, write_folder
+from ritizen_cases import CASES, attention, layer, lightning, mamba2, model, parallel, plain_logits, random_config, random_tensors, row_error, write_folder
 from test_gpu_mopilorn import check, run_trace, tokens
 from test_gpu_parts import context, runtime
 from test_gpu_sonalix import CUTS, as_float, bind, part_tol, rel_rows, step_mixer
@@ -84,6 +84,37 @@ def test_replay_as_captured_graphs(models, name, dtype, regime):
     outs, runner = run_trace(folder, dtype, steps, CASES[name]["block_size"], cuda_graphs=True)
     check(steps, outs, ref, scale, TOL[dtype])
     assert runner.core.runner.num_graph_kernels > 0
+
+
+def test_long_runs_go_in_chunks_eager_and_as_captured_graphs(tmp_path, monkeypatch):
+    """Whole models whose steps bring hundreds of tokens a sequence to a state space in bfloat16, by boxes (a state of 128 rows) and by
+    copies: prompts, portions behind them on the state that they left and single tokens after, run eagerly and as graphs, are the plain
+    implementation's within rounding, and the long steps do go in chunks."""
+    from kvforge_b200 import ops
+
+    config = model(131, 64, [
+        layer("mamba2", mamba2(4, 64, 128, 1), 72),
+        layer("attention", attention(4, 2, 16, 24), 40),
+        layer("mamba2", mamba2(8, 24, 40, 1, conv=3, norm_groups=2), 48),
+    ], max_positions=600)  # fmt: skip
+    folder, reqs, ref, scale, _ = build(tmp_path, "long", config, random_tensors(config, 29), [424, 424])
+    at, steps = dict.fromkeys(reqs, 0), []
+    for cut in [(200, 150), (200, 250)] + [(1, 1)] * 6 + [(18, 18)]:
+        entries, end = [], []
+        for rid, k in zip(reqs, cut):
+            entries.append({"id": rid, "tokens": reqs[rid][at[rid] : at[rid] + k], "want": [k - 1]})
+            at[rid] += k
+            if at[rid] == 424:
+                end.append(rid)
+        steps.append({"step": len(steps), "entries": entries, "end": end})
+    took, real = [], ops.state_space
+    monkeypatch.setattr(ops, "state_space", lambda *a, **kw: (took.append((a[0].shape[0], kw.get("raw") is not None)), real(*a, **kw))[1])
+    for graphs in (False, True):
+        took.clear()
+        outs, runner = run_trace(folder, "bfloat16", steps, 16, max_live=2, cuda_graphs=graphs)
+        check(steps, outs, ref, scale, TOL["bfloat16"])
+        assert {form for n, form in took if n >= 350} == {True} and not any(form for n, form in took if n < 128)
+        assert not graphs or any(key[0] >= 350 and not key[-1] for key in runner.core.runner._graphs)
 
 
 @pytest.mark.parametrize("name", ["a", "d"])
